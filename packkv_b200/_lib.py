@@ -104,6 +104,7 @@ SIGNATURES = {
 }
 
 _lib = None
+_host = None
 
 
 class PackKVLibraryError(RuntimeError):
@@ -124,6 +125,26 @@ def lib() -> ctypes.CDLL:
             fn.restype, fn.argtypes = res, args
         _lib = handle
     return _lib
+
+
+# the library functions of csrc/host.cpp, in the order of its struct Library
+_HOST_FUNCTIONS = ("pkv_decode_attention", "pkv_decode_attention_append", "pkv_decode_attention_exchange", "pkv_decode_attention_split",
+                   "pkv_attention_plan", "pkv_encode_tensor", "pkv_encode_tensor_ordered", "pkv_encode_tensor_static", "pkv_value_median_order",
+                   "pkv_append_residual", "pkv_rope")
+
+
+def host():
+    """The native host path (csrc/host.cpp), bound to the loaded library."""
+    global _host
+    if _host is None:
+        try:
+            from . import _host as module
+        except ImportError as e:
+            raise PackKVLibraryError(f"packkv_b200/_host.so does not load ({e}): build it with `python -m packkv_b200.build`. There is no fallback.") from e
+        handle = lib()
+        module.bind(*(ctypes.cast(getattr(handle, name), ctypes.c_void_p).value for name in _HOST_FUNCTIONS))
+        _host = module
+    return _host
 
 
 def check(status: int, what: str) -> None:

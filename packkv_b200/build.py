@@ -1,4 +1,5 @@
-"""Builds packkv_b200/libpackkv_sm100.so in-tree with nvcc for sm_100a.
+"""Builds packkv_b200/libpackkv_sm100.so (the kernels and the C ABI, nvcc for sm_100a) and packkv_b200/_host.so (the host
+path of packkv_b200.ops, a CPython extension over torch's tensors) in-tree.
 
     python -m packkv_b200.build [--force]
 
@@ -16,6 +17,8 @@ CSRC = os.path.join(PKG, "csrc")
 OBJ = os.path.join(PKG, "build")
 LIB = os.path.join(PKG, "libpackkv_sm100.so")
 SOURCES = ["pack.cu", "quant.cu", "attn.cu", "legacy.cu", "cache.cu", "reorder.cu", "fused_encode.cu", "encode_entry.cu", "capi.cu"]
+HOST_SOURCE = os.path.join(CSRC, "host.cpp")
+HOST_LIB = os.path.join(PKG, "_host.so")
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
     "-Xcompiler", "-fPIC", "-Xptxas", "-v",
@@ -34,6 +37,20 @@ def _stale(target: str, deps) -> bool:
     return any(os.path.getmtime(d) > t for d in deps)
 
 
+def _host_command():
+    import sysconfig
+
+    import torch
+    root = os.path.dirname(torch.__file__)
+    cuda = os.environ.get("CUDA_HOME", "/usr/local/cuda")
+    include = [os.path.join(root, "include"), os.path.join(root, "include", "torch", "csrc", "api", "include"), os.path.join(cuda, "include"),
+               sysconfig.get_paths()["include"]]
+    lib = os.path.join(root, "lib")
+    return (["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden", "-Wall", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}"]
+            + [x for i in include for x in ("-isystem", i)] + [HOST_SOURCE, "-o", HOST_LIB]
+            + [f"-L{lib}", "-ltorch_python", "-ltorch", "-ltorch_cpu", "-lc10_cuda", "-lc10"])
+
+
 def build(force: bool = False, verbose: bool = False) -> str:
     os.makedirs(OBJ, exist_ok=True)
     headers = [os.path.join(CSRC, f) for f in os.listdir(CSRC) if f.endswith((".cuh", ".h"))]
@@ -46,6 +63,11 @@ def build(force: bool = False, verbose: bool = False) -> str:
             jobs.append((s, o))
 
     def compile_one(job):
+        if job is None:
+            r = subprocess.run(_host_command(), capture_output=True, text=True)
+            if r.returncode != 0:
+                raise RuntimeError(f"g++ failed for {HOST_SOURCE}:\n{r.stdout}\n{r.stderr}")
+            return
         s, o = job
         r = subprocess.run([_nvcc()] + NVCC_FLAGS + ["-c", s, "-o", o], capture_output=True, text=True)
         if r.returncode != 0:
@@ -55,8 +77,9 @@ def build(force: bool = False, verbose: bool = False) -> str:
         if verbose:
             print(r.stderr)
 
+    host = [None] if force or _stale(HOST_LIB, [HOST_SOURCE, headers[-1]]) else []
     with ThreadPoolExecutor(max_workers=8) as pool:
-        list(pool.map(compile_one, jobs))
+        list(pool.map(compile_one, jobs + host))
     objs = [os.path.join(OBJ, s.replace(".cu", ".o")) for s in SOURCES]
     if force or jobs or _stale(LIB, objs):
         r = subprocess.run([_nvcc(), "-shared", "-o", LIB] + objs, capture_output=True, text=True)

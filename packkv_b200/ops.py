@@ -207,9 +207,8 @@ class CompressedLayer:
 
 
 def _check_layer_shapes(L: "CompressedLayer", batch: int) -> None:
-    """Host-side bounds of everything the attention kernel indexes from n_comp, kv_heads and the block sizes:
-    a layer whose metadata disagrees with its arrays (a caller mistake, a truncated or corrupt blob) must raise
-    here instead of reading outside the arrays on the device."""
+    """Bounds of everything the attention kernel indexes from n_comp, kv_heads and the block sizes, for layers that are
+    read from blobs (serialize.py); a launch checks the same in csrc/host.cpp."""
     if L.cbk not in (64, 128) or L.cbv not in (64, 128) or L.n_comp <= 0 or L.kv_heads <= 0:
         raise RuntimeError("not supported") if L.cbk == 32 or L.cbv == 32 else ValueError("bad layer metadata")
     nkb, nvb = (L.n_comp // L.cbk) * L.kv_heads, (L.n_comp // L.cbv) * 2 * L.kv_heads
@@ -258,94 +257,8 @@ def decode_attention(q: torch.Tensor, layer: Optional[CompressedLayer], k_res: O
     (extra > 0 with cluster 1: the first `extra` pairs get nsplit + 1 CTAs).
     plan_only: nothing is launched and the plan (cluster, nsplit, launches, extra) that would be used is returned.
     """
-    _require_cuda(q, k_res, v_res, out, flags, scratch)
-    if q.dim() != 3 or q.shape[2] != 128 or not q.is_contiguous():
-        raise ValueError("q must be a contiguous (B, Hq, 128) tensor")
-    if q.dtype not in (torch.float16, torch.bfloat16):
-        raise ValueError("q must be fp16 or bf16")
-    B, Hq, D = q.shape
-    if layer is not None:
-        kv_heads = layer.kv_heads
-    elif kv_heads is None:
-        kv_heads = k_res.shape[1]
-    if Hq % kv_heads:
-        raise ValueError("q heads must be a multiple of kv heads")
-    if out is None:
-        out = torch.empty_like(q)
-    if flags is None:
-        flags = new_flags(q.device)
-    a = _lib.AttnArgs()
-    a.q, a.out = q.data_ptr(), out.data_ptr()
-    n_comp = 0 if layer is None else layer.n_comp
-    if n_comp > 0:
-        L = layer
-        for t in (L.k_scale, L.k_zero, L.v_scale, L.v_zero):
-            if t.dtype != q.dtype or not t.is_contiguous():
-                raise ValueError("scale / zero tensors must be contiguous and of q's dtype")
-        _check_layer_shapes(L, B)
-        a.k_stream, a.k_seq_stride, a.k_capacity = L.k_stream.data_ptr(), L.k_stream.stride(0), L.k_stream.shape[1] & ~15
-        a.k_info, a.k_info_seq_stride = L.k_info.data_ptr(), L.k_info.shape[1]
-        a.k_scale, a.k_zero = L.k_scale.data_ptr(), L.k_zero.data_ptr()
-        a.v_stream, a.v_seq_stride, a.v_capacity = L.v_stream.data_ptr(), L.v_stream.stride(0), L.v_stream.shape[1] & ~15
-        a.v_info, a.v_info_seq_stride = L.v_info.data_ptr(), L.v_info.shape[1]
-        a.v_scale, a.v_zero = L.v_scale.data_ptr(), L.v_zero.data_ptr()
-        a.param_tokens = L.v_scale.shape[1]
-        a.param_blocks = L.k_scale.shape[2] if L.k_mode == K_CHANNEL else 0
-        if L.k_mode == K_TOKEN and L.k_scale.shape[1] != L.v_scale.shape[1]:
-            raise ValueError("token-mode K and V parameter arrays must have the same row length")
-        a.cbk, a.cbv, a.bits_k, a.bits_v = L.cbk, L.cbv, L.bits_k, L.bits_v
-        a.k_mode, a.high_precision_zero = L.k_mode, int(L.high_precision_zero)
-    if n_res > 0:
-        if k_res.dtype != q.dtype or v_res.dtype != q.dtype or k_res.stride(3) != 1 or k_res.stride(2) != 128:
-            raise ValueError("residual tensors must be (B, Hkv, R, 128) with contiguous rows, in q's dtype")
-        if k_res.stride() != v_res.stride():
-            raise ValueError("k_res and v_res must share strides")
-        a.k_res, a.v_res = k_res.data_ptr(), v_res.data_ptr()
-        a.res_seq_stride, a.res_head_stride = k_res.stride(0), k_res.stride(1)
-    a.n_res, a.batch, a.kv_heads, a.group, a.n_comp = n_res, B, kv_heads, Hq // kv_heads, n_comp
-    a.is_bf16 = int(q.dtype == torch.bfloat16)
-    a.scaling = float(D ** -0.5 if scaling is None else scaling)
-    a.flags = flags.data_ptr()
-    if append is not None:
-        k_new, v_new, cos, sin = append
-        _require_cuda(k_new, v_new, cos, sin)
-        if n_res < 1 or k_new.shape != (B, kv_heads, 1, 128) or v_new.shape != k_new.shape or k_new.stride(3) != 1 or v_new.stride(3) != 1 \
-                or k_new.dtype != q.dtype or v_new.dtype != q.dtype:
-            raise ValueError("append needs k_new / v_new of shape (B, Hkv, 1, 128) in q's dtype with contiguous channels")
-        ap = _lib.AttnAppend()
-        ap.new_k, ap.new_v = k_new.data_ptr(), v_new.data_ptr()
-        ap.k_stride_b, ap.k_stride_h, ap.v_stride_b, ap.v_stride_h = k_new.stride(0), k_new.stride(1), v_new.stride(0), v_new.stride(1)
-        if cos is not None:
-            if cos.dtype != q.dtype or sin.dtype != q.dtype or cos.shape[-2:] != (1, 128) or sin.shape != cos.shape or not cos.is_contiguous() \
-                    or not sin.is_contiguous():
-                raise ValueError("cos / sin must be contiguous (B or 1, 1, 128) tensors of q's dtype")
-            ap.cos, ap.sin, ap.cs_stride_b = cos.data_ptr(), sin.data_ptr(), (0 if cos.shape[0] == 1 else 128)
-        ap.res_capacity = k_res.shape[2]
-    else:
-        ap = None
-    if scratch is not None or plan is not None or plan_only:
-        pl = _lib.AttnPlan()
-        if plan is not None:
-            pl.cluster, pl.nsplit, pl.launches = plan[:3]
-            pl.extra = plan[3] if len(plan) > 3 else 0
-        if scratch is not None and (scratch.dtype != torch.uint8 or not scratch.is_contiguous() or scratch.data_ptr() % 256):
-            raise ValueError("scratch must be a contiguous uint8 tensor aligned to 256 bytes (new_attention_scratch)")
-        sbytes = 0 if scratch is None else scratch.numel()
-        if plan_only:
-            _lib.check(_lib.lib().pkv_attention_plan(ctypes.byref(a), ctypes.byref(pl), sbytes, int(exchange is not None)), "attention_plan")
-            return (pl.cluster, pl.nsplit, pl.launches, pl.extra)
-        st = _lib.lib().pkv_decode_attention_split(ctypes.byref(a), ctypes.byref(ap) if ap is not None else None,
-                                                   ctypes.byref(exchange) if exchange is not None else None, ctypes.byref(pl),
-                                                   scratch.data_ptr() if scratch is not None else None, sbytes, _stream_ptr())
-    elif ap is not None:
-        st = _lib.lib().pkv_decode_attention_append(ctypes.byref(a), ctypes.byref(ap), ctypes.byref(exchange) if exchange is not None else None,
-                                                    _stream_ptr())
-    elif exchange is None:
-        st = _lib.lib().pkv_decode_attention(ctypes.byref(a), _stream_ptr())
-    else:
-        st = _lib.lib().pkv_decode_attention_exchange(ctypes.byref(a), ctypes.byref(exchange), _stream_ptr())
-    _lib.check(st, "decode_attention")
-    return out
+    return _lib.host().decode_attention(q, layer, k_res, v_res, n_res, scaling, out, flags, kv_heads, None if exchange is None else ctypes.addressof(exchange),
+                                        append, scratch, plan, plan_only)
 
 
 def new_attention_scratch(device, nbytes: int = 32 << 20) -> torch.Tensor:
@@ -369,47 +282,14 @@ def exchange_wait(arrivals: torch.Tensor, n_ranks: int, expected: int, flags: to
 def rope(x: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor, out: Optional[torch.Tensor] = None) -> torch.Tensor:
     """(x * cos) + (rotate_half(x) * sin) with the reference's per-op rounding.
     x (B, H, T, D) with contiguous channels; cos/sin (B or 1, T, D)."""
-    _require_cuda(x, cos, sin, out)
-    if x.dim() != 4 or x.stride(3) != 1 or x.dtype not in (torch.float16, torch.bfloat16):
-        raise ValueError("x must be (B, H, T, D) fp16/bf16 with contiguous channels")
-    B, H, T, D = x.shape
-    cos, sin = cos.to(x.dtype).contiguous(), sin.to(x.dtype).contiguous()
-    if cos.shape[-2:] != (T, D) or sin.shape != cos.shape:
-        raise ValueError("cos/sin must be (B or 1, T, D)")
-    if out is None:
-        out = torch.empty(B, H, T, D, dtype=x.dtype, device=x.device)
-    cs_stride = 0 if cos.shape[0] == 1 else T * D
-    st = _lib.lib().pkv_rope(x.data_ptr(), x.stride(0), x.stride(1), x.stride(2), cos.data_ptr(), sin.data_ptr(), cs_stride,
-                             out.data_ptr(), out.stride(0), out.stride(1), out.stride(2), B, H, T, D,
-                             int(x.dtype == torch.bfloat16), _stream_ptr())
-    _lib.check(st, "rope")
-    return out
+    return _lib.host().rope(x, cos, sin, out)
 
 
 def append_residual(k_new: torch.Tensor, v_new: torch.Tensor, k_res: torch.Tensor, v_res: torch.Tensor, position: int,
                     cos: Optional[torch.Tensor] = None, sin: Optional[torch.Tensor] = None) -> None:
     """Writes the new tokens (B, H, T, 128) into rows [position, position+T) of the residual buffers
     (B, H, capacity, 128): K after RoPE (skipped when cos/sin are None), V as is.  One launch."""
-    _require_cuda(k_new, v_new, k_res, v_res, cos, sin)
-    B, H, T, D = k_new.shape
-    if D != 128 or v_new.shape != k_new.shape or k_new.stride(3) != 1 or v_new.stride(3) != 1:
-        raise ValueError("k_new and v_new must be (B, H, T, 128) with contiguous channels")
-    if k_res.shape != v_res.shape or k_res.stride() != v_res.stride() or k_res.stride(3) != 1 or k_res.stride(2) != 128:
-        raise ValueError("k_res and v_res must be (B, H, capacity, 128) with contiguous rows and equal strides")
-    if k_res.dtype != k_new.dtype or v_new.dtype != k_new.dtype or k_new.dtype not in (torch.float16, torch.bfloat16):
-        raise ValueError("dtype mismatch")
-    cs_stride = 0
-    if cos is not None:
-        cos, sin = cos.to(k_new.dtype).contiguous(), sin.to(k_new.dtype).contiguous()
-        if cos.shape[-2:] != (T, D) or sin.shape != cos.shape:
-            raise ValueError("cos/sin must be (B or 1, T, 128)")
-        cs_stride = 0 if cos.shape[0] == 1 else T * D
-    st = _lib.lib().pkv_append_residual(
-        k_new.data_ptr(), k_new.stride(0), k_new.stride(1), k_new.stride(2), v_new.data_ptr(), v_new.stride(0), v_new.stride(1), v_new.stride(2),
-        cos.data_ptr() if cos is not None else None, sin.data_ptr() if sin is not None else None, cs_stride,
-        k_res.data_ptr(), v_res.data_ptr(), k_res.stride(0), k_res.stride(1), k_res.shape[2], position, B, H, T,
-        int(k_new.dtype == torch.bfloat16), _stream_ptr())
-    _lib.check(st, "append_residual")
+    _lib.host().append_residual(k_new, v_new, k_res, v_res, position, cos, sin)
 
 
 def dequantize(codes: torch.Tensor, scale: torch.Tensor, zero: torch.Tensor, heads: int, block: int, mode: int, *,
@@ -427,22 +307,6 @@ def dequantize(codes: torch.Tensor, scale: torch.Tensor, zero: torch.Tensor, hea
     return out
 
 
-def _encode_args(which: str, x, block, rel, mode, bits, hp, cb, scale, zero, stream, info, stream_bytes, flags, first_token):
-    B, H, S, D = x.shape
-    a = _lib.EncodeArgs()
-    a.x, a.stride_b, a.stride_h, a.stride_s = x.data_ptr(), x.stride(0), x.stride(1), x.stride(2)
-    a.scale, a.zero = scale.data_ptr(), zero.data_ptr()
-    a.param_blocks = scale.shape[2] if mode == K_CHANNEL else 0
-    a.param_tokens = scale.shape[1] if mode == K_TOKEN else 0
-    a.stream, a.stream_seq_stride, a.capacity = stream.data_ptr(), stream.stride(0), stream.shape[1]
-    a.block_info, a.info_seq_stride, a.stream_bytes = info.data_ptr(), info.shape[1], stream_bytes.data_ptr()
-    a.flags = flags.data_ptr()
-    a.batch, a.heads, a.tokens, a.first_token, a.qblock, a.cb = B, H, S, first_token, block, cb
-    a.which = 0 if which == "k" else 1
-    a.bits, a.mode, a.high_precision_zero, a.is_bf16, a.rel = bits, mode, int(hp), int(x.dtype == torch.bfloat16), float(rel)
-    return a
-
-
 def encode_tensor(which: str, x: torch.Tensor, block: int, rel: float, mode: int, bits: int, cb: int, *,
                   scale: torch.Tensor, zero: torch.Tensor, stream: torch.Tensor, info: torch.Tensor,
                   stream_bytes: torch.Tensor, flags: torch.Tensor, first_token: int = 0,
@@ -453,45 +317,15 @@ def encode_tensor(which: str, x: torch.Tensor, block: int, rel: float, mode: int
     allocated when not given.  `order` (B, S/order_block, order_block) uint8 (value_median_order): rows are read
     through it, i.e. the tokens of every reorder block are stored in that order (single-pass modes only:
     RuntimeError("not supported") otherwise)."""
-    _require_cuda(x, scale, zero, stream, info, stream_bytes, flags, scratch)
-    if x.dim() != 4 or x.shape[3] != 128 or x.stride(3) != 1 or x.dtype not in (torch.float16, torch.bfloat16):
-        raise ValueError("x must be (B, H, S, 128) fp16/bf16 with contiguous channels")
-    B, H, S, D = x.shape
-    if S % block or S % cb:
-        raise ValueError("Tensor shape is not divisible by block size")
-    need = B * S * H * D
-    if scratch is None:
-        scratch = torch.empty(max(need, 16), dtype=torch.uint8, device=x.device)
-    a = _encode_args(which, x, block, rel, mode, bits, high_precision_zero, cb, scale, zero, stream, info, stream_bytes, flags, first_token)
-    if order is not None:
-        _require_cuda(order)
-        if order.dtype != torch.uint8 or not order.is_contiguous() or order.numel() != B * S:
-            raise ValueError("order must be a contiguous uint8 tensor with one entry per token")
-        st = _lib.lib().pkv_encode_tensor_ordered(ctypes.byref(a), order.data_ptr(), order_block, scratch.data_ptr(), scratch.numel(), _stream_ptr())
-    else:
-        st = _lib.lib().pkv_encode_tensor(ctypes.byref(a), scratch.data_ptr(), scratch.numel(), _stream_ptr())
-    _lib.check(st, f"encode_tensor({which})")
+    _lib.host().encode_tensor(which, x, block, rel, mode, bits, cb, scale, zero, stream, info, stream_bytes, flags, first_token, high_precision_zero,
+                              scratch, order, order_block)
 
 
 def value_median_order(v: torch.Tensor, block: int, rel: float, flags: Optional[torch.Tensor] = None) -> torch.Tensor:
     """Token order of every block by descending lower median of the V codes (stable on ties), computed from
     fp16/bf16 V (B, H <= 8, S, 128) without a code matrix: the same order as median_order on quantised codes.
     Returns (B, S/block, block) uint8."""
-    _require_cuda(v, flags)
-    if v.dim() != 4 or v.shape[3] != 128 or v.stride(3) != 1 or v.dtype not in (torch.float16, torch.bfloat16):
-        raise ValueError("v must be (B, H, S, 128) fp16/bf16 with contiguous channels")
-    B, H, S, _ = v.shape
-    if S % block:
-        raise ValueError("Tensor shape is not divisible by block size")
-    order = torch.empty(B, S // block, block, dtype=torch.uint8, device=v.device)
-    a = _lib.EncodeArgs()
-    a.x, a.stride_b, a.stride_h, a.stride_s = v.data_ptr(), v.stride(0), v.stride(1), v.stride(2)
-    a.batch, a.heads, a.tokens, a.which, a.mode = B, H, S, 1, K_TOKEN
-    a.is_bf16, a.rel = int(v.dtype == torch.bfloat16), float(rel)
-    a.flags = (flags if flags is not None else new_flags(v.device)).data_ptr()
-    st = _lib.lib().pkv_value_median_order(ctypes.byref(a), order.data_ptr(), block, _stream_ptr())
-    _lib.check(st, "value_median_order")
-    return order
+    return _lib.host().value_median_order(v, block, rel, flags)
 
 
 def encode_tensor_static(which: str, x: torch.Tensor, block: int, rel: float, mode: int, bits: int, cb: int, *,
@@ -504,14 +338,8 @@ def encode_tensor_static(which: str, x: torch.Tensor, block: int, rel: float, mo
     exceed that (ValueError otherwise), and calls must not overlap on the GPU because they share
     it.  The first call on a device resolves the array's address: make it before capturing streams.
     Results are identical to encode_tensor's."""
-    _require_cuda(x, scale, zero, stream, info, stream_bytes, flags)
-    if x.dim() != 4 or x.shape[3] != 128 or x.stride(3) != 1 or x.dtype not in (torch.float16, torch.bfloat16):
-        raise ValueError("x must be (B, H, S, 128) fp16/bf16 with contiguous channels")
-    if x.shape[2] % block or x.shape[2] % cb:
-        raise ValueError("Tensor shape is not divisible by block size")
-    a = _encode_args(which, x, block, rel, mode, bits, high_precision_zero, cb, scale, zero, stream, info, stream_bytes, flags, first_token)
-    st = _lib.lib().pkv_encode_tensor_static(ctypes.byref(a), _stream_ptr())
-    _lib.check(st, f"encode_tensor_static({which})")
+    _lib.host().encode_tensor(which, x, block, rel, mode, bits, cb, scale, zero, stream, info, stream_bytes, flags, first_token, high_precision_zero,
+                              False, None, 0)
 
 
 def median_order(v_codes: torch.Tensor, heads: int, block: int, want_keys: bool = False):
