@@ -270,6 +270,32 @@ int32_t pkv_dequantize(const uint8_t* codes, int64_t codes_seq_stride, const voi
                        void* cuda_stream);
 
 /*
+ * Dense view of one tensor of a layer: rows [0, n_comp) of out are the packed tokens, unpacked and dequantised as
+ * pkv_{k,v}_decode followed by pkv_dequantize give them, rows [n_comp, n_comp + n_res) the first n_res rows of the
+ * uncompressed residual (models/cache/packkv_quant.py:45-85).  One launch, no scratch.
+ * out (batch, heads, n_comp + n_res, dim): dim 8..128, a multiple of 8, is the number of channels kept of every 128;
+ * 16-byte aligned, strides in elements and multiples of 8.  res (batch, heads, >= n_res, 128), aligned likewise.
+ * order (optional): (batch, ...) uint8 with order_seq_stride bytes between sequences, entry t = source row, inside its
+ * group of order_block tokens, of stored token t; the rows come back in source order.
+ * cb 64 or 128; K per channel needs qblock = cb.  A block that the table places outside the stream, or that is cut
+ * short, sets PKV_FLAG_BAD_STREAM and reads as codes 0 from there on.
+ */
+typedef struct pkv_dense_args {
+    const uint8_t* stream; int64_t stream_seq_stride, capacity;
+    const uint32_t* block_info; int64_t info_seq_stride;
+    const void* scale; const void* zero; int32_t param_blocks, param_tokens;   /* as in pkv_quantize */
+    const uint8_t* order; int64_t order_seq_stride;
+    const void* res; int64_t res_stride_b, res_stride_h;                        /* strides in elements, rows of 128 */
+    void* out; int64_t o_stride_b, o_stride_h, o_stride_s;
+    uint32_t* flags;
+    int32_t batch, heads, dim, n_comp, n_res;
+    int32_t order_block, qblock, cb;
+    int32_t which, bits, mode, high_precision_zero, is_bf16;                    /* as in pkv_encode_args */
+} pkv_dense_args;
+
+int32_t pkv_dense(const pkv_dense_args* args_host, void* cuda_stream);
+
+/*
  * Fused decompress-attention decode: out = softmax(q K^T * scaling) V for ONE new query token
  * per sequence over (compressed tokens + uncompressed residual tokens), reading the packed
  * streams directly.  Replaces the chain kq_mat_vec_mul -> fused_kq -> torch softmax ->

@@ -66,7 +66,22 @@ class EncodeArgs(ctypes.Structure):
     ]
 
 
+class DenseArgs(ctypes.Structure):
+    _fields_ = [
+        ("stream", _p), ("stream_seq_stride", _i64), ("capacity", _i64),
+        ("block_info", _p), ("info_seq_stride", _i64),
+        ("scale", _p), ("zero", _p), ("param_blocks", _i32), ("param_tokens", _i32),
+        ("order", _p), ("order_seq_stride", _i64),
+        ("res", _p), ("res_stride_b", _i64), ("res_stride_h", _i64),
+        ("out", _p), ("o_stride_b", _i64), ("o_stride_h", _i64), ("o_stride_s", _i64), ("flags", _p),
+        ("batch", _i32), ("heads", _i32), ("dim", _i32), ("n_comp", _i32), ("n_res", _i32),
+        ("order_block", _i32), ("qblock", _i32), ("cb", _i32),
+        ("which", _i32), ("bits", _i32), ("mode", _i32), ("high_precision_zero", _i32), ("is_bf16", _i32),
+    ]
+
+
 SIGNATURES = {
+    "pkv_dense": (_i32, [ctypes.POINTER(DenseArgs), _p]),
     "pkv_encode_tensor": (_i32, [ctypes.POINTER(EncodeArgs), _p, _i64, _p]),
     "pkv_encode_tensor_static": (_i32, [ctypes.POINTER(EncodeArgs), _p]),
     "pkv_encode_tensor_ordered": (_i32, [ctypes.POINTER(EncodeArgs), _p, _i32, _p, _i64, _p]),

@@ -16,7 +16,7 @@ PKG = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(PKG, "csrc")
 OBJ = os.path.join(PKG, "build")
 LIB = os.path.join(PKG, "libpackkv_sm100.so")
-SOURCES = ["pack.cu", "quant.cu", "attn.cu", "legacy.cu", "cache.cu", "reorder.cu", "fused_encode.cu", "encode_entry.cu", "capi.cu"]
+SOURCES = ["pack.cu", "quant.cu", "attn.cu", "legacy.cu", "cache.cu", "dense.cu", "reorder.cu", "fused_encode.cu", "encode_entry.cu", "capi.cu"]
 HOST_SOURCE = os.path.join(CSRC, "host.cpp")
 HOST_LIB = os.path.join(PKG, "_host.so")
 NVCC_FLAGS = [

@@ -291,23 +291,10 @@ class PackKVCache(_HFCache):
         L = self._layers[layer_idx]
         self._flush(L)
         D = self.head_dim if self.head_dim < 128 else 128
-        k_res, v_res = L.k_res[:, :, : L.n_res, :D], L.v_res[:, :, : L.n_res, :D]
         if L.n_comp == 0:
-            return k_res.clone(), v_res.clone()
-        C, cfg = L.comp, self._config()
-        H = C.kv_heads
-        kc, _ = ops.decode_codes("k", C.k_stream, C.k_info, L.n_comp, H * 128, C.cbk, C.bits_k, flags=self.flags)
-        vc, _ = ops.decode_codes("v", C.v_stream, C.v_info, L.n_comp, H * 128, C.cbv, C.bits_v, flags=self.flags)
-        kd = ops.dequantize(kc, C.k_scale, C.k_zero, H, cfg.block_size, C.k_mode, high_precision_zero=C.high_precision_zero)
-        vd = ops.dequantize(vc, C.v_scale, C.v_zero, H, cfg.block_size, ops.K_TOKEN, high_precision_zero=C.high_precision_zero)
-        if C.order is not None:   # undo the in-block reordering: original position of every stored row
-            block = cfg.block_size
-            pos = (C.order.to(torch.int64) + torch.arange(L.n_comp // block, device=kd.device).view(1, -1, 1) * block).reshape(kd.shape[0], -1)
-            inv = torch.empty_like(pos)
-            inv.scatter_(1, pos, torch.arange(L.n_comp, device=kd.device).expand_as(pos))
-            idx = inv.view(kd.shape[0], 1, L.n_comp, 1).expand_as(kd)
-            kd, vd = torch.gather(kd, 2, idx), torch.gather(vd, 2, idx)
-        return torch.cat([kd[..., :D], k_res], dim=2), torch.cat([vd[..., :D], v_res], dim=2)
+            return L.k_res[:, :, : L.n_res, :D].clone(), L.v_res[:, :, : L.n_res, :D].clone()
+        block = self._config().block_size
+        return (ops.dense("k", L.comp, L.k_res, L.n_res, D, block, self.flags), ops.dense("v", L.comp, L.v_res, L.n_res, D, block, self.flags))
 
     def attend(self, query_states: torch.Tensor, layer_idx: int, scaling: Optional[float] = None) -> torch.Tensor:
         """Decode attention for one new token: query_states (B, Hq, 1, 128) after RoPE ->

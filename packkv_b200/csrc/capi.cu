@@ -147,6 +147,11 @@ int32_t pkv_dequantize(const uint8_t* codes, int64_t codes_seq_stride, const voi
     return launch_dequantize(q, static_cast<cudaStream_t>(cuda_stream));
 }
 
+int32_t pkv_dense(const pkv_dense_args* args_host, void* cuda_stream) {
+    if (!args_host) return kBadArgument;
+    return launch_dense(*args_host, static_cast<cudaStream_t>(cuda_stream));
+}
+
 int32_t pkv_decode_attention(const pkv_attn_args* args_host, void* cuda_stream) {
     if (!args_host) return kBadArgument;
     return launch_attention(*args_host, nullptr, nullptr, nullptr, nullptr, 0, false, static_cast<cudaStream_t>(cuda_stream));

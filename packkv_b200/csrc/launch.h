@@ -94,6 +94,7 @@ int launch_gather_params(const void* src, void* dst, int64_t row_len, int first,
                          int block, cudaStream_t st);
 int launch_rope(const RopeArgs& r, cudaStream_t st);
 int launch_append(const AppendArgs& r, cudaStream_t st);
+int launch_dense(const pkv_dense_args& a, cudaStream_t st);
 int launch_dequantize(const DequantArgs& q, cudaStream_t st);
 int launch_quantize(const QuantArgs& q, cudaStream_t st);
 // single-pass encoder (fused_encode.cu); the request is the C ABI's argument block

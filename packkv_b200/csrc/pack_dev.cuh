@@ -1,4 +1,4 @@
-// Device helpers shared by the bit-pack kernels (pack.cu, fused_encode.cu).
+// Device helpers shared by the bit-pack kernels (pack.cu, fused_encode.cu, dense.cu).
 #pragma once
 #include "common.cuh"
 
@@ -20,6 +20,31 @@ __device__ __forceinline__ void store_pack_smem(uint8_t* dst, uint64_t w, int le
 #pragma unroll
     for (int i = 0; i < 4; i++)
         if (i < len) q[i] = (uint16_t)(w >> (16 * i));
+}
+
+// Copies `size` bytes (plus up to 16 bytes of slack on either side, inside the stream
+// allocation) from global `src` into shared memory so that the shared copy of src[0] has
+// the same address modulo 16.  Returns the shared pointer that mirrors src.
+__device__ __forceinline__ const uint8_t* warp_copy_in(uint8_t* sbuf16, const uint8_t* src, int size, int lane,
+                                                       const uint8_t* lo, const uint8_t* hi) {
+    int phase = (int)(reinterpret_cast<uintptr_t>(src) & 15);
+    const uint8_t* a = src - phase;                 // 16-byte aligned start
+    int total = (phase + size + 15) & ~15;
+    for (int i = 16 * lane; i < total; i += 16 * 32) {
+        const uint8_t* p = a + i;
+        uint4 v = make_uint4(0, 0, 0, 0);
+        if (p >= lo && p + 16 <= hi) {
+            v = *reinterpret_cast<const uint4*>(p);
+        } else {                                    // ragged edge of the allocation
+            unsigned q[4] = {0, 0, 0, 0};
+#pragma unroll
+            for (int b = 0; b < 16; b++)
+                if (p + b >= lo && p + b < hi) q[b >> 2] |= (unsigned)p[b] << (8 * (b & 3));
+            v = make_uint4(q[0], q[1], q[2], q[3]);
+        }
+        *reinterpret_cast<uint4*>(sbuf16 + i) = v;
+    }
+    return sbuf16 + phase;
 }
 
 // Copies `size` bytes from shared `src` to global `dst`; both have the same address modulo

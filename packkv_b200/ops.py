@@ -307,6 +307,36 @@ def dequantize(codes: torch.Tensor, scale: torch.Tensor, zero: torch.Tensor, hea
     return out
 
 
+def dense(which: str, layer: CompressedLayer, res: Optional[torch.Tensor], n_res: int, dim: int, block: int,
+          flags: torch.Tensor) -> torch.Tensor:
+    """Rows of K or V of a layer as the reference's cache returns them, (B, H, n_comp + n_res, dim): the packed tokens
+    dequantised (in source order when the layer is reordered) and the first n_res rows of the residual behind them.
+    `block` is the quantisation block; dim < 128 keeps the first channels of every head.  One launch."""
+    get = lambda name: getattr(layer, f"{which}_{name}")
+    stream, info, scale, zero = get("stream"), get("info"), get("scale"), get("zero")
+    B, H, n, cb = stream.shape[0], layer.kv_heads, layer.n_comp, layer.cbk if which == "k" else layer.cbv
+    mode = layer.k_mode if which == "k" else K_TOKEN
+    _require_cuda(stream, info, scale, zero, res, layer.order, flags)
+    pb, pt = _param_extents(scale, mode)
+    if n % block or n % cb or info.dim() != 3 or info.shape[1] < (n // cb) * H * (1 if which == "k" else 2) or not info.is_contiguous() \
+            or stream.dim() != 2 or stream.stride(1) != 1 or (pb < n // block if mode == K_CHANNEL else pt < n) \
+            or not scale.is_contiguous() or not zero.is_contiguous() or zero.shape != scale.shape or any(t.shape[0] != B for t in (info, scale)):
+        raise ValueError("dense: the layer's tables do not cover its tokens")
+    if layer.order is not None and (not layer.order.is_contiguous() or layer.order.numel() != B * n):
+        raise ValueError("dense: order must hold one entry per token")
+    if n_res and (res.dim() != 4 or res.shape[:2] != (B, H) or res.shape[2] < n_res or res.shape[3] != 128 or res.stride(3) != 1 or res.stride(2) != 128
+                  or res.dtype != scale.dtype):
+        raise ValueError("dense: the residual must be (B, H, >= n_res, 128) rows of the layer's element type")
+    out = torch.empty(B, H, n + n_res, dim, dtype=scale.dtype, device=scale.device)
+    a = _lib.DenseArgs(stream.data_ptr(), stream.stride(0), stream.shape[1], info.data_ptr(), info.shape[1], scale.data_ptr(), zero.data_ptr(), pb, pt,
+                       None if layer.order is None else layer.order.data_ptr(), n, res.data_ptr() if n_res else None,
+                       res.stride(0) if n_res else 0, res.stride(1) if n_res else 0, out.data_ptr(), out.stride(0), out.stride(1), out.stride(2),
+                       flags.data_ptr(), B, H, dim, n, n_res, block if layer.order is None else layer.order.shape[2], block, cb, 0 if which == "k" else 1,
+                       layer.bits_k if which == "k" else layer.bits_v, mode, int(layer.high_precision_zero), int(scale.dtype == torch.bfloat16))
+    _lib.check(_lib.lib().pkv_dense(ctypes.byref(a), _stream_ptr()), "dense")
+    return out
+
+
 def encode_tensor(which: str, x: torch.Tensor, block: int, rel: float, mode: int, bits: int, cb: int, *,
                   scale: torch.Tensor, zero: torch.Tensor, stream: torch.Tensor, info: torch.Tensor,
                   stream_bytes: torch.Tensor, flags: torch.Tensor, first_token: int = 0,

@@ -1,0 +1,64 @@
+"""GPU: the dense view of a layer (pkv_dense) against the oracle's quantise -> dequantise on CPU, bit for bit: every
+element is the result of the same two rounded operations."""
+import pytest
+import torch
+
+from helpers import layer_from_oracle
+from oracle import quant as Q
+from packkv_b200 import encode, ops, synth
+from packkv_b200.config import QuantMode, RepackMethod
+
+pytestmark = pytest.mark.gpu
+
+
+def _check(layer, kd, vd, k_res, v_res, n_res, dim, block, flags):
+    for which, dense, res in (("k", kd, k_res), ("v", vd, v_res)):
+        got = ops.dense(which, layer, res, n_res, dim, block, flags).cpu()
+        want = torch.cat([dense[..., :dim], res[:, :, :n_res, :dim].cpu()], dim=2)
+        assert got.shape == want.shape
+        assert torch.equal(got.view(torch.int16), want.view(torch.int16)), which
+    assert int(flags.item()) == 0
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("k_mode", ["channel", "token"])
+@pytest.mark.parametrize("bits,block,dim,n_res,hp", [(4, 64, 128, 133, False), (3, 64, 96, 1, False), (2, 128, 128, 0, False), (4, 128, 72, 16, True),
+                                                     (3, 128, 64, 17, True)])
+def test_dense_matches_the_oracle(cuda_device, dtype, k_mode, bits, block, dim, n_res, hp):
+    dev = cuda_device
+    B, H, S = 2, 3, 384
+    k, v = synth.synth_kv(B, H, S, 128, seed=bits * 10 + block, dtype=dtype)
+    k[0, 0, 16:32], v[1, 1, 16:32] = k[0, 0, 16:17], 0.01  # packs of width 0
+    k[1, 2, 5] *= 300                                      # and one far outside the rest
+    rel = synth.rel_for_bits(bits)
+    layer, kd, vd = layer_from_oracle(k, v, block=block, bits_k=bits, bits_v=bits, k_mode=k_mode, cbk=block, cbv=block, rel_k=rel, rel_v=rel, device=dev, hp=hp)
+    res = [torch.randn(B, H, 192, 128).to(dtype).to(dev) for _ in range(2)]
+    _check(layer, kd, vd, *res, n_res, dim, block, ops.new_flags(dev))
+
+
+@pytest.mark.parametrize("cbv", [64, 128])
+def test_dense_returns_reordered_tokens_in_source_order(cuda_device, cbv):
+    dev = cuda_device
+    B, H, S = 2, 2, 256
+    k, v = synth.synth_kv(B, H, S, 128, seed=3, dtype=torch.bfloat16)
+    rel = synth.rel_for_bits(4)
+    layer = encode.compress_kv(k.to(dev), v.to(dev), block=64, bits_k=4, bits_v=4, k_rel=rel, v_rel=rel, k_mode=QuantMode.ChannelQuant, cbk=64, cbv=cbv,
+                               repack_method=RepackMethod.MEDIAN)
+    assert not torch.equal(layer.order[0, 0].cpu(), torch.arange(64, dtype=torch.uint8))
+    kd, vd = (Q.dequant(*Q.quant_ints(x, 64, rel, mode, False)) for x, mode in ((k, "channel"), (v, "token")))
+    res = torch.zeros(B, H, 192, 128, dtype=torch.bfloat16, device=dev)
+    _check(layer, kd, vd, res, res, 3, 128, 64, ops.new_flags(dev))
+
+
+def test_dense_flags_blocks_outside_the_stream(cuda_device):
+    dev = cuda_device
+    k, v = synth.synth_kv(1, 2, 128, 128, seed=4, dtype=torch.float16)
+    rel = synth.rel_for_bits(4)
+    layer, kd, _ = layer_from_oracle(k, v, block=64, bits_k=4, bits_v=4, k_mode="channel", cbk=64, cbv=64, rel_k=rel, rel_v=rel, device=dev)
+    layer.k_info[0, 1, 0] = layer.k_stream.shape[1]
+    flags = ops.new_flags(dev)
+    got = ops.dense("k", layer, None, 0, 128, 64, flags).cpu()
+    assert int(flags.item()) == 4
+    assert torch.equal(got[:, 0], kd[:, 0]) and torch.equal(got[:, 1, 64:], kd[:, 1, 64:])
+    want = layer.k_zero[0, 1, 0].cpu() * layer.k_scale[0, 1, 0].cpu()             # codes 0
+    assert torch.equal(got[0, 1, :64], want.expand(64, 128))
