@@ -255,6 +255,7 @@ struct AttnDev {
     int rows;            // score rows kept per tile (q heads of the group, rounded up to even)
     int slot;            // bytes of one staging slot
     int nslots;          // staging slots per warp: 2 = the next block is copied while this one is unpacked
+    int team;            // single launch: the warps of a CTA share its tiles (see TEAM)
     int vpair;           // 64-token V blocks: an item is the pair of blocks of one token block (both channel halves)
     int kbound, vbound;  // largest legal block size in bytes
     int prow;            // bytes of one row of the score / probability tile
@@ -314,7 +315,11 @@ __device__ __forceinline__ unsigned deq(unsigned biased, typename Tr<T>::T2 add,
 // come back, global max and sum, V phase, per-cluster rows to the scratch, the pair's last cluster adds them up.
 enum AttnPass : int { kFused = 0, kScores = 1, kValues = 2 };
 
-template <typename T, int KMODE, bool HP, int PASS>
+// TEAM (single launch only): the four warps of a CTA share its tiles instead of owning tiles each.  Warp w takes the K rounds
+// w, w + 4, ... of a block and, of the head's 128 V channels, w's 32 (the block headers say where a round or segment starts);
+// the scores of a tile lie in the first warp's region.  For launches whose time is the latency of one warp's tile: with one
+// tile to a warp and one warp to a scheduler, a round or segment of 16 x 128 codes is about 1 us of dependent instructions.
+template <typename T, int KMODE, bool HP, int PASS, bool TEAM>
 __global__ void __launch_bounds__(kAW * 32, PASS == 1 ? PKV_ATTN_CTAS_SCORES : PASS == 2 ? PKV_ATTN_CTAS_VALUES : kMaxCtasPerSm) attn_decode_kernel(const AttnDev P) {
     using T2 = typename Tr<T>::T2;
     constexpr unsigned MAGIC = Tr<T>::kMagic2;
@@ -340,6 +345,8 @@ __global__ void __launch_bounds__(kAW * 32, PASS == 1 ? PKV_ATTN_CTAS_SCORES : P
     const int q_heads = a.kv_heads * G;
     const int n_warps = kAW * n_vctas;
     const int gw = vrank * kAW + wic;                  // warp index among all warps of the pair
+    static_assert(!TEAM || (PASS == kFused && kAW == 4), "a team is the four warps of a single-launch CTA");
+    const int tw = TEAM ? vrank : gw, tstep = TEAM ? n_vctas : n_warps;   // tiles tw, tw + tstep, ... are this warp's (or its team's)
     const int pair = b * a.kv_heads + h;
     const int ml_stride = P.cluster * part_stride;     // CTAs a pair's scratch rows are laid out for
 
@@ -351,7 +358,7 @@ __global__ void __launch_bounds__(kAW * 32, PASS == 1 ? PKV_ATTN_CTAS_SCORES : P
     const unsigned raw_a = wbase_a + P.off_raw;        // parameters as copied from global memory
     const unsigned perm_a = wbase_a + P.off_perm;      // per-token parameters in pair order: [tile] scale, [tile] zero
     const unsigned desc_a = wbase_a + P.off_desc;      // V: per channel-owner lane (pack offsets, lengths, minima)
-    const unsigned stile_a = wbase_a + P.off_stile;    // [tpw][rows][prow] scores -> probabilities
+    const unsigned stile_a = (TEAM ? smem_addr(smem) : wbase_a) + P.off_stile;    // [tpw][rows][prow] scores -> probabilities
     const unsigned rst_a = wbase_a + P.off_rst;        // [rtw][rows][16] residual scores -> probabilities
     unsigned lutm_a = smem_addr(cs->lutm);
     const unsigned bar_a = smem_addr(&cs->mbar[wic][0]);
@@ -368,13 +375,14 @@ __global__ void __launch_bounds__(kAW * 32, PASS == 1 ? PKV_ATTN_CTAS_SCORES : P
     __syncthreads();
     asm volatile("" : "+r"(lutm_a) :: "memory");        // reads of the table stay behind the barrier
 
-    const int my_tiles = gw < P.tiles_total ? (P.tiles_total - gw + n_warps - 1) / n_warps : 0;
+    const int my_tiles = tw < P.tiles_total ? (P.tiles_total - tw + tstep - 1) / tstep : 0;
     // residual tiles are dealt from the last warp backwards (the compressed tiles are dealt from
     // the first warp forwards, so the warps with one tile fewer take them)
     const int n_rt = (a.n_res + 15) >> 4, rslot = n_warps - 1 - gw;
     const int my_rt = rslot < n_rt ? (n_rt - rslot + n_warps - 1) / n_warps : 0;
-    const int nkb = 1 << P.nkb_shift, nvi = 1 << P.nvi_shift;   // K blocks / V blocks per tile
-    const int k_items = PASS == kValues ? 0 : my_tiles << P.nkb_shift, v_items = PASS == kScores ? 0 : my_tiles << P.nvi_shift;
+    const int nvi_shift = TEAM && !P.vpair ? 0 : P.nvi_shift;   // a team's warp reads one channel half: its block of a 128-token tile
+    const int nkb = 1 << P.nkb_shift, nvi = 1 << nvi_shift;     // K blocks / V items per tile
+    const int k_items = PASS == kValues ? 0 : my_tiles << P.nkb_shift, v_items = PASS == kScores ? 0 : my_tiles << nvi_shift;
     const int total_items = k_items + v_items;
     const int k_rounds = a.cbk >> 4;
     const int lbk = len_field_bits(a.bits_k), lbv = len_field_bits(a.bits_v);
@@ -404,13 +412,17 @@ __global__ void __launch_bounds__(kAW * 32, PASS == 1 ? PKV_ATTN_CTAS_SCORES : P
     auto load_info = [&](int n) -> uint4 {
         if (n < k_items) {
             const int tl = n >> P.nkb_shift, i = n & (nkb - 1);
-            const uint2 e = __ldg(kinfo_h + (((gw + tl * n_warps) << P.nkb_shift) + i) * a.kv_heads);
+            const uint2 e = __ldg(kinfo_h + (((tw + tl * tstep) << P.nkb_shift) + i) * a.kv_heads);
             return make_uint4(e.x, e.y, 0, 0);
         }
         const int m = n - k_items;
-        const int tl = m >> P.nvi_shift, vi = m & (nvi - 1);
+        const int tl = m >> nvi_shift, vi = m & (nvi - 1);
+        if (TEAM) {
+            const uint2 e = __ldg(vinfo_h + (((tw + tl * tstep) << nvi_shift) + vi) * (2 * a.kv_heads) + (wic >> 1));
+            return make_uint4(e.x, e.y, 0, 0);
+        }
         if (P.vpair) {
-            const uint2* p = vinfo_h + (((gw + tl * n_warps) << P.nvi_shift) + vi) * (2 * a.kv_heads);
+            const uint2* p = vinfo_h + (((gw + tl * n_warps) << nvi_shift) + vi) * (2 * a.kv_heads);
             const uint2 e0 = __ldg(p), e1 = __ldg(p + 1);
             return make_uint4(e0.x, e0.y, e1.x, e1.y);
         }
@@ -437,23 +449,23 @@ __global__ void __launch_bounds__(kAW * 32, PASS == 1 ? PKV_ATTN_CTAS_SCORES : P
         if (is_k) {
             const int tl = n >> P.nkb_shift, i = n & (nkb - 1);
             if (KMODE == kKChannel) {
-                const int off_e = (((gw + tl * n_warps) << P.nkb_shift) + i) * kD;
+                const int off_e = (((tw + tl * tstep) << P.nkb_shift) + i) * kD;
                 p0 = kpar_s + off_e; p1 = kpar_z + off_e; pbytes = 2 * kD;
             } else if (i == 0) {
-                const int t0 = (gw + tl * n_warps) << P.tile_shift;
+                const int t0 = (tw + tl * tstep) << P.tile_shift;
                 p0 = kpar_s + t0; p1 = kpar_z + t0; pbytes = 2 * P.tile;
             }
         } else {
             const int m = n - k_items;
-            const int tl = m >> P.nvi_shift, vi = m & (nvi - 1);
-            if (vi == 0 || (!P.vpair && vi == 0)) {
-                const int t0 = (gw + tl * n_warps) << P.tile_shift;
+            const int tl = m >> nvi_shift, vi = m & (nvi - 1);
+            if (vi == 0) {
+                const int t0 = (tw + tl * tstep) << P.tile_shift;
                 p0 = vpar_s + t0; p1 = vpar_z + t0; pbytes = 2 * P.tile;
             }
         }
         pk0 = check_block(inf.x, inf.y, base, cap, bound);
-        pk1 = (!is_k && P.vpair) ? check_block(inf.z, inf.w, base, cap, bound) : 0u;
-        if ((pk0 == 0 || (!is_k && P.vpair && pk1 == 0)) && lane == 0) atomicOr(a.flags, kFlagBadStream);
+        pk1 = (!TEAM && !is_k && P.vpair) ? check_block(inf.z, inf.w, base, cap, bound) : 0u;
+        if ((pk0 == 0 || (!TEAM && !is_k && P.vpair && pk1 == 0)) && lane == 0) atomicOr(a.flags, kFlagBadStream);
         if (lane == 0) {
             const unsigned slot = n & ns_mask;
             const unsigned dst = wbase_a + slot * P.slot, bar = bar_a + 8 * slot;
@@ -547,6 +559,14 @@ __global__ void __launch_bounds__(kAW * 32, PASS == 1 ? PKV_ATTN_CTAS_SCORES : P
     // of the lower-row registers (6,2) (4,0) (14,10) (12,8), slot g + 8 the token after it
     const int tau = ((g >> 2) << 3) + ((g & 1) ? ((g & 2) ? 0 : 2) : ((g & 2) ? 4 : 6));
 
+    // where part i of a block (K round, V segment) starts behind the table of part ends at the block's beginning; a table
+    // that no encoder writes reads as 0, so that the part stays inside the staged bytes
+    auto part_start = [&](unsigned blk, int i, int part_bound) -> int {
+        const int at = i ? (int)lds16(blk + 2 * (i - 1)) : 0;
+        if (at > i * part_bound || (at & 1)) { bad_len = true; return 0; }
+        return at;
+    };
+
     T2 mpk0 = as_t2<T2>(Tr<T>::pack2(-INFINITY, -INFINITY)), mpk1 = mpk0;   // running max of this lane's scores, heads 2c and 2c+1
 
     // ============================================================================ phase 1: K tiles
@@ -554,7 +574,8 @@ __global__ void __launch_bounds__(kAW * 32, PASS == 1 ? PKV_ATTN_CTAS_SCORES : P
     auto k_block = [&](auto bits_tag, unsigned blk, int i, unsigned st, const T2 (&ksd)[4], const T2 (&kzb)[4]) {
         constexpr int BK = decltype(bits_tag)::value, LBK = len_field_bits(BK);
         int pos = 2 * k_rounds;
-        for (int r = 0; r < k_rounds; r++) {
+        for (int r = TEAM ? wic : 0; r < k_rounds; r += TEAM ? kAW : 1) {
+            if (TEAM) pos = 2 * k_rounds + part_start(blk, r, 16 * BK + 16 * LBK + 256 * BK);
             const unsigned hdr = blk + pos;
             unsigned lens4 = spread_const<LBK>(lane_word<4 * LBK>(hdr + 16 * BK, lane));   // byte j = length of pack j
             const unsigned mins4 = spread_const<BK>(lane_word<4 * BK>(hdr, lane));
@@ -801,7 +822,7 @@ __global__ void __launch_bounds__(kAW * 32, PASS == 1 ? PKV_ATTN_CTAS_SCORES : P
             const unsigned st = stile_a + tl * P.rows * P.prow + 4 * lane;
 #pragma unroll
             for (int r = 0; r < 8; r++) {
-                if (r < P.rows) {
+                if (r < P.rows && (!TEAM || (r & (kAW - 1)) == wic)) {   // a team's rows are shared out
                     const float m = cs->cl_m[r];
                     for (int ch = 0; ch < chunks; ch++) {
                         const float2 x = Tr<T>::unpack2(lds32(st + r * P.prow + 128 * ch));
@@ -949,6 +970,7 @@ __global__ void __launch_bounds__(kAW * 32, PASS == 1 ? PKV_ATTN_CTAS_SCORES : P
     for (int i = 0; i < 8; i++)
 #pragma unroll
         for (int j = 0; j < 4; j++) o[i][j] = 0.f;
+    float ot[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};   // TEAM: this warp's 32 channels over the team's tiles
 
     // One V block (cbv tokens x 64 channels).  A segment is 64 tokens x 32 channels; lane l of the warp owns
     // channel l's four packs in the stream (lengths, minima, offsets), while the mma wants lane (g, c) to hold
@@ -961,7 +983,7 @@ __global__ void __launch_bounds__(kAW * 32, PASS == 1 ? PKV_ATTN_CTAS_SCORES : P
         const int rpw = a.cbv == 128 ? 2 : 1;           // segments of 64 tokens per 32 channels
         int pos = 4 * rpw;
         auto segment = [&](auto w_tag, int rr) {
-            constexpr int W = decltype(w_tag)::value, SEL = 2 * HH + W;
+            constexpr int SEL = 2 * HH + decltype(w_tag)::value;
             const int tok_seg = tok_blk + rr * 64;     // first token (in the tile) of the segment
             const unsigned hdr = blk + pos;
             unsigned lens4 = spread_const<LBV>(lane_word<4 * LBV>(hdr + 16 * BV, lane));   // byte q = length of pack q (tokens 16q..16q+15)
@@ -1014,12 +1036,20 @@ __global__ void __launch_bounds__(kAW * 32, PASS == 1 ? PKV_ATTN_CTAS_SCORES : P
 #pragma unroll
                 for (int s = 0; s < 4; s++) {
                     const unsigned af[4] = {x[0][2 * s], x[1][2 * s], x[0][2 * s + 1], x[1][2 * s + 1]};
-                    Tr<T>::mma(o[2 * SEL + mt], af, pw[2 * s], pw[2 * s + 1]);
+                    Tr<T>::mma(TEAM ? ot[mt] : o[2 * SEL + mt], af, pw[2 * s], pw[2 * s + 1]);
                 }
             }
             __syncwarp();                              // descriptors are rewritten by the next segment
             pos += 16 * BV + 16 * LBV + 2 * (int)(t012 + (tot >> 24));
         };
+        if (TEAM) {
+#pragma unroll 1
+            for (int rr = 0; rr < rpw; rr++) {
+                pos = 4 * rpw + part_start(blk, (wic & 1) * rpw + rr, 16 * BV + 16 * LBV + 256 * BV);
+                segment(std::integral_constant<int, 0>{}, rr);
+            }
+            return;
+        }
         // (unrolling these two loops as well was measured slower: 122 against 117 us per layer)
 #pragma unroll 1
         for (int rr = 0; rr < rpw; rr++) segment(std::integral_constant<int, 0>{}, rr);
@@ -1027,22 +1057,43 @@ __global__ void __launch_bounds__(kAW * 32, PASS == 1 ? PKV_ATTN_CTAS_SCORES : P
         for (int rr = 0; rr < rpw; rr++) segment(std::integral_constant<int, 1>{}, rr);
     };
 
+    // scores -> probabilities rounded to the element type, in place, pair order: unit u = (row, group of eight tokens, e)
+    const int pr_shift = P.tile_shift - 2, units = P.rows << pr_shift;
+    if (TEAM) {
+        // all of the team's tiles at once; the two units of a group of eight, which read what the other one writes, are
+        // neighbouring lanes of a warp
+        for (int u0 = 0; u0 < my_tiles * units; u0 += kAW * 32) {
+            const int v = u0 + threadIdx.x, tl = v / units, u = v - tl * units;
+            const int r = u >> pr_shift, rem = u & ((1 << pr_shift) - 1), q8 = rem >> 1, e = rem & 1;
+            const unsigned row = stile_a + (tl * P.rows + r) * P.prow + 16 * q8;
+            unsigned w0 = 0, w1 = 0;
+            if (tl < my_tiles) {
+                const float M = cs->gM[r], I = cs->gInvL[r];
+                const float2 xa = Tr<T>::unpack2(lds32(row + 4 * e)), xb = Tr<T>::unpack2(lds32(row + 4 * e + 8));
+                const unsigned pa = Tr<T>::pack2(fast_exp(xa.x - M) * I, fast_exp(xa.y - M) * I);
+                const unsigned pb = Tr<T>::pack2(fast_exp(xb.x - M) * I, fast_exp(xb.y - M) * I);
+                pair_words(pa, pb, w0, w1);
+            }
+            __syncwarp();
+            if (tl < my_tiles) sts64(row + 8 * (1 - e), w0, w1);
+        }
+        __syncthreads();
+    }
+
     for (int n = k_items; n < total_items; n++) {
         cur_pk0 = nxt_pk0; cur_pk1 = nxt_pk1;
         wait_item(n);
         if (dead) { cur_pk0 = 0; cur_pk1 = 0; }
         __syncwarp();
         const int m = n - k_items;
-        const int tl = m >> P.nvi_shift, vi = m & (nvi - 1);
+        const int tl = m >> nvi_shift, vi = m & (nvi - 1);
         const unsigned st_a = stile_a + tl * P.rows * P.prow;
 
         if (vi == 0 && !dead) {
             // the tile's V scales and zero-points, pair order
             permute_params();
-            // scores -> probabilities rounded to the element type, in place, pair order: unit u = (row, group of
-            // eight tokens, e); loads of up to four units per lane, a warp barrier, then the stores
-            const int pr_shift = P.tile_shift - 2, units = P.rows << pr_shift;
-            for (int u0 = 0; u0 < units; u0 += 128) {
+            // the tile's probabilities: loads of up to four units per lane, a warp barrier, then the stores
+            for (int u0 = 0; !TEAM && u0 < units; u0 += 128) {
                 unsigned w0[4], w1[4];
 #pragma unroll
                 for (int it = 0; it < 4; it++) {
@@ -1081,14 +1132,14 @@ __global__ void __launch_bounds__(kAW * 32, PASS == 1 ? PKV_ATTN_CTAS_SCORES : P
         asm volatile("" : "+r"(sbase) :: "memory");        // the reads of the blocks stay behind the wait for their copy
         if (!(PKV_ABL & 1)) {
 #pragma unroll 1
-            for (int sub = 0; sub < (P.vpair ? 2 : 1); sub++) {
+            for (int sub = 0; sub < (!TEAM && P.vpair ? 2 : 1); sub++) {
                 const unsigned pk = sub ? cur_pk1 : cur_pk0;
                 if (pk == 0) continue;
                 const unsigned blk = sbase + sub * half_slot + (pk & 15);
                 const int hh = P.vpair ? sub : vi;                       // which 64-channel half of the head
                 const int tok_blk = P.vpair ? (vi << 6) : 0;             // token offset of the block in the tile
                 auto by_half = [&](auto bits_tag) {
-                    if (hh) v_block(bits_tag, std::integral_constant<int, 1>{}, blk, tok_blk, st_a);
+                    if (!TEAM && hh) v_block(bits_tag, std::integral_constant<int, 1>{}, blk, tok_blk, st_a);
                     else v_block(bits_tag, std::integral_constant<int, 0>{}, blk, tok_blk, st_a);
                 };
                 switch (a.bits_v) {
@@ -1149,6 +1200,14 @@ __global__ void __launch_bounds__(kAW * 32, PASS == 1 ? PKV_ATTN_CTAS_SCORES : P
     __syncwarp();
     // a launch that follows under programmatic stream serialisation (the exchange's wait) may be set up from here on
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    if (TEAM) {
+#pragma unroll
+        for (int mt = 0; mt < 8; mt++)
+            if ((mt >> 1) == wic) {
+#pragma unroll
+                for (int j = 0; j < 4; j++) o[mt][j] += ot[mt & 1][j];
+            }
+    }
     // ---- warp accumulators -> this warp's shared region: red[head][channel] --------------------
     float* red = reinterpret_cast<float*>(wbase);
 #pragma unroll
@@ -1229,9 +1288,9 @@ static int env_int(const char* name) {
     return v ? std::atoi(v) : 0;
 }
 
-template <typename T, int KM, bool HPV, int PASS>
+template <typename T, int KM, bool HPV, int PASS, bool TEAM>
 static int launch_one(const AttnDev& P, dim3 grid, int smem, cudaStream_t st) {
-    auto kern = attn_decode_kernel<T, KM, HPV, PASS>;
+    auto kern = attn_decode_kernel<T, KM, HPV, PASS, TEAM>;
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return kCudaError;
     if (P.cluster > 8 && cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) return kCudaError;
     cudaLaunchConfig_t cfg = {};
@@ -1261,17 +1320,17 @@ static int launch_one(const AttnDev& P, dim3 grid, int smem, cudaStream_t st) {
     return cudaLaunchKernelEx(&cfg, kern, P) == cudaSuccess ? kOk : kCudaError;
 }
 
-template <typename T, int PASS>
+template <typename T, int PASS, bool TEAM = false>
 static int launch_pass(const AttnDev& P, dim3 grid, int smem, cudaStream_t st) {
     const AttnArgs& a = P.a;
     if (a.k_mode == kKChannel)
-        return a.high_precision_zero ? launch_one<T, kKChannel, true, PASS>(P, grid, smem, st) : launch_one<T, kKChannel, false, PASS>(P, grid, smem, st);
-    return a.high_precision_zero ? launch_one<T, kKToken, true, PASS>(P, grid, smem, st) : launch_one<T, kKToken, false, PASS>(P, grid, smem, st);
+        return a.high_precision_zero ? launch_one<T, kKChannel, true, PASS, TEAM>(P, grid, smem, st) : launch_one<T, kKChannel, false, PASS, TEAM>(P, grid, smem, st);
+    return a.high_precision_zero ? launch_one<T, kKToken, true, PASS, TEAM>(P, grid, smem, st) : launch_one<T, kKToken, false, PASS, TEAM>(P, grid, smem, st);
 }
 
 template <typename T>
 static int launch_typed(const AttnDev& P, dim3 grid, int smem, cudaStream_t st) {
-    if (P.nsplit == 1 && P.sc_count == nullptr) return launch_pass<T, kFused>(P, grid, smem, st);
+    if (P.nsplit == 1 && P.sc_count == nullptr) return P.team ? launch_pass<T, kFused, true>(P, grid, smem, st) : launch_pass<T, kFused>(P, grid, smem, st);
 #ifdef PKV_DEBUG_PASS   // measurement builds: one of the two launches alone (the results are then meaningless)
     static const int only = env_int("PKV_ATTN_ONLY_PASS");
     if (only == 1) return launch_pass<T, kScores>(P, grid, smem, st);
@@ -1290,7 +1349,8 @@ static int plan_smem(AttnDev& P, int cl, int nsplit, int nslots, int slot) {
     P.nsplit = nsplit;
     P.nslots = nslots;
     P.slot = slot;
-    P.tpw = (P.tiles_total + n_warps - 1) / n_warps;
+    const int owners = P.team ? cl : n_warps;                 // a team's tiles lie in the first warp's region; the others' stay empty
+    P.tpw = (P.tiles_total + owners - 1) / owners;
     P.rtw = ((a.n_res + 15) / 16 + n_warps - 1) / n_warps;
     int off = nslots * slot;
     if (off < 16 * 272) off = 16 * 272;                       // the residual V tile borrows the staging slots
@@ -1462,13 +1522,18 @@ int launch_attention(const AttnArgs& a, const AttnExchange* xch, const AttnAppen
     // per cluster of the pair.  Clusters are placed inside one GPC: about 7 % of the slots stay unusable for them
     // (136 clusters of 4 fit at once, 144 do not), and clusters above the portable size schedule badly once they
     // fill more than half the GPU.
-    auto plan_cost = [&](long ctas, int cl, int per_sm, double avg_upw, int upw_max, double fixed, int ns) {
+    auto plan_cost = [&](long ctas, int cl, int per_sm, double avg_upw, double upw_dealt, double upw_placed, double fixed, int ns, int launches, bool team) {
         long slots = (long)kSmCount * per_sm;
         if (cl > 1) slots = (long)((double)slots * 0.93 / cl) * cl;
         if (slots < cl) slots = cl;
         const long waves = (ctas + slots - 1) / slots;
         const long on_gpu = ctas < slots ? ctas : slots;
         const int sm_warps = (int)((on_gpu + kSmCount - 1) / kSmCount) * kAW;
+        // On a busy SM it makes no difference who holds the residual tiles; on an idle one it is the longest warp's time
+        // (counted for clusters that place well), and so are the hand-over and the second start of two launches.
+        const bool idle = sm_warps <= 8;
+        const double upw_max = team || (idle && !(cl & (cl - 1))) ? upw_placed : upw_dealt;
+        if (idle && launches == 2) fixed += 1.0;
         // (a launch ends with its longest warps running alone, below the saturated rate: three quarters of the
         // difference between the longest and the average warp count as if every warp had them)
         const double eff_upw = avg_upw + 0.75 * (upw_max - avg_upw);
@@ -1477,7 +1542,29 @@ int launch_attention(const AttnArgs& a, const AttnExchange* xch, const AttnAppen
         double cost = (double)waves * (thr > lat ? thr : lat);
         if (ns == 1) cost *= 1.02;                              // the copy of the next block is not overlapped (it comes from L2)
         if (cl > 8) cost *= 2 * ctas > slots ? 1.4 : 1.1;
+        if (team && sm_warps > 8) cost *= 1.15;                 // a team's extra instructions count once the SM is busy (11 x 2154, 2 bits: 39 us against 35)
+        if (team && (cl & (cl - 1))) cost *= 1.06;              // short launches: clusters of 3..11 cost 1 to 2 us more than 4 or 8
         return cost;
+    };
+    // Units of the longest warp.  Compressed tiles are dealt from the first owner (warp, or CTA of a team) on, residual
+    // tiles from the last warp backwards: with owners to spare nobody has one more of both (700 tokens, one sequence:
+    // 14.6 us with the 12 residual tiles beside the compressed ones, 16.7 us behind them).
+    const auto longest = [&](int owners, double unit, int warps_per_owner) {
+        const int T = P.tiles_total, n_warps = owners * warps_per_owner;
+        const int q = T / owners, more_t = T % owners, p = n_rt / n_warps, more_r = (n_rt % n_warps + warps_per_owner - 1) / warps_per_owner;
+        if (more_t + more_r > owners) return (q + 1) * unit + p + 1;
+        double most = q * unit + p;
+        if (more_t && most < (q + 1) * unit + p) most = (q + 1) * unit + p;
+        if (more_r && most < q * unit + p + 1) most = q * unit + p + 1;
+        return most;
+    };
+    // A team (see TEAM) turns a warp's whole tiles into quarters of the CTA's tiles, for about 15 % more instructions (every
+    // warp stages the block; tables and probabilities are shared).  It pays where warps have one tile or none: the time is
+    // then one tile's latency (one sequence x 700 tokens, 8 KV heads: 28.1 us a launch before, 14.6 as a team; two sequences
+    // x 825: 20.6 and 14.6).  With two tiles to a warp the launch is bound by issue (42 x 521: 32 us, 37 as a team).  The rule
+    // looks at one pair only, so that a forced plan computes the same bits whatever the batch.
+    const auto team_wins = [&](int cl) {
+        return kAW == 4 && P.tiles_total > 0 && P.tiles_total <= kAW * cl && 1.15 * ((P.tiles_total + cl - 1) / cl) < kAW;
     };
     static const int kSplits[] = {1, 2, 3, 4, 6, 8, 12, 16, 24, 32, 48, 64};
     int best_cl = 0, best_ns = 1, best_split = 1, best_launches = 1, best_extra = -1;
@@ -1494,6 +1581,7 @@ int launch_attention(const AttnArgs& a, const AttnExchange* xch, const AttnAppen
                 for (int ns = 2; ns >= 1; ns--) {
                     if (env_slots && ns != env_slots) continue;
                     AttnDev Q = P;
+                    Q.team = launches == 1 && team_wins(cl);
                     const int smem = plan_smem(Q, cl, split, ns, slot);
                     if (smem > 227 * 1024) continue;
                     if (launches == 2 && (!scratch || scratch_layout(pairs, cl, split, Q.dump_bytes).total > scratch_bytes)) continue;
@@ -1501,9 +1589,10 @@ int launch_attention(const AttnArgs& a, const AttnExchange* xch, const AttnAppen
                     if (per_sm > kMaxCtasPerSm) per_sm = kMaxCtasPerSm;
                     if (per_sm < 1) continue;
                     const int n_warps = kAW * cl * split;
-                    const int upw = ((P.tiles_total + n_warps - 1) / n_warps) * unit_tile + ((n_rt + n_warps - 1) / n_warps);
+                    const double placed = Q.team ? longest(cl, 1.15 / kAW * unit_tile, kAW) : longest(n_warps, unit_tile, 1);
+                    const double dealt = (double)((P.tiles_total + n_warps - 1) / n_warps) * unit_tile + (n_rt + n_warps - 1) / n_warps;
                     const double fixed = launches == 2 ? 4.0 + 0.05 * split : 3.0;
-                    const double cost = plan_cost(pairs * cl * split, cl, per_sm, pair_units / n_warps, upw, fixed, ns);
+                    const double cost = plan_cost(pairs * cl * split, cl, per_sm, (Q.team ? 1.15 : 1.0) * pair_units / n_warps, dealt, placed, fixed, ns, launches, Q.team);
                     if (cost < best_cost - 1e-9) { best_cost = cost; best_cl = cl; best_ns = ns; best_split = split; best_launches = launches; best_extra = -1; }
                 }
             }
@@ -1532,8 +1621,8 @@ int launch_attention(const AttnArgs& a, const AttnExchange* xch, const AttnAppen
                 if (fit < per_sm && want_extra == 0) continue;
                 const long ctas = pairs * base + extra;
                 const int n_warps = kAW * base;
-                const int upw = ((P.tiles_total + n_warps - 1) / n_warps) * unit_tile + ((n_rt + n_warps - 1) / n_warps);
-                const double cost = plan_cost(ctas, 1, fit, pair_units * pairs / ((double)ctas * kAW), upw, 4.0 + 0.05 * (base + 1), ns);
+                const double dealt = (double)((P.tiles_total + n_warps - 1) / n_warps) * unit_tile + (n_rt + n_warps - 1) / n_warps;
+                const double cost = plan_cost(ctas, 1, fit, pair_units * pairs / ((double)ctas * kAW), dealt, longest(n_warps, unit_tile, 1), 4.0 + 0.05 * (base + 1), ns, 2, false);
                 if (cost < best_cost - 1e-9 || want_extra > 0) {
                     best_cost = cost; best_cl = 1; best_ns = ns; best_split = base; best_launches = 2; best_extra = extra;
                     found = true;
@@ -1544,6 +1633,7 @@ int launch_attention(const AttnArgs& a, const AttnExchange* xch, const AttnAppen
         }
     }
     if (best_cl == 0) return kUnsupported;
+    P.team = best_launches == 1 && team_wins(best_cl);
     const int smem = plan_smem(P, best_cl, best_split, best_ns, slot);
     P.extra = best_extra;
     if (best_launches == 2) {

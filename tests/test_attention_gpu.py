@@ -433,3 +433,21 @@ def test_uneven_ctas_per_pair(cuda_device, k_mode):
         assert _rel_err(outs[-1].float().cpu(), ref, dtype) <= TOL, plan
         assert ops.decode_attention(qd, layer, kr, vr, n_res, scratch=scratch, plan=plan, plan_only=True) == plan
     assert torch.equal(outs[1], outs[4])
+
+
+@pytest.mark.parametrize("cl,n_comp,n_res,block,cbk,cbv,bits,k_mode,hp", [
+    (4, 256, 129, 64, 64, 64, 4, "channel", False),      # one tile of 64 tokens to a CTA, residual tiles beside them
+    (8, 128, 191, 64, 64, 64, 3, "token", False),        # CTAs without a tile
+    (3, 320, 1, 64, 64, 64, 2, "channel", True),         # uneven tiles, one residual token
+    (2, 256, 17, 64, 64, 128, 4, "token", False),        # 128-token tiles of 64-token K blocks
+    (16, 1664, 130, 128, 128, 64, 2, "channel", False),  # 128-token K blocks (two rounds to a warp), 64-token V blocks
+    (5, 1280, 0, 128, 128, 128, 3, "token", True),       # two tiles to a CTA, no residual
+    (1, 128, 5, 64, 64, 128, 4, "channel", False)])
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+def test_team_form_matches_reference(cuda_device, dtype, cl, n_comp, n_res, block, cbk, cbv, bits, k_mode, hp):
+    """Single launches in which the four warps of a CTA share its tiles (the rule takes it for these sizes and cluster
+    sizes), at groups of 1, 4 and 7 q heads."""
+    for G in (1, 4, 7):
+        err = _run_case(cuda_device, dtype, 2, 2, G, n_comp, n_res, block=block, cbk=cbk, cbv=cbv, bits_k=bits, bits_v=bits, k_mode=k_mode,
+                        seed=60 + cl + G, hp=hp, plan=(cl, 1, 1), repeats=2)
+        assert err <= TOL, (G, err)
