@@ -58,6 +58,11 @@ constexpr unsigned kChainSpins = 1u << 24;  // polls of a look-back before it gi
 
 // The CTA's place in the launch: ticket t -> (sequence, link).  All threads call; one barrier.
 __device__ __forceinline__ void chain_place(const FusedArgs& a, unsigned* sh_word, int& b, int& link) {
+    if (a.links == 1) {          // nothing before it in its sequence: no place to take, no status to publish
+        b = (int)(blockIdx.x + gridDim.x * blockIdx.y);
+        link = 0;
+        return;
+    }
     if (threadIdx.x == 0) *sh_word = atomicAdd(a.ticket, 1u);
     __syncthreads();
     // sequences take turns: the links of one sequence that are in flight at the same time are few, so a look-back
@@ -112,7 +117,7 @@ __device__ __forceinline__ bool chain_offset(const FusedArgs& a, int b, int link
 #endif
     // successors must not hang on a link that gave up: it publishes its own bytes on top of what it has
     if (lane == 0) {
-        *reinterpret_cast<volatile unsigned long long*>(st + link) = (2ull << 32) | (excl + total);
+        if (a.links > 1) *reinterpret_cast<volatile unsigned long long*>(st + link) = (2ull << 32) | (excl + total);
         if (link == a.links - 1) a.stream_bytes[b] = excl + total;
         if (!ok) atomicOr(a.flags, kFlagTimeout);
     }
@@ -299,17 +304,22 @@ __device__ __forceinline__ int k_encode_rounds_packed(const T* x, int64_t ss, co
         unsigned before = 0;
 #pragma unroll
         for (int j = 0; j < 4; j++) {
-            const unsigned step = 1u << len[j];
-            unsigned wt = 0, wb = 0, ones = 0;
+            // 16-bit lanes, four tokens each (token 0 and 4, 8 and 12 highest): w = w * 2^len + code for two of them per
+            // multiply-add, then the minimum is taken off all four fields at once (min * (1 + 2^len + ... + 2^(3 len))).
+            // A lane stays below 2^16: four codes below 2^4 at steps of at most 2^4.  Against one multiply-add and one
+            // extraction per code: 1.6 instead of 2.8 instructions per code.
+            const unsigned step = 1u << len[j], sel = (j & 1) ? 0x7632u : 0x5410u;
+            const unsigned(&cj)[16] = j < 2 ? c01 : c23;
+            unsigned za = __byte_perm(cj[0], cj[4], sel), zb = __byte_perm(cj[8], cj[12], sel);
 #pragma unroll
-            for (int t = 0; t < 8; t++) {
-                const unsigned ct = j < 2 ? c01[t] : c23[t], cb = j < 2 ? c01[t + 8] : c23[t + 8];
-                wt = wt * step + ((j & 1) ? ct >> 16 : ct & 0xFFFFu);
-                wb = wb * step + ((j & 1) ? cb >> 16 : cb & 0xFFFFu);
-                ones = ones * step + 1u;
+            for (int t = 1; t < 4; t++) {
+                za = za * step + __byte_perm(cj[t], cj[t + 4], sel);
+                zb = zb * step + __byte_perm(cj[t + 8], cj[t + 12], sel);
             }
-            wt -= mnj[j] * ones;
-            wb -= mnj[j] * ones;
+            const unsigned low = mnj[j] * ((1u + step) * (1u + step * step)) * 0x00010001u;
+            za -= low;
+            zb -= low;
+            const unsigned wt = ((za & 0xFFFFu) << (4 * len[j])) | (za >> 16), wb = ((zb & 0xFFFFu) << (4 * len[j])) | (zb >> 16);
             const uint64_t w = ((uint64_t)wt << (8 * len[j])) | wb;
             store_pack_smem(packs + 2 * (before + ((exc >> (8 * j)) & 0xFFu)), w, len[j]);
             before += (tot >> (8 * j)) & 0xFFu;
@@ -331,8 +341,9 @@ __device__ __forceinline__ int k_encode_rounds_packed(const T* x, int64_t ss, co
 #define PKV_K_WARPS 4
 #endif
 constexpr int kKWarps = PKV_K_WARPS;   // warps (= consecutive blocks of a sequence's stream) per CTA of the channel-mode K kernel
-template <typename T, bool CONTIG, int BITS, bool ORDERED = false>
-__global__ void __launch_bounds__(kKWarps * 32, 768 / (kKWarps * 32)) k_fused_encode_kernel(FusedArgs a) {
+constexpr int kKWarpsOne = 8;          // and when that many blocks are all there is of a sequence: one CTA then needs no look-back
+template <typename T, bool CONTIG, int BITS, bool ORDERED, int NW>
+__global__ void __launch_bounds__(NW * 32, 768 / (NW * 32)) k_fused_encode_kernel(FusedArgs a) {
     constexpr bool HP = false;
     const int64_t ss = CONTIG ? 128 : a.ss;
     extern __shared__ __align__(16) uint8_t smem[];
@@ -340,16 +351,16 @@ __global__ void __launch_bounds__(kKWarps * 32, 768 / (kKWarps * 32)) k_fused_en
     const int lane = lane_id(), wic = threadIdx.x >> 5;
     const int nctx = a.tokens / a.cb;
     const int64_t per_seq = (int64_t)nctx * a.heads;
-    __shared__ unsigned sh_word, sh_sizes[kKWarps];
+    __shared__ unsigned sh_word, sh_sizes[NW];
     const bool direct = a.status != nullptr;
     int b, rem, link = 0;
     int64_t warp = 0;
     if (direct) {
-        // the CTA's warps take kKWarps consecutive blocks of one sequence's stream
+        // the CTA's warps take NW consecutive blocks of one sequence's stream
         chain_place(a, &sh_word, b, link);
-        rem = link * kKWarps + wic;
+        rem = link * NW + wic;
     } else {
-        warp = (int64_t)blockIdx.x * kKWarps + wic;
+        warp = (int64_t)blockIdx.x * NW + wic;
         if (warp >= per_seq * a.batch) return;
         b = (int)(warp / per_seq);
         rem = (int)(warp % per_seq);
@@ -368,7 +379,7 @@ __global__ void __launch_bounds__(kKWarps * 32, 768 / (kKWarps * 32)) k_fused_en
     // (min/max of element-type values is exact, so the fp32 detour is not needed here)
     using T2 = typename QT<T>::T2;
     T2 lo01 = QT<T>::init2(INFINITY), lo23 = lo01, hi01 = QT<T>::init2(-INFINITY), hi23 = hi01;
-#pragma unroll 8
+#pragma unroll 16
     for (int t = 0; t < a.cb; t++) {
         const uint2 raw = __ldg(reinterpret_cast<const uint2*>(x + (int64_t)t * ss));
         const T2 v01 = *reinterpret_cast<const T2*>(&raw.x), v23 = *reinterpret_cast<const T2*>(&raw.y);
@@ -397,9 +408,9 @@ __global__ void __launch_bounds__(kKWarps * 32, 768 / (kKWarps * 32)) k_fused_en
     }   // active
     if (direct) {
         if (lane == 0) sh_sizes[wic] = (unsigned)pos;
-        const int64_t left = per_seq - (int64_t)link * kKWarps;
-        chain_store(a, b, link, sh_sizes, (int)(left < kKWarps ? left : kKWarps), &sh_word,
-                    (int64_t)a.first_cb * a.heads + (int64_t)link * kKWarps, kKWarps, [&](int j) { return smem + j * slot_smem; });
+        const int64_t left = per_seq - (int64_t)link * NW;
+        chain_store(a, b, link, sh_sizes, (int)(left < NW ? left : NW), &sh_word,
+                    (int64_t)a.first_cb * a.heads + (int64_t)link * NW, NW, [&](int j) { return smem + j * slot_smem; });
     } else {
         store_slot(a.slots + (int64_t)warp * a.slot_stride, stage, pos, lane);
         if (lane == 0) a.info[((int64_t)b * a.info_seq_stride + (int64_t)(a.first_cb + cbi) * a.heads + h) * 2 + 1] = (unsigned)pos;
@@ -525,10 +536,10 @@ __device__ __forceinline__ void chunk_to_pack(const uint4& cw, int& len, uint64_
 // reference's token mode reduces over dims [1, 4], utils/compute.py:405-410): half a warp per token.
 // Writes (scale, zero, 1/scale, packed code bias or 0) to prm[] and scale / zero to the caller's arrays.
 // ord[t] = source row (inside the block) of stored row t; WRITE = false keeps the parameters in shared memory only.
-template <typename T, int CB, bool WRITE = true>
+template <typename T, int CB, bool WRITE = true, int NW = 8>
 __device__ __forceinline__ bool token_params_pass(const FusedArgs& a, const T* xb, float4* prm, const uint8_t* ord, int b, int cbi, int lane, int wic) {
     bool bad = false;
-    for (int t = 2 * wic + (lane >> 4); t < CB; t += 16) {     // 8 channels per lane
+    for (int t = 2 * wic + (lane >> 4); t < CB; t += 2 * NW) {     // 8 channels per lane
         const T* xt = xb + (int64_t)ord[t] * a.ss + 8 * (lane & 15);
         using T2 = typename QT<T>::T2;
         T2 lo2 = QT<T>::init2(INFINITY), hi2 = QT<T>::init2(-INFINITY);
@@ -564,10 +575,10 @@ __device__ __forceinline__ bool token_params_pass(const FusedArgs& a, const T* x
 }
 
 // Source row (inside a block of CB tokens) of every stored row: the identity, or the caller's reorder of every
-// order_block tokens.  256 threads; ends with a CTA barrier.
-template <int CB>
+// order_block tokens.  NW warps; ends with a CTA barrier.
+template <int CB, int NW = 8>
 __device__ __forceinline__ void load_row_order(const FusedArgs& a, uint8_t* ord, int b, int cbi) {
-    for (int t = threadIdx.x; t < CB; t += 256) {
+    for (int t = threadIdx.x; t < CB; t += 32 * NW) {
         unsigned src = t;
         if (a.order) {
             const int ob = a.order_block, sub = t / ob;
@@ -578,8 +589,14 @@ __device__ __forceinline__ void load_row_order(const FusedArgs& a, uint8_t* ord,
     __syncthreads();
 }
 
-template <typename T, bool HP, int BITS, int CB>
-__global__ void __launch_bounds__(256, 3) v_fused_encode_kernel(FusedArgs a) {
+// finished blocks that a warp of the V kernel holds in the direct form until their offsets are known
+__host__ __device__ constexpr int v_slots(int heads, int nw) { return (2 * heads + nw - 1) / nw; }
+
+// NW warps: 8, or 16 for launches of no more CTAs than SMs, whose time is that of one CTA (every warp then packs one block
+// of an 8-head token block instead of two, and the parameter pass has half the rows to a warp): with the K kernel's
+// single-CTA form, 16 sequences x 64 tokens take 98 us for four layers' K and V instead of 121
+template <typename T, bool HP, int BITS, int CB, int NW>
+__global__ void __launch_bounds__(NW * 32, NW == 8 ? 3 : 1) v_fused_encode_kernel(FusedArgs a) {
     extern __shared__ __align__(16) uint8_t smem[];
     constexpr int LB = len_field_bits(BITS);
     const int lane = lane_id(), wic = threadIdx.x >> 5;
@@ -591,20 +608,20 @@ __global__ void __launch_bounds__(256, 3) v_fused_encode_kernel(FusedArgs a) {
     constexpr int PPT = CB == 32 ? 2 : 4, RPW = CB == 128 ? 2 : 1;
     const VGeom g(CB, BITS);
     const int bound16 = (g.head_bytes + g.nseg * (g.min_bytes + g.len_bytes + 32 * PPT * 2 * BITS) + 15) & ~15;
-    const int wstride = CB * 64 + (direct ? 2 : 1) * bound16;
+    const int wstride = CB * 64 + (direct ? v_slots(a.heads, NW) : 1) * bound16;
     float4* prm = reinterpret_cast<float4*>(smem);           // [cb] (scale, zero, 1/scale, fast)
     uint8_t* wbase = smem + 32 * CB + wic * wstride;
     uint8_t* ctile = wbase;                                  // [cb][64] codes
     const T* xb = reinterpret_cast<const T*>(a.x) + (int64_t)b * a.sb + (int64_t)cbi * CB * a.ss;
-    uint8_t* ord = smem + 32 * CB + 8 * wstride;
-    load_row_order<CB>(a, ord, b, cbi);
+    uint8_t* ord = smem + 32 * CB + NW * wstride;
+    load_row_order<CB, NW>(a, ord, b, cbi);
 
     // pass 1: per-token statistics across every head and channel
-    bool bad = token_params_pass<T, CB>(a, xb, prm, ord, b, cbi, lane, wic);
+    bool bad = token_params_pass<T, CB, true, NW>(a, xb, prm, ord, b, cbi, lane, wic);
     // one decision for the whole CTA: the packed conversion needs every token's parameters in range
     __syncthreads();
     bool mine_ok = true, mine_half = true;
-    for (int t = threadIdx.x; t < CB; t += 256) {
+    for (int t = threadIdx.x; t < CB; t += 32 * NW) {
         mine_ok = mine_ok && __float_as_uint(prm[t].w) != 0u;
         mine_half = mine_half && reinterpret_cast<const uint4*>(prm + CB)[t].w != 0u;
     }
@@ -614,10 +631,10 @@ __global__ void __launch_bounds__(256, 3) v_fused_encode_kernel(FusedArgs a) {
     // pass 2: quantise + pack, one warp per V block
     unsigned seen = 0;
     const int nvb = 2 * a.heads;
-    for (int vb = wic; vb < nvb; vb += 8) {
+    for (int vb = wic; vb < nvb; vb += NW) {
         const int h = vb >> 1, half = vb & 1;
         const T* src = xb + (int64_t)h * a.sh + 64 * half;
-        uint8_t* stage = wbase + CB * 64 + (direct ? (vb >> 3) * bound16 : 0);
+        uint8_t* stage = wbase + CB * 64 + (direct ? (vb / NW) * bound16 : 0);
         __syncwarp();
         seen |= all_half ? v_quantise_tile<T, CB, 2>(src, a.ss, prm, ord, ctile, lane)
                          : all_packed ? v_quantise_tile<T, CB, 1>(src, a.ss, prm, ord, ctile, lane) : v_quantise_tile<T, CB, 0>(src, a.ss, prm, ord, ctile, lane);
@@ -674,8 +691,8 @@ __global__ void __launch_bounds__(256, 3) v_fused_encode_kernel(FusedArgs a) {
         }
     }
     if (direct)
-        chain_store(a, b, cbi, sh_sizes, nvb, &sh_word, (int64_t)(a.first_cb + cbi) * nvb, 8,
-                    [&](int j) { return smem + 32 * CB + (j & 7) * wstride + CB * 64 + (j >> 3) * bound16; });
+        chain_store(a, b, cbi, sh_sizes, nvb, &sh_word, (int64_t)(a.first_cb + cbi) * nvb, NW,
+                    [&](int j) { return smem + 32 * CB + (j % NW) * wstride + CB * 64 + (j / NW) * bound16; });
     bad = bad || (seen & ~(((1u << BITS) - 1u) * 0x00010001u)) != 0;
     if (__any_sync(0xffffffffu, bad) && lane == 0) atomicOr(a.flags, kFlagCodeRange);
 }
@@ -981,7 +998,8 @@ static int launch_fused_t(const FusedEncodeRequest& r, uint8_t* slots, const uin
     // (PKV_ENCODE_PATH=slots: measurements, tests).
     static const bool env_slots = [] { const char* v = std::getenv("PKV_ENCODE_PATH"); return v && std::string(v) == "slots"; }();
     const bool per_token_kernel = r.which == 1 || r.mode == 1;
-    const int links = per_token_kernel ? nctx : (nctx * r.heads + kKWarps - 1) / kKWarps;
+    const bool k_one = !per_token_kernel && nctx * r.heads <= kKWarpsOne;
+    const int links = per_token_kernel ? nctx : k_one ? 1 : (nctx * r.heads + kKWarps - 1) / kKWarps;
     const int64_t chain_bytes = 256 + (int64_t)r.batch * links * 8;
     // (128-token blocks in the per-token kernels: a second staging buffer per warp would leave one CTA per SM; measured
     // 2.55 ms against 2.28 ms for the slots form on the 4-bit sweep configuration)
@@ -992,7 +1010,7 @@ static int launch_fused_t(const FusedEncodeRequest& r, uint8_t* slots, const uin
         a.status = reinterpret_cast<unsigned long long*>(slots + 256);
         a.links = links;
         a.stream = r.stream; a.stream_seq_stride = r.stream_seq_stride; a.capacity = r.capacity; a.stream_bytes = reinterpret_cast<unsigned*>(r.stream_bytes);
-        if (cudaMemsetAsync(slots, 0, (size_t)chain_bytes, st) != cudaSuccess) return kCudaError;
+        if (links > 1 && cudaMemsetAsync(slots, 0, (size_t)chain_bytes, st) != cudaSuccess) return kCudaError;
     }
     if (r.which == 0) {
         const KGeom g(r.cb, BITS);
@@ -1000,8 +1018,8 @@ static int launch_fused_t(const FusedEncodeRequest& r, uint8_t* slots, const uin
         a.slot_stride = bound16;
         blocks_per_seq = nctx * r.heads;
         const int64_t nwarps = (int64_t)blocks_per_seq * r.batch;
-        const int smem = kKWarps * bound16 + 16;
-        const unsigned grid = direct ? (unsigned)links * r.batch : (unsigned)((nwarps + kKWarps - 1) / kKWarps);
+        const int nw = direct && k_one ? kKWarpsOne : kKWarps, smem = nw * bound16 + 16;
+        const unsigned grid = direct ? (unsigned)links * r.batch : (unsigned)((nwarps + nw - 1) / nw);
         if (r.mode == 1) {                       // per-token parameters: CTA per (sequence, token block)
             const int smem_t = 32 * r.cb + 8 * (r.cb * 128 + bound16) + r.cb + 16;
             auto launch_kt = [&](auto kern) {
@@ -1014,34 +1032,34 @@ static int launch_fused_t(const FusedEncodeRequest& r, uint8_t* slots, const uin
             else if (r.cb == 64) rc = launch_kt(kt_fused_encode_kernel<T, BITS, 64>);
             else rc = launch_kt(kt_fused_encode_kernel<T, BITS, 128>);
             if (rc != kOk) return rc;
-        } else if (a.order) {
-            auto kern = k_fused_encode_kernel<T, false, BITS, true>;
-            if (opt_in_smem(kern, smem)) return kCudaError;
-            kern<<<grid, kKWarps * 32, smem, st>>>(a);
-        } else if (r.stride_s == 128) {
-            auto kern = k_fused_encode_kernel<T, true, BITS>;
-            if (opt_in_smem(kern, smem)) return kCudaError;
-            kern<<<grid, kKWarps * 32, smem, st>>>(a);
         } else {
-            auto kern = k_fused_encode_kernel<T, false, BITS>;
-            if (opt_in_smem(kern, smem)) return kCudaError;
-            kern<<<grid, kKWarps * 32, smem, st>>>(a);
+            auto launch_k = [&](auto kern) {
+                if (opt_in_smem(kern, smem)) return (int)kCudaError;
+                kern<<<grid, nw * 32, smem, st>>>(a);
+                return (int)kOk;
+            };
+            const bool one = nw == kKWarpsOne;
+            const int rc = a.order ? (one ? launch_k(k_fused_encode_kernel<T, false, BITS, true, kKWarpsOne>) : launch_k(k_fused_encode_kernel<T, false, BITS, true, kKWarps>))
+                           : r.stride_s == 128 ? (one ? launch_k(k_fused_encode_kernel<T, true, BITS, false, kKWarpsOne>) : launch_k(k_fused_encode_kernel<T, true, BITS, false, kKWarps>))
+                                               : (one ? launch_k(k_fused_encode_kernel<T, false, BITS, false, kKWarpsOne>) : launch_k(k_fused_encode_kernel<T, false, BITS, false, kKWarps>));
+            if (rc != kOk) return rc;
         }
     } else {
         const VGeom g(r.cb, BITS);
         bound16 = (g.head_bytes + g.nseg * (g.min_bytes + g.len_bytes + 32 * g.ppt * 2 * BITS) + 15) & ~15;
         a.slot_stride = bound16;
         blocks_per_seq = nctx * 2 * r.heads;
-        const int smem = 32 * r.cb + 8 * (r.cb * 64 + (direct ? 2 : 1) * bound16) + r.cb + 16;
+        const int nw = 2 * r.heads > 8 && (int64_t)nctx * r.batch <= 148 ? 16 : 8;
+        const int smem = 32 * r.cb + nw * (r.cb * 64 + (direct ? v_slots(r.heads, nw) : 1) * bound16) + r.cb + 16;
         auto launch_v = [&](auto kern) {
             if (opt_in_smem(kern, smem)) return (int)kCudaError;
-            kern<<<dim3(nctx, r.batch), 256, smem, st>>>(a);
+            kern<<<dim3(nctx, r.batch), nw * 32, smem, st>>>(a);
             return (int)kOk;
         };
         int rc = kOk;
-        if (r.cb == 32) rc = launch_v(v_fused_encode_kernel<T, HP, BITS, 32>);
-        else if (r.cb == 64) rc = launch_v(v_fused_encode_kernel<T, HP, BITS, 64>);
-        else rc = launch_v(v_fused_encode_kernel<T, HP, BITS, 128>);
+        if (r.cb == 32) rc = nw == 16 ? launch_v(v_fused_encode_kernel<T, HP, BITS, 32, 16>) : launch_v(v_fused_encode_kernel<T, HP, BITS, 32, 8>);
+        else if (r.cb == 64) rc = nw == 16 ? launch_v(v_fused_encode_kernel<T, HP, BITS, 64, 16>) : launch_v(v_fused_encode_kernel<T, HP, BITS, 64, 8>);
+        else rc = nw == 16 ? launch_v(v_fused_encode_kernel<T, HP, BITS, 128, 16>) : launch_v(v_fused_encode_kernel<T, HP, BITS, 128, 8>);
         if (rc != kOk) return rc;
     }
     if (direct) return cudaGetLastError() == cudaSuccess ? kOk : kCudaError;

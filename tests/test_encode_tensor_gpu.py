@@ -135,3 +135,27 @@ def test_direct_and_slot_forms(cuda_device, which, mode, H, S):
         assert int(bufs["stream_bytes"][b].item()) == ws.size
         assert np.array_equal(bufs["stream"][b, : ws.size].cpu().numpy(), ws)
         assert np.array_equal(bufs["info"][b].cpu().numpy().view(np.uint32), wi)
+
+
+@pytest.mark.parametrize("which,mode", [("k", ops.K_CHANNEL), ("v", ops.K_TOKEN), ("k", ops.K_TOKEN)])
+@pytest.mark.parametrize("H,S,block,bits", [(8, 64, 64, 4), (5, 128, 64, 3), (8, 64 * 60, 64, 2), (8, 32, 32, 4), (7, 256, 128, 4), (6, 128, 128, 2)])
+def test_launch_forms_by_size(cuda_device, which, mode, H, S, block, bits):
+    """Sequences of one CTA (no look-back: one token block, or at most eight K blocks), V launches of few CTAs (16 warps
+    each) and of more than the GPU has SMs (8 warps), in one call and behind tokens that are already there."""
+    dev, dtype, B = cuda_device, torch.bfloat16, 3
+    rel = synth.rel_for_bits(bits)
+    k, v = synth.synth_kv(B, H, 2 * S, 128, seed=51, dtype=dtype, apply_rope=True)
+    x = k if which == "k" else v
+    want, z, s = _oracle(x, which, mode, block, bits, False)
+    bufs = _bufs(B, H, 2 * S, block, bits, which, mode, dtype, dev)
+    for t0 in (0, S):
+        ops.encode_tensor(which, x[:, :, t0:t0 + S].to(dev), block, rel, mode, bits, block, first_token=t0, **bufs)
+    torch.cuda.synchronize()
+    assert int(bufs["flags"].item()) == 0
+    for b in range(B):
+        ws, wi = want[b]
+        assert int(bufs["stream_bytes"][b].item()) == ws.size
+        assert np.array_equal(bufs["stream"][b, : ws.size].cpu().numpy(), ws)
+        assert np.array_equal(bufs["info"][b].cpu().numpy().view(np.uint32), wi)
+    assert torch.equal(bufs["scale"].cpu().view(torch.int16), s.reshape(bufs["scale"].shape).contiguous().view(torch.int16))
+    assert torch.equal(bufs["zero"].cpu().view(torch.int16), z.reshape(bufs["zero"].shape).contiguous().view(torch.int16))
