@@ -258,6 +258,18 @@ int32_t pkv_rope(const void* x, int64_t x_stride_b, int64_t x_stride_h, int64_t 
                  void* cuda_stream);
 
 /*
+ * Rows of heads with 64 <= dim <= 128 channels widened to 128: K rotated when cos is given (as pkv_rope), V (may be null,
+ * with v_out) copied, into rows [position, position + tokens) of (batch, heads, capacity, 128) buffers.  Channels
+ * dim..127 repeat the row's first 128 - dim channels, or are zero with zero_tail.  The cache packs such heads as
+ * 128-channel blocks: copies leave the quantisation parameters of the real channels as they are.
+ */
+int32_t pkv_widen_rows(const void* k, int64_t k_stride_b, int64_t k_stride_h, int64_t k_stride_s, const void* v,
+                       int64_t v_stride_b, int64_t v_stride_h, int64_t v_stride_s, const void* cos, const void* sin,
+                       int64_t cs_stride_b, void* k_out, void* v_out, int64_t o_stride_b, int64_t o_stride_h,
+                       int32_t capacity, int32_t position, int32_t batch, int32_t heads, int32_t tokens, int32_t dim,
+                       int32_t zero_tail, int32_t is_bf16, void* cuda_stream);
+
+/*
  * Dense reconstruction of quantised tokens, (code + zero) * scale or code * scale + min with the
  * reference's roundings (utils/compute.py:173-178).  codes (batch, tokens, heads*128) as written
  * by pkv_quantize / pkv_{k,v}_decode; scale/zero laid out as in pkv_quantize, the first token of

@@ -93,6 +93,7 @@ SIGNATURES = {
     "pkv_median_order": (_i32, [_p, _i64, _p, _p] + [_i32] * 4 + [_p]),
     "pkv_gather_rows": (_i32, [_p, _p, _i64, _p] + [_i32] * 4 + [_p]),
     "pkv_append_residual": (_i32, [_p, _i64, _i64, _i64, _p, _i64, _i64, _i64, _p, _p, _i64, _p, _p, _i64, _i64] + [_i32] * 6 + [_p]),
+    "pkv_widen_rows": (_i32, [_p, _i64, _i64, _i64, _p, _i64, _i64, _i64, _p, _p, _i64, _p, _p, _i64, _i64] + [_i32] * 8 + [_p]),
     "pkv_greedy_order": (_i32, [_p, _p, _i64, _p] + [_i32] * 5 + [_p]),
     "pkv_size_model": (_i32, [_p, _i64] + [_i32] * 4 + [_p, _p, _p]),
     "pkv_gather_params": (_i32, [_p, _p, _i64, _i32, _p] + [_i32] * 3 + [_p]),
@@ -145,7 +146,7 @@ def lib() -> ctypes.CDLL:
 # the library functions of csrc/host.cpp, in the order of its struct Library
 _HOST_FUNCTIONS = ("pkv_decode_attention", "pkv_decode_attention_append", "pkv_decode_attention_exchange", "pkv_decode_attention_split",
                    "pkv_attention_plan", "pkv_encode_tensor", "pkv_encode_tensor_ordered", "pkv_encode_tensor_static", "pkv_value_median_order",
-                   "pkv_append_residual", "pkv_rope")
+                   "pkv_append_residual", "pkv_rope", "pkv_widen_rows")
 
 
 def host():

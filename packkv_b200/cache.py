@@ -159,7 +159,12 @@ class PackKVCache(_HFCache):
         C, block = L.comp, cfg.block_size
         if self.flags is None:
             self.flags = ops.new_flags(k.device)
-        if cfg.repack_method in (RepackMethod.MEDIAN, RepackMethod.GREEDY):
+        first, order = L.n_comp, None
+        if cfg.repack_method == RepackMethod.MEDIAN and encode.median_in_one_pass(k, v, block, C):
+            # the order straight from V; the encoders then read their rows through it
+            order = ops.value_median_order(v, block, cfg.v_quant_scale_rel, flags=self.flags)
+            C.order = order if C.order is None else torch.cat([C.order, order], dim=1)
+        if order is None and cfg.repack_method in (RepackMethod.MEDIAN, RepackMethod.GREEDY):
             # quantise, reorder the tokens of each new block (median of the V codes, or greedy packs), pack
             kq = ops.quantize(k, block, cfg.k_quant_scale_rel, C.k_mode, bits=C.bits_k, high_precision_zero=C.high_precision_zero,
                               flags=self.flags, scale=C.k_scale, zero=C.k_zero, first_token=L.n_comp)
@@ -178,13 +183,12 @@ class PackKVCache(_HFCache):
                              stream_bytes=C.v_bytes, flags=self.flags, first_cb=L.n_comp // C.cbv)
             C.order = order if C.order is None else torch.cat([C.order, order], dim=1)
         else:
-            scratch = torch.empty(max(16, B * n * H * 128), dtype=torch.uint8, device=k.device)
+            more = dict(flags=self.flags, first_token=first, high_precision_zero=C.high_precision_zero,
+                        scratch=torch.empty(max(16, B * n * H * 128), dtype=torch.uint8, device=k.device), order=order, order_block=block)
             ops.encode_tensor("k", k, block, cfg.k_quant_scale_rel, C.k_mode, C.bits_k, C.cbk, scale=C.k_scale, zero=C.k_zero,
-                              stream=C.k_stream, info=C.k_info, stream_bytes=C.k_bytes, flags=self.flags, first_token=L.n_comp,
-                              high_precision_zero=C.high_precision_zero, scratch=scratch)
+                              stream=C.k_stream, info=C.k_info, stream_bytes=C.k_bytes, **more)
             ops.encode_tensor("v", v, block, cfg.v_quant_scale_rel, ops.K_TOKEN, C.bits_v, C.cbv, scale=C.v_scale, zero=C.v_zero,
-                              stream=C.v_stream, info=C.v_info, stream_bytes=C.v_bytes, flags=self.flags, first_token=L.n_comp,
-                              high_precision_zero=C.high_precision_zero, scratch=scratch)
+                              stream=C.v_stream, info=C.v_info, stream_bytes=C.v_bytes, **more)
         L.n_comp += n
         C.n_comp = L.n_comp
 
@@ -198,65 +202,100 @@ class PackKVCache(_HFCache):
         self._flush(L)
         B, H, T, D = key_states.shape
         if D != 128 and (D > 128 or D < 64 or D % 8):
-            raise RuntimeError("not supported")   # streams are built from 128-channel blocks; 64..120 are padded, see _widen
+            raise RuntimeError("not supported")   # streams are built from 128-channel blocks; 64..120 are widened, see _append
         if cfg.enable_quant and cfg.block_size not in (64, 128):
             # the codec packs 32-token blocks too, but the attention kernel reads 64- and 128-token blocks only:
             # refuse here, not at the first attend()
             raise RuntimeError("not supported: PackKVCache needs block_size 64 or 128")
         # the reference's models pass K before RoPE together with sin/cos; the installed transformers rotates K itself
         cos, sin = (cache_kwargs["cos"], cache_kwargs["sin"]) if cache_kwargs is not None and "cos" in cache_kwargs and "sin" in cache_kwargs else (None, None)
-        if D != 128 and cfg.enable_quant:
+        if not cfg.enable_quant:
+            return self._update_dense(L, key_states, value_states, cos, sin, layer_idx)
+        total = L.n_res + T
+        n_c = compress_block_count(total, cfg.block_size, cfg.buffer_size) * cfg.block_size
+        if n_c == 0 and L.k_res is not None and T == 1 and D == 128 and not self.materialize and key_states.dtype in (torch.float16, torch.bfloat16):
+            # the common decode step: the fused attention to follow writes the token into the residual itself (attend() below)
             if cos is not None:
-                key_states, cos, sin = ops.rope(key_states, cos, sin), None, None
-            key_states, value_states = self._widen(key_states), self._widen(value_states)
-            D = 128
-        if cfg.enable_quant and L.k_res is not None:
-            total = L.n_res + T
-            if compress_block_count(total, cfg.block_size, cfg.buffer_size) == 0:
-                # the common decode step: rotate K and copy V straight into the residual.  With one new token and
-                # the fused attention to follow, the attention launch does it itself (attend() below); otherwise one launch
-                if T == 1 and not self.materialize and key_states.dtype in (torch.float16, torch.bfloat16):
-                    if cos is not None:
-                        cos, sin = cos.to(key_states.dtype).contiguous(), sin.to(key_states.dtype).contiguous()
-                    L.pending = (key_states, value_states, cos, sin)
-                else:
-                    ops.append_residual(key_states, value_states, L.k_res, L.v_res, L.n_res, cos, sin)
-                L.n_res = total
-                return self._step_result(layer_idx, T)
+                cos, sin = cos.to(key_states.dtype).contiguous(), sin.to(key_states.dtype).contiguous()
+            L.pending = (key_states, value_states, cos, sin)
+            L.n_res = total
+            return self._step_result(layer_idx, T)
+        if key_states.stride(3) != 1 or value_states.stride(3) != 1:
+            key_states, value_states = key_states.contiguous(), value_states.contiguous()
+        if value_states.dtype != key_states.dtype:
+            value_states = value_states.to(key_states.dtype)
+        if L.k_res is None:
+            L.k_res = key_states.new_empty(B, H, cfg.buffer_size + cfg.block_size, 128)
+            L.v_res = torch.empty_like(L.k_res)
+
+        def part(t, lo, hi):                     # tokens lo..hi of the cos / sin tables
+            return None if t is None else t[..., lo:hi, :]
+
+        if n_c == 0:
+            self._append(L.k_res, L.v_res, L.n_res, key_states, value_states, cos, sin)
+            L.n_res = total
+        elif L.n_res == 0:
+            # the first tokens: what is packed goes through the rotation (and the widening) once, what stays behind
+            # straight into the residual
+            k_head, v_head = key_states[:, :, :n_c], value_states[:, :, :n_c]
+            if D != 128:
+                k_wide, v_wide = (key_states.new_empty(B, H, n_c, 128) for _ in range(2))
+                self._append(k_wide, v_wide, 0, k_head, v_head, part(cos, 0, n_c), part(sin, 0, n_c))
+                k_head, v_head = k_wide, v_wide
+            else:
+                k_head = ops.rope(k_head, part(cos, 0, n_c), part(sin, 0, n_c)) if cos is not None else k_head.contiguous()
+            self._compress(L, k_head, v_head, cfg)
+            if total > n_c:
+                self._append(L.k_res, L.v_res, 0, key_states[:, :, n_c:], value_states[:, :, n_c:], part(cos, n_c, T), part(sin, n_c, T))
+            L.n_res = total - n_c
+        else:
+            # the residual overflows: its first blocks are packed, the rows behind them start a new one
+            k_all, v_all = L.k_res, L.v_res
+            if total > k_all.shape[2]:
+                k_all = key_states.new_empty(B, H, total, 128)
+                v_all = torch.empty_like(k_all)
+                self._append(k_all, v_all, 0, L.k_res[:, :, : L.n_res], L.v_res[:, :, : L.n_res], None, None)
+            self._append(k_all, v_all, L.n_res, key_states, value_states, cos, sin)
+            self._compress(L, k_all[:, :, :n_c], v_all[:, :, :n_c], cfg)
+            k_res = torch.empty_like(L.k_res)
+            v_res = torch.empty_like(k_res)
+            if total > n_c:
+                self._append(k_res, v_res, 0, k_all[:, :, n_c:total], v_all[:, :, n_c:total], None, None)
+            L.k_res, L.v_res, L.n_res = k_res, v_res, total - n_c
+        return self._step_result(layer_idx, T)
+
+    @staticmethod
+    def _update_dense(L: "_Layer", key_states, value_states, cos, sin, layer_idx: int):
+        """enable_quant off: the cache keeps (and, when asked, collects) the uncompressed K and V."""
         k_new = ops.rope(key_states, cos, sin) if cos is not None else key_states.contiguous()
         v_new = value_states
-        if not cfg.enable_quant:
-            L.k_res = k_new if L.k_res is None else torch.cat([L.k_res[:, :, : L.n_res], k_new], dim=2)
-            L.v_res = v_new.clone() if L.v_res is None else torch.cat([L.v_res[:, :, : L.n_res], v_new], dim=2)
-            L.n_res += T
-            ex = PackKVCacheConfigStatic.extract_cache
-            if ex is not None:
-                ex.key_caches.setdefault(0, {})[layer_idx - 1] = L.k_res
-                ex.value_caches.setdefault(0, {})[layer_idx - 1] = L.v_res
-            return L.k_res, L.v_res
+        L.k_res = k_new if L.k_res is None else torch.cat([L.k_res[:, :, : L.n_res], k_new], dim=2)
+        L.v_res = v_new.clone() if L.v_res is None else torch.cat([L.v_res[:, :, : L.n_res], v_new], dim=2)
+        L.n_res += key_states.shape[2]
+        ex = PackKVCacheConfigStatic.extract_cache
+        if ex is not None:
+            ex.key_caches.setdefault(0, {})[layer_idx - 1] = L.k_res
+            ex.value_caches.setdefault(0, {})[layer_idx - 1] = L.v_res
+        return L.k_res, L.v_res
 
-        block, recent = cfg.block_size, cfg.buffer_size
-        total = L.n_res + T
-        n_c = compress_block_count(total, block, recent) * block
-        res_cap = recent + block
-        if L.k_res is None:
-            L.k_res = torch.empty(B, H, res_cap, D, dtype=k_new.dtype, device=k_new.device)
-            L.v_res = torch.empty(B, H, res_cap, D, dtype=k_new.dtype, device=k_new.device)
-        if n_c == 0:
-            L.k_res[:, :, L.n_res: total] = k_new
-            L.v_res[:, :, L.n_res: total] = v_new
-            L.n_res = total
+    @staticmethod
+    def _append(k_rows: torch.Tensor, v_rows: torch.Tensor, position: int, k: torch.Tensor, v: torch.Tensor, cos, sin) -> None:
+        """Tokens (B, H, T, D) into rows [position, position + T) of 128 channels: K rotated when cos is given; rows of
+        64 <= D < 128 are widened, the tail repeating the first 128 - D channels.  The streams are built from 128-channel
+        blocks; with copies in the tail the per-channel K parameters of the real channels and the per-token minima / maxima
+        of V (and token-mode K) are unchanged, so codes and parameters of the real channels are exactly the reference's for
+        head_dim D.  attend() pads q with zeros, so the copies add nothing to the scores, and drops the output's tail."""
+        if not k.is_cuda or k.dtype not in (torch.float16, torch.bfloat16):
+            # kept uncompressed as it is (packing and attention refuse it)
+            if cos is not None:
+                k = ops.rope(k, cos, sin)
+            tail = k_rows.shape[3] - k.shape[3]
+            k, v = (torch.cat([t, t[..., :tail]], dim=-1) if tail else t for t in (k, v))
+            k_rows[:, :, position: position + k.shape[2]], v_rows[:, :, position: position + k.shape[2]] = k, v
+        elif k.shape[3] == 128:
+            ops.append_residual(k, v, k_rows, v_rows, position, cos, sin)
         else:
-            if L.n_res:
-                k_all = torch.cat([L.k_res[:, :, : L.n_res], k_new], dim=2)
-                v_all = torch.cat([L.v_res[:, :, : L.n_res], v_new], dim=2)
-            else:
-                k_all, v_all = k_new, v_new
-            self._compress(L, k_all[:, :, :n_c], v_all[:, :, :n_c], cfg)
-            L.n_res = total - n_c
-            L.k_res[:, :, : L.n_res] = k_all[:, :, n_c:]
-            L.v_res[:, :, : L.n_res] = v_all[:, :, n_c:]
-        return self._step_result(layer_idx, T)
+            ops.widen_rows(k, v, k_rows, v_rows, position, cos, sin)
 
     def _flush(self, L: "_Layer") -> None:
         """Writes a decode step's token that no attend() has consumed into the residual (one launch)."""
@@ -269,15 +308,6 @@ class PackKVCache(_HFCache):
         """Makes the residual buffers of every layer complete (call before reading them from outside)."""
         for L in self._layers:
             self._flush(L)
-
-    @staticmethod
-    def _widen(x: torch.Tensor) -> torch.Tensor:
-        """(B, H, T, D) with 64 <= D < 128 -> (B, H, T, 128): the tail repeats the first 128 - D channels.  The
-        streams are built from 128-channel blocks; with copies in the tail the per-channel K parameters of the real
-        channels and the per-token minima / maxima of V (and token-mode K) are unchanged, so codes and parameters
-        of the real channels are exactly the reference's for head_dim D.  attend() pads q with zeros, so the copies
-        add nothing to the scores, and drops the tail of the output."""
-        return torch.cat([x, x[..., : 128 - x.shape[-1]]], dim=-1)
 
     def _step_result(self, layer_idx: int, T: int):
         if T > 1 or self.materialize:
@@ -305,12 +335,13 @@ class PackKVCache(_HFCache):
             raise ValueError("attend handles one query token per sequence; use dense() for prefill")
         if self.flags is None:
             self.flags = ops.new_flags(query_states.device)
-        q = query_states.reshape(B, Hq, D)
         if D != 128:
             if scaling is None:
                 scaling = D ** -0.5
-            q = torch.nn.functional.pad(q, (0, 128 - D))       # zeros: the copied channels of K add nothing
-        q = q.contiguous()
+            q = query_states.new_empty(B, Hq, 128)             # zeros behind it: the copied channels of K add nothing
+            ops.widen_rows(query_states if query_states.stride(3) == 1 else query_states.contiguous(), None, q.view(B, Hq, 1, 128), None, zero_tail=True)
+        else:
+            q = query_states.reshape(B, Hq, D).contiguous()
         kv_heads = L.comp.kv_heads if L.comp is not None else L.k_res.shape[1]
         pending, L.pending = L.pending, None
         if self._scratch is None and B * kv_heads <= 64:

@@ -714,7 +714,7 @@ __global__ void __launch_bounds__(kAW * 32, PASS == 1 ? PKV_ATTN_CTAS_SCORES : P
     // A fragments come straight from the uncompressed rows: lane (g, c) reads channels
     // 32m + 8c .. +7 (m = 0..3) of tokens g and g+8 and pairs them in the order of pair_shuffle.
     // The decode step's new token: the warp that owns the residual tile of row n_res - 1 rotates K (the
-    // arithmetic of rope_kernel: both products rounded to the element type, then their sum) and copies V into
+    // arithmetic of rows_kernel: both products rounded to the element type, then their sum) and copies V into
     // that row first; its own loads of the tile below then see the row (plain loads and cp.async, no read-only path).
     if (P.ap.new_k != nullptr && my_rt > 0) {
         const int tn = a.n_res - 1, tile_n = tn >> 4;

@@ -111,9 +111,21 @@ int32_t pkv_append_residual(const void* k, int64_t k_stride_b, int64_t k_stride_
                             int64_t cs_stride_b, void* k_res, void* v_res, int64_t res_stride_b, int64_t res_stride_h,
                             int32_t res_capacity, int32_t position, int32_t batch, int32_t heads, int32_t tokens,
                             int32_t is_bf16, void* cuda_stream) {
-    AppendArgs r{k, k_stride_b, k_stride_h, k_stride_s, v, v_stride_b, v_stride_h, v_stride_s, cos, sin, cs_stride_b,
-                 k_res, v_res, res_stride_b, res_stride_h, res_capacity, position, batch, heads, tokens, is_bf16};
-    return launch_append(r, static_cast<cudaStream_t>(cuda_stream));
+    if (!v || !v_res) return (int64_t)batch * tokens == 0 ? kOk : kBadArgument;
+    const RowsArgs r{k, k_stride_b, k_stride_h, k_stride_s, v, v_stride_b, v_stride_h, v_stride_s, cos, sin, cs_stride_b,
+                     k_res, v_res, res_stride_b, res_stride_h, 128, res_capacity, position, batch, heads, tokens, 128, 128, 0, is_bf16};
+    return launch_rows(r, static_cast<cudaStream_t>(cuda_stream));
+}
+
+int32_t pkv_widen_rows(const void* k, int64_t k_stride_b, int64_t k_stride_h, int64_t k_stride_s, const void* v,
+                       int64_t v_stride_b, int64_t v_stride_h, int64_t v_stride_s, const void* cos, const void* sin,
+                       int64_t cs_stride_b, void* k_out, void* v_out, int64_t o_stride_b, int64_t o_stride_h,
+                       int32_t capacity, int32_t position, int32_t batch, int32_t heads, int32_t tokens, int32_t dim,
+                       int32_t zero_tail, int32_t is_bf16, void* cuda_stream) {
+    if (dim < 64) return kUnsupported;
+    const RowsArgs r{k, k_stride_b, k_stride_h, k_stride_s, v, v_stride_b, v_stride_h, v_stride_s, cos, sin, cs_stride_b,
+                     k_out, v_out, o_stride_b, o_stride_h, 128, capacity, position, batch, heads, tokens, dim, 128, zero_tail, is_bf16};
+    return launch_rows(r, static_cast<cudaStream_t>(cuda_stream));
 }
 
 int32_t pkv_greedy_order(const uint8_t* k_codes, const uint8_t* v_codes, int64_t codes_seq_stride, uint8_t* order,
@@ -132,9 +144,10 @@ int32_t pkv_rope(const void* x, int64_t x_stride_b, int64_t x_stride_h, int64_t 
                  const void* sin, int64_t cs_stride_b, void* out, int64_t o_stride_b, int64_t o_stride_h,
                  int64_t o_stride_s, int32_t batch, int32_t heads, int32_t tokens, int32_t dim, int32_t is_bf16,
                  void* cuda_stream) {
-    RopeArgs r{x, x_stride_b, x_stride_h, x_stride_s, cos, sin, cs_stride_b, out, o_stride_b, o_stride_h, o_stride_s,
-               batch, heads, tokens, dim, is_bf16};
-    return launch_rope(r, static_cast<cudaStream_t>(cuda_stream));
+    if (!cos || !sin) return (int64_t)batch * tokens == 0 ? kOk : kBadArgument;
+    const RowsArgs r{x, x_stride_b, x_stride_h, x_stride_s, nullptr, 0, 0, 0, cos, sin, cs_stride_b,
+                     out, nullptr, o_stride_b, o_stride_h, o_stride_s, tokens, 0, batch, heads, tokens, dim, dim, 0, is_bf16};
+    return launch_rows(r, static_cast<cudaStream_t>(cuda_stream));
 }
 
 int32_t pkv_dequantize(const uint8_t* codes, int64_t codes_seq_stride, const void* scale, const void* zero,

@@ -39,6 +39,7 @@ struct Library {
     decltype(&pkv_value_median_order) value_order;
     decltype(&pkv_append_residual) append;
     decltype(&pkv_rope) rope;
+    decltype(&pkv_widen_rows) widen;
 } lib{};
 
 // thrown once a Python exception is set
@@ -392,6 +393,28 @@ PyObject* append_residual(PyObject* const* p) {
     Py_RETURN_NONE;
 }
 
+// k (B, H, T, 64 <= D <= 128), v or None, k_out, v_out or None (B, H, capacity, 128), position, cos, sin, zero_tail
+PyObject* widen_rows(PyObject* const* p) {
+    const at::Tensor &k = cuda(p[0], "k"), &ko = cuda(p[2], "k_out");
+    const at::Tensor *v = maybe_cuda(p[1], "v"), *vo = maybe_cuda(p[3], "v_out"), *cos = maybe_cuda(p[5], "cos"), *sin = maybe_cuda(p[6], "sin");
+    check(k.dim() == 4 && k.size(3) >= 64 && k.size(3) <= 128 && k.size(3) % 8 == 0 && k.stride(3) == 1 && half_type(k),
+          "k must be (B, H, T, 64..128) fp16/bf16 with contiguous channels");
+    check((v == nullptr) == (vo == nullptr) && (cos == nullptr) == (sin == nullptr), "v with v_out and cos with sin");
+    check(!v || (v->sizes() == k.sizes() && v->stride(3) == 1 && v->scalar_type() == k.scalar_type()), "v must have k's shape and type and contiguous channels");
+    check(ko.dim() == 4 && ko.size(0) == k.size(0) && ko.size(1) == k.size(1) && ko.size(3) == 128 && ko.stride(3) == 1 && ko.stride(2) == 128 &&
+              ko.scalar_type() == k.scalar_type() && (!vo || (vo->sizes() == ko.sizes() && vo->strides() == ko.strides() && vo->scalar_type() == k.scalar_type())),
+          "k_out and v_out must be (B, H, capacity, 128) with contiguous rows and equal strides");
+    const int64_t T = k.size(2), D = k.size(3);
+    std::unique_ptr<Tables> cs;
+    if (cos) cs = std::make_unique<Tables>(*cos, *sin, k.scalar_type(), T, D, "cos/sin must be (B or 1, T, D)");
+    check_status(lib.widen(k.data_ptr(), k.stride(0), k.stride(1), k.stride(2), v ? v->data_ptr() : nullptr, v ? v->stride(0) : 0, v ? v->stride(1) : 0,
+                           v ? v->stride(2) : 0, cs ? cs->cos.data_ptr() : nullptr, cs ? cs->sin.data_ptr() : nullptr, cs ? cs->stride_b : 0,
+                           ko.data_ptr(), vo ? vo->data_ptr() : nullptr, ko.stride(0), ko.stride(1), extent(ko.size(2)), extent(integer(p[4])),
+                           extent(k.size(0)), extent(k.size(1)), extent(T), extent(D), truth(p[7]), is_bf16(k), stream()),
+                 "widen_rows");
+    Py_RETURN_NONE;
+}
+
 // x, cos, sin, out -> out
 PyObject* rope(PyObject* const* p) {
     const at::Tensor &x = cuda(p[0], "x"), &cos = cuda(p[1], "cos"), &sin = cuda(p[2], "sin");
@@ -453,6 +476,7 @@ PyMethodDef methods[] = {
     FAST(value_median_order, 4, "ops.value_median_order"),
     FAST(append_residual, 7, "ops.append_residual"),
     FAST(rope, 4, "ops.rope"),
+    FAST(widen_rows, 8, "ops.widen_rows"),
     {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "_host", "native host path of packkv_b200.ops", -1, methods};
 

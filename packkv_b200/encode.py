@@ -23,6 +23,18 @@ def stream_capacity(which: str, n_tokens: int, kv_heads: int, cb: int, bits: int
     return _pad16((n_tokens // cb) * nhid * ops.block_bound(which, cb, bits)) + 16
 
 
+def _median_in_one_pass(k: torch.Tensor, v: torch.Tensor, block: int, cbk: int, cbv: int, k_mode: int, high_precision_zero: bool) -> bool:
+    """Whether value_median_order and the ordered single-pass encoder take these tensors."""
+    return (not high_precision_zero and block == 64 and k.shape[1] <= 8 and cbv % 64 == 0 and (cbk == block if k_mode == ops.K_CHANNEL else cbk % 64 == 0)
+            and k.stride(3) == 1 and v.stride(3) == 1 and all(t.stride(i) % 8 == 0 for t in (k, v) for i in range(3)))
+
+
+def median_in_one_pass(k: torch.Tensor, v: torch.Tensor, block: int, layer: ops.CompressedLayer) -> bool:
+    """The same for tokens that are packed behind those of a layer (rows on 16-byte boundaries)."""
+    return (_median_in_one_pass(k, v, block, layer.cbk, layer.cbv, layer.k_mode, layer.high_precision_zero)
+            and k.data_ptr() % 16 == 0 and v.data_ptr() % 16 == 0)
+
+
 def compress_kv(k: torch.Tensor, v: torch.Tensor, *, block: int, bits_k: int, bits_v: int,
                 k_rel: float, v_rel: float, k_mode: QuantMode = QuantMode.ChannelQuant,
                 cbk: Optional[int] = None, cbv: Optional[int] = None, high_precision_zero: bool = False,
@@ -60,10 +72,7 @@ def compress_kv(k: torch.Tensor, v: torch.Tensor, *, block: int, bits_k: int, bi
     k_info = torch.empty(B, (cap_tok // cbk) * H, 2, dtype=torch.int32, device=dev)
     v_info = torch.empty(B, (cap_tok // cbv) * 2 * H, 2, dtype=torch.int32, device=dev)
     k_bytes, v_bytes = zeros[:B], zeros[B:2 * B]
-    fused_median = (repack_method == RepackMethod.MEDIAN and not high_precision_zero and block == 64 and H <= 8 and cbv % 64 == 0
-                    and (cbk == block if km == ops.K_CHANNEL else cbk % 64 == 0)
-                    and k.stride(3) == 1 and v.stride(3) == 1 and all(t.stride(i) % 8 == 0 for t in (k, v) for i in range(3)))
-    if fused_median:
+    if repack_method == RepackMethod.MEDIAN and _median_in_one_pass(k, v, block, cbk, cbv, km, high_precision_zero):
         # the order straight from V, then the single-pass encoder reads K and V rows through it: no code matrix in HBM
         order = ops.value_median_order(v, block, v_rel, flags=flags)
         scratch = torch.empty(max(16, B * S * H * D), dtype=torch.uint8, device=dev)

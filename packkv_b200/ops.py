@@ -292,6 +292,13 @@ def append_residual(k_new: torch.Tensor, v_new: torch.Tensor, k_res: torch.Tenso
     _lib.host().append_residual(k_new, v_new, k_res, v_res, position, cos, sin)
 
 
+def widen_rows(k: torch.Tensor, v: Optional[torch.Tensor], k_out: torch.Tensor, v_out: Optional[torch.Tensor], position: int = 0,
+               cos: Optional[torch.Tensor] = None, sin: Optional[torch.Tensor] = None, zero_tail: bool = False) -> None:
+    """append_residual for heads of 64 <= D < 128 channels (B, H, T, D): the rows of k_out / v_out (B, H, capacity, 128) are
+    widened, channels D.. repeating the row's first 128 - D (zeros with zero_tail).  v and v_out may be None.  One launch."""
+    _lib.host().widen_rows(k, v, k_out, v_out, position, cos, sin, zero_tail)
+
+
 def dequantize(codes: torch.Tensor, scale: torch.Tensor, zero: torch.Tensor, heads: int, block: int, mode: int, *,
                first_token: int = 0, high_precision_zero: bool = False, out: Optional[torch.Tensor] = None) -> torch.Tensor:
     """codes (B, T, heads*128) uint8 + scale/zero -> dense (B, heads, T, 128) in scale's dtype."""

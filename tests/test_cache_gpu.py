@@ -225,3 +225,31 @@ def test_config_contract_and_disabled_quant(cuda_device):
     cfg = _cfg(QuantMethod.KIVI, k_rel=0.1, v_rel=0.2)
     assert PackKVCacheConfig.from_str(str(cfg)) == cfg and hash(PackKVCacheConfig.from_str(str(cfg))) == hash(cfg)
     assert C.bits_for_rel(0.1) == 4 and C.bits_for_rel(0.2) == 3 and C.bits_for_rel(1 / 14) == 4 and C.bits_for_rel(0.5) == 2
+
+
+@pytest.mark.parametrize("D", [128, 96])
+@pytest.mark.parametrize("repack", [RepackMethod.NONE, RepackMethod.MEDIAN])
+def test_prompts_in_pieces_match_reference_cache(cuda_device, D, repack):
+    """Pieces that leave the residual short of a block, fill it past its capacity (300 tokens behind 130 of 256 rows), cross
+    a block boundary one token at a time, and end on it, from strided projections: dense rows bit-identical."""
+    dev, dtype, B, H = cuda_device, torch.bfloat16, 2, 2
+    cfg = _cfg(QuantMethod.KIVI, repack=repack)
+    C.PackKVCacheConfigStatic.config = cfg
+    try:
+        cache = C.PackKVCache(B, H, D, 1, materialize=True)
+        oracle = Q.CacheLayerOracle(64, 192, cfg.k_quant_scale_rel, cfg.v_quant_scale_rel, "channel", "token")
+        pieces = [30, 100, 300, 1, 40, 1, 64]
+        k, v = synth.synth_kv(B, H, sum(pieces), D, seed=12, dtype=dtype)
+        cos, sin = synth.rope_tables(sum(pieces), D, dtype=dtype)
+        t = 0
+        for n in pieces:
+            def part(x):
+                return x[:, :, t:t + n]
+            Ko, Vo = oracle.update(part(k), part(v), cos[:, t:t + n], sin[:, t:t + n])
+            Kg, Vg = cache.update(*(part(x).to(dev).transpose(1, 2).contiguous().transpose(1, 2) for x in (k, v)), 0,
+                                  {"cos": cos[:, t:t + n].to(dev), "sin": sin[:, t:t + n].to(dev)})
+            assert torch.equal(Kg.cpu(), Ko) and torch.equal(Vg.cpu(), Vo), t
+            t += n
+        cache.check_flags()
+    finally:
+        C.PackKVCacheConfigStatic.config = None
