@@ -1312,10 +1312,18 @@ static int launch_one(const AttnDev& P, dim3 grid, int smem, cudaStream_t st) {
         cfg.numAttrs = 2;
     }
     if (P.cluster > 8) {
-        // a non-portable cluster size with this much shared memory may not be schedulable at all: say so
-        int clusters = 0;
-        if (cudaOccupancyMaxActiveClusters(&clusters, kern, &cfg) != cudaSuccess) { cudaGetLastError(); return kCudaError; }
-        if (clusters < 1) return kUnsupported;
+        // a non-portable cluster size with this much shared memory may not be schedulable at all: say so.  The answer
+        // depends on the kernel, the device and these two sizes; each thread remembers the last one (the steps of a decode
+        // loop ask the same thing again)
+        thread_local int seen_device = -1, seen_cluster = 0, seen_smem = 0;
+        int device = 0;
+        if (cudaGetDevice(&device) != cudaSuccess) { cudaGetLastError(); return kCudaError; }
+        if (device != seen_device || P.cluster != seen_cluster || smem != seen_smem) {
+            int clusters = 0;
+            if (cudaOccupancyMaxActiveClusters(&clusters, kern, &cfg) != cudaSuccess) { cudaGetLastError(); return kCudaError; }
+            if (clusters < 1) return kUnsupported;
+            seen_device = device; seen_cluster = P.cluster; seen_smem = smem;
+        }
     }
     return cudaLaunchKernelEx(&cfg, kern, P) == cudaSuccess ? kOk : kCudaError;
 }
@@ -1341,39 +1349,51 @@ static int launch_typed(const AttnDev& P, dim3 grid, int smem, cudaStream_t st) 
 }
 
 
-// shared memory of one CTA for a cluster of `cl` CTAs with `nslots` staging slots per warp; fills the layout fields
-static int plan_smem(AttnDev& P, int cl, int nsplit, int nslots, int slot) {
+// Shared memory of one CTA for a cluster of `cl` CTAs with `nslots` staging slots per warp.  A value of its own, not
+// written into AttnDev: the planner lays out a hundred candidates per call, and copying the launch arguments for each
+// was most of its 15 us (3 to 8 us now, 4 on a short context).
+struct CtaLayout {
+    int tpw, rtw, out_off, off_xch, off_raw, off_perm, off_desc, off_stile, off_rst, warp_smem, dump_bytes, cta_off, total;
+};
+static CtaLayout lay_out(const AttnDev& P, bool team, int cl, int nsplit, int nslots, int slot) {
     const AttnArgs& a = P.a;
+    CtaLayout L;
     const int n_warps = kAW * cl * nsplit;
-    P.cluster = cl;
-    P.nsplit = nsplit;
-    P.nslots = nslots;
-    P.slot = slot;
-    const int owners = P.team ? cl : n_warps;                 // a team's tiles lie in the first warp's region; the others' stay empty
-    P.tpw = (P.tiles_total + owners - 1) / owners;
-    P.rtw = ((a.n_res + 15) / 16 + n_warps - 1) / n_warps;
+    const int owners = team ? cl : n_warps;                   // a team's tiles lie in the first warp's region; the others' stay empty
+    L.tpw = (P.tiles_total + owners - 1) / owners;
+    L.rtw = ((a.n_res + 15) / 16 + n_warps - 1) / n_warps;
     int off = nslots * slot;
     if (off < 16 * 272) off = 16 * 272;                       // the residual V tile borrows the staging slots
     if (off < 8 * kD * 4) off = 8 * kD * 4;                   // and so do the parked accumulators
-    P.out_off = off;                                          // the CTA's reduced rows sit behind them
-    P.off_xch = off; off += 2048;                             // (>= 2 * kD * 4 bytes: two heads' rows per warp)
+    L.out_off = off;                                          // the CTA's reduced rows sit behind them
+    L.off_xch = off; off += 2048;                             // (>= 2 * kD * 4 bytes: two heads' rows per warp)
     // The parameter staging, the pair-order parameters and the V descriptors are idle while the K exchange tile
     // is in use when K has per-channel parameters and the next item is only copied after the current one is
     // done (one slot): the parameters of a block are in registers before its first round.  They share the tile then.
     const int raw_bytes = 4 * P.tile > 4 * kD ? 4 * P.tile : 4 * kD;
     if (a.k_mode == kKChannel && nslots == 1 && raw_bytes + 4 * P.tile + 384 <= 2048) {
-        P.off_raw = P.off_xch; P.off_perm = P.off_raw + raw_bytes; P.off_desc = P.off_perm + 4 * P.tile;
+        L.off_raw = L.off_xch; L.off_perm = L.off_raw + raw_bytes; L.off_desc = L.off_perm + 4 * P.tile;
     } else {
-        P.off_raw = off; off += raw_bytes;
-        P.off_perm = off; off += 4 * P.tile;
-        P.off_desc = off; off += 384;
+        L.off_raw = off; off += raw_bytes;
+        L.off_perm = off; off += 4 * P.tile;
+        L.off_desc = off; off += 384;
     }
-    P.off_stile = off; off += P.tpw * P.rows * P.prow;
-    P.off_rst = off; off += P.rtw * P.rows * 32;
-    P.warp_smem = (off + 15) & ~15;
-    P.dump_bytes = P.warp_smem - P.off_stile;
-    P.cta_off = kAW * P.warp_smem;
-    return P.cta_off + (int)sizeof(CtaShared);
+    L.off_stile = off; off += L.tpw * P.rows * P.prow;
+    L.off_rst = off; off += L.rtw * P.rows * 32;
+    L.warp_smem = (off + 15) & ~15;
+    L.dump_bytes = L.warp_smem - L.off_stile;
+    L.cta_off = kAW * L.warp_smem;
+    L.total = L.cta_off + (int)sizeof(CtaShared);
+    return L;
+}
+// the chosen plan's layout into the launch arguments
+static int plan_smem(AttnDev& P, int cl, int nsplit, int nslots, int slot) {
+    const CtaLayout L = lay_out(P, P.team, cl, nsplit, nslots, slot);
+    P.cluster = cl; P.nsplit = nsplit; P.nslots = nslots; P.slot = slot;
+    P.tpw = L.tpw; P.rtw = L.rtw; P.out_off = L.out_off;
+    P.off_xch = L.off_xch; P.off_raw = L.off_raw; P.off_perm = L.off_perm; P.off_desc = L.off_desc; P.off_stile = L.off_stile; P.off_rst = L.off_rst;
+    P.warp_smem = L.warp_smem; P.dump_bytes = L.dump_bytes; P.cta_off = L.cta_off;
+    return L.total;
 }
 
 // partition of the caller's scratch for the two-launch form
@@ -1578,21 +1598,24 @@ int launch_attention(const AttnArgs& a, const AttnExchange* xch, const AttnAppen
                 if (want_launches && launches != want_launches) continue;
                 if (launches == 1 && split > 1) continue;
                 if (launches == 2 && split == 1 && want_launches != 2) continue;   // one cluster in two launches: only on request
+                if (launches == 2 && !scratch) continue;
+                // more clusters than give every tile a warp of its own only add to the hand-over
+                if (launches == 2 && !want_split && !want_launches && !want_cl && split > 1 && kAW * cl * split >= 2 * (P.tiles_total + n_rt)) continue;
+                const bool team = launches == 1 && team_wins(cl);
                 for (int ns = 2; ns >= 1; ns--) {
                     if (env_slots && ns != env_slots) continue;
-                    AttnDev Q = P;
-                    Q.team = launches == 1 && team_wins(cl);
-                    const int smem = plan_smem(Q, cl, split, ns, slot);
+                    const CtaLayout Q = lay_out(P, team, cl, split, ns, slot);
+                    const int smem = Q.total;
                     if (smem > 227 * 1024) continue;
-                    if (launches == 2 && (!scratch || scratch_layout(pairs, cl, split, Q.dump_bytes).total > scratch_bytes)) continue;
+                    if (launches == 2 && scratch_layout(pairs, cl, split, Q.dump_bytes).total > scratch_bytes) continue;
                     int per_sm = (228 * 1024) / (smem + 1024);
                     if (per_sm > kMaxCtasPerSm) per_sm = kMaxCtasPerSm;
                     if (per_sm < 1) continue;
                     const int n_warps = kAW * cl * split;
-                    const double placed = Q.team ? longest(cl, 1.15 / kAW * unit_tile, kAW) : longest(n_warps, unit_tile, 1);
+                    const double placed = team ? longest(cl, 1.15 / kAW * unit_tile, kAW) : longest(n_warps, unit_tile, 1);
                     const double dealt = (double)((P.tiles_total + n_warps - 1) / n_warps) * unit_tile + (n_rt + n_warps - 1) / n_warps;
                     const double fixed = launches == 2 ? 4.0 + 0.05 * split : 3.0;
-                    const double cost = plan_cost(pairs * cl * split, cl, per_sm, (Q.team ? 1.15 : 1.0) * pair_units / n_warps, dealt, placed, fixed, ns, launches, Q.team);
+                    const double cost = plan_cost(pairs * cl * split, cl, per_sm, (team ? 1.15 : 1.0) * pair_units / n_warps, dealt, placed, fixed, ns, launches, team);
                     if (cost < best_cost - 1e-9) { best_cost = cost; best_cl = cl; best_ns = ns; best_split = split; best_launches = launches; best_extra = -1; }
                 }
             }
@@ -1612,8 +1635,8 @@ int launch_attention(const AttnArgs& a, const AttnExchange* xch, const AttnAppen
             bool found = false;
             for (int ns = 2; ns >= 1; ns--) {
                 if (env_slots && ns != env_slots) continue;
-                AttnDev Q = P;
-                const int smem = plan_smem(Q, 1, base, ns, slot);
+                const CtaLayout Q = lay_out(P, false, 1, base, ns, slot);
+                const int smem = Q.total;
                 if (smem > 227 * 1024) continue;
                 if (scratch_layout(pairs, 1, base + 1, Q.dump_bytes).total > scratch_bytes) continue;
                 int fit = (228 * 1024) / (smem + 1024);
