@@ -256,6 +256,7 @@ struct AttnDev {
     int slot;            // bytes of one staging slot
     int nslots;          // staging slots per warp: 2 = the next block is copied while this one is unpacked
     int team;            // single launch: the warps of a CTA share its tiles (see TEAM)
+    int early;           // single launch that may start while the one before drains (launch_attention)
     int vpair;           // 64-token V blocks: an item is the pair of blocks of one token block (both channel halves)
     int kbound, vbound;  // largest legal block size in bytes
     int prow;            // bytes of one row of the score / probability tile
@@ -374,6 +375,13 @@ __global__ void __launch_bounds__(kAW * 32, PASS == 1 ? PKV_ATTN_CTAS_SCORES : P
     }
     __syncthreads();
     asm volatile("" : "+r"(lutm_a) :: "memory");        // reads of the table stay behind the barrier
+    if (PASS != kValues) {
+        // Small single launches are started under programmatic stream serialisation (P.early): the lines above overlap the
+        // end of the launch before; nothing it may have written (q, tables, residual) is touched before it is complete, and
+        // the launch after this one may be set up from here on.
+        asm volatile("griddepcontrol.wait;" ::: "memory");
+        if (PASS == kFused && P.early) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    }
 
     const int my_tiles = tw < P.tiles_total ? (P.tiles_total - tw + tstep - 1) / tstep : 0;
     // residual tiles are dealt from the last warp backwards (the compressed tiles are dealt from
@@ -1304,9 +1312,10 @@ static int launch_one(const AttnDev& P, dim3 grid, int smem, cudaStream_t st) {
     attr[0].val.clusterDim.y = 1;
     attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
+    // a launch may start while the one before it drains; it waits for it on the device (griddepcontrol.wait): the second of
+    // two launches with its first copies under way, a small single launch with its shared memory set up
     cfg.numAttrs = 1;
-    if (PASS == kValues) {
-        // the second launch may start while the first one drains; it waits for it on the device (griddepcontrol.wait)
+    if (PASS == kValues || P.early) {
         attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
         attr[1].val.programmaticStreamSerializationAllowed = 1;
         cfg.numAttrs = 2;
@@ -1659,6 +1668,10 @@ int launch_attention(const AttnArgs& a, const AttnExchange* xch, const AttnAppen
     P.team = best_launches == 1 && team_wins(best_cl);
     const int smem = plan_smem(P, best_cl, best_split, best_ns, slot);
     P.extra = best_extra;
+    // At most one CTA per SM: 8 KV heads x 700 tokens 14.3 -> 13.0 us a launch.  Fuller launches stay ordered: their CTAs would
+    // be placed around those still running, unevenly (11 x 2154: 30 -> 34 us; two launches 0 to 5 % slower).  So do launches
+    // with an exchange: the launch before may be its wait, which does not wait for the launch before itself.
+    P.early = best_launches == 1 && !xch && pairs * best_cl <= kSmCount;
     if (best_launches == 2) {
         const ScratchLayout L = scratch_layout(pairs, best_cl, best_extra >= 0 ? best_split + 1 : best_split, P.dump_bytes);
         if (!scratch || L.total > scratch_bytes) return kBadArgument;

@@ -451,3 +451,34 @@ def test_team_form_matches_reference(cuda_device, dtype, cl, n_comp, n_res, bloc
         err = _run_case(cuda_device, dtype, 2, 2, G, n_comp, n_res, block=block, cbk=cbk, cbv=cbv, bits_k=bits, bits_v=bits, k_mode=k_mode,
                         seed=60 + cl + G, hp=hp, plan=(cl, 1, 1), repeats=2)
         assert err <= TOL, (G, err)
+
+
+@pytest.mark.parametrize("n_comp,plan", [(256, None), (2048, None), (2048, (2, 3, 2))])
+def test_back_to_back_steps_equal_synchronised_steps(cuda_device, n_comp, plan):
+    """A launch may start while the one before it drains: 40 steps, each appending a row that the next ones attend to and
+    writing its output where the next step's query comes from, give the same bits as with a synchronisation after each."""
+    dev, dtype = cuda_device, torch.bfloat16
+    B, H, G, n0, steps = 2, 2, 4, 129, 40
+    k, v = synth.synth_kv(B, H, n_comp, 128, seed=8, dtype=dtype, apply_rope=True)
+    layer, _, _ = layer_from_oracle(k, v, block=64, bits_k=4, bits_v=4, k_mode="channel", cbk=64, cbv=64, rel_k=synth.rel_for_bits(4),
+                                    rel_v=synth.rel_for_bits(4), device=dev)
+    g = torch.Generator().manual_seed(3)
+    res = [torch.randn(B, H, 192, 128, generator=g).to(dtype).to(dev) for _ in range(2)]
+    new = [torch.randn(steps, B, H, 1, 128, generator=g).to(dtype).to(dev) for _ in range(2)]
+    got = []
+    for wait in (True, False):
+        k_res, v_res = (t.clone() for t in res)
+        x = torch.randn(B, H * G, 128, generator=torch.Generator().manual_seed(4)).to(dtype).to(dev)
+        y, flags, scratch = torch.empty_like(x), ops.new_flags(dev), ops.new_attention_scratch(dev)
+        torch.cuda.synchronize()
+        for n in range(steps):
+            ops.decode_attention(x, layer, k_res, v_res, n0 + n + 1, out=y, flags=flags, append=(new[0][n], new[1][n], None, None), scratch=scratch, plan=plan,
+                                 scaling=1.0)
+            x, y = y, x
+            if wait:
+                torch.cuda.synchronize()
+        torch.cuda.synchronize()
+        assert int(flags.item()) == 0
+        got.append((x, y, k_res, v_res))
+    for a, b in zip(*got):
+        assert torch.equal(a.view(torch.int16), b.view(torch.int16))
