@@ -323,6 +323,8 @@ class PackKVCache(_HFCache):
         D = self.head_dim if self.head_dim < 128 else 128
         if L.n_comp == 0:
             return L.k_res[:, :, : L.n_res, :D].clone(), L.v_res[:, :, : L.n_res, :D].clone()
+        if self.flags is None:            # a restored cache that has neither packed a block nor attended yet
+            self.flags = ops.new_flags(L.comp.k_stream.device)
         block = self._config().block_size
         return (ops.dense("k", L.comp, L.k_res, L.n_res, D, block, self.flags), ops.dense("v", L.comp, L.v_res, L.n_res, D, block, self.flags))
 

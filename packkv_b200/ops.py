@@ -315,7 +315,7 @@ def dequantize(codes: torch.Tensor, scale: torch.Tensor, zero: torch.Tensor, hea
 
 
 def dense(which: str, layer: CompressedLayer, res: Optional[torch.Tensor], n_res: int, dim: int, block: int,
-          flags: torch.Tensor) -> torch.Tensor:
+          flags: Optional[torch.Tensor] = None) -> torch.Tensor:
     """Rows of K or V of a layer as the reference's cache returns them, (B, H, n_comp + n_res, dim): the packed tokens
     dequantised (in source order when the layer is reordered) and the first n_res rows of the residual behind them.
     `block` is the quantisation block; dim < 128 keeps the first channels of every head.  One launch."""
@@ -324,6 +324,8 @@ def dense(which: str, layer: CompressedLayer, res: Optional[torch.Tensor], n_res
     B, H, n, cb = stream.shape[0], layer.kv_heads, layer.n_comp, layer.cbk if which == "k" else layer.cbv
     mode = layer.k_mode if which == "k" else K_TOKEN
     _require_cuda(stream, info, scale, zero, res, layer.order, flags)
+    if flags is None:
+        flags = new_flags(stream.device)
     pb, pt = _param_extents(scale, mode)
     if n % block or n % cb or info.dim() != 3 or info.shape[1] < (n // cb) * H * (1 if which == "k" else 2) or not info.is_contiguous() \
             or stream.dim() != 2 or stream.stride(1) != 1 or (pb < n // block if mode == K_CHANNEL else pt < n) \

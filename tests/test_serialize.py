@@ -99,3 +99,30 @@ def test_restored_layer_and_cache_decode_identically(cuda_device):
         cache.check_flags(); twin.check_flags()
     finally:
         PackKVCacheConfigStatic.config = None
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("repack", ["NONE", "MEDIAN"])
+@pytest.mark.parametrize("materialize", [False, True])
+def test_restored_cache_returns_the_dense_view(cuda_device, repack, materialize):
+    """The first call on a restored cache is dense(), or an update() that returns dense rows: nothing has packed a block or
+    attended yet."""
+    from packkv_b200 import synth
+    from packkv_b200.cache import PackKVCache, PackKVCacheConfigStatic
+    from packkv_b200.config import PackKVCacheConfig, QuantMethod, RepackMethod
+    dev, dtype, B, H, S = cuda_device, torch.bfloat16, 2, 2, 400
+    PackKVCacheConfigStatic.config = PackKVCacheConfig("synthetic", QuantMethod.KIVI, RepackMethod[repack], False, 64, 192, 16, 1 / 14, 1 / 14)
+    try:
+        k, v = synth.synth_kv(B, H, S + 3, 128, seed=32, dtype=dtype, device=dev)
+        cache = PackKVCache(B, H, 128, 1, materialize=materialize)
+        cache.update(k[:, :, :S], v[:, :, :S], 0)
+        twin = serialize.loads_cache(serialize.dumps_cache(cache), dev, materialize=materialize)
+        if not materialize:
+            for a, b in zip(cache.dense(0), twin.dense(0)):
+                assert torch.equal(a, b)
+        for lo, hi in ((S, S + 1), (S + 1, S + 3)):          # one token, and several that do not fill a block
+            for a, b in zip(*(c.update(k[:, :, lo:hi], v[:, :, lo:hi], 0) for c in (cache, twin))):
+                assert (a is None and b is None) or torch.equal(a, b)
+        twin.check_flags()
+    finally:
+        PackKVCacheConfigStatic.config = None
