@@ -288,7 +288,8 @@ int32_t pkv_dequantize(const uint8_t* codes, int64_t codes_seq_stride, const voi
  * out (batch, heads, n_comp + n_res, dim): dim 8..128, a multiple of 8, is the number of channels kept of every 128;
  * 16-byte aligned, strides in elements and multiples of 8.  res (batch, heads, >= n_res, 128), aligned likewise.
  * order (optional): (batch, ...) uint8 with order_seq_stride bytes between sequences, entry t = source row, inside its
- * group of order_block tokens, of stored token t; the rows come back in source order.
+ * group of order_block tokens, of stored token t; the rows come back in source order.  A group whose entries are not a
+ * permutation raises PKV_FLAG_BAD_STREAM and comes back in stored order.
  * cb 64 or 128; K per channel needs qblock = cb.  A block that the table places outside the stream, or that is cut
  * short, sets PKV_FLAG_BAD_STREAM and reads as codes 0 from there on.
  */

@@ -98,6 +98,20 @@ __device__ __forceinline__ void load_token_params(const pkv_dense_args& a, int b
     }
 }
 
+// Whether a reorder group of n entries names every row of the group once.  Warp-cooperative.
+__device__ __forceinline__ bool is_permutation(const uint8_t* group, int n, int lane) {
+    bool ok = true;
+    for (int w = 0; w < n; w += 32) {                 // rows w .. w + 31
+        unsigned seen = 0;
+        for (int i = lane; i < n; i += 32) {
+            const unsigned v = group[i] - (unsigned)w;
+            if (v < 32u) seen |= 1u << v;
+        }
+        ok = __reduce_or_sync(0xffffffffu, seen) == (n - w >= 32 ? 0xffffffffu : (1u << (n - w)) - 1u) && ok;
+    }
+    return ok;
+}
+
 // 16 residual rows of one (sequence, head) behind the dequantised ones
 __device__ __forceinline__ void copy_residual(const pkv_dense_args& a, int64_t item, int lane) {
     const int per = (a.n_res + 15) >> 4, chunks = a.dim >> 3;
@@ -167,10 +181,24 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32) dense_kernel(pkv_dense_args
     }
     __syncwarp();
     bool cut = bad;
-    const uint8_t* ord = a.order ? a.order + (int64_t)b * a.order_seq_stride + (int64_t)cbi * a.cb : nullptr;
     T* out = reinterpret_cast<T*>(a.out) + b * a.o_stride_b + h * a.o_stride_h + (int64_t)cbi * a.cb * a.o_stride_s;
-    // row of stored token t of this block: the reorder moves tokens inside groups of order_block
-    const auto row = [&](int t) { return out + (ord ? (t / a.order_block) * a.order_block + ord[t] : t) * a.o_stride_s; };
+    // The reorder moves tokens inside groups of order_block.  Its entries say where rows are stored, so a group that is no
+    // permutation (a corrupt blob) is flagged and stays in stored order: every row is written, none outside its group.
+    const uint8_t* ord = a.order && a.order_block > 1 ? a.order + (int64_t)b * a.order_seq_stride + (int64_t)cbi * a.cb : nullptr;
+    uint64_t moved = 0;                                // bit g: group g of this block is a permutation
+    if (ord)
+        for (int g = 0; g * a.order_block < a.cb; g++) {
+            if (is_permutation(ord + g * a.order_block, a.order_block, lane)) moved |= 1ull << g;
+            else bad = true;
+        }
+    const auto row = [&](int t) {                      // of stored token t of this block
+        int at = t;
+        if (ord) {
+            const int g = t / a.order_block;
+            if ((moved >> g) & 1) at = g * a.order_block + ord[t];
+        }
+        return out + at * a.o_stride_s;
+    };
     const T2 bias = DT<T>::dup(MAGIC == 0x64006400u ? 1024.f : 128.f);
 
     if (WHICH == 0) {

@@ -231,6 +231,14 @@ def _check_layer_shapes(L: "CompressedLayer", batch: int) -> None:
         raise ValueError("token-mode k_scale / k_zero must be (B, >= n_comp)")
     if L.k_stream.dim() != 2 or L.v_stream.dim() != 2 or L.k_stream.stride(1) != 1 or L.v_stream.stride(1) != 1:
         raise ValueError("streams must be (B, capacity) with contiguous bytes")
+    _check_order(L, batch)
+
+
+def _check_order(L: "CompressedLayer", batch: int) -> None:
+    """One byte for every packed token.  The values are looked at on the device (dense.cu): reading them here would synchronise."""
+    if L.order is not None and (L.order.dtype != torch.uint8 or L.order.dim() != 3 or L.order.shape[0] != batch
+                                or L.order.shape[1] * L.order.shape[2] != L.n_comp or not L.order.is_contiguous()):
+        raise ValueError("order must be a contiguous (B, n_comp / block, block) uint8 tensor")
 
 
 # changes whenever the attention kernel changes in a way that can change its DRAM traffic (keys recorded profiler figures)
@@ -331,8 +339,7 @@ def dense(which: str, layer: CompressedLayer, res: Optional[torch.Tensor], n_res
             or stream.dim() != 2 or stream.stride(1) != 1 or (pb < n // block if mode == K_CHANNEL else pt < n) \
             or not scale.is_contiguous() or not zero.is_contiguous() or zero.shape != scale.shape or any(t.shape[0] != B for t in (info, scale)):
         raise ValueError("dense: the layer's tables do not cover its tokens")
-    if layer.order is not None and (not layer.order.is_contiguous() or layer.order.numel() != B * n):
-        raise ValueError("dense: order must hold one entry per token")
+    _check_order(layer, B)
     if n_res and (res.dim() != 4 or res.shape[:2] != (B, H) or res.shape[2] < n_res or res.shape[3] != 128 or res.stride(3) != 1 or res.stride(2) != 128
                   or res.dtype != scale.dtype):
         raise ValueError("dense: the residual must be (B, H, >= n_res, 128) rows of the layer's element type")

@@ -62,3 +62,41 @@ def test_dense_flags_blocks_outside_the_stream(cuda_device):
     assert torch.equal(got[:, 0], kd[:, 0]) and torch.equal(got[:, 1, 64:], kd[:, 1, 64:])
     want = layer.k_zero[0, 1, 0].cpu() * layer.k_scale[0, 1, 0].cpu()             # codes 0
     assert torch.equal(got[0, 1, :64], want.expand(64, 128))
+
+
+@pytest.mark.parametrize("cbv", [64, 128])
+@pytest.mark.parametrize("entry", [255, 64, 7])
+def test_dense_keeps_groups_that_are_no_permutation_in_stored_order(cuda_device, cbv, entry):
+    """An entry outside its group, or one that is there twice, in the last group of the last sequence and in one before
+    others: flagged, the group's rows in stored order, every other row and the residual untouched."""
+    dev = cuda_device
+    B, H, S, n_res = 2, 2, 256, 5
+    k, v = synth.synth_kv(B, H, S, 128, seed=6, dtype=torch.float16, device=dev)
+    rel = synth.rel_for_bits(4)
+    layer = encode.compress_kv(k, v, block=64, bits_k=4, bits_v=4, k_rel=rel, v_rel=rel, cbk=64, cbv=cbv, repack_method=RepackMethod.MEDIAN)
+    res = torch.randn(B, H, 192, 128, device=dev).half()
+    want = {which: ops.dense(which, layer, res, n_res, 128, 64) for which in "kv"}
+    broken = layer.order.clone()
+    for b, g in ((0, 1), (B - 1, S // 64 - 1)):
+        stored = layer.order[b, g].long() + 64 * g
+        for which in "kv":
+            want[which][b, :, 64 * g:64 * g + 64] = want[which][b][:, stored]
+        row = int((broken[b, g] != entry).nonzero()[0])
+        broken[b, g, row] = entry
+    layer.order = broken
+    for which in "kv":
+        flags = ops.new_flags(dev)
+        got = ops.dense(which, layer, res, n_res, 128, 64, flags)
+        assert int(flags.item()) == 4
+        assert torch.equal(got, want[which])
+
+
+def test_dense_refuses_an_order_of_another_form(cuda_device):
+    dev = cuda_device
+    k, v = synth.synth_kv(1, 1, 128, 128, seed=7, dtype=torch.float16, device=dev)
+    layer = encode.compress_kv(k, v, block=64, bits_k=4, bits_v=4, k_rel=1 / 14, v_rel=1 / 14, repack_method=RepackMethod.MEDIAN)
+    order = layer.order
+    for other in (order.int(), order[:, :1], order.view(1, 128), torch.zeros(1, 2, 128, dtype=torch.uint8, device=dev)[..., ::2]):
+        layer.order = other
+        with pytest.raises(ValueError):
+            ops.dense("k", layer, None, 0, 128, 64)

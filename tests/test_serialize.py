@@ -60,6 +60,11 @@ def test_rejects_metadata_that_disagrees_with_the_arrays():
             ops._check_layer_shapes(L, 2)
     with pytest.raises(ValueError):
         ops._check_layer_shapes(_fake_layer(), 3)          # q with another batch size
+    for other in (torch.int32, None):                      # the dense view stores rows where the order says
+        L = _fake_layer(order=True)
+        L.order = L.order[:, :1] if other is None else L.order.to(other)
+        with pytest.raises(ValueError):
+            serialize.loads_layer(serialize.dumps_layer(L), device="cpu")
     L = _fake_layer()
     L.v_info = L.v_info[:, :3]
     with pytest.raises(ValueError):
