@@ -1438,13 +1438,16 @@ __global__ void exchange_wait_kernel(uint32_t* arrivals, int n_ranks, unsigned e
     if (!all && lane == 0) atomicOr(flags, kFlagTimeout);
     if (all && consume && lane < n_ranks) atomicSub(arrivals + lane, expected);   // resolved where the peers' additions are: this GPU's L2
     __threadfence_system();
+    // the launch before is complete too, whatever became of the arrivals: what follows is then ordered behind both, also a
+    // launch that starts early and waits for this one only
+    asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
 int launch_exchange_wait(uint32_t* arrivals, int n_ranks, unsigned expected, unsigned max_polls, unsigned* flags, bool consume, cudaStream_t st) {
     if (!arrivals || !flags || n_ranks < 1 || n_ranks > 8) return kBadArgument;
     // The wait needs nothing from the launch before it but this rank's own arrivals, which are counted like the
-    // others': it may start while that launch drains (programmatic stream serialisation, no device-side wait) and
-    // ends when the last rank has arrived.  Launches after it are ordered behind both.
+    // others': it may start while that launch drains (programmatic stream serialisation) and ends when the last rank
+    // has arrived and that launch is complete.  Launches after it are ordered behind both.
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(1, 1, 1);
     cfg.blockDim = dim3(32, 1, 1);
@@ -1670,7 +1673,7 @@ int launch_attention(const AttnArgs& a, const AttnExchange* xch, const AttnAppen
     P.extra = best_extra;
     // At most one CTA per SM: 8 KV heads x 700 tokens 14.3 -> 13.0 us a launch.  Fuller launches stay ordered: their CTAs would
     // be placed around those still running, unevenly (11 x 2154: 30 -> 34 us; two launches 0 to 5 % slower).  So do launches
-    // with an exchange: the launch before may be its wait, which does not wait for the launch before itself.
+    // with an exchange, which were not measured.
     P.early = best_launches == 1 && !xch && pairs * best_cl <= kSmCount;
     if (best_launches == 2) {
         const ScratchLayout L = scratch_layout(pairs, best_cl, best_extra >= 0 ? best_split + 1 : best_split, P.dump_bytes);

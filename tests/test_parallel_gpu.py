@@ -127,6 +127,41 @@ def test_exchange_wait_gives_up(cuda_device):
     assert int(flags.item()) == 0
 
 
+def test_launches_behind_a_wait_are_ordered_behind_the_launch_before_it(cuda_device):
+    """A wait that gives up at once stands between two attention launches, the second of which may start early and reads what
+    the first one writes: the same bits as with a synchronisation after each."""
+    from packkv_b200 import _lib, encode, ops, synth
+    from packkv_b200.config import QuantMode
+    dev, dtype, B, H, G, S = cuda_device, torch.bfloat16, 4, 8, 4, 4096
+    args = dict(block=64, bits_k=4, bits_v=4, k_rel=1 / 14, v_rel=1 / 14, k_mode=QuantMode.ChannelQuant)
+    k, v = synth.synth_kv(B, H, S, 128, seed=6, dtype=dtype, device=dev, apply_rope=True)
+    long, short = encode.compress_kv(k, v, **args), encode.compress_kv(k[:1, :, :256], v[:1, :, :256], **args)
+    q = synth.synth_q(B, H * G, 128, seed=6, dtype=dtype, device=dev)[:, :, 0].contiguous()
+    scratch, arrivals, waits = ops.new_attention_scratch(dev), torch.zeros(2, dtype=torch.int32, device=dev), ops.new_flags(dev)
+    assert ops.decode_attention(q[:1], short, None, None, 0, scratch=scratch, plan_only=True)[2] == 1
+    got = []
+    for sync in (True, False):
+        x, y, flags = torch.zeros_like(q), torch.empty_like(q[:1]), ops.new_flags(dev)
+        torch.cuda.synchronize()
+        for _ in range(20):
+            ops.decode_attention(q + x, long, None, None, 0, out=x, flags=flags, scratch=scratch, scaling=1.0)
+            if sync:
+                torch.cuda.synchronize()
+            ops.exchange_wait(arrivals, 2, 1, waits, max_polls=1)
+            if sync:
+                torch.cuda.synchronize()
+            ops.decode_attention(x[-1:], short, None, None, 0, out=y, flags=flags, scratch=scratch, scaling=1.0)
+            if sync:
+                torch.cuda.synchronize()
+            x[0] = y[0]
+        torch.cuda.synchronize()
+        assert int(flags.item()) == 0
+        got.append((x, y))
+    assert int(waits.item()) == _lib.FLAG_TIMEOUT
+    for a, b in zip(*got):
+        assert torch.equal(a.view(torch.int16), b.view(torch.int16))
+
+
 def test_consuming_wait_serves_every_step(cuda_device):
     """The wait that takes a step's arrivals off the counters again: three steps with the same call, the counters end
     at zero; a step whose arrivals are missing gives up with the flag and takes nothing."""
