@@ -105,7 +105,7 @@ int extent(int64_t v) {
 bool half_type(const at::Tensor& t) { return t.scalar_type() == at::kHalf || t.scalar_type() == at::kBFloat16; }
 int is_bf16(const at::Tensor& t) { return t.scalar_type() == at::kBFloat16; }
 
-// the library's calls run without the interpreter lock: a launch may wait for room in the stream's queue
+// the library's launches run without the interpreter lock: one may wait for room in the stream's queue
 template <typename F> int32_t unlocked(F call) {
     PyThreadState* state = PyEval_SaveThread();
     const int32_t st = call();
@@ -385,10 +385,12 @@ PyObject* append_residual(PyObject* const* p) {
         check(sin != nullptr, "cos/sin must be (B or 1, T, 128)");
         cs = std::make_unique<Tables>(*cos, *sin, k.scalar_type(), T, 128, "cos/sin must be (B or 1, T, 128)");
     }
-    check_status(lib.append(k.data_ptr(), k.stride(0), k.stride(1), k.stride(2), v.data_ptr(), v.stride(0), v.stride(1), v.stride(2),
-                            cs ? cs->cos.data_ptr() : nullptr, cs ? cs->sin.data_ptr() : nullptr, cs ? cs->stride_b : 0, kr.data_ptr(), vr.data_ptr(),
-                            kr.stride(0), kr.stride(1), extent(kr.size(2)), extent(integer(p[4])), extent(k.size(0)), extent(k.size(1)), extent(T),
-                            is_bf16(k), stream()),
+    const int capacity = extent(kr.size(2)), position = extent(integer(p[4])), batch = extent(k.size(0)), heads = extent(k.size(1)), tokens = extent(T);
+    check_status(unlocked([&, on = stream()] {
+                     return lib.append(k.data_ptr(), k.stride(0), k.stride(1), k.stride(2), v.data_ptr(), v.stride(0), v.stride(1), v.stride(2),
+                                       cs ? cs->cos.data_ptr() : nullptr, cs ? cs->sin.data_ptr() : nullptr, cs ? cs->stride_b : 0, kr.data_ptr(),
+                                       vr.data_ptr(), kr.stride(0), kr.stride(1), capacity, position, batch, heads, tokens, is_bf16(k), on);
+                 }),
                  "append_residual");
     Py_RETURN_NONE;
 }
@@ -407,10 +409,14 @@ PyObject* widen_rows(PyObject* const* p) {
     const int64_t T = k.size(2), D = k.size(3);
     std::unique_ptr<Tables> cs;
     if (cos) cs = std::make_unique<Tables>(*cos, *sin, k.scalar_type(), T, D, "cos/sin must be (B or 1, T, D)");
-    check_status(lib.widen(k.data_ptr(), k.stride(0), k.stride(1), k.stride(2), v ? v->data_ptr() : nullptr, v ? v->stride(0) : 0, v ? v->stride(1) : 0,
-                           v ? v->stride(2) : 0, cs ? cs->cos.data_ptr() : nullptr, cs ? cs->sin.data_ptr() : nullptr, cs ? cs->stride_b : 0,
-                           ko.data_ptr(), vo ? vo->data_ptr() : nullptr, ko.stride(0), ko.stride(1), extent(ko.size(2)), extent(integer(p[4])),
-                           extent(k.size(0)), extent(k.size(1)), extent(T), extent(D), truth(p[7]), is_bf16(k), stream()),
+    const int capacity = extent(ko.size(2)), position = extent(integer(p[4])), batch = extent(k.size(0)), heads = extent(k.size(1)), tokens = extent(T);
+    const bool zero_tail = truth(p[7]);
+    check_status(unlocked([&, on = stream()] {
+                     return lib.widen(k.data_ptr(), k.stride(0), k.stride(1), k.stride(2), v ? v->data_ptr() : nullptr, v ? v->stride(0) : 0,
+                                      v ? v->stride(1) : 0, v ? v->stride(2) : 0, cs ? cs->cos.data_ptr() : nullptr, cs ? cs->sin.data_ptr() : nullptr,
+                                      cs ? cs->stride_b : 0, ko.data_ptr(), vo ? vo->data_ptr() : nullptr, ko.stride(0), ko.stride(1), capacity, position,
+                                      batch, heads, tokens, (int)D, zero_tail, is_bf16(k), on);
+                 }),
                  "widen_rows");
     Py_RETURN_NONE;
 }
@@ -423,9 +429,11 @@ PyObject* rope(PyObject* const* p) {
     const Tables cs(cos, sin, x.scalar_type(), x.size(2), x.size(3), "cos/sin must be (B or 1, T, D)");
     at::Tensor own;
     if (!out) { own = at::empty(x.sizes(), x.options()); out = &own; }
-    check_status(lib.rope(x.data_ptr(), x.stride(0), x.stride(1), x.stride(2), cs.cos.data_ptr(), cs.sin.data_ptr(), cs.stride_b, out->data_ptr(),
-                          out->stride(0), out->stride(1), out->stride(2), extent(x.size(0)), extent(x.size(1)), extent(x.size(2)), extent(x.size(3)),
-                          is_bf16(x), stream()),
+    const int batch = extent(x.size(0)), heads = extent(x.size(1)), tokens = extent(x.size(2)), dim = extent(x.size(3));
+    check_status(unlocked([&, on = stream()] {
+                     return lib.rope(x.data_ptr(), x.stride(0), x.stride(1), x.stride(2), cs.cos.data_ptr(), cs.sin.data_ptr(), cs.stride_b,
+                                     out->data_ptr(), out->stride(0), out->stride(1), out->stride(2), batch, heads, tokens, dim, is_bf16(x), on);
+                 }),
                  "rope");
     if (p[3] != Py_None) return Py_NewRef(p[3]);
     return THPVariable_Wrap(own);
