@@ -190,9 +190,10 @@ void fill_layer(PyObject* layer, const at::Tensor& q, int64_t batch, int64_t n_c
 }
 
 void fill_append(PyObject* append, const at::Tensor& q, const at::Tensor& k_res, int64_t batch, int64_t kv_heads, int64_t n_res, pkv_attn_append& ap) {
-    check(PyTuple_Check(append) && PyTuple_GET_SIZE(append) == 4, "append is (k_new, v_new, cos, sin)");
-    const at::Tensor &k = cuda(PyTuple_GET_ITEM(append, 0), "k_new"), &v = cuda(PyTuple_GET_ITEM(append, 1), "v_new");
-    const at::Tensor *cos = maybe_cuda(PyTuple_GET_ITEM(append, 2), "cos"), *sin = maybe_cuda(PyTuple_GET_ITEM(append, 3), "sin");
+    check(PySequence_Fast_GET_SIZE(append) == 4, "append is (k_new, v_new, cos, sin)");
+    PyObject** it = PySequence_Fast_ITEMS(append);
+    const at::Tensor &k = cuda(it[0], "k_new"), &v = cuda(it[1], "v_new");
+    const at::Tensor *cos = maybe_cuda(it[2], "cos"), *sin = maybe_cuda(it[3], "sin");
     check(n_res >= 1 && k.dim() == 4 && k.size(0) == batch && k.size(1) == kv_heads && k.size(2) == 1 && k.size(3) == 128 && v.sizes() == k.sizes() &&
               k.stride(3) == 1 && v.stride(3) == 1 && k.scalar_type() == q.scalar_type() && v.scalar_type() == q.scalar_type(),
           "append needs k_new / v_new of shape (B, Hkv, 1, 128) in q's dtype with contiguous channels");
@@ -248,9 +249,10 @@ PyObject* decode_attention(PyObject* const* p) {
     a.flags = static_cast<uint32_t*>(flags->data_ptr());
     pkv_attn_append ap{};
     const bool has_append = p[10] != Py_None;
+    const Held append(has_append ? PySequence_Fast(p[10], "append is (k_new, v_new, cos, sin)") : Py_NewRef(Py_None));   // any iterable
     if (has_append) {
         check(n_res >= 1 && k_res, "append needs k_new / v_new of shape (B, Hkv, 1, 128) in q's dtype with contiguous channels");
-        fill_append(p[10], q, *k_res, batch, kv_heads, n_res, ap);
+        fill_append(append.o, q, *k_res, batch, kv_heads, n_res, ap);
     }
     const pkv_attn_exchange* xch = p[9] == Py_None ? nullptr : reinterpret_cast<const pkv_attn_exchange*>(integer(p[9]));
     const bool plan_only = truth(p[13]);
@@ -260,7 +262,7 @@ PyObject* decode_attention(PyObject* const* p) {
         if (p[12] != Py_None) {
             const Held seq(PySequence_Fast(p[12], "plan is (cluster, nsplit, launches[, extra])"));
             const Py_ssize_t n = PySequence_Fast_GET_SIZE(seq.o);
-            check(n == 3 || n == 4, "plan is (cluster, nsplit, launches[, extra])");
+            check(n >= 3, "plan is (cluster, nsplit, launches[, extra])");
             PyObject** it = PySequence_Fast_ITEMS(seq.o);
             plan.cluster = extent(integer(it[0])); plan.nsplit = extent(integer(it[1])); plan.launches = extent(integer(it[2]));
             plan.extra = n > 3 ? extent(integer(it[3])) : 0;

@@ -37,3 +37,17 @@ def test_no_call_holds_the_interpreter_lock(stubbed):
     ops.widen_rows(_empty(B, H, 1, 96), None, res, None)
     ops.value_median_order(_empty(B, H, 64, 128), 64, 0.1)
     ops.decode_attention(_empty(B, H * G, 128), None, res, res, 1)
+
+
+
+def test_append_and_plan_take_any_sequence(stubbed):
+    q, res, new, cs = _empty(B, H * G, 128), _empty(B, H, R, 128), _empty(B, H, 1, 128), _empty(1, 1, 128)
+    for append in ((new, new, cs, cs), [new, new, cs, cs], iter((new, new, None, None))):
+        ops.decode_attention(q, None, res, res, 1, append=append)
+    for plan in ((0, 0, 1), [0, 0, 1, 0], (0, 0, 1, 0, 7)):
+        ops.decode_attention(q, None, res, res, 1, plan=plan)
+    for append in ((new, new, cs), (new, new, cs, cs, cs), 3):
+        with pytest.raises((ValueError, TypeError)):
+            ops.decode_attention(q, None, res, res, 1, append=append)
+    with pytest.raises(ValueError):
+        ops.decode_attention(q, None, res, res, 1, plan=(0, 0))
