@@ -290,7 +290,8 @@ int32_t pkv_dequantize(const uint8_t* codes, int64_t codes_seq_stride, const voi
  * order (optional): (batch, ...) uint8 with order_seq_stride bytes between sequences, entry t = source row, inside its
  * group of order_block tokens, of stored token t; the rows come back in source order.  A group whose entries are not a
  * permutation raises PKV_FLAG_BAD_STREAM and comes back in stored order.
- * cb 64 or 128; K per channel needs qblock = cb.  A block that the table places outside the stream, or that is cut
+ * cb 64 or 128; K per channel: qblock a multiple of 16 that divides n_comp; order_block divides n_comp, at most 256.
+ * A block that the table places outside the stream, or that is cut
  * short, sets PKV_FLAG_BAD_STREAM and reads as codes 0 from there on.
  */
 typedef struct pkv_dense_args {

@@ -112,6 +112,24 @@ __device__ __forceinline__ bool is_permutation(const uint8_t* group, int n, int 
     return ok;
 }
 
+// Row, relative to the stream block's first, of every token of the block.  The reorder moves tokens inside groups of
+// order_block, which may begin or end in another block.  Its entries say where rows are stored, so a group that is no
+// permutation (a corrupt blob) stays in stored order: every row is written, none outside its group.  False if there is one.
+__device__ __forceinline__ bool place_rows(const pkv_dense_args& a, int b, int cbi, int16_t* place, int lane) {
+    const int first = cbi * a.cb, ob = a.order_block;
+    for (int t = lane; t < a.cb; t += 32) place[t] = (int16_t)t;
+    if (!a.order || ob == 1) return true;
+    __syncwarp();
+    bool ok = true;
+    const uint8_t* ord = a.order + (int64_t)b * a.order_seq_stride;
+    for (int g = first / ob * ob; g < first + a.cb; g += ob) {
+        if (!is_permutation(ord + g, ob, lane)) { ok = false; continue; }
+        for (int i = lane; i < ob; i += 32)
+            if (g + i >= first && g + i < first + a.cb) place[g + i - first] = (int16_t)(g - first + ord[g + i]);
+    }
+    return ok;
+}
+
 // 16 residual rows of one (sequence, head) behind the dequantised ones
 __device__ __forceinline__ void copy_residual(const pkv_dense_args& a, int64_t item, int lane) {
     const int per = (a.n_res + 15) >> 4, chunks = a.dim >> 3;
@@ -135,11 +153,15 @@ __host__ __device__ int dense_bound(int cb, int bits) {
     const VGeom g(cb, bits);
     return g.head_bytes + g.nseg * (g.min_bytes + g.len_bytes + 32 * g.ppt * 2 * bits);
 }
-template <int WHICH>
-__host__ __device__ int dense_slot(int cb, int bits) { return ((dense_bound<WHICH>(cb, bits) + 48 + 15) & ~15) + 4 * cb; }   // the block, then its token parameters
+// the block, its token parameters, and in the general form the row of every token
+template <int WHICH, bool GENERAL>
+__host__ __device__ int dense_slot(int cb, int bits) { return ((dense_bound<WHICH>(cb, bits) + 48 + 15) & ~15) + 4 * cb + (GENERAL ? 2 * cb : 0); }
 
-// WHICH 0: K, parameters per (head, block, channel) or, with TOKEN, per token; WHICH 1: V, per token
-template <typename T, int WHICH, int BITS, bool HP, bool TOKEN>
+// WHICH 0: K, parameters per (head, block, channel) or, with TOKEN, per token; WHICH 1: V, per token.
+// GENERAL: layers that are reordered, or whose channel parameters change inside a stream block or span several.  Rows come
+// from a table in shared memory (V of 4 x 8064 tokens x 8 heads, 4 bits: 33 us; 50 with a division and a byte of the order
+// for every row); plain layers keep a kernel without either (27 us; 34 with the order as a run-time branch).
+template <typename T, int WHICH, int BITS, bool HP, bool TOKEN, bool GENERAL>
 __global__ void __launch_bounds__(kWarpsPerCta * 32) dense_kernel(pkv_dense_args a) {
     using T2 = typename DT<T>::T2;
     constexpr unsigned MAGIC = DT<T>::kMagic2;
@@ -155,15 +177,16 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32) dense_kernel(pkv_dense_args
     }
     const int b = (int)(item / per_seq), rem = (int)(item % per_seq), cbi = rem / nblk, hb = rem % nblk;
     const int h = WHICH == 0 ? hb : hb >> 1;
-    uint8_t* slot = smem + wic * dense_slot<WHICH>(a.cb, BITS);
-    unsigned* tscale = reinterpret_cast<unsigned*>(slot + dense_slot<WHICH>(a.cb, BITS) - 4 * a.cb);
+    uint8_t* slot = smem + wic * dense_slot<WHICH, GENERAL>(a.cb, BITS);
+    unsigned* tscale = reinterpret_cast<unsigned*>(slot + dense_slot<WHICH, false>(a.cb, BITS) - 4 * a.cb);
     unsigned* tzero = tscale + a.cb / 2;
+    int16_t* place = reinterpret_cast<int16_t*>(tzero + a.cb / 2);
     const uint32_t* bi = a.block_info + (b * a.info_seq_stride + rem) * 2;
     const unsigned off = bi[0], size = bi[1];
     if (TOKEN) load_token_params<T>(a, b, cbi * a.cb, a.cb, tscale, tzero, lane);
     T2 cscale[4], czero[4];
-    if (!TOKEN) {
-        const int64_t pi = (((int64_t)b * a.heads + h) * a.param_blocks + cbi) * 128 + 4 * lane;
+    const auto channel_params = [&](int t) {          // of token t of this block
+        const int64_t pi = (((int64_t)b * a.heads + h) * a.param_blocks + (GENERAL ? (cbi * a.cb + t) / a.qblock : cbi)) * 128 + 4 * lane;
         const uint2 s = __ldg(reinterpret_cast<const uint2*>(reinterpret_cast<const T*>(a.scale) + pi));
         const uint2 z = __ldg(reinterpret_cast<const uint2*>(reinterpret_cast<const T*>(a.zero) + pi));
 #pragma unroll
@@ -171,7 +194,8 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32) dense_kernel(pkv_dense_args
             cscale[j] = pair_of<T2>(__byte_perm(j < 2 ? s.x : s.y, 0, (j & 1) ? 0x3232 : 0x1010));
             czero[j] = pair_of<T2>(__byte_perm(j < 2 ? z.x : z.y, 0, (j & 1) ? 0x3232 : 0x1010));
         }
-    }
+    };
+    if (!TOKEN) channel_params(0);
     // a block that the table places outside the stream, or that is cut short, reads as codes 0 from there on
     bool bad = (int64_t)off + size > a.capacity || (int)size > dense_bound<WHICH>(a.cb, BITS) || (int)size < (WHICH == 0 ? a.cb / 8 : a.cb == 128 ? 8 : 4);
     const uint8_t* blk = slot;
@@ -179,26 +203,11 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32) dense_kernel(pkv_dense_args
         const uint8_t* base = a.stream + b * a.stream_seq_stride;
         blk = warp_copy_in(slot, base + off, (int)size, lane, base, base + a.capacity);
     }
-    __syncwarp();
     bool cut = bad;
     T* out = reinterpret_cast<T*>(a.out) + b * a.o_stride_b + h * a.o_stride_h + (int64_t)cbi * a.cb * a.o_stride_s;
-    // The reorder moves tokens inside groups of order_block.  Its entries say where rows are stored, so a group that is no
-    // permutation (a corrupt blob) is flagged and stays in stored order: every row is written, none outside its group.
-    const uint8_t* ord = a.order && a.order_block > 1 ? a.order + (int64_t)b * a.order_seq_stride + (int64_t)cbi * a.cb : nullptr;
-    uint64_t moved = 0;                                // bit g: group g of this block is a permutation
-    if (ord)
-        for (int g = 0; g * a.order_block < a.cb; g++) {
-            if (is_permutation(ord + g * a.order_block, a.order_block, lane)) moved |= 1ull << g;
-            else bad = true;
-        }
-    const auto row = [&](int t) {                      // of stored token t of this block
-        int at = t;
-        if (ord) {
-            const int g = t / a.order_block;
-            if ((moved >> g) & 1) at = g * a.order_block + ord[t];
-        }
-        return out + at * a.o_stride_s;
-    };
+    if (GENERAL) bad |= !place_rows(a, b, cbi, place, lane);
+    __syncwarp();
+    const auto row = [&](int t) { return out + (GENERAL ? place[t] : t) * a.o_stride_s; };   // of stored token t of this block
     const T2 bias = DT<T>::dup(MAGIC == 0x64006400u ? 1024.f : 128.f);
 
     if (WHICH == 0) {
@@ -206,6 +215,7 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32) dense_kernel(pkv_dense_args
         int pos = g.head_bytes;
         const bool inside = 4 * lane < a.dim;
         for (int r = 0; r < g.rounds; r++) {
+            if (GENERAL && !TOKEN && a.qblock != a.cb && r > 0) channel_params(16 * r);
             unsigned u[4][2][4] = {};                     // [channel][group of eight][k]
             if (!cut && pos + g.min_bytes + g.len_bytes <= (int)size) {
                 PackHeads<BITS> ph;
@@ -301,22 +311,26 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32) dense_kernel(pkv_dense_args
     if (__any_sync(0xffffffffu, bad) && lane == 0) atomicOr(a.flags, kFlagBadStream);
 }
 
-template <typename T, int WHICH, int BITS, bool HP, bool TOKEN>
+template <typename T, int WHICH, int BITS, bool HP, bool TOKEN, bool GENERAL>
 static int start(const pkv_dense_args& a, cudaStream_t st) {
-    const int smem = kWarpsPerCta * dense_slot<WHICH>(a.cb, BITS);
-    if (smem > 48 * 1024 &&
-        cudaFuncSetAttribute(dense_kernel<T, WHICH, BITS, HP, TOKEN>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
-        return kCudaError;
+    const auto kern = dense_kernel<T, WHICH, BITS, HP, TOKEN, GENERAL>;
+    const int smem = kWarpsPerCta * dense_slot<WHICH, GENERAL>(a.cb, BITS);
+    if (smem > 48 * 1024 && cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return kCudaError;
     const int64_t items = (int64_t)a.batch * ((int64_t)(a.n_comp / a.cb) * (WHICH == 0 ? a.heads : 2 * a.heads) + (int64_t)a.heads * ((a.n_res + 15) >> 4));
     const int64_t ctas = (items + kWarpsPerCta - 1) / kWarpsPerCta;
     if (ctas > 0x7FFFFFFF) return kBadArgument;
-    dense_kernel<T, WHICH, BITS, HP, TOKEN><<<(unsigned)ctas, kWarpsPerCta * 32, smem, st>>>(a);
+    kern<<<(unsigned)ctas, kWarpsPerCta * 32, smem, st>>>(a);
     return cudaGetLastError() == cudaSuccess ? kOk : kCudaError;
 }
 
+template <typename T, int WHICH, int BITS, bool HP, bool TOKEN>
+static int pick_form(const pkv_dense_args& a, cudaStream_t st) {
+    const bool general = a.order || (!TOKEN && a.qblock != a.cb);
+    return general ? start<T, WHICH, BITS, HP, TOKEN, true>(a, st) : start<T, WHICH, BITS, HP, TOKEN, false>(a, st);
+}
 template <typename T, int WHICH, int BITS, bool TOKEN>
 static int pick_zero(const pkv_dense_args& a, cudaStream_t st) {
-    return a.high_precision_zero ? start<T, WHICH, BITS, true, TOKEN>(a, st) : start<T, WHICH, BITS, false, TOKEN>(a, st);
+    return a.high_precision_zero ? pick_form<T, WHICH, BITS, true, TOKEN>(a, st) : pick_form<T, WHICH, BITS, false, TOKEN>(a, st);
 }
 template <typename T, int BITS>
 static int pick_mode(const pkv_dense_args& a, cudaStream_t st) {
@@ -331,7 +345,8 @@ static int pick_bits(const pkv_dense_args& a, cudaStream_t st) {
 int launch_dense(const pkv_dense_args& a, cudaStream_t st) {
     if ((a.which != 0 && a.which != 1) || a.batch < 0 || a.heads <= 0 || a.n_comp < 0 || a.n_res < 0 || a.dim <= 0) return kBadArgument;
     if (a.bits < 2 || a.bits > 4 || (a.cb != 64 && a.cb != 128) || (a.mode != PKV_K_CHANNEL && a.mode != PKV_K_TOKEN) || a.dim > 128 || a.dim % 8) return kUnsupported;
-    if (a.which == 1 ? a.mode != PKV_K_TOKEN : a.mode == PKV_K_CHANNEL && a.qblock != a.cb) return kUnsupported;
+    // a round of 16 tokens has one set of channel parameters
+    if (a.which == 1 ? a.mode != PKV_K_TOKEN : a.mode == PKV_K_CHANNEL && (a.qblock <= 0 || a.qblock % 16)) return kUnsupported;
     if (a.n_comp % a.cb) return kBadArgument;
     if ((int64_t)a.batch * ((int64_t)a.n_comp + a.n_res) == 0) return kOk;
     // rows are written in 8-byte (K) and 16-byte (residual) pieces
@@ -340,9 +355,9 @@ int launch_dense(const pkv_dense_args& a, cudaStream_t st) {
     if (a.n_res && (!a.res || !aligned(a.res) || ((a.res_stride_b | a.res_stride_h) & 7))) return kBadArgument;
     if (a.n_comp) {
         if (!a.stream || !a.block_info || !a.scale || !a.zero || (reinterpret_cast<uintptr_t>(a.stream) & 1) || (a.stream_seq_stride & 1)) return kBadArgument;
-        if (a.mode == PKV_K_CHANNEL ? a.param_blocks < a.n_comp / a.cb || (reinterpret_cast<uintptr_t>(a.scale) & 7) || (reinterpret_cast<uintptr_t>(a.zero) & 7)
+        if (a.mode == PKV_K_CHANNEL ? a.n_comp % a.qblock || a.param_blocks < a.n_comp / a.qblock || (reinterpret_cast<uintptr_t>(a.scale) & 7) || (reinterpret_cast<uintptr_t>(a.zero) & 7)
                                     : a.param_tokens < a.n_comp) return kBadArgument;
-        if (a.order && (a.order_block <= 0 || a.cb % a.order_block || a.order_seq_stride < a.n_comp)) return kBadArgument;
+        if (a.order && (a.order_block <= 0 || a.order_block > 256 || a.n_comp % a.order_block || a.order_seq_stride < a.n_comp)) return kBadArgument;
     }
     return a.is_bf16 ? pick_bits<__nv_bfloat16>(a, st) : pick_bits<__half>(a, st);
 }

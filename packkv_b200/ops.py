@@ -335,7 +335,7 @@ def dense(which: str, layer: CompressedLayer, res: Optional[torch.Tensor], n_res
     if flags is None:
         flags = new_flags(stream.device)
     pb, pt = _param_extents(scale, mode)
-    if n % block or n % cb or info.dim() != 3 or info.shape[1] < (n // cb) * H * (1 if which == "k" else 2) or not info.is_contiguous() \
+    if (mode == K_CHANNEL and n % block) or n % cb or info.dim() != 3 or info.shape[1] < (n // cb) * H * (1 if which == "k" else 2) or not info.is_contiguous() \
             or stream.dim() != 2 or stream.stride(1) != 1 or (pb < n // block if mode == K_CHANNEL else pt < n) \
             or not scale.is_contiguous() or not zero.is_contiguous() or zero.shape != scale.shape or any(t.shape[0] != B for t in (info, scale)):
         raise ValueError("dense: the layer's tables do not cover its tokens")

@@ -100,3 +100,31 @@ def test_dense_refuses_an_order_of_another_form(cuda_device):
         layer.order = other
         with pytest.raises(ValueError):
             ops.dense("k", layer, None, 0, 128, 64)
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("k_mode,block,cbk,cbv,S,repack", [
+    ("channel", 64, 128, 128, 384, RepackMethod.NONE), ("channel", 128, 64, 64, 384, RepackMethod.NONE), ("channel", 32, 128, 64, 256, RepackMethod.NONE),
+    ("token", 128, 64, 64, 256, RepackMethod.MEDIAN), ("token", 128, 64, 128, 256, RepackMethod.GREEDY), ("token", 64, 128, 128, 256, RepackMethod.MEDIAN)])
+def test_dense_takes_quantisation_blocks_of_other_sizes_than_the_streams(cuda_device, dtype, k_mode, block, cbk, cbv, S, repack):
+    """compress_kv stores such layers; a reorder block may span stream blocks, and parameters change inside one."""
+    dev, B, H, rel = cuda_device, 2, 2, synth.rel_for_bits(4)
+    k, v = synth.synth_kv(B, H, S, 128, seed=block + cbk, dtype=dtype)
+    layer = encode.compress_kv(k.to(dev), v.to(dev), block=block, bits_k=4, bits_v=4, k_rel=rel, v_rel=rel, cbk=cbk, cbv=cbv, repack_method=repack,
+                               k_mode=QuantMode.ChannelQuant if k_mode == "channel" else QuantMode.TokenQuant)
+    res = torch.zeros(B, H, 192, 128, dtype=dtype, device=dev)
+    flags = ops.new_flags(dev)
+    for which, x, mode in (("k", k, k_mode), ("v", v, "token")):
+        want = Q.dequant(*Q.quant_ints(x, block, rel, mode, False))
+        got = ops.dense(which, layer, res, 0, 128, block, flags).cpu()
+        assert torch.equal(got.view(torch.int16), want.view(torch.int16)), which
+    assert int(flags.item()) == 0
+
+
+def test_dense_of_per_token_layers_needs_no_whole_quantisation_block(cuda_device):
+    dev, rel = cuda_device, synth.rel_for_bits(4)
+    k, v = synth.synth_kv(1, 2, 192, 128, seed=9, dtype=torch.float16)
+    layer = encode.compress_kv(k.to(dev), v.to(dev), block=64, bits_k=4, bits_v=4, k_rel=rel, v_rel=rel, k_mode=QuantMode.TokenQuant)
+    for which, x in (("k", k), ("v", v)):
+        want = Q.dequant(*Q.quant_ints(x, 64, rel, "token", False))
+        assert torch.equal(ops.dense(which, layer, None, 0, 128, 128).cpu(), want)
