@@ -220,6 +220,8 @@ class PackKVCache(_HFCache):
             L.pending = (key_states, value_states, cos, sin)
             L.n_res = total
             return self._step_result(layer_idx, T)
+        if cos is not None and (cos.dim() < 2 or cos.shape[-2] != T or sin.shape != cos.shape):
+            raise ValueError("cos/sin must be (B or 1, T, D)")      # parts of longer tables would rotate by other positions
         if key_states.stride(3) != 1 or value_states.stride(3) != 1:
             key_states, value_states = key_states.contiguous(), value_states.contiguous()
         if value_states.dtype != key_states.dtype:

@@ -253,3 +253,22 @@ def test_prompts_in_pieces_match_reference_cache(cuda_device, D, repack):
         cache.check_flags()
     finally:
         C.PackKVCacheConfigStatic.config = None
+
+
+@pytest.mark.parametrize("D", [128, 96])
+def test_update_refuses_rotation_tables_of_another_length(cuda_device, D):
+    dev, dtype = cuda_device, torch.bfloat16
+    C.PackKVCacheConfigStatic.config = _cfg(QuantMethod.KIVI)
+    try:
+        cache = C.PackKVCache(1, 2, D, 1)
+        cos, sin = synth.rope_tables(500, D, device=dev, dtype=dtype)
+        for T in (400, 10, 1):                               # a prompt that is packed, tokens that stay behind, a decode step
+            k, v = synth.synth_kv(1, 2, T, D, seed=5, dtype=dtype, device=dev)
+            for n in (T + 1, 500):
+                with pytest.raises(ValueError):
+                    cache.update(k, v, 0, {"cos": cos[:, :n], "sin": sin[:, :n]})
+                    cache.flush()
+            if T > 1:
+                cache.update(k, v, 0, {"cos": cos[:, :T], "sin": sin[:, :T]})
+    finally:
+        C.PackKVCacheConfigStatic.config = None
