@@ -1,6 +1,6 @@
 // Native host path of the per-step entry points: reads the tensors of a call, checks everything the kernels index
 // from, fills the C ABI's argument blocks and calls the library.  packkv_b200.ops keeps the public names; this module
-// (packkv_b200/_host.so) is what they run.
+// (packkv_b200/_host.so) is what they run.  Not looked at: the other ranks' addresses in an exchange block.
 //
 // Why native: a decode step on a short context is a 10-20 us launch, and the same checks written in Python
 // (about 120 tensor attribute calls and 40 ctypes field stores) took 33 us per call, 15 us per encoder call.
@@ -101,6 +101,11 @@ bool truth(PyObject* o) {
 int extent(int64_t v) {
     if (v < INT32_MIN || v > INT32_MAX) fail(PyExc_OverflowError, "extent %lld does not fit 32 bits", (long long)v);
     return (int)v;
+}
+// the device status word
+uint32_t* status_word(const at::Tensor& flags) {
+    check(flags.itemsize() == 4 && flags.numel() >= 1, "flags must hold a 32-bit word (new_flags)");
+    return static_cast<uint32_t*>(flags.data_ptr());
 }
 bool half_type(const at::Tensor& t) { return t.scalar_type() == at::kHalf || t.scalar_type() == at::kBFloat16; }
 int is_bf16(const at::Tensor& t) { return t.scalar_type() == at::kBFloat16; }
@@ -204,6 +209,7 @@ void fill_append(PyObject* append, const at::Tensor& q, const at::Tensor& k_res,
                   cos->size(-1) == 128 && sin->sizes() == cos->sizes() && cos->is_contiguous() && sin->is_contiguous(),
               "cos / sin must be contiguous (B or 1, 1, 128) tensors of q's dtype");
         ap.cos = cos->data_ptr(); ap.sin = sin->data_ptr(); ap.cs_stride_b = cos->size(0) == 1 ? 0 : 128;
+        check(ap.cs_stride_b == 0 || cos->numel() >= batch * 128, "cos / sin must be contiguous (B or 1, 1, 128) tensors of q's dtype");
     }
     ap.res_capacity = extent(k_res.size(2));
 }
@@ -232,6 +238,7 @@ PyObject* decode_attention(PyObject* const* p) {
     at::Tensor own_out, own_flags;
     if (!out) { own_out = at::empty_like(q); out = &own_out; }
     if (!flags) { own_flags = new_flags(q); flags = &own_flags; }
+    check(out->scalar_type() == q.scalar_type() && out->is_contiguous() && out->numel() >= q.numel(), "out must be contiguous, of q's dtype and size");
     pkv_attn_args a{};
     a.q = q.data_ptr(); a.out = out->data_ptr();
     if (n_comp > 0) fill_layer(p[1], q, batch, n_comp, kv_heads, a);
@@ -240,13 +247,16 @@ PyObject* decode_attention(PyObject* const* p) {
                   k_res->stride(3) == 1 && k_res->stride(2) == 128,
               "residual tensors must be (B, Hkv, R, 128) with contiguous rows, in q's dtype");
         check(k_res->strides() == v_res->strides(), "k_res and v_res must share strides");
+        for (const at::Tensor* t : {k_res, v_res})
+            check(t->size(0) >= batch && t->size(1) >= kv_heads && t->size(2) >= n_res && t->size(3) == 128,
+                  "residual tensors must hold n_res rows of 128 channels for every sequence and KV head");
         a.k_res = k_res->data_ptr(); a.v_res = v_res->data_ptr();
         a.res_seq_stride = k_res->stride(0); a.res_head_stride = k_res->stride(1);
     }
     a.n_res = extent(n_res); a.batch = extent(batch); a.kv_heads = extent(kv_heads); a.group = extent(q_heads / kv_heads); a.n_comp = extent(n_comp);
     a.is_bf16 = is_bf16(q);
     a.scaling = p[5] == Py_None ? (float)std::pow(128.0, -0.5) : (float)number(p[5]);
-    a.flags = static_cast<uint32_t*>(flags->data_ptr());
+    a.flags = status_word(*flags);
     pkv_attn_append ap{};
     const bool has_append = p[10] != Py_None;
     const Held append(has_append ? PySequence_Fast(p[10], "append is (k_new, v_new, cos, sin)") : Py_NewRef(Py_None));   // any iterable
@@ -292,6 +302,26 @@ void check_source(const at::Tensor& x) {
     check(x.dim() == 4 && x.size(3) == 128 && x.stride(3) == 1 && half_type(x), "x must be (B, H, S, 128) fp16/bf16 with contiguous channels");
 }
 
+// What the encoder writes behind the `first` tokens that are there: parameters, block table, streams and their lengths.
+// (Blocks that do not fit a stream's capacity are skipped and flagged on the device.)
+void check_tables(int64_t batch, int64_t heads, int64_t tokens, int64_t first, int64_t block, int64_t cb, int64_t mode, bool is_k, const at::Tensor& x,
+                  const at::Tensor& scale, const at::Tensor& zero, const at::Tensor& strm, const at::Tensor& info, const at::Tensor& bytes) {
+    if (mode != PKV_K_CHANNEL && mode != PKV_K_TOKEN) fail(PyExc_RuntimeError, "not supported");
+    check(first >= 0, "first_token must not be negative");
+    const char* const what = "scale / zero must be contiguous tensors of x's dtype with room for all tokens: (B, H, blocks, 128) per channel, (B, tokens) per token";
+    check(scale.dim() >= (mode == PKV_K_CHANNEL ? 3 : 2), what);
+    const int64_t room = scale.size(mode == PKV_K_CHANNEL ? 2 : 1), need = mode == PKV_K_CHANNEL ? first / block + tokens / block : first + tokens;
+    const int64_t rows = mode == PKV_K_CHANNEL ? batch * heads : batch, width = mode == PKV_K_CHANNEL ? 128 : 1;
+    for (const at::Tensor* t : {&scale, &zero})
+        check(t->scalar_type() == x.scalar_type() && t->is_contiguous() && room >= need && t->numel() >= ((rows - 1) * room + need) * width, what);
+    check(strm.dim() == 2 && strm.itemsize() == 1 && strm.stride(1) == 1 && strm.size(0) >= batch, "stream must be (B, capacity) with contiguous bytes");
+    const int64_t entries = (first / cb + tokens / cb) * heads * (is_k ? 1 : 2);
+    check(info.dim() >= 2 && info.itemsize() == 4 && info.is_contiguous() && info.numel() >= 2 * ((batch - 1) * info.size(1) + entries) &&
+              (batch <= 1 || info.size(1) >= entries),
+          "info must be a contiguous (B, blocks, 2) table with room for all blocks");
+    check(bytes.itemsize() == 4 && bytes.is_contiguous() && bytes.numel() >= batch, "stream_bytes must hold a 32-bit count for every sequence");
+}
+
 // which ('k' or 'v'), x, block, rel, mode, bits, cb, scale, zero, stream, info, stream_bytes, flags, first_token,
 // high_precision_zero, scratch (tensor or None: allocated here; False: the library's own), order, order_block
 PyObject* encode_tensor(PyObject* const* p) {
@@ -303,17 +333,19 @@ PyObject* encode_tensor(PyObject* const* p) {
     check_source(x);
     const int64_t block = integer(p[2]), mode = integer(p[4]), cb = integer(p[6]), batch = x.size(0), heads = x.size(1), tokens = x.size(2);
     check(block > 0 && cb > 0 && tokens % block == 0 && tokens % cb == 0, "Tensor shape is not divisible by block size");
+    const bool is_k = which[0] == 'k';
+    check_tables(batch, heads, tokens, integer(p[13]), block, cb, mode, is_k, x, scale, zero, strm, info, bytes);
     pkv_encode_args a{};
     a.x = x.data_ptr(); a.stride_b = x.stride(0); a.stride_h = x.stride(1); a.stride_s = x.stride(2);
     a.scale = scale.data_ptr(); a.zero = zero.data_ptr();
     a.param_blocks = mode == PKV_K_CHANNEL ? extent(scale.size(2)) : 0;
-    a.param_tokens = mode == PKV_K_TOKEN ? extent(scale.size(1)) : 0;
+    a.param_tokens = mode == PKV_K_CHANNEL ? 0 : extent(scale.size(1));
     a.stream = static_cast<uint8_t*>(strm.data_ptr()); a.stream_seq_stride = strm.stride(0); a.capacity = strm.size(1);
     a.block_info = static_cast<uint32_t*>(info.data_ptr()); a.info_seq_stride = info.size(1);
     a.stream_bytes = static_cast<uint32_t*>(bytes.data_ptr());
-    a.flags = static_cast<uint32_t*>(flags.data_ptr());
+    a.flags = status_word(flags);
     a.batch = extent(batch); a.heads = extent(heads); a.tokens = extent(tokens); a.first_token = extent(integer(p[13]));
-    a.qblock = extent(block); a.cb = extent(cb); a.which = which[0] == 'k' ? 0 : 1;
+    a.qblock = extent(block); a.cb = extent(cb); a.which = is_k ? 0 : 1;
     a.bits = extent(integer(p[5])); a.mode = extent(mode); a.high_precision_zero = truth(p[14]); a.is_bf16 = is_bf16(x); a.rel = (float)number(p[3]);
     const char* what = a.which == 0 ? "encode_tensor(k)" : "encode_tensor(v)";
     if (p[15] == Py_False) {
@@ -354,7 +386,7 @@ PyObject* value_median_order(PyObject* const* p) {
     a.x = v.data_ptr(); a.stride_b = v.stride(0); a.stride_h = v.stride(1); a.stride_s = v.stride(2);
     a.batch = extent(v.size(0)); a.heads = extent(v.size(1)); a.tokens = extent(v.size(2)); a.which = 1; a.mode = PKV_K_TOKEN;
     a.is_bf16 = is_bf16(v); a.rel = (float)number(p[2]);
-    a.flags = static_cast<uint32_t*>(flags->data_ptr());
+    a.flags = status_word(*flags);
     const int rows = extent(block);
     check_status(unlocked([&, on = stream()] { return lib.value_order(&a, static_cast<uint8_t*>(order.data_ptr()), rows, on); }), "value_median_order");
     return THPVariable_Wrap(order);
@@ -365,10 +397,11 @@ PyObject* value_median_order(PyObject* const* p) {
 struct Tables {
     at::Tensor cos, sin;
     int64_t stride_b = 0;
-    Tables(const at::Tensor& c, const at::Tensor& s, at::ScalarType dtype, int64_t tokens, int64_t dim, const char* what)
+    Tables(const at::Tensor& c, const at::Tensor& s, at::ScalarType dtype, int64_t batch, int64_t tokens, int64_t dim, const char* what)
         : cos(c.to(dtype).contiguous()), sin(s.to(dtype).contiguous()) {
         check(cos.dim() >= 2 && cos.size(-2) == tokens && cos.size(-1) == dim && sin.sizes() == cos.sizes(), what);
         stride_b = cos.size(0) == 1 ? 0 : tokens * dim;
+        check(stride_b == 0 || cos.numel() >= batch * stride_b, what);
     }
 };
 
@@ -378,14 +411,15 @@ PyObject* append_residual(PyObject* const* p) {
     const at::Tensor *cos = maybe_cuda(p[5], "cos"), *sin = maybe_cuda(p[6], "sin");
     check(k.dim() == 4 && k.size(3) == 128 && v.sizes() == k.sizes() && k.stride(3) == 1 && v.stride(3) == 1,
           "k_new and v_new must be (B, H, T, 128) with contiguous channels");
-    check(kr.dim() == 4 && kr.sizes() == vr.sizes() && kr.strides() == vr.strides() && kr.stride(3) == 1 && kr.stride(2) == 128,
+    check(kr.dim() == 4 && kr.sizes() == vr.sizes() && kr.strides() == vr.strides() && kr.stride(3) == 1 && kr.stride(2) == 128 &&
+              kr.size(0) >= k.size(0) && kr.size(1) >= k.size(1) && kr.size(3) == 128,
           "k_res and v_res must be (B, H, capacity, 128) with contiguous rows and equal strides");
     check(kr.scalar_type() == k.scalar_type() && v.scalar_type() == k.scalar_type() && half_type(k), "dtype mismatch");
     const int64_t T = k.size(2);
     std::unique_ptr<Tables> cs;
     if (cos) {
         check(sin != nullptr, "cos/sin must be (B or 1, T, 128)");
-        cs = std::make_unique<Tables>(*cos, *sin, k.scalar_type(), T, 128, "cos/sin must be (B or 1, T, 128)");
+        cs = std::make_unique<Tables>(*cos, *sin, k.scalar_type(), k.size(0), T, 128, "cos/sin must be (B or 1, T, 128)");
     }
     const int capacity = extent(kr.size(2)), position = extent(integer(p[4])), batch = extent(k.size(0)), heads = extent(k.size(1)), tokens = extent(T);
     check_status(unlocked([&, on = stream()] {
@@ -410,7 +444,7 @@ PyObject* widen_rows(PyObject* const* p) {
           "k_out and v_out must be (B, H, capacity, 128) with contiguous rows and equal strides");
     const int64_t T = k.size(2), D = k.size(3);
     std::unique_ptr<Tables> cs;
-    if (cos) cs = std::make_unique<Tables>(*cos, *sin, k.scalar_type(), T, D, "cos/sin must be (B or 1, T, D)");
+    if (cos) cs = std::make_unique<Tables>(*cos, *sin, k.scalar_type(), k.size(0), T, D, "cos/sin must be (B or 1, T, D)");
     const int capacity = extent(ko.size(2)), position = extent(integer(p[4])), batch = extent(k.size(0)), heads = extent(k.size(1)), tokens = extent(T);
     const bool zero_tail = truth(p[7]);
     check_status(unlocked([&, on = stream()] {
@@ -428,9 +462,12 @@ PyObject* rope(PyObject* const* p) {
     const at::Tensor &x = cuda(p[0], "x"), &cos = cuda(p[1], "cos"), &sin = cuda(p[2], "sin");
     const at::Tensor* out = maybe_cuda(p[3], "out");
     check(x.dim() == 4 && x.stride(3) == 1 && half_type(x), "x must be (B, H, T, D) fp16/bf16 with contiguous channels");
-    const Tables cs(cos, sin, x.scalar_type(), x.size(2), x.size(3), "cos/sin must be (B or 1, T, D)");
+    const Tables cs(cos, sin, x.scalar_type(), x.size(0), x.size(2), x.size(3), "cos/sin must be (B or 1, T, D)");
     at::Tensor own;
     if (!out) { own = at::empty(x.sizes(), x.options()); out = &own; }
+    bool holds = out->dim() == 4 && out->scalar_type() == x.scalar_type() && out->stride(3) == 1;
+    for (int i = 0; i < 4; i++) holds = holds && out->size(i) >= x.size(i);
+    check(holds, "out must be of x's size and dtype with contiguous channels");
     const int batch = extent(x.size(0)), heads = extent(x.size(1)), tokens = extent(x.size(2)), dim = extent(x.size(3));
     check_status(unlocked([&, on = stream()] {
                      return lib.rope(x.data_ptr(), x.stride(0), x.stride(1), x.stride(2), cs.cos.data_ptr(), cs.sin.data_ptr(), cs.stride_b,
