@@ -19,6 +19,8 @@ LIB = os.path.join(PKG, "libpackkv_sm100.so")
 SOURCES = ["pack.cu", "quant.cu", "attn.cu", "legacy.cu", "cache.cu", "dense.cu", "reorder.cu", "fused_encode.cu", "encode_entry.cu", "capi.cu"]
 HOST_SOURCE = os.path.join(CSRC, "host.cpp")
 HOST_LIB = os.path.join(PKG, "_host.so")
+HOST_STAMP = os.path.join(OBJ, "_host.stamp")
+HEADER = os.path.join(os.path.dirname(PKG), "include", "packkv_sm100.h")
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
     "-Xcompiler", "-fPIC", "-Xptxas", "-v",
@@ -51,10 +53,25 @@ def _host_command():
             + [f"-L{lib}", "-ltorch_python", "-ltorch", "-ltorch_cpu", "-lc10_cuda", "-lc10"])
 
 
+def _host_key() -> str:
+    """What _host.so was built with and against: it shares the layout of torch's and CPython's classes."""
+    import sysconfig
+
+    import torch
+    return "\n".join([torch.__version__, str(sysconfig.get_config_var("SOABI"))] + _host_command())
+
+
+def _host_stale() -> bool:
+    if _stale(HOST_LIB, [HOST_SOURCE, HEADER]) or not os.path.exists(HOST_STAMP):
+        return True
+    with open(HOST_STAMP) as f:
+        return f.read() != _host_key()
+
+
 def build(force: bool = False, verbose: bool = False) -> str:
     os.makedirs(OBJ, exist_ok=True)
     headers = [os.path.join(CSRC, f) for f in os.listdir(CSRC) if f.endswith((".cuh", ".h"))]
-    headers.append(os.path.join(os.path.dirname(PKG), "include", "packkv_sm100.h"))
+    headers.append(HEADER)
     jobs = []
     for src in SOURCES:
         s = os.path.join(CSRC, src)
@@ -67,6 +84,8 @@ def build(force: bool = False, verbose: bool = False) -> str:
             r = subprocess.run(_host_command(), capture_output=True, text=True)
             if r.returncode != 0:
                 raise RuntimeError(f"g++ failed for {HOST_SOURCE}:\n{r.stdout}\n{r.stderr}")
+            with open(HOST_STAMP, "w") as f:
+                f.write(_host_key())
             return
         s, o = job
         r = subprocess.run([_nvcc()] + NVCC_FLAGS + ["-c", s, "-o", o], capture_output=True, text=True)
@@ -77,7 +96,7 @@ def build(force: bool = False, verbose: bool = False) -> str:
         if verbose:
             print(r.stderr)
 
-    host = [None] if force or _stale(HOST_LIB, [HOST_SOURCE, headers[-1]]) else []
+    host = [None] if force or _host_stale() else []
     with ThreadPoolExecutor(max_workers=8) as pool:
         list(pool.map(compile_one, jobs + host))
     objs = [os.path.join(OBJ, s.replace(".cu", ".o")) for s in SOURCES]
