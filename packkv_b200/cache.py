@@ -73,6 +73,11 @@ class _Layer:
 
 
 class PackKVCache(_HFCache):
+    """Compressed K and V of a model's layers behind the reference's update() / get_seq_length() (packkv_cache.py:22-38).
+
+    The buffers of a layer are the cache's own: a residual that overflows continues in new buffers, and a store that is full
+    in a larger one, so an address read from outside is good until the next update()."""
+
     def __init__(self, batch_size, head_num, head_dim, layer_num, materialize: bool = False, decode_handles: bool = False):
         if _HFCache is not object:
             try:
@@ -220,8 +225,6 @@ class PackKVCache(_HFCache):
             L.pending = (key_states, value_states, cos, sin)
             L.n_res = total
             return self._step_result(layer_idx, T)
-        if cos is not None and (cos.dim() < 2 or cos.shape[-2] != T or sin.shape != cos.shape):
-            raise ValueError("cos/sin must be (B or 1, T, D)")      # parts of longer tables would rotate by other positions
         if key_states.stride(3) != 1 or value_states.stride(3) != 1:
             key_states, value_states = key_states.contiguous(), value_states.contiguous()
         if value_states.dtype != key_states.dtype:
@@ -239,6 +242,8 @@ class PackKVCache(_HFCache):
         elif L.n_res == 0:
             # the first tokens: what is packed goes through the rotation (and the widening) once, what stays behind
             # straight into the residual
+            if cos is not None and (cos.dim() < 2 or cos.shape[-2] != T or sin.shape != cos.shape):
+                raise ValueError("cos/sin must be (B or 1, T, D)")      # parts of longer tables would rotate by other positions
             k_head, v_head = key_states[:, :, :n_c], value_states[:, :, :n_c]
             if D != 128:
                 k_wide, v_wide = (key_states.new_empty(B, H, n_c, 128) for _ in range(2))

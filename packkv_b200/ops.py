@@ -231,13 +231,14 @@ def _check_layer_shapes(L: "CompressedLayer", batch: int) -> None:
         raise ValueError("token-mode k_scale / k_zero must be (B, >= n_comp)")
     if L.k_stream.dim() != 2 or L.v_stream.dim() != 2 or L.k_stream.stride(1) != 1 or L.v_stream.stride(1) != 1:
         raise ValueError("streams must be (B, capacity) with contiguous bytes")
-    _check_order(L, batch)
+    if L.order is not None:
+        _check_order(L, batch)
 
 
 def _check_order(L: "CompressedLayer", batch: int) -> None:
     """One byte for every packed token.  The values are looked at on the device (dense.cu): reading them here would synchronise."""
-    if L.order is not None and (L.order.dtype != torch.uint8 or L.order.dim() != 3 or L.order.shape[0] != batch
-                                or L.order.shape[1] * L.order.shape[2] != L.n_comp or not L.order.is_contiguous()):
+    order, shape = L.order, L.order.shape
+    if order.dtype is not torch.uint8 or len(shape) != 3 or shape[0] != batch or shape[1] * shape[2] != L.n_comp or not order.is_contiguous():
         raise ValueError("order must be a contiguous (B, n_comp / block, block) uint8 tensor")
 
 
@@ -337,9 +338,12 @@ def dense(which: str, layer: CompressedLayer, res: Optional[torch.Tensor], n_res
     pb, pt = _param_extents(scale, mode)
     if (mode == K_CHANNEL and n % block) or n % cb or info.dim() != 3 or info.shape[1] < (n // cb) * H * (1 if which == "k" else 2) or not info.is_contiguous() \
             or stream.dim() != 2 or stream.stride(1) != 1 or (pb < n // block if mode == K_CHANNEL else pt < n) \
-            or not scale.is_contiguous() or not zero.is_contiguous() or zero.shape != scale.shape or any(t.shape[0] != B for t in (info, scale)):
+            or not scale.is_contiguous() or not zero.is_contiguous() or zero.shape != scale.shape or info.shape[0] != B or scale.shape[0] != B:
         raise ValueError("dense: the layer's tables do not cover its tokens")
-    _check_order(layer, B)
+    order_block = block
+    if layer.order is not None:
+        _check_order(layer, B)
+        order_block = layer.order.shape[2]
     if n_res and (res.dim() != 4 or res.shape[:2] != (B, H) or res.shape[2] < n_res or res.shape[3] != 128 or res.stride(3) != 1 or res.stride(2) != 128
                   or res.dtype != scale.dtype):
         raise ValueError("dense: the residual must be (B, H, >= n_res, 128) rows of the layer's element type")
@@ -347,7 +351,7 @@ def dense(which: str, layer: CompressedLayer, res: Optional[torch.Tensor], n_res
     a = _lib.DenseArgs(stream.data_ptr(), stream.stride(0), stream.shape[1], info.data_ptr(), info.shape[1], scale.data_ptr(), zero.data_ptr(), pb, pt,
                        None if layer.order is None else layer.order.data_ptr(), n, res.data_ptr() if n_res else None,
                        res.stride(0) if n_res else 0, res.stride(1) if n_res else 0, out.data_ptr(), out.stride(0), out.stride(1), out.stride(2),
-                       flags.data_ptr(), B, H, dim, n, n_res, block if layer.order is None else layer.order.shape[2], block, cb, 0 if which == "k" else 1,
+                       flags.data_ptr(), B, H, dim, n, n_res, order_block, block, cb, 0 if which == "k" else 1,
                        layer.bits_k if which == "k" else layer.bits_v, mode, int(layer.high_precision_zero), int(scale.dtype == torch.bfloat16))
     _lib.check(_lib.lib().pkv_dense(ctypes.byref(a), _stream_ptr()), "dense")
     return out
