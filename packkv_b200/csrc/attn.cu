@@ -55,7 +55,6 @@ constexpr int kAW = PKV_ATTN_WARPS;   // warps per CTA (1, 2 or 4)
 #endif
 constexpr int kMaxCtasPerSm = PKV_ATTN_CTAS;  // register budget: 65536 / (128 * 4) -> 128 per thread, 96 for 5
 constexpr int kD = 128;           // head dimension
-constexpr int kSmCount = 148;
 constexpr unsigned kWaitSpins = 1u << 22;   // bounded mbarrier wait (each try suspends for a while by itself)
 #ifndef PKV_ATTN_CTAS_SCORES
 #define PKV_ATTN_CTAS_SCORES PKV_ATTN_CTAS   // the two-launch form's kernels may take other register budgets
@@ -1561,8 +1560,11 @@ int launch_attention(const AttnArgs& a, const AttnExchange* xch, const AttnAppen
         const long waves = (ctas + slots - 1) / slots;
         const long on_gpu = ctas < slots ? ctas : slots;
         const int sm_warps = (int)((on_gpu + kSmCount - 1) / kSmCount) * kAW;
-        // On a busy SM it makes no difference who holds the residual tiles; on an idle one it is the longest warp's time
-        // (counted for clusters that place well), and so are the hand-over and the second start of two launches.
+        // On a busy SM it makes no difference who holds the residual tiles; on an idle one it is the longest warp's time,
+        // and so are the hand-over and the second start of two launches.  Powers of two only: that, like the 6 % of a team
+        // below, is fitted to short launches, where 4, 8 and 16 CTAs to a cluster beat their neighbours by up to 2 us
+        // (one sequence x 700 tokens, 8 KV heads, us for 3..16: 19.0 14.2 14.9 15.1 14.2 12.4 13.6 14.3 14.9 13.8 14.6 15.5
+        // 15.8 13.8; two x 825: 19.5 17.1 15.2 15.5 16.1 13.2 14.4 15.5 16.0 15.0 15.9 17.2 17.6 15.5).
         const bool idle = sm_warps <= 8;
         const double upw_max = team || (idle && !(cl & (cl - 1))) ? upw_placed : upw_dealt;
         if (idle && launches == 2) fixed += 1.0;
@@ -1575,7 +1577,7 @@ int launch_attention(const AttnArgs& a, const AttnExchange* xch, const AttnAppen
         if (ns == 1) cost *= 1.02;                              // the copy of the next block is not overlapped (it comes from L2)
         if (cl > 8) cost *= 2 * ctas > slots ? 1.4 : 1.1;
         if (team && sm_warps > 8) cost *= 1.15;                 // a team's extra instructions count once the SM is busy (11 x 2154, 2 bits: 39 us against 35)
-        if (team && (cl & (cl - 1))) cost *= 1.06;              // short launches: clusters of 3..11 cost 1 to 2 us more than 4 or 8
+        if (team && (cl & (cl - 1))) cost *= 1.06;
         return cost;
     };
     // Units of the longest warp.  Compressed tiles are dealt from the first owner (warp, or CTA of a team) on, residual

@@ -3,8 +3,8 @@
 //                 apply_rotary_pos_emb_single (utils/compute.py:22-43): (t*cos) + (rotate_half(t)*sin), each op
 //                 rounded to the element type; V copied.  One launch.
 //   dequantize  : codes + scale/zero -> dense K or V exactly as the reference's cache does it,
-//                 (code + zero) * scale or code * scale + min (utils/compute.py:173-178); used when a
-//                 caller asks for the dense history (prefill attention, debugging).
+//                 (code + zero) * scale or code * scale + min (utils/compute.py:173-178), for codes of any
+//                 quantisation mode; a packed layer goes through dense.cu instead.
 #include "common.cuh"
 #include "launch.h"
 
@@ -133,7 +133,7 @@ int launch_rows(const RowsArgs& r, cudaStream_t st) {
     const int64_t chunks = (int64_t)r.batch * r.tokens * (r.dim / 16);
     if (!(at & 15) && !(strides & 7) && r.dim % 16 == 0 && r.width % 8 == 0 && chunks * r.heads < (1LL << 31)) {
         // four heads to a thread once that still gives every SM 1024 threads
-        const int hpt = chunks * r.heads >= 4LL * 148 * 1024 ? 4 : 1;
+        const int hpt = chunks * r.heads >= 4LL * kSmCount * 1024 ? 4 : 1;
         const unsigned items = (unsigned)(chunks * ((r.heads + hpt - 1) / hpt));
         if (r.is_bf16) rows_kernel<__nv_bfloat16><<<(items + 255) / 256, 256, 0, st>>>(r, hpt, items);
         else rows_kernel<__half><<<(items + 255) / 256, 256, 0, st>>>(r, hpt, items);

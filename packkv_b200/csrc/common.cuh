@@ -16,6 +16,7 @@ namespace pkv {
 
 constexpr int kPackTokens = 16;
 constexpr int kLanes = 32;
+constexpr int kSmCount = 148;
 
 // status codes returned by the C ABI and OR-ed bit flags written to the device status word
 enum Status : int {

@@ -1049,7 +1049,7 @@ static int launch_fused_t(const FusedEncodeRequest& r, uint8_t* slots, const uin
         bound16 = (g.head_bytes + g.nseg * (g.min_bytes + g.len_bytes + 32 * g.ppt * 2 * BITS) + 15) & ~15;
         a.slot_stride = bound16;
         blocks_per_seq = nctx * 2 * r.heads;
-        const int nw = 2 * r.heads > 8 && (int64_t)nctx * r.batch <= 148 ? 16 : 8;
+        const int nw = 2 * r.heads > 8 && (int64_t)nctx * r.batch <= kSmCount ? 16 : 8;
         const int smem = 32 * r.cb + nw * (r.cb * 64 + (direct ? v_slots(r.heads, nw) : 1) * bound16) + r.cb + 16;
         auto launch_v = [&](auto kern) {
             if (opt_in_smem(kern, smem)) return (int)kCudaError;
