@@ -46,6 +46,19 @@ def test_argument_blocks_match_the_header_layout():
         assert fields == [n for n, _ in ctype._fields_], cname
 
 
+def test_dense_block_matches_the_header_layout():
+    with open(os.path.join(ROOT, "include", "packkv_sm100.h")) as f:
+        body = re.search(r"typedef struct pkv_dense_args \{(.*?)\} pkv_dense_args", f.read(), re.S).group(1)
+    types = {"const uint8_t*": _lib._p, "const uint32_t*": _lib._p, "uint32_t*": _lib._p, "const void*": _lib._p, "void*": _lib._p,
+             "int64_t": _lib._i64, "int32_t": _lib._i32}
+    want = []
+    for decl in re.sub(r"/\*.*?\*/", "", body, flags=re.S).split(";"):
+        if decl.strip():
+            kind, names = re.match(r"\s*((?:const )?\w+\*?) (.*)", decl, re.S).groups()
+            want += [(name.strip(), types[kind]) for name in names.split(",")]
+    assert want == list(_lib.DenseArgs._fields_)
+
+
 def test_missing_library_fails_loudly(monkeypatch):
     monkeypatch.setattr(_lib, "_lib", None)
     monkeypatch.setattr(_lib, "LIB_PATH", "/nonexistent/libpackkv_sm100.so")
