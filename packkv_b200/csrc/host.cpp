@@ -104,7 +104,7 @@ int extent(int64_t v) {
 }
 // the device status word
 uint32_t* status_word(const at::Tensor& flags) {
-    check(flags.itemsize() == 4 && flags.numel() >= 1, "flags must hold a 32-bit word (new_flags)");
+    check(flags.nbytes() >= 4 && reinterpret_cast<uintptr_t>(flags.data_ptr()) % 4 == 0, "flags must hold a 32-bit word (new_flags)");
     return static_cast<uint32_t*>(flags.data_ptr());
 }
 bool half_type(const at::Tensor& t) { return t.scalar_type() == at::kHalf || t.scalar_type() == at::kBFloat16; }
@@ -319,7 +319,7 @@ void check_tables(int64_t batch, int64_t heads, int64_t tokens, int64_t first, i
     check(info.dim() >= 2 && info.itemsize() == 4 && info.is_contiguous() && info.numel() >= 2 * ((batch - 1) * info.size(1) + entries) &&
               (batch <= 1 || info.size(1) >= entries),
           "info must be a contiguous (B, blocks, 2) table with room for all blocks");
-    check(bytes.itemsize() == 4 && bytes.is_contiguous() && bytes.numel() >= batch, "stream_bytes must hold a 32-bit count for every sequence");
+    check((bytes.itemsize() == 4 || (batch <= 1 && bytes.itemsize() > 4)) && bytes.is_contiguous() && bytes.numel() >= batch, "stream_bytes must hold a 32-bit count for every sequence");
 }
 
 // which ('k' or 'v'), x, block, rel, mode, bits, cb, scale, zero, stream, info, stream_bytes, flags, first_token,

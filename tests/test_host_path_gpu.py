@@ -72,7 +72,7 @@ def test_attention_checks_what_the_kernel_indexes(stubbed):
     _accepted_and_refused(
         call,
         [dict(), dict(k=big, v=big), dict(k=big[:B, :H], v=big[:B, :H]), dict(out=torch.empty_like(q)), dict(out=_empty(B, 1, H * G * 128)),
-         dict(flags=_empty(2, dtype=torch.int32))],
+         dict(flags=_empty(2, dtype=torch.int32)), dict(flags=_empty(1, dtype=torch.int64))],
         [dict(n_res=R + 1),                                                   # more rows than the residual has
          dict(k=res[: B - 1], v=res[: B - 1]), dict(k=res[:, : H - 1], v=res[:, : H - 1]),
          dict(v=res[:1]), dict(v=res[:, :1]), dict(v=res[:, :, : R - 1]),     # V with K's strides, not its sizes
