@@ -444,6 +444,16 @@ int32_t pkv_attention_plan(const pkv_attn_args* args_host, pkv_attn_plan* plan_i
                            int32_t with_exchange);
 
 /*
+ * The same step for heads of head_dim channels, 64 <= head_dim < 128, a multiple of 8, whose stored rows are widened to 128
+ * channels, the tail repeating the row's first 128 - head_dim (pkv_widen_rows).  q is (batch, q heads, head_dim); the new
+ * token's rows and cos / sin have head_dim channels, any alignment, and are widened as they are written into the residual.
+ * out is (batch, q heads, 128): the first head_dim channels of a row are the head's, the rest repeat.
+ * append_host and scratch may be NULL.
+ */
+int32_t pkv_decode_attention_narrow(const pkv_attn_args* args_host, const pkv_attn_append* append_host, int32_t head_dim,
+                                    void* scratch, int64_t scratch_bytes, void* cuda_stream);
+
+/*
  * Set-up helpers of the exchange; the only entry points that allocate or touch address-space mappings (they
  * synchronise, call them once, outside the decode loop).  pkv_exchange_alloc returns `bytes` of zeroed device
  * memory on the current device (its own cudaMalloc, so that it can be exported) and the 64-byte

@@ -105,6 +105,7 @@ SIGNATURES = {
     "pkv_decode_attention_append": (_i32, [ctypes.POINTER(AttnArgs), ctypes.POINTER(AttnAppend), ctypes.POINTER(AttnExchange), _p]),
     "pkv_decode_attention_split": (_i32, [ctypes.POINTER(AttnArgs), ctypes.POINTER(AttnAppend), ctypes.POINTER(AttnExchange), ctypes.POINTER(AttnPlan),
                                           _p, _i64, _p]),
+    "pkv_decode_attention_narrow": (_i32, [ctypes.POINTER(AttnArgs), ctypes.POINTER(AttnAppend), _i32, _p, _i64, _p]),
     "pkv_attention_plan": (_i32, [ctypes.POINTER(AttnArgs), ctypes.POINTER(AttnPlan), _i64, _i32]),
     "pkv_exchange_wait": (_i32, [_p, _i32, ctypes.c_uint32, ctypes.c_uint32, _p, _p]),
     "pkv_exchange_wait_consume": (_i32, [_p, _i32, ctypes.c_uint32, ctypes.c_uint32, _p, _p]),
@@ -146,7 +147,7 @@ def lib() -> ctypes.CDLL:
 # the library functions of csrc/host.cpp, in the order of its struct Library
 _HOST_FUNCTIONS = ("pkv_decode_attention", "pkv_decode_attention_append", "pkv_decode_attention_exchange", "pkv_decode_attention_split",
                    "pkv_attention_plan", "pkv_encode_tensor", "pkv_encode_tensor_ordered", "pkv_encode_tensor_static", "pkv_value_median_order",
-                   "pkv_append_residual", "pkv_rope", "pkv_widen_rows")
+                   "pkv_append_residual", "pkv_rope", "pkv_widen_rows", "pkv_decode_attention_narrow")
 
 
 def host():

@@ -256,6 +256,7 @@ struct AttnDev {
     int nslots;          // staging slots per warp: 2 = the next block is copied while this one is unpacked
     int team;            // single launch: the warps of a CTA share its tiles (see TEAM)
     int early;           // single launch that may start while the one before drains (launch_attention)
+    int dim;             // channels of q's rows and of the new token's: 128, or a narrow head's 64 .. 120 (the stored rows repeat their first ones behind them)
     int vpair;           // 64-token V blocks: an item is the pair of blocks of one token block (both channel halves)
     int kbound, vbound;  // largest legal block size in bytes
     int prow;            // bytes of one row of the score / probability tile
@@ -543,10 +544,11 @@ __global__ void __launch_bounds__(kAW * 32, PASS == 1 ? PKV_ATTN_CTAS_SCORES : P
     unsigned qf[4][2][2];
     {
         const uint4* qp = reinterpret_cast<const uint4*>(
-            reinterpret_cast<const T*>(a.q) + ((int64_t)(b * q_heads + h * G + min(g, G - 1))) * kD + 8 * c);
+            reinterpret_cast<const T*>(a.q) + ((int64_t)(b * q_heads + h * G + min(g, G - 1))) * P.dim + 8 * c);
 #pragma unroll
         for (int m = 0; m < 4; m++) {
-            const uint4 v = g < G ? __ldg(qp + 4 * m) : make_uint4(0, 0, 0, 0);
+            // the repeated channels behind a narrow head's own add nothing to its scores: q is 0 there
+            const uint4 v = g < G && 32 * m + 8 * c < P.dim ? __ldg(qp + 4 * m) : make_uint4(0, 0, 0, 0);
             unsigned f0[2], f1[2];
             pair_shuffle(v, f0, f1);
             qf[0][m >> 1][m & 1] = f0[0]; qf[1][m >> 1][m & 1] = f0[1];
@@ -726,7 +728,32 @@ __global__ void __launch_bounds__(kAW * 32, PASS == 1 ? PKV_ATTN_CTAS_SCORES : P
     if (P.ap.new_k != nullptr && my_rt > 0) {
         const int tn = a.n_res - 1, tile_n = tn >> 4;
         if (tile_n % n_warps == rslot) {
-            if (lane < 16) {
+            if (P.dim != kD) {
+                // A narrow head's row, widened as rows_kernel does it: channels dim .. 127 repeat the first ones.  One channel at a
+                // time (any alignment, any even dim), all loads in flight together.
+                const T* x = reinterpret_cast<const T*>(P.ap.new_k) + (int64_t)b * P.ap.k_stride_b + (int64_t)h * P.ap.k_stride_h;
+                const T* y = reinterpret_cast<const T*>(P.ap.new_v) + (int64_t)b * P.ap.v_stride_b + (int64_t)h * P.ap.v_stride_h;
+                const T* cs = reinterpret_cast<const T*>(P.ap.cos) + (int64_t)b * P.ap.cs_stride_b;
+                const T* sn = reinterpret_cast<const T*>(P.ap.sin) + (int64_t)b * P.ap.cs_stride_b;
+                const int half = P.dim >> 1;
+                T kv[4], vv[4];
+#pragma unroll
+                for (int i = 0; i < 4; i++) {
+                    const int w = lane + 32 * i, d = w < P.dim ? w : w - P.dim;
+                    kv[i] = x[d]; vv[i] = y[d];
+                    if (P.ap.cos != nullptr) {
+                        const float rot = d < half ? -Tr<T>::to_float(x[d + half]) : Tr<T>::to_float(x[d - half]);
+                        const float a0 = Tr<T>::round(Tr<T>::to_float(kv[i]) * Tr<T>::to_float(cs[d]));
+                        const float c0 = Tr<T>::round(rot * Tr<T>::to_float(sn[d]));
+                        kv[i] = Tr<T>::from_float(a0 + c0);
+                    }
+                }
+#pragma unroll
+                for (int i = 0; i < 4; i++) {
+                    const_cast<T*>(kres)[(int64_t)tn * kD + lane + 32 * i] = kv[i];
+                    const_cast<T*>(vres)[(int64_t)tn * kD + lane + 32 * i] = vv[i];
+                }
+            } else if (lane < 16) {
                 const T* x = reinterpret_cast<const T*>(P.ap.new_k) + (int64_t)b * P.ap.k_stride_b + (int64_t)h * P.ap.k_stride_h;
                 const int d0 = 8 * lane;
                 uint4 xv = *reinterpret_cast<const uint4*>(x + d0);
@@ -760,10 +787,10 @@ __global__ void __launch_bounds__(kAW * 32, PASS == 1 ? PKV_ATTN_CTAS_SCORES : P
     if (my_rt > 0) {
         unsigned qr[8][2];
         const uint4* qp = reinterpret_cast<const uint4*>(
-            reinterpret_cast<const T*>(a.q) + ((int64_t)(b * q_heads + h * G + min(g, G - 1))) * kD + 8 * c);
+            reinterpret_cast<const T*>(a.q) + ((int64_t)(b * q_heads + h * G + min(g, G - 1))) * P.dim + 8 * c);
 #pragma unroll
         for (int m = 0; m < 4; m++) {
-            const uint4 v = g < G ? __ldg(qp + 4 * m) : make_uint4(0, 0, 0, 0);
+            const uint4 v = g < G && 32 * m + 8 * c < P.dim ? __ldg(qp + 4 * m) : make_uint4(0, 0, 0, 0);
             pair_shuffle(v, qr[2 * m], qr[2 * m + 1]);
         }
         for (int k = 0; k < my_rt; k++) {
@@ -1465,7 +1492,8 @@ int launch_exchange_wait(uint32_t* arrivals, int n_ranks, unsigned expected, uns
 
 // plan_io: in: cluster / nsplit / launches to force (0 = choose); out: what was chosen.  dry_run: plan only.
 int launch_attention(const AttnArgs& a, const AttnExchange* xch, const AttnAppend* ap, AttnPlan* plan_io, void* scratch, int64_t scratch_bytes,
-                     bool dry_run, cudaStream_t st) {
+                     bool dry_run, cudaStream_t st, int head_dim) {
+    if (head_dim < kD / 2 || head_dim > kD || head_dim % 8) return kUnsupported;
     if (a.batch <= 0 || a.kv_heads <= 0 || a.group < 1 || a.group > 8) return a.group > 8 ? kUnsupported : kBadArgument;
     if (a.n_comp < 0 || a.n_res < 0 || a.n_comp + a.n_res == 0) return kBadArgument;
     if (!a.q || !a.out || !a.flags) return kBadArgument;
@@ -1494,11 +1522,12 @@ int launch_attention(const AttnArgs& a, const AttnExchange* xch, const AttnAppen
     AttnDev P{};
     P.extra = -1;
     P.a = a;
+    P.dim = head_dim;
     if (ap) {
         if (!ap->new_k || !ap->new_v || a.n_res < 1 || a.n_res > ap->res_capacity || ((ap->cos == nullptr) != (ap->sin == nullptr))) return kBadArgument;
-        if ((reinterpret_cast<uintptr_t>(ap->new_k) & 15) || (reinterpret_cast<uintptr_t>(ap->new_v) & 15) || (ap->k_stride_b & 7) || (ap->k_stride_h & 7) ||
+        if (head_dim == kD && ((reinterpret_cast<uintptr_t>(ap->new_k) & 15) || (reinterpret_cast<uintptr_t>(ap->new_v) & 15) || (ap->k_stride_b & 7) || (ap->k_stride_h & 7) ||
             (ap->v_stride_b & 7) || (ap->v_stride_h & 7) || (reinterpret_cast<uintptr_t>(ap->cos) & 15) || (reinterpret_cast<uintptr_t>(ap->sin) & 15) ||
-            (ap->cs_stride_b & 7))
+            (ap->cs_stride_b & 7)))
             return kBadArgument;
         P.ap = *ap;
     }

@@ -187,6 +187,12 @@ int32_t pkv_decode_attention_split(const pkv_attn_args* args_host, const pkv_att
     return launch_attention(*args_host, exchange_host, append_host, plan_io, scratch, scratch_bytes, false, static_cast<cudaStream_t>(cuda_stream));
 }
 
+int32_t pkv_decode_attention_narrow(const pkv_attn_args* args_host, const pkv_attn_append* append_host, int32_t head_dim, void* scratch,
+                                    int64_t scratch_bytes, void* cuda_stream) {
+    if (!args_host) return kBadArgument;
+    return launch_attention(*args_host, nullptr, append_host, nullptr, scratch, scratch_bytes, false, static_cast<cudaStream_t>(cuda_stream), head_dim);
+}
+
 int32_t pkv_attention_plan(const pkv_attn_args* args_host, pkv_attn_plan* plan_io, int64_t scratch_bytes, int32_t with_exchange) {
     if (!args_host || !plan_io) return kBadArgument;
     // the plan depends on sizes only: any non-null, aligned address stands for the scratch, and a block that is never

@@ -40,6 +40,7 @@ struct Library {
     decltype(&pkv_append_residual) append;
     decltype(&pkv_rope) rope;
     decltype(&pkv_widen_rows) widen;
+    decltype(&pkv_decode_attention_narrow) attention_narrow;
 } lib{};
 
 // thrown once a Python exception is set
@@ -194,33 +195,37 @@ void fill_layer(PyObject* layer, const at::Tensor& q, int64_t batch, int64_t n_c
     a.k_mode = extent(mode); a.high_precision_zero = truth(h_hp.o);
 }
 
-void fill_append(PyObject* append, const at::Tensor& q, const at::Tensor& k_res, int64_t batch, int64_t kv_heads, int64_t n_res, pkv_attn_append& ap) {
+void fill_append(PyObject* append, const at::Tensor& q, const at::Tensor& k_res, int64_t batch, int64_t kv_heads, int64_t n_res, int64_t dim, pkv_attn_append& ap) {
     check(PySequence_Fast_GET_SIZE(append) == 4, "append is (k_new, v_new, cos, sin)");
     PyObject** it = PySequence_Fast_ITEMS(append);
     const at::Tensor &k = cuda(it[0], "k_new"), &v = cuda(it[1], "v_new");
     const at::Tensor *cos = maybe_cuda(it[2], "cos"), *sin = maybe_cuda(it[3], "sin");
-    check(n_res >= 1 && k.dim() == 4 && k.size(0) == batch && k.size(1) == kv_heads && k.size(2) == 1 && k.size(3) == 128 && v.sizes() == k.sizes() &&
+    check(n_res >= 1 && k.dim() == 4 && k.size(0) == batch && k.size(1) == kv_heads && k.size(2) == 1 && k.size(3) == dim && v.sizes() == k.sizes() &&
               k.stride(3) == 1 && v.stride(3) == 1 && k.scalar_type() == q.scalar_type() && v.scalar_type() == q.scalar_type(),
           "append needs k_new / v_new of shape (B, Hkv, 1, 128) in q's dtype with contiguous channels");
     ap.new_k = k.data_ptr(); ap.new_v = v.data_ptr();
     ap.k_stride_b = k.stride(0); ap.k_stride_h = k.stride(1); ap.v_stride_b = v.stride(0); ap.v_stride_h = v.stride(1);
     if (cos) {
         check(sin && cos->scalar_type() == q.scalar_type() && sin->scalar_type() == q.scalar_type() && cos->dim() >= 2 && cos->size(-2) == 1 &&
-                  cos->size(-1) == 128 && sin->sizes() == cos->sizes() && cos->is_contiguous() && sin->is_contiguous(),
+                  cos->size(-1) == dim && sin->sizes() == cos->sizes() && cos->is_contiguous() && sin->is_contiguous(),
               "cos / sin must be contiguous (B or 1, 1, 128) tensors of q's dtype");
-        ap.cos = cos->data_ptr(); ap.sin = sin->data_ptr(); ap.cs_stride_b = cos->size(0) == 1 ? 0 : 128;
-        check(ap.cs_stride_b == 0 || cos->numel() >= batch * 128, "cos / sin must be contiguous (B or 1, 1, 128) tensors of q's dtype");
+        ap.cos = cos->data_ptr(); ap.sin = sin->data_ptr(); ap.cs_stride_b = cos->size(0) == 1 ? 0 : dim;
+        check(ap.cs_stride_b == 0 || cos->numel() >= batch * dim, "cos / sin must be contiguous (B or 1, 1, 128) tensors of q's dtype");
     }
     ap.res_capacity = extent(k_res.size(2));
 }
 
 // q, layer, k_res, v_res, n_res, scaling, out, flags, kv_heads, exchange (address of its block), append, scratch, plan, plan_only
-PyObject* decode_attention(PyObject* const* p) {
+// NARROW: q and the appended rows have 64 .. 120 channels; no exchange, plan or out
+template <bool NARROW> PyObject* decode_attention_of(PyObject* const* p) {
     const at::Tensor& q = cuda(p[0], "q");
     const at::Tensor *k_res = maybe_cuda(p[2], "k_res"), *v_res = maybe_cuda(p[3], "v_res");
     const at::Tensor *out = maybe_cuda(p[6], "out"), *flags = maybe_cuda(p[7], "flags"), *scratch = maybe_cuda(p[11], "scratch");
     const int64_t n_res = integer(p[4]);
-    check(q.dim() == 3 && q.size(2) == 128 && q.is_contiguous(), "q must be a contiguous (B, Hq, 128) tensor");
+    if (NARROW)
+        check(q.dim() == 3 && q.size(2) >= 64 && q.size(2) < 128 && q.size(2) % 8 == 0 && q.is_contiguous(), "q must be a contiguous (B, Hq, 64 .. 120) tensor");
+    else
+        check(q.dim() == 3 && q.size(2) == 128 && q.is_contiguous(), "q must be a contiguous (B, Hq, 128) tensor");
     check(half_type(q), "q must be fp16 or bf16");
     const int64_t batch = q.size(0), q_heads = q.size(1);
     int64_t n_comp = 0, kv_heads;
@@ -236,7 +241,7 @@ PyObject* decode_attention(PyObject* const* p) {
     }
     check(kv_heads > 0 && q_heads % kv_heads == 0, "q heads must be a multiple of kv heads");
     at::Tensor own_out, own_flags;
-    if (!out) { own_out = at::empty_like(q); out = &own_out; }
+    if (!out) { own_out = NARROW ? at::empty({batch, q_heads, 128}, q.options()) : at::empty_like(q); out = &own_out; }
     if (!flags) { own_flags = new_flags(q); flags = &own_flags; }
     check(out->scalar_type() == q.scalar_type() && out->is_contiguous() && out->numel() >= q.numel(), "out must be contiguous, of q's dtype and size");
     pkv_attn_args a{};
@@ -262,12 +267,20 @@ PyObject* decode_attention(PyObject* const* p) {
     const Held append(has_append ? PySequence_Fast(p[10], "append is (k_new, v_new, cos, sin)") : Py_NewRef(Py_None));   // any iterable
     if (has_append) {
         check(n_res >= 1 && k_res, "append needs k_new / v_new of shape (B, Hkv, 1, 128) in q's dtype with contiguous channels");
-        fill_append(append.o, q, *k_res, batch, kv_heads, n_res, ap);
+        fill_append(append.o, q, *k_res, batch, kv_heads, n_res, q.size(2), ap);
     }
     const pkv_attn_exchange* xch = p[9] == Py_None ? nullptr : reinterpret_cast<const pkv_attn_exchange*>(integer(p[9]));
     const bool plan_only = truth(p[13]);
     int32_t st;
-    if (scratch || p[12] != Py_None || plan_only) {
+    if (NARROW) {
+        if (scratch)
+            check(scratch->scalar_type() == at::kByte && scratch->is_contiguous() && reinterpret_cast<uintptr_t>(scratch->data_ptr()) % 256 == 0,
+                  "scratch must be a contiguous uint8 tensor aligned to 256 bytes (new_attention_scratch)");
+        st = unlocked([&, on = stream()] {
+            return lib.attention_narrow(&a, has_append ? &ap : nullptr, (int32_t)q.size(2), scratch ? scratch->data_ptr() : nullptr,
+                                        scratch ? scratch->numel() : 0, on);
+        });
+    } else if (scratch || p[12] != Py_None || plan_only) {
         pkv_attn_plan plan{};
         if (p[12] != Py_None) {
             const Held seq(PySequence_Fast(p[12], "plan is (cluster, nsplit, launches[, extra])"));
@@ -295,6 +308,14 @@ PyObject* decode_attention(PyObject* const* p) {
     check_status(st, "decode_attention");
     if (p[6] != Py_None) return Py_NewRef(p[6]);
     return THPVariable_Wrap(own_out);
+}
+
+PyObject* decode_attention(PyObject* const* p) { return decode_attention_of<false>(p); }
+
+// q, layer, k_res, v_res, n_res, scaling, flags, kv_heads, append, scratch
+PyObject* decode_attention_narrow(PyObject* const* p) {
+    PyObject* const all[14] = {p[0], p[1], p[2], p[3], p[4], p[5], Py_None, p[6], p[7], Py_None, p[8], p[9], Py_None, Py_False};
+    return decode_attention_of<true>(all);
 }
 
 // ---- encoder ------------------------------------------------------------------------------------------------------------
@@ -519,6 +540,7 @@ PyObject* bind(PyObject*, PyObject* const* args, Py_ssize_t n) {
 PyMethodDef methods[] = {
     {"bind", (PyCFunction)(void (*)(void))bind, METH_FASTCALL, "addresses of the library's functions"},
     FAST(decode_attention, 14, "ops.decode_attention"),
+    FAST(decode_attention_narrow, 10, "ops.decode_attention for heads of 64 .. 120 channels"),
     FAST(encode_tensor, 18, "ops.encode_tensor / ops.encode_tensor_static"),
     FAST(value_median_order, 4, "ops.value_median_order"),
     FAST(append_residual, 7, "ops.append_residual"),

@@ -6,7 +6,7 @@ import torch
 
 from oracle import quant as Q
 from packkv_b200 import cache as C
-from packkv_b200 import synth
+from packkv_b200 import ops, synth
 from packkv_b200.config import PackKVCacheConfig, QuantMethod, RepackMethod
 
 pytestmark = pytest.mark.gpu
@@ -270,5 +270,53 @@ def test_update_refuses_rotation_tables_of_another_length(cuda_device, D):
                     cache.flush()
             if T > 1:
                 cache.update(k, v, 0, {"cos": cos[:, :T], "sin": sin[:, :T]})
+    finally:
+        C.PackKVCacheConfigStatic.config = None
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("D", [64, 72, 96, 120])
+@pytest.mark.parametrize("tables", ["row", "rows", None])
+def test_narrow_decode_step_inside_the_attention_launch(cuda_device, D, dtype, tables):
+    """Heads below 128 channels: the launch that attends widens the step's rows and reads the narrow q.  Residual rows bit for bit those of
+    widen_rows (halves of 32 .. 60 channels, rows at odd addresses, tables for one or all sequences), outputs those of a q that is padded
+    and rows that are written beforehand, with and without packed blocks and without an attend() between two steps."""
+    dev, B, H, G = cuda_device, 2, 2, 3
+    C.PackKVCacheConfigStatic.config = _cfg(QuantMethod.PackKV)
+    try:
+        for S0 in (3, 270):
+            new, old = C.PackKVCache(B, H * G, D, 1), C.PackKVCache(B, H * G, D, 1)
+            old._narrow_step = lambda *a: False                    # its rows are written by update()
+            new._scratch = ops.new_attention_scratch(dev)
+            k, v = synth.synth_kv(B, H, S0, D, seed=S0, dtype=dtype, device=dev)
+            for cache in (new, old):
+                cache.update(k, v, 0)
+            for t in range(5):
+                gen = torch.Generator(device=dev).manual_seed(t)
+                buf = torch.randn(2, B, H, D + 1, generator=gen, device=dev).to(dtype)
+                kn, vn = (x[..., t % 2: t % 2 + D].unsqueeze(2) for x in buf)
+                q = torch.randn(B, H * G, 1, D, generator=gen, device=dev).to(dtype)
+                kw = None
+                if tables:
+                    cs = torch.randn(2, B if tables == "rows" else 1, 1, D, generator=gen, device=dev).to(dtype)
+                    kw = {"cos": cs[0], "sin": cs[1]}
+                for cache in (new, old):
+                    cache.update(kn, vn, 0, kw)
+                assert new._layers[0].pending is not None and old._layers[0].pending is None
+                if t == 2:
+                    continue                                       # the next update writes the row itself
+                wide = torch.zeros(B, H * G, 128, dtype=dtype, device=dev)
+                wide[..., :D] = q[:, :, 0]
+                L = old._layers[0]
+                want = ops.decode_attention(wide, L.comp if L.n_comp else None, L.k_res, L.v_res, L.n_res, scaling=D ** -0.5, kv_heads=H, scratch=new._scratch)
+                got = new.attend(q, 0)
+                assert got.shape == (B, 1, H * G, D) and torch.equal(got[:, 0], want[..., :D])
+                N = new._layers[0]
+                assert torch.equal(N.k_res[:, :, : N.n_res], L.k_res[:, :, : L.n_res]) and torch.equal(N.v_res[:, :, : N.n_res], L.v_res[:, :, : L.n_res])
+            new.check_flags()
+        other = torch.randn(B, H * G, 1, 128, device=dev).to(dtype)
+        new.update(kn, vn, 0, kw)
+        old.update(kn, vn, 0, kw)
+        assert torch.equal(new.attend(other, 0), old.attend(other, 0))   # a wider query than the rows of the step
     finally:
         C.PackKVCacheConfigStatic.config = None
