@@ -53,6 +53,18 @@ def compress_block_count(length: int, block: int, recent: int) -> int:
     return max(0, (length + block - length % block - recent) // block)
 
 
+def _zeroed(device, **specs) -> Dict[str, torch.Tensor]:
+    """Zeroed tensors, name=(shape, dtype), in one allocation that one launch clears: the ten tensors of a layer took ten launches (two layers
+    of 4 x 8191 tokens: 638 us with them, 592 without).  Each starts on a 256-byte boundary, as an allocation of its own would at least."""
+    sizes = {name: math.prod(shape) * dtype.itemsize for name, (shape, dtype) in specs.items()}
+    store = torch.zeros(sum((n + 255) // 256 * 256 for n in sizes.values()), dtype=torch.uint8, device=device)
+    out, at = {}, 0
+    for name, (shape, dtype) in specs.items():
+        out[name] = store[at: at + sizes[name]].view(dtype).view(shape)
+        at += (sizes[name] + 255) // 256 * 256
+    return out
+
+
 class PackKVHandle:
     """Stands in for the K (or V) tensor of a decode step: names the cache and the layer."""
     __slots__ = ("cache", "layer_idx")
@@ -124,16 +136,13 @@ class PackKVCache(_HFCache):
         bits_k, bits_v = bits_for_rel(cfg.k_quant_scale_rel), bits_for_rel(cfg.v_quant_scale_rel)
         k_mode = cfg.quant_method.value[0]
         B = self.batch_size
+        k_params = (B, kv_heads, cap // block, 128) if k_mode == QuantMode.ChannelQuant else (B, cap)
         new = ops.CompressedLayer(
-            k_stream=torch.zeros(B, encode.stream_capacity("k", cap, kv_heads, block, bits_k), dtype=torch.uint8, device=device),
-            k_info=torch.zeros(B, (cap // block) * kv_heads, 2, dtype=torch.int32, device=device),
-            k_bytes=torch.zeros(B, dtype=torch.int32, device=device),
-            k_scale=torch.zeros((B, kv_heads, cap // block, 128) if k_mode == QuantMode.ChannelQuant else (B, cap), dtype=dtype, device=device),
-            k_zero=torch.zeros((B, kv_heads, cap // block, 128) if k_mode == QuantMode.ChannelQuant else (B, cap), dtype=dtype, device=device),
-            v_stream=torch.zeros(B, encode.stream_capacity("v", cap, kv_heads, block, bits_v), dtype=torch.uint8, device=device),
-            v_info=torch.zeros(B, (cap // block) * 2 * kv_heads, 2, dtype=torch.int32, device=device),
-            v_bytes=torch.zeros(B, dtype=torch.int32, device=device),
-            v_scale=torch.zeros(B, cap, dtype=dtype, device=device), v_zero=torch.zeros(B, cap, dtype=dtype, device=device),
+            **_zeroed(device,
+                      k_stream=((B, encode.stream_capacity("k", cap, kv_heads, block, bits_k)), torch.uint8),
+                      k_info=((B, (cap // block) * kv_heads, 2), torch.int32), k_bytes=((B,), torch.int32), k_scale=(k_params, dtype), k_zero=(k_params, dtype),
+                      v_stream=((B, encode.stream_capacity("v", cap, kv_heads, block, bits_v)), torch.uint8),
+                      v_info=((B, (cap // block) * 2 * kv_heads, 2), torch.int32), v_bytes=((B,), torch.int32), v_scale=((B, cap), dtype), v_zero=((B, cap), dtype)),
             n_comp=0, kv_heads=kv_heads, cbk=block, cbv=block, bits_k=bits_k, bits_v=bits_v,
             k_mode=ops.K_CHANNEL if k_mode == QuantMode.ChannelQuant else ops.K_TOKEN,
             high_precision_zero=bool(cfg.high_precision_zero_point))
