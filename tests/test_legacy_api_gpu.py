@@ -110,3 +110,43 @@ def test_error_behaviour(cuda_device):
     # CUDA tensors are accepted directly
     size = packkv_cuda.k_encode_cpu(block.to(cuda_device), buf.to(cuda_device), info.to(cuda_device), 64, 128, 64, 128, 4)
     assert size == 8 + 4 * (64 + 48)
+
+
+@pytest.mark.parametrize("extra", [-1, 0, 1])
+@pytest.mark.parametrize("chunks", [1, 2, 3, 5])
+def test_host_buffers_through_chunks(cuda_device, chunks, extra):
+    """Host tensors on their way through the page-locked chunks: sizes around whole chunks, page-locked and ordinary ones."""
+    from packkv_b200 import api
+    n = chunks * api._CHUNK + extra
+    src = torch.randint(0, 256, (n,), dtype=torch.uint8)
+    for host, back in ((src, torch.zeros_like(src)), (src.pin_memory(), torch.zeros(n, dtype=torch.uint8, pin_memory=True))):
+        dev = torch.zeros(n, dtype=torch.uint8, device=cuda_device)
+        api._upload(host, dev)
+        api._download(dev, back)
+        assert torch.equal(back, src) and torch.equal(dev.cpu(), src)
+
+
+@pytest.mark.parametrize("which,cb,hb", [("k", 64, 128), ("v", 128, 64)])
+def test_decode_takes_what_the_table_refers_to(cuda_device, which, cb, hb):
+    """The packed bytes are the front of a larger host buffer (more than a chunk of it in use); a table entry beyond the buffer is refused,
+    one that ends in its unused part is read there."""
+    ctx, hidden = 4096, 2048
+    codes = torch.randint(0, 16, (ctx, hidden), dtype=torch.uint8)
+    info = torch.zeros((ctx // cb) * (hidden // hb), 2, dtype=U32)
+    packed, back = torch.zeros(ctx, hidden, dtype=torch.uint8), torch.zeros(ctx, hidden, dtype=torch.uint8)
+    size = getattr(packkv_cuda, which + "_encode_cpu")(codes, packed, info, ctx, hidden, cb, hb, 4)
+    assert (2 << 20) < size < packed.numel()
+    decode = getattr(packkv_cuda, which + "_decode_cpu")
+    decode(packed, info, back, ctx, hidden, cb, hb, 4)
+    assert torch.equal(back, codes)
+    entries = info.view(torch.int32)
+    off, n = entries[3].tolist()
+    packed.view(-1)[size + 64: size + 64 + n] = packed.view(-1)[off: off + n].clone()
+    entries[3, 0] = size + 64
+    back.zero_()
+    decode(packed, info, back, ctx, hidden, cb, hb, 4)
+    assert torch.equal(back, codes)
+    for bad in (packed.numel() - 2, -64):                       # past the buffer's end; an offset of nearly 2^32
+        entries[3, 0] = bad
+        with pytest.raises(ValueError):
+            decode(packed, info, back, ctx, hidden, cb, hb, 4)
