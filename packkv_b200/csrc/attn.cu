@@ -289,7 +289,7 @@ struct CtaShared {
     float cl_m[8];       // this CTA's max per head
     float cl_l[8];       // this CTA's sum of exp(s - cl_m) per head
     float wm[kAW][8];    // per-warp scratch
-    float gM[8], gInvL[8];
+    float gM[kAW][8], gInvL[kAW][8];   // global maximum and reciprocal sum, a copy for every warp
     unsigned lutm[8];    // (2^len - 1) * 0x00010001 per pack length 0..4 (see unpack8)
     unsigned last;       // two-launch form: this cluster is the pair's last one to deliver its rows
     unsigned pad_[3];
@@ -908,19 +908,32 @@ __global__ void __launch_bounds__(kAW * 32, PASS == 1 ? PKV_ATTN_CTAS_SCORES : P
     if constexpr (PASS == kFused) {
         // ---- cluster exchange: global max and sum ---------------------------------------------------
         cluster.sync();
-        if (threadIdx.x < 8) {
-            float M = -INFINITY;
-            for (int r = 0; r < P.cluster; r++) M = fmaxf(M, cluster.map_shared_rank(cs, r)->cl_m[threadIdx.x]);
-            float L = 0.f;
-            for (int r = 0; r < P.cluster; r++) {
+        // lane: head lane & 7 of the CTAs (lane >> 3) + 4 i, all remote loads in flight together; every warp for itself, so that no
+        // barrier follows
+        float mr[4], lr[4], M = -INFINITY, L = 0.f;
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const int r = (lane >> 3) + 4 * i;
+            mr[i] = -INFINITY; lr[i] = 0.f;
+            if (r < P.cluster) {
                 const CtaShared* o = cluster.map_shared_rank(cs, r);
-                const float mr = o->cl_m[threadIdx.x];
-                if (mr != -INFINITY) L += o->cl_l[threadIdx.x] * fast_exp(mr - M);
+                mr[i] = o->cl_m[lane & 7]; lr[i] = o->cl_l[lane & 7];
             }
-            cs->gM[threadIdx.x] = M;
-            cs->gInvL[threadIdx.x] = L > 0.f ? 1.f / L : 0.f;
         }
-        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < 4; i++) M = fmaxf(M, mr[i]);
+        M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, 8));
+        M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, 16));
+#pragma unroll
+        for (int i = 0; i < 4; i++)
+            if (mr[i] != -INFINITY) L += lr[i] * fast_exp(mr[i] - M);
+        L += __shfl_xor_sync(0xffffffffu, L, 8);
+        L += __shfl_xor_sync(0xffffffffu, L, 16);
+        if (lane < 8) {
+            cs->gM[wic][lane] = M;
+            cs->gInvL[wic][lane] = L > 0.f ? 1.f / L : 0.f;
+        }
+        __syncwarp();
     }
     if constexpr (PASS == kScores) {
         // ---- first launch ends here: this CTA's max and sum and every warp's score region go to the scratch ----
@@ -989,17 +1002,17 @@ __global__ void __launch_bounds__(kAW * 32, PASS == 1 ? PKV_ATTN_CTAS_SCORES : P
             if (lane == 0) cs->wm[wic][r] = l;
         }
         __syncthreads();
-        if (threadIdx.x < 8) {
+        if (lane < 8) {
             float L = 0.f;
 #pragma unroll
-            for (int w = 0; w < kAW; w++) L += cs->wm[w][threadIdx.x];
+            for (int w = 0; w < kAW; w++) L += cs->wm[w][lane];
             float M = -INFINITY;
 #pragma unroll
-            for (int r = 0; r < 8; r++) if (r == (int)threadIdx.x) M = M8[r];
-            cs->gM[threadIdx.x] = M;
-            cs->gInvL[threadIdx.x] = L > 0.f ? 1.f / L : 0.f;
+            for (int r = 0; r < 8; r++) if (r == lane) M = M8[r];
+            cs->gM[wic][lane] = M;
+            cs->gInvL[wic][lane] = L > 0.f ? 1.f / L : 0.f;
         }
-        __syncthreads();
+        __syncwarp();
     }
 
     // ============================================================================ phase 2: V tiles
@@ -1106,7 +1119,7 @@ __global__ void __launch_bounds__(kAW * 32, PASS == 1 ? PKV_ATTN_CTAS_SCORES : P
             const unsigned row = stile_a + (tl * P.rows + r) * P.prow + 16 * q8;
             unsigned w0 = 0, w1 = 0;
             if (tl < my_tiles) {
-                const float M = cs->gM[r], I = cs->gInvL[r];
+                const float M = cs->gM[wic][r], I = cs->gInvL[wic][r];
                 const float2 xa = Tr<T>::unpack2(lds32(row + 4 * e)), xb = Tr<T>::unpack2(lds32(row + 4 * e + 8));
                 const unsigned pa = Tr<T>::pack2(fast_exp(xa.x - M) * I, fast_exp(xa.y - M) * I);
                 const unsigned pb = Tr<T>::pack2(fast_exp(xb.x - M) * I, fast_exp(xb.y - M) * I);
@@ -1139,7 +1152,7 @@ __global__ void __launch_bounds__(kAW * 32, PASS == 1 ? PKV_ATTN_CTAS_SCORES : P
                     if (u < units) {
                         const int r = u >> pr_shift, rem = u & ((1 << pr_shift) - 1), q8 = rem >> 1, e = rem & 1;
                         const unsigned ad = st_a + r * P.prow + 16 * q8 + 4 * e;
-                        const float M = cs->gM[r], I = cs->gInvL[r];
+                        const float M = cs->gM[wic][r], I = cs->gInvL[wic][r];
                         const float2 xa = Tr<T>::unpack2(lds32(ad)), xb = Tr<T>::unpack2(lds32(ad + 8));
                         const unsigned pa = Tr<T>::pack2(fast_exp(xa.x - M) * I, fast_exp(xa.y - M) * I);
                         const unsigned pb = Tr<T>::pack2(fast_exp(xb.x - M) * I, fast_exp(xb.y - M) * I);
@@ -1212,7 +1225,7 @@ __global__ void __launch_bounds__(kAW * 32, PASS == 1 ? PKV_ATTN_CTAS_SCORES : P
 #pragma unroll
             for (int r = 0; r < 8; r++) {
                 if (r < P.rows) {
-                    const float M = cs->gM[r], I = cs->gInvL[r];
+                    const float M = cs->gM[wic][r], I = cs->gInvL[wic][r];
                     const unsigned ad = rst_a + (k * P.rows + r) * 32 + 4 * lane;
                     const float2 x = Tr<T>::unpack2(lds32(ad));
                     sts32(ad, Tr<T>::pack2(x.x == -INFINITY ? 0.f : fast_exp(x.x - M) * I, x.y == -INFINITY ? 0.f : fast_exp(x.y - M) * I));
@@ -1268,51 +1281,69 @@ __global__ void __launch_bounds__(kAW * 32, PASS == 1 ? PKV_ATTN_CTAS_SCORES : P
         }
     }
     cluster.sync();
-    if (rank == 0) {
+    // The cluster's CTAs share out the G * 128 sums, one to a thread, whose remote loads are in flight together.  With the first CTA adding
+    // them all, one remote load after the other, this was the last 1.7 us of 13 (8 KV heads x 700 tokens, 4 heads to a group; 11.5 now) and
+    // 8 of the 31 us of two launches with 7 heads to a group (10 pairs x 5333 tokens; 26.7 now).  With an exchange the first CTA
+    // delivers alone: it announces one arrival.
+    const bool spread = P.x.n_ranks == 0;
+    if (spread || rank == 0) {
+        const int first = (spread ? rank : 0) * kThreads + (int)threadIdx.x, stride = (spread ? P.cluster : 1) * kThreads;
+        const auto cluster_sum = [&](int e) {
+            const int hd = e / kD, d = e % kD;
+            float x[16], v = 0.f;
+#pragma unroll
+            for (int r = 0; r < 16; r++) x[r] = r < P.cluster ? cluster.map_shared_rank(cta_out_row(smem, P.warp_smem, P.out_off, hd), r)[d] : 0.f;
+#pragma unroll
+            for (int r = 0; r < 16; r++) v += x[r];
+            return v;
+        };
+        const auto put = [&](int e, float v) {
+            const T r = Tr<T>::from_float(v);
+            const int64_t idx = (int64_t)(b * q_heads + h * G) * kD + e;
+            reinterpret_cast<T*>(a.out)[idx] = r;
+            // head-sharded decode: the same row goes into this rank's slice of every rank's gathered buffer
+            for (int p = 0; p < P.x.n_ranks; p++)
+                reinterpret_cast<T*>(P.x.gathered[p])[(int64_t)P.x.rank * a.batch * q_heads * kD + idx] = r;
+        };
         bool deliver = true;
         if constexpr (PASS == kValues) {
-            // this cluster's rows go to the scratch; the cluster that finds all the others' there adds them up
+            // this cluster's rows go to the scratch; the CTA that finds all the others' there adds them up
             float* part = P.sc_part + ((int64_t)pair * part_stride + split) * 8 * kD;
-            for (int d = threadIdx.x; d < kD; d += kThreads) {
-                for (int hd = 0; hd < G; hd++) {
-                    float v = 0.f;
-                    for (int r = 0; r < P.cluster; r++) v += cluster.map_shared_rank(cta_out_row(smem, P.warp_smem, P.out_off, hd), r)[d];
-                    __stcg(part + hd * kD + d, v);
-                }
-            }
+            for (int e = first; e < G * kD; e += stride) __stcg(part + e, cluster_sum(e));
             __threadfence();
             __syncthreads();
-            if (threadIdx.x == 0) cs->last = atomicAdd(P.sc_count + pair, 1u) == (unsigned)(n_splits - 1) ? 1u : 0u;
+            if (threadIdx.x == 0) cs->last = atomicAdd(P.sc_count + pair, 1u) == (unsigned)((spread ? n_vctas : n_splits) - 1) ? 1u : 0u;
             __syncthreads();
             deliver = cs->last != 0;
-            if (deliver) __threadfence();
-        }
-        if (deliver) {
-            for (int d = threadIdx.x; d < kD; d += kThreads) {
-                for (int hd = 0; hd < G; hd++) {
-                    float v = 0.f;
-                    if constexpr (PASS == kValues) {
-                        for (int sp = 0; sp < n_splits; sp++) v += __ldcg(P.sc_part + (((int64_t)pair * part_stride + sp) * 8 + hd) * kD + d);
-                    } else {
-                        for (int r = 0; r < P.cluster; r++) v += cluster.map_shared_rank(cta_out_row(smem, P.warp_smem, P.out_off, hd), r)[d];
+            if (deliver) {
+                __threadfence();
+                for (int d = threadIdx.x; d < kD; d += kThreads) {
+                    float v[8];
+#pragma unroll
+                    for (int hd = 0; hd < 8; hd++) v[hd] = 0.f;
+                    const float* rows = P.sc_part + (int64_t)pair * part_stride * 8 * kD + d;
+#pragma unroll 4
+                    for (int sp = 0; sp < n_splits; sp++) {
+#pragma unroll
+                        for (int hd = 0; hd < 8; hd++)
+                            if (hd < G) v[hd] += __ldcg(rows + (sp * 8 + hd) * kD);
                     }
-                    const T r = Tr<T>::from_float(v);
-                    const int64_t idx = ((int64_t)(b * q_heads + h * G + hd)) * kD + d;
-                    reinterpret_cast<T*>(a.out)[idx] = r;
-                    // head-sharded decode: the same row goes into this rank's slice of every rank's gathered buffer
-                    for (int p = 0; p < P.x.n_ranks; p++)
-                        reinterpret_cast<T*>(P.x.gathered[p])[(int64_t)P.x.rank * a.batch * q_heads * kD + idx] = r;
+#pragma unroll
+                    for (int hd = 0; hd < 8; hd++)
+                        if (hd < G) put(hd * kD + d, v[hd]);
                 }
+                if (threadIdx.x == 0) P.sc_count[pair] = 0u;   // ready for the next launch on this scratch
             }
-            if (PASS == kValues && threadIdx.x == 0) P.sc_count[pair] = 0u;   // ready for the next launch on this scratch
-            if (P.x.n_ranks > 0) {
-                __threadfence_system();                // the rows are visible to the other GPUs before the arrival is
-                __syncthreads();
-                if ((int)threadIdx.x < P.x.n_ranks) atomicAdd_system(P.x.arrivals[threadIdx.x] + P.x.rank, 1u);
-            }
+        } else {
+            for (int e = first; e < G * kD; e += stride) put(e, cluster_sum(e));
+        }
+        if (deliver && P.x.n_ranks > 0) {
+            __threadfence_system();                // the rows are visible to the other GPUs before the arrival is
+            __syncthreads();
+            if ((int)threadIdx.x < P.x.n_ranks) atomicAdd_system(P.x.arrivals[threadIdx.x] + P.x.rank, 1u);
         }
     }
-    cluster.sync();   // keep every CTA's shared memory alive until rank 0 has read it
+    cluster.sync();   // keep every CTA's shared memory alive until the others have read it
     }   // PASS != kScores
 }
 
