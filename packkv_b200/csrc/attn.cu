@@ -66,9 +66,6 @@ constexpr unsigned kWaitSpins = 1u << 22;   // bounded mbarrier wait (each try s
 #ifndef PKV_ATTN_CTAS_VALUES
 #define PKV_ATTN_CTAS_VALUES PKV_ATTN_CTAS
 #endif
-#ifndef PKV_ONE_CHAIN
-#define PKV_ONE_CHAIN 0
-#endif
 #ifndef PKV_ABL
 #define PKV_ABL 0
 #endif
@@ -95,6 +92,12 @@ template <> struct Tr<__half> {
             : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
             : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
     }
+    static __device__ __forceinline__ void mma0(float (&d)[4], const unsigned (&a)[4], unsigned b0, unsigned b1) {   // accumulators that start at 0
+        asm volatile(
+            "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};\n"
+            : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+            : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(0.f));
+    }
 };
 
 template <> struct Tr<__nv_bfloat16> {
@@ -115,6 +118,12 @@ template <> struct Tr<__nv_bfloat16> {
             "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
             : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
             : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+    }
+    static __device__ __forceinline__ void mma0(float (&d)[4], const unsigned (&a)[4], unsigned b0, unsigned b1) {   // accumulators that start at 0
+        asm volatile(
+            "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};\n"
+            : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+            : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(0.f));
     }
 };
 
@@ -192,7 +201,7 @@ __device__ __forceinline__ unsigned ldp16(unsigned a) { unsigned short v; asm("l
 __device__ __forceinline__ unsigned ldp8(unsigned a) { unsigned v; asm("ld.shared.u8 %0, [%1];" : "=r"(v) : "r"(a)); return v; }
 // 64-bit window at shared address a (2-byte aligned): three aligned 32-bit loads, two funnel shifts
 __device__ __forceinline__ void ldp_u64_align2(unsigned a, unsigned& lo, unsigned& hi) {
-    const unsigned wa = a & ~3u, sh = (a & 2u) * 8u;
+    const unsigned wa = a & ~3u, sh = a << 3;           // the funnel shift takes the low five bits: 0 or 16
     const unsigned w0 = ldp32(wa), w1 = ldp32(wa + 4), w2 = ldp32(wa + 8);
     lo = __funnelshift_r(w0, w1, sh);
     hi = __funnelshift_r(w1, w2, sh);
@@ -592,7 +601,7 @@ __global__ void __launch_bounds__(kAW * 32, PASS == 1 ? PKV_ATTN_CTAS_SCORES : P
             const unsigned hdr = blk + pos;
             unsigned lens4 = spread_const<LBK>(lane_word<4 * LBK>(hdr + 16 * BK, lane));   // byte j = length of pack j
             const unsigned mins4 = spread_const<BK>(lane_word<4 * BK>(hdr, lane));
-            if ((lens4 + 0x03030303u) & 0x08080808u) { lens4 = 0; bad_len = true; }   // no encoder writes a length above 4
+            if (LBK > 2 && ((lens4 + 0x03030303u) & 0x08080808u)) { lens4 = 0; bad_len = true; }   // no encoder writes a length above 4
             const unsigned inc = warp_inclusive_sum(lens4);
             const unsigned tot = __shfl_sync(0xffffffffu, inc, 31);
             const unsigned exc2 = (inc - lens4) << 1;                 // byte j = byte offset of this lane's pack j in its group
@@ -604,7 +613,7 @@ __global__ void __launch_bounds__(kAW * 32, PASS == 1 ? PKV_ATTN_CTAS_SCORES : P
                 sw[0] = lds128(perm_a + 2 * tk0); sw[1] = lds128(perm_a + 2 * tk0 + 16);
                 zw[0] = lds128(perm_a + 2 * P.tile + 2 * tk0); zw[1] = lds128(perm_a + 2 * P.tile + 2 * tk0 + 16);
             }
-            float accs[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};   // two chains hide the mma latency
+            float accs[2][4];                                         // two chains hide the mma latency
 #pragma unroll
             for (int j = 0; j < 4; j++) {
                 unsigned lo, hi;
@@ -645,7 +654,8 @@ __global__ void __launch_bounds__(kAW * 32, PASS == 1 ? PKV_ATTN_CTAS_SCORES : P
                 for (int ap = 0; ap < 2; ap++) {
                     unsigned af[4];
                     ldmatrix_x4_trans(kldm[ap] + (j & 1) * 1024, af);
-                    Tr<T>::mma(accs[PKV_ONE_CHAIN ? 0 : ap], af, qf[j][ap][0], qf[j][ap][1]);
+                    if (j == 0) Tr<T>::mma0(accs[ap], af, qf[j][ap][0], qf[j][ap][1]);
+                    else Tr<T>::mma(accs[ap], af, qf[j][ap][0], qf[j][ap][1]);
                 }
             }
             // scores rounded like the reference: matmul output, then * scaling; fragment rows g and g + 8 are the
@@ -653,8 +663,10 @@ __global__ void __launch_bounds__(kAW * 32, PASS == 1 ? PKV_ATTN_CTAS_SCORES : P
             // only the stores are predicated, no branch)
             {
                 const unsigned row0 = st + (2 * c) * P.prow + 2 * (tk0 + tau);
-                const unsigned p0 = Tr<T>::pack2(Tr<T>::round(accs[0][0] + accs[1][0]) * a.scaling, Tr<T>::round(accs[0][2] + accs[1][2]) * a.scaling);
-                const unsigned p1 = Tr<T>::pack2(Tr<T>::round(accs[0][1] + accs[1][1]) * a.scaling, Tr<T>::round(accs[0][3] + accs[1][3]) * a.scaling);
+                const float2 s0 = Tr<T>::unpack2(Tr<T>::pack2(accs[0][0] + accs[1][0], accs[0][2] + accs[1][2]));
+                const float2 s1 = Tr<T>::unpack2(Tr<T>::pack2(accs[0][1] + accs[1][1], accs[0][3] + accs[1][3]));
+                const unsigned p0 = Tr<T>::pack2(s0.x * a.scaling, s0.y * a.scaling);
+                const unsigned p1 = Tr<T>::pack2(s1.x * a.scaling, s1.y * a.scaling);
                 if (col_live) sts32(row0, p0);
                 if (col_live) sts32(row0 + P.prow, p1);
                 mpk0 = __hmax2(mpk0, as_t2<T2>(p0));
@@ -1039,7 +1051,7 @@ __global__ void __launch_bounds__(kAW * 32, PASS == 1 ? PKV_ATTN_CTAS_SCORES : P
             const unsigned hdr = blk + pos;
             unsigned lens4 = spread_const<LBV>(lane_word<4 * LBV>(hdr + 16 * BV, lane));   // byte q = length of pack q (tokens 16q..16q+15)
             const unsigned mins4 = spread_const<BV>(lane_word<4 * BV>(hdr, lane));
-            if ((lens4 + 0x03030303u) & 0x08080808u) { lens4 = 0; bad_len = true; }
+            if (LBV > 2 && ((lens4 + 0x03030303u) & 0x08080808u)) { lens4 = 0; bad_len = true; }
             const unsigned inc = warp_inclusive_sum(lens4);
             const unsigned tot = __shfl_sync(0xffffffffu, inc, 31);
             const unsigned packs = hdr + 16 * BV + 16 * LBV;
