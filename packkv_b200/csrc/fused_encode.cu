@@ -20,6 +20,7 @@
 //            fixed-stride SLOTS in scratch memory with the size in block_info[blk][1]; per-sequence
 //            exclusive scan (scan_sizes_kernel, pack.cu); one warp per block copies its slot to its
 //            final offset.  The block bytes are written, read and written once more.
+#include <cooperative_groups.h>
 #include <cstdlib>
 #include <string>
 
@@ -27,6 +28,8 @@
 #include "launch.h"
 #include "pack_dev.cuh"
 #include "quant_dev.cuh"
+
+namespace cg = cooperative_groups;
 
 namespace pkv {
 
@@ -182,154 +185,156 @@ __device__ __forceinline__ void store_slot(uint8_t* slot, const uint8_t* stage, 
 }
 
 // ------------------------------------------------------------------------------------------ K
-// rounds of one K block: quantise 16 tokens x 4 channels per lane, pack, append to `stage`
-// ORDERED: stored row t of the block is source row ordp[t] (16-byte aligned table of the block's rows)
-template <typename T, bool HP, int BITS, bool FAST, bool ORDERED>
-__device__ __forceinline__ int k_encode_rounds(const T* x, int64_t ss, const uint8_t* ordp, const Quantiser<T, HP>& q0, const Quantiser<T, HP>& q1,
-                                               const Quantiser<T, HP>& q2, const Quantiser<T, HP>& q3, const KGeom& g, uint8_t* stage,
-                                               int lane, bool& bad) {
-    constexpr int LB = len_field_bits(BITS);
+// One round of a K block: quantise 16 tokens x 4 channels per lane and pack them at `at`: minima, lengths, packs.  row(t) gives the
+// lane's four elements of the round's token t.  Returns the round's bytes.
+template <typename T, bool HP, int BITS, bool FAST, typename Row>
+__device__ __forceinline__ unsigned k_encode_round(Row row, const Quantiser<T, HP>& q0, const Quantiser<T, HP>& q1, const Quantiser<T, HP>& q2,
+                                                   const Quantiser<T, HP>& q3, uint8_t* at, int lane, unsigned& over) {
+    constexpr int LB = len_field_bits(BITS), kMin = 16 * BITS, kLen = 16 * LB;
     const int z0 = (int)q0.zero, z1 = (int)q1.zero, z2 = (int)q2.zero, z3 = (int)q3.zero;
-    int pos = g.head_bytes;
-    unsigned round_end = 0, over = 0;
-    for (int r = 0; r < g.rounds; r++) {
-        unsigned u[16];                               // four channel codes per token, one byte each
-        unsigned mnj[4] = {255u, 255u, 255u, 255u}, mxj[4] = {0u, 0u, 0u, 0u};
-        uint4 ob = make_uint4(0, 0, 0, 0);
-        if (ORDERED) ob = __ldg(reinterpret_cast<const uint4*>(ordp + 16 * r));
-        const unsigned ow[4] = {ob.x, ob.y, ob.z, ob.w};
+    unsigned u[16];                                   // four channel codes per token, one byte each
+    unsigned mnj[4] = {255u, 255u, 255u, 255u}, mxj[4] = {0u, 0u, 0u, 0u};
 #pragma unroll
-        for (int t = 0; t < 16; t++) {
-            const int row = ORDERED ? (int)((ow[t >> 2] >> (8 * (t & 3))) & 0xFFu) : r * 16 + t;
-            const uint2 raw = __ldg(reinterpret_cast<const uint2*>(x + (int64_t)row * ss));
-            const T* e = reinterpret_cast<const T*>(&raw);
-            const unsigned c0 = q0.template code_u8<FAST>(QT<T>::ld(e), z0), c1 = q1.template code_u8<FAST>(QT<T>::ld(e + 1), z1);
-            const unsigned c2 = q2.template code_u8<FAST>(QT<T>::ld(e + 2), z2), c3 = q3.template code_u8<FAST>(QT<T>::ld(e + 3), z3);
-            mnj[0] = min(mnj[0], c0); mxj[0] = max(mxj[0], c0);
-            mnj[1] = min(mnj[1], c1); mxj[1] = max(mxj[1], c1);
-            mnj[2] = min(mnj[2], c2); mxj[2] = max(mxj[2], c2);
-            mnj[3] = min(mnj[3], c3); mxj[3] = max(mxj[3], c3);
-            u[t] = c0 | (c1 << 8) | (c2 << 16) | (c3 << 24);
-        }
-        unsigned minword = 0, lenword = 0, lens4 = 0;
-        int len[4];
-#pragma unroll
-        for (int j = 0; j < 4; j++) {
-            over |= mxj[j] >> BITS;
-            len[j] = min(bit_length_u32(mxj[j] - mnj[j]), BITS);
-            minword |= (mnj[j] & ((1u << BITS) - 1u)) << (j * BITS);
-            lenword |= (unsigned)len[j] << (j * LB);
-            lens4 |= (unsigned)len[j] << (8 * j);
-        }
-        store_lane_fields_w<4 * BITS>(stage + pos, lane, minword);
-        store_lane_fields_w<4 * LB>(stage + pos + g.min_bytes, lane, lenword);
-        const unsigned inc = warp_inclusive_sum(lens4);
-        const unsigned tot = __shfl_sync(0xffffffffu, inc, 31);
-        const unsigned exc = inc - lens4;
-        uint8_t* packs = stage + pos + g.min_bytes + g.len_bytes;
-        unsigned before = 0;
-#pragma unroll
-        for (int j = 0; j < 4; j++) {
-            // tokens 0..7 and 8..15 as two words of at most 32 bits: w = w * 2^len + code, then the
-            // minimum is taken off all eight fields at once (min * (1 + 2^len + ... + 2^(7 len)))
-            const unsigned step = 1u << len[j];
-            unsigned wt = 0, wb = 0, ones = 0;
-#pragma unroll
-            for (int t = 0; t < 8; t++) {
-                wt = wt * step + __byte_perm(u[t], 0, 0x4440 + j);
-                wb = wb * step + __byte_perm(u[t + 8], 0, 0x4440 + j);
-                ones = ones * step + 1u;
-            }
-            wt -= mnj[j] * ones;
-            wb -= mnj[j] * ones;
-            const uint64_t w = ((uint64_t)wt << (8 * len[j])) | wb;
-            store_pack_smem(packs + 2 * (before + ((exc >> (8 * j)) & 0xFFu)), w, len[j]);
-            before += (tot >> (8 * j)) & 0xFFu;
-        }
-        const unsigned round_size = g.min_bytes + g.len_bytes + 2 * before;
-        round_end += round_size;
-        if (lane == 0) *reinterpret_cast<uint16_t*>(stage + 2 * r) = (uint16_t)round_end;
-        pos += round_size;
+    for (int t = 0; t < 16; t++) {
+        const uint2 raw = row(t);
+        const T* e = reinterpret_cast<const T*>(&raw);
+        const unsigned c0 = q0.template code_u8<FAST>(QT<T>::ld(e), z0), c1 = q1.template code_u8<FAST>(QT<T>::ld(e + 1), z1);
+        const unsigned c2 = q2.template code_u8<FAST>(QT<T>::ld(e + 2), z2), c3 = q3.template code_u8<FAST>(QT<T>::ld(e + 3), z3);
+        mnj[0] = min(mnj[0], c0); mxj[0] = max(mxj[0], c0);
+        mnj[1] = min(mnj[1], c1); mxj[1] = max(mxj[1], c1);
+        mnj[2] = min(mnj[2], c2); mxj[2] = max(mxj[2], c2);
+        mnj[3] = min(mnj[3], c3); mxj[3] = max(mxj[3], c3);
+        u[t] = c0 | (c1 << 8) | (c2 << 16) | (c3 << 24);
     }
-    bad = bad || over != 0;
-    return pos;
+    unsigned minword = 0, lenword = 0, lens4 = 0;
+    int len[4];
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+        over |= mxj[j] >> BITS;
+        len[j] = min(bit_length_u32(mxj[j] - mnj[j]), BITS);
+        minword |= (mnj[j] & ((1u << BITS) - 1u)) << (j * BITS);
+        lenword |= (unsigned)len[j] << (j * LB);
+        lens4 |= (unsigned)len[j] << (8 * j);
+    }
+    store_lane_fields_w<4 * BITS>(at, lane, minword);
+    store_lane_fields_w<4 * LB>(at + kMin, lane, lenword);
+    const unsigned inc = warp_inclusive_sum(lens4);
+    const unsigned tot = __shfl_sync(0xffffffffu, inc, 31);
+    const unsigned exc = inc - lens4;
+    uint8_t* packs = at + kMin + kLen;
+    unsigned before = 0;
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+        // tokens 0..7 and 8..15 as two words of at most 32 bits: w = w * 2^len + code, then the
+        // minimum is taken off all eight fields at once (min * (1 + 2^len + ... + 2^(7 len)))
+        const unsigned step = 1u << len[j];
+        unsigned wt = 0, wb = 0, ones = 0;
+#pragma unroll
+        for (int t = 0; t < 8; t++) {
+            wt = wt * step + __byte_perm(u[t], 0, 0x4440 + j);
+            wb = wb * step + __byte_perm(u[t + 8], 0, 0x4440 + j);
+            ones = ones * step + 1u;
+        }
+        wt -= mnj[j] * ones;
+        wb -= mnj[j] * ones;
+        const uint64_t w = ((uint64_t)wt << (8 * len[j])) | wb;
+        store_pack_smem(packs + 2 * (before + ((exc >> (8 * j)) & 0xFFu)), w, len[j]);
+        before += (tot >> (8 * j)) & 0xFFu;
+    }
+    return kMin + kLen + 2 * before;
 }
 
-// The same rounds for blocks whose four quantisers are packable(): two channels per instruction
+// The same round for blocks whose four quantisers are packable(): two channels per instruction
 // from the conversion to the pack minimum / maximum (16-bit lanes), then one multiply-add per code
 // into the pack words.
-template <typename T, int BITS, bool HALF, bool ORDERED>
-__device__ __forceinline__ int k_encode_rounds_packed(const T* x, int64_t ss, const uint8_t* ordp, const Quantiser<T, false>& q0, const Quantiser<T, false>& q1,
-                                                      const Quantiser<T, false>& q2, const Quantiser<T, false>& q3, const KGeom& g,
-                                                      uint8_t* stage, int lane, bool& bad) {
-    constexpr int LB = len_field_bits(BITS);
-    const unsigned k01 = packed_code_bias(q0, q1), k23 = packed_code_bias(q2, q3);
-    const HalfQuotient<T> h01(q0, q1), h23(q2, q3);      // used when every quantiser is in the half domain
+template <typename T>
+struct PackedQuantisers {
+    unsigned k01, k23;
+    HalfQuotient<T> h01, h23;                         // used when every quantiser is in the half domain
+    __device__ __forceinline__ PackedQuantisers(const Quantiser<T, false>& q0, const Quantiser<T, false>& q1, const Quantiser<T, false>& q2, const Quantiser<T, false>& q3)
+        : k01(packed_code_bias(q0, q1)), k23(packed_code_bias(q2, q3)), h01(q0, q1), h23(q2, q3) {}
+};
+template <typename T, int BITS, bool HALF, typename Row>
+__device__ __forceinline__ unsigned k_encode_round_packed(Row row, const Quantiser<T, false>& q0, const Quantiser<T, false>& q1, const Quantiser<T, false>& q2,
+                                                          const Quantiser<T, false>& q3, const PackedQuantisers<T>& pq, uint8_t* at, int lane, unsigned& over) {
+    constexpr int LB = len_field_bits(BITS), kMin = 16 * BITS, kLen = 16 * LB;
+    unsigned c01[16], c23[16];
+    unsigned mn01 = 0xFFFFFFFFu, mx01 = 0u, mn23 = 0xFFFFFFFFu, mx23 = 0u;
+#pragma unroll
+    for (int t = 0; t < 16; t++) {
+        const uint2 raw = row(t);
+        c01[t] = HALF ? pq.h01.codes(raw.x) : packed_codes<T>(raw.x, q0, q1, pq.k01);
+        c23[t] = HALF ? pq.h23.codes(raw.y) : packed_codes<T>(raw.y, q2, q3, pq.k23);
+        mn01 = min_u16x2(mn01, c01[t]); mx01 = max_u16x2(mx01, c01[t]);
+        mn23 = min_u16x2(mn23, c23[t]); mx23 = max_u16x2(mx23, c23[t]);
+    }
+    over |= mx01 | mx23;
+    const unsigned mnj[4] = {mn01 & 0xFFFFu, mn01 >> 16, mn23 & 0xFFFFu, mn23 >> 16};
+    const unsigned d01 = mx01 - mn01, d23 = mx23 - mn23;     // lane-wise: no borrow, max >= min
+    const unsigned dj[4] = {d01 & 0xFFFFu, d01 >> 16, d23 & 0xFFFFu, d23 >> 16};
+    unsigned minword = 0, lenword = 0, lens4 = 0;
+    int len[4];
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+        len[j] = min(bit_length_u32(dj[j]), BITS);
+        minword |= (mnj[j] & ((1u << BITS) - 1u)) << (j * BITS);
+        lenword |= (unsigned)len[j] << (j * LB);
+        lens4 |= (unsigned)len[j] << (8 * j);
+    }
+    store_lane_fields_w<4 * BITS>(at, lane, minword);
+    store_lane_fields_w<4 * LB>(at + kMin, lane, lenword);
+    const unsigned inc = warp_inclusive_sum(lens4);
+    const unsigned tot = __shfl_sync(0xffffffffu, inc, 31);
+    const unsigned exc = inc - lens4;
+    uint8_t* packs = at + kMin + kLen;
+    unsigned before = 0;
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+        // 16-bit lanes, four tokens each (token 0 and 4, 8 and 12 highest): w = w * 2^len + code for two of them per
+        // multiply-add, then the minimum is taken off all four fields at once (min * (1 + 2^len + ... + 2^(3 len))).
+        // A lane stays below 2^16: four codes below 2^4 at steps of at most 2^4.  Against one multiply-add and one
+        // extraction per code: 1.6 instead of 2.8 instructions per code.
+        const unsigned step = 1u << len[j], sel = (j & 1) ? 0x7632u : 0x5410u;
+        const unsigned(&cj)[16] = j < 2 ? c01 : c23;
+        unsigned za = __byte_perm(cj[0], cj[4], sel), zb = __byte_perm(cj[8], cj[12], sel);
+#pragma unroll
+        for (int t = 1; t < 4; t++) {
+            za = za * step + __byte_perm(cj[t], cj[t + 4], sel);
+            zb = zb * step + __byte_perm(cj[t + 8], cj[t + 12], sel);
+        }
+        const unsigned low = mnj[j] * ((1u + step) * (1u + step * step)) * 0x00010001u;
+        za -= low;
+        zb -= low;
+        const unsigned wt = ((za & 0xFFFFu) << (4 * len[j])) | (za >> 16), wb = ((zb & 0xFFFFu) << (4 * len[j])) | (zb >> 16);
+        const uint64_t w = ((uint64_t)wt << (8 * len[j])) | wb;
+        store_pack_smem(packs + 2 * (before + ((exc >> (8 * j)) & 0xFFu)), w, len[j]);
+        before += (tot >> (8 * j)) & 0xFFu;
+    }
+    return kMin + kLen + 2 * before;
+}
+
+// rounds of one K block, appended to `stage` behind the table of round ends
+// MODE 0: scalar conversion, 1: two elements per instruction in fp32, 2: in the element type
+// ORDERED: stored row t of the block is source row ordp[t] (16-byte aligned table of the block's rows)
+template <typename T, int BITS, int MODE, bool ORDERED>
+__device__ __forceinline__ int k_encode_rounds(const T* x, int64_t ss, const uint8_t* ordp, const Quantiser<T, false>& q0, const Quantiser<T, false>& q1,
+                                               const Quantiser<T, false>& q2, const Quantiser<T, false>& q3, const KGeom& g, uint8_t* stage, int lane, bool& bad) {
+    const PackedQuantisers<T> pq(q0, q1, q2, q3);
     int pos = g.head_bytes;
-    unsigned round_end = 0, over = 0;
+    unsigned over = 0;
     for (int r = 0; r < g.rounds; r++) {
-        unsigned c01[16], c23[16];
-        unsigned mn01 = 0xFFFFFFFFu, mx01 = 0u, mn23 = 0xFFFFFFFFu, mx23 = 0u;
         uint4 ob = make_uint4(0, 0, 0, 0);
         if (ORDERED) ob = __ldg(reinterpret_cast<const uint4*>(ordp + 16 * r));
         const unsigned ow[4] = {ob.x, ob.y, ob.z, ob.w};
-#pragma unroll
-        for (int t = 0; t < 16; t++) {
-            const int row = ORDERED ? (int)((ow[t >> 2] >> (8 * (t & 3))) & 0xFFu) : r * 16 + t;
-            const uint2 raw = __ldg(reinterpret_cast<const uint2*>(x + (int64_t)row * ss));
-            c01[t] = HALF ? h01.codes(raw.x) : packed_codes<T>(raw.x, q0, q1, k01);
-            c23[t] = HALF ? h23.codes(raw.y) : packed_codes<T>(raw.y, q2, q3, k23);
-            mn01 = min_u16x2(mn01, c01[t]); mx01 = max_u16x2(mx01, c01[t]);
-            mn23 = min_u16x2(mn23, c23[t]); mx23 = max_u16x2(mx23, c23[t]);
-        }
-        over |= mx01 | mx23;
-        const unsigned mnj[4] = {mn01 & 0xFFFFu, mn01 >> 16, mn23 & 0xFFFFu, mn23 >> 16};
-        const unsigned d01 = mx01 - mn01, d23 = mx23 - mn23;     // lane-wise: no borrow, max >= min
-        const unsigned dj[4] = {d01 & 0xFFFFu, d01 >> 16, d23 & 0xFFFFu, d23 >> 16};
-        unsigned minword = 0, lenword = 0, lens4 = 0;
-        int len[4];
-#pragma unroll
-        for (int j = 0; j < 4; j++) {
-            len[j] = min(bit_length_u32(dj[j]), BITS);
-            minword |= (mnj[j] & ((1u << BITS) - 1u)) << (j * BITS);
-            lenword |= (unsigned)len[j] << (j * LB);
-            lens4 |= (unsigned)len[j] << (8 * j);
-        }
-        store_lane_fields_w<4 * BITS>(stage + pos, lane, minword);
-        store_lane_fields_w<4 * LB>(stage + pos + g.min_bytes, lane, lenword);
-        const unsigned inc = warp_inclusive_sum(lens4);
-        const unsigned tot = __shfl_sync(0xffffffffu, inc, 31);
-        const unsigned exc = inc - lens4;
-        uint8_t* packs = stage + pos + g.min_bytes + g.len_bytes;
-        unsigned before = 0;
-#pragma unroll
-        for (int j = 0; j < 4; j++) {
-            // 16-bit lanes, four tokens each (token 0 and 4, 8 and 12 highest): w = w * 2^len + code for two of them per
-            // multiply-add, then the minimum is taken off all four fields at once (min * (1 + 2^len + ... + 2^(3 len))).
-            // A lane stays below 2^16: four codes below 2^4 at steps of at most 2^4.  Against one multiply-add and one
-            // extraction per code: 1.6 instead of 2.8 instructions per code.
-            const unsigned step = 1u << len[j], sel = (j & 1) ? 0x7632u : 0x5410u;
-            const unsigned(&cj)[16] = j < 2 ? c01 : c23;
-            unsigned za = __byte_perm(cj[0], cj[4], sel), zb = __byte_perm(cj[8], cj[12], sel);
-#pragma unroll
-            for (int t = 1; t < 4; t++) {
-                za = za * step + __byte_perm(cj[t], cj[t + 4], sel);
-                zb = zb * step + __byte_perm(cj[t + 8], cj[t + 12], sel);
-            }
-            const unsigned low = mnj[j] * ((1u + step) * (1u + step * step)) * 0x00010001u;
-            za -= low;
-            zb -= low;
-            const unsigned wt = ((za & 0xFFFFu) << (4 * len[j])) | (za >> 16), wb = ((zb & 0xFFFFu) << (4 * len[j])) | (zb >> 16);
-            const uint64_t w = ((uint64_t)wt << (8 * len[j])) | wb;
-            store_pack_smem(packs + 2 * (before + ((exc >> (8 * j)) & 0xFFu)), w, len[j]);
-            before += (tot >> (8 * j)) & 0xFFu;
-        }
-        const unsigned round_size = g.min_bytes + g.len_bytes + 2 * before;
-        round_end += round_size;
-        if (lane == 0) *reinterpret_cast<uint16_t*>(stage + 2 * r) = (uint16_t)round_end;
-        pos += round_size;
+        const auto row = [&](int t) {
+            const int at = ORDERED ? (int)((ow[t >> 2] >> (8 * (t & 3))) & 0xFFu) : r * 16 + t;
+            return __ldg(reinterpret_cast<const uint2*>(x + (int64_t)at * ss));
+        };
+        pos += MODE == 0 ? k_encode_round<T, false, BITS, false>(row, q0, q1, q2, q3, stage + pos, lane, over)
+                         : k_encode_round_packed<T, BITS, MODE == 2>(row, q0, q1, q2, q3, pq, stage + pos, lane, over);
+        if (lane == 0) *reinterpret_cast<uint16_t*>(stage + 2 * r) = (uint16_t)(pos - g.head_bytes);
     }
-    bad = bad || (over & ~(((1u << BITS) - 1u) * 0x00010001u)) != 0;
+    bad = bad || (MODE == 0 ? over : over & ~(((1u << BITS) - 1u) * 0x00010001u)) != 0;
     return pos;
 }
 
@@ -401,9 +406,9 @@ __global__ void __launch_bounds__(NW * 32, 768 / (NW * 32)) k_fused_encode_kerne
     const bool half_ok = __all_sync(0xffffffffu, q0.half_domain() && q1.half_domain() && q2.half_domain() && q3.half_domain());
     // reordered blocks (order_block == cb here): the table of this block's rows
     const uint8_t* ordp = ORDERED ? a.order + ((int64_t)b * nctx + cbi) * a.cb : nullptr;
-    if (!HP && half_ok) pos = k_encode_rounds_packed<T, BITS, true, ORDERED>(x, ss, ordp, q0, q1, q2, q3, g, stage, lane, bad);
-    else if (!HP && packable) pos = k_encode_rounds_packed<T, BITS, false, ORDERED>(x, ss, ordp, q0, q1, q2, q3, g, stage, lane, bad);
-    else pos = k_encode_rounds<T, HP, BITS, false, ORDERED>(x, ss, ordp, q0, q1, q2, q3, g, stage, lane, bad);
+    if (half_ok) pos = k_encode_rounds<T, BITS, 2, ORDERED>(x, ss, ordp, q0, q1, q2, q3, g, stage, lane, bad);
+    else if (packable) pos = k_encode_rounds<T, BITS, 1, ORDERED>(x, ss, ordp, q0, q1, q2, q3, g, stage, lane, bad);
+    else pos = k_encode_rounds<T, BITS, 0, ORDERED>(x, ss, ordp, q0, q1, q2, q3, g, stage, lane, bad);
     __syncwarp();
     }   // active
     if (direct) {
@@ -432,65 +437,56 @@ __global__ void __launch_bounds__(NW * 32, 768 / (NW * 32)) k_fused_encode_kerne
 template <int CB>
 __device__ __forceinline__ int v_swz(int ch) { return ((ch >> 1) ^ (ch >> 3)) & (CB / 16 - 1); }
 
-// Quantises one V block into the tile.  Lane (r0 = lane >> 3, cg = lane & 7) loads 8 channels
-// (16 bytes) of tokens r0, r0+4, r0+8, ... and, per pack, turns its 4 tokens x 8 channels into one
-// 4-token word per channel.  PACKED: two channels per instruction (all tokens packable()).
-// Returns the OR of all codes in 16-bit lanes for the range check.
+// Codes of the eight channels a lane holds of token `tok`, two to a word.
 template <typename T, int CB, int MODE>     // MODE 0: scalar conversion, 1: two elements per instruction in fp32, 2: in the element type
-__device__ __forceinline__ unsigned v_quantise_tile(const T* src, int64_t ss, const float4* prm, const uint8_t* ord, uint8_t* tile, int lane) {
-    constexpr bool PACKED = MODE == 1;
+__device__ __forceinline__ void v_quantise_row(const uint4& raw, const float4* prm, int tok, unsigned (&c)[4]) {
     const uint4* prmh = reinterpret_cast<const uint4*>(prm + CB);   // per token: r, -128*scale, r/128 (element-type pairs), code bias
-    const int r0 = lane >> 3, cg = lane & 7;
-    unsigned seen = 0;
+    const unsigned rw[4] = {raw.x, raw.y, raw.z, raw.w};
+    if (MODE == 2) {
+        const uint4 ph = prmh[tok];
+        HalfQuotient<T> hq;
+        hq.r = *reinterpret_cast<const typename QT<T>::T2*>(&ph.x);
+        hq.nsp = *reinterpret_cast<const typename QT<T>::T2*>(&ph.y);
+        hq.rp = *reinterpret_cast<const typename QT<T>::T2*>(&ph.z);
+        hq.kab = ph.w;
+        hq.magic = QT<T>::dup((float)(QT<T>::kIntBits == 0x6600u ? 1536 : 192));
+        hq.pre = QT<T>::dup(QT<T>::kPre);
+#pragma unroll
+        for (int i = 0; i < 4; i++) c[i] = hq.codes(rw[i]);
+        return;
+    }
+    const float4 pr = prm[tok];                            // scale, zero, 1/scale
+    Quantiser<T, false> qz;
+    qz.scale = pr.x; qz.zero = pr.y; qz.rcp = pr.z;
+    if (MODE == 1) {
+        const unsigned kab = __float_as_uint(pr.w);
+#pragma unroll
+        for (int i = 0; i < 4; i++) c[i] = packed_codes<T>(rw[i], qz, qz, kab);
+    } else {
+        const int zi = (int)pr.y;
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const float2 f = QT<T>::to_float2(rw[i]);
+            c[i] = qz.template code_u8<false>(f.x, zi) | (qz.template code_u8<false>(f.y, zi) << 16);
+        }
+    }
+}
+
+// A lane's place in the tile of 64 channels: lane (r0 = lane >> 3, cg = lane & 7) turns its 4 tokens x 8 channels of a pack into one
+// 4-token word per channel.
+template <int CB>
+struct TileLane {
     uint8_t* wr[4];                                        // row of channel 8cg + 2i at this lane's word, before the chunk swizzle
     int sw[4];
+    __device__ __forceinline__ TileLane(uint8_t* tile, int lane) {
+        const int r0 = lane >> 3, cg = lane & 7;
 #pragma unroll
-    for (int i = 0; i < 4; i++) {
-        wr[i] = tile + (8 * cg + 2 * i) * CB + 4 * r0;
-        sw[i] = v_swz<CB>(8 * cg + 2 * i) << 4;           // channels 8cg + 2i and + 1 share the swizzle
-    }
-    const T* lsrc = src + 8 * cg;
-#pragma unroll 1
-    for (int p = 0; p < CB / 16; p++) {
-        unsigned c[4][4];                                  // [token k][channel pair i] as 16-bit lanes
-#pragma unroll
-        for (int k = 0; k < 4; k++) {
-            const int tok = 16 * p + 4 * k + r0;
-            const uint4 raw = __ldg(reinterpret_cast<const uint4*>(lsrc + (int64_t)ord[tok] * ss));
-            const unsigned rw[4] = {raw.x, raw.y, raw.z, raw.w};
-            if (MODE == 2) {
-                const uint4 ph = prmh[tok];
-                HalfQuotient<T> hq;
-                hq.r = *reinterpret_cast<const typename QT<T>::T2*>(&ph.x);
-                hq.nsp = *reinterpret_cast<const typename QT<T>::T2*>(&ph.y);
-                hq.rp = *reinterpret_cast<const typename QT<T>::T2*>(&ph.z);
-                hq.kab = ph.w;
-                hq.magic = QT<T>::dup((float)(QT<T>::kIntBits == 0x6600u ? 1536 : 192));
-                hq.pre = QT<T>::dup(QT<T>::kPre);
-#pragma unroll
-                for (int i = 0; i < 4; i++) c[k][i] = hq.codes(rw[i]);
-#pragma unroll
-                for (int i = 0; i < 4; i++) seen |= c[k][i];
-                continue;
-            }
-            const float4 pr = prm[tok];                    // scale, zero, 1/scale
-            Quantiser<T, false> qz;
-            qz.scale = pr.x; qz.zero = pr.y; qz.rcp = pr.z;
-            if (PACKED) {
-                const unsigned kab = __float_as_uint(pr.w);
-#pragma unroll
-                for (int i = 0; i < 4; i++) c[k][i] = packed_codes<T>(rw[i], qz, qz, kab);
-            } else {
-                const int zi = (int)pr.y;
-#pragma unroll
-                for (int i = 0; i < 4; i++) {
-                    const float2 f = QT<T>::to_float2(rw[i]);
-                    c[k][i] = qz.template code_u8<false>(f.x, zi) | (qz.template code_u8<false>(f.y, zi) << 16);
-                }
-            }
-#pragma unroll
-            for (int i = 0; i < 4; i++) seen |= c[k][i];
+        for (int i = 0; i < 4; i++) {
+            wr[i] = tile + (8 * cg + 2 * i) * CB + 4 * r0;
+            sw[i] = v_swz<CB>(8 * cg + 2 * i) << 4;       // channels 8cg + 2i and + 1 share the swizzle
         }
+    }
+    __device__ __forceinline__ void store(int p, const unsigned (&c)[4][4]) const {   // [token k][channel pair i] as 16-bit lanes
 #pragma unroll
         for (int i = 0; i < 4; i++) {
             // (even channel | odd channel) x tokens 0..3 -> one word per channel
@@ -499,6 +495,30 @@ __device__ __forceinline__ unsigned v_quantise_tile(const T* src, int64_t ss, co
             *reinterpret_cast<unsigned*>(at) = __byte_perm(x, y, 0x5410);
             *reinterpret_cast<unsigned*>(at + CB) = __byte_perm(x, y, 0x7632);
         }
+    }
+};
+
+// Quantises one V block into the tile.  Lane (r0 = lane >> 3, cg = lane & 7) loads 8 channels
+// (16 bytes) of tokens r0, r0+4, r0+8, ...
+// Returns the OR of all codes in 16-bit lanes for the range check.
+template <typename T, int CB, int MODE>
+__device__ __forceinline__ unsigned v_quantise_tile(const T* src, int64_t ss, const float4* prm, const uint8_t* ord, uint8_t* tile, int lane) {
+    const int r0 = lane >> 3;
+    unsigned seen = 0;
+    const TileLane<CB> out(tile, lane);
+    const T* lsrc = src + 8 * (lane & 7);
+#pragma unroll 1
+    for (int p = 0; p < CB / 16; p++) {
+        unsigned c[4][4];
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            const int tok = 16 * p + 4 * k + r0;
+            const uint4 raw = __ldg(reinterpret_cast<const uint4*>(lsrc + (int64_t)ord[tok] * ss));
+            v_quantise_row<T, CB, MODE>(raw, prm, tok, c[k]);
+#pragma unroll
+            for (int i = 0; i < 4; i++) seen |= c[k][i];
+        }
+        out.store(p, c);
     }
     return seen;
 }
@@ -532,6 +552,85 @@ __device__ __forceinline__ void chunk_to_pack(const uint4& cw, int& len, uint64_
     wd = ((uint64_t)wt << (8 * len)) | wb;
 }
 
+// One segment of a V block (PPT packs of 16 tokens for each of 32 channels) from the tile: this lane's channel row and swizzle.
+// Minima, lengths, packs at `at`; returns the segment's bytes.
+template <int CB, int BITS>
+__device__ __forceinline__ unsigned v_pack_segment(const uint8_t* row, int swz, int r, uint8_t* at, int lane) {
+    constexpr int LB = len_field_bits(BITS), PPT = CB == 32 ? 2 : 4, kMin = BITS * PPT * 4, kLen = LB * PPT * 4;
+    unsigned minword = 0, lenword = 0, lens4 = 0;
+    uint64_t wd[4];
+    int len[4];
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+        len[q] = 0; wd[q] = 0;
+        if (q < PPT) {
+            // word r0 of the chunk: bytes k = tokens r0 + 4k of the pack
+            const uint4 cw = *reinterpret_cast<const uint4*>(row + (((r * PPT + q) ^ swz) << 4));
+            unsigned mn1;
+            chunk_to_pack<BITS>(cw, len[q], wd[q], mn1);
+            minword |= (mn1 & ((1u << BITS) - 1u)) << (q * BITS);
+            lenword |= (unsigned)len[q] << (q * LB);
+            lens4 |= (unsigned)len[q] << (8 * q);
+        }
+    }
+    store_lane_fields_w<PPT * BITS>(at, lane, minword);
+    store_lane_fields_w<PPT * LB>(at + kMin, lane, lenword);
+    const unsigned inc = warp_inclusive_sum(lens4);
+    const unsigned tot = __shfl_sync(0xffffffffu, inc, 31);
+    const unsigned exc = inc - lens4;
+    uint8_t* packs = at + kMin + kLen;
+    unsigned before = 0;
+#pragma unroll
+    for (int q = 0; q < 4; q++)
+        if (q < PPT) {
+            store_pack_smem(packs + 2 * (before + ((exc >> (8 * q)) & 0xFFu)), wd[q], len[q]);
+            before += (tot >> (8 * q)) & 0xFFu;
+        }
+    return kMin + kLen + 2 * before;
+}
+
+// One round (16 tokens x 128 channels) of a K block with per-token parameters from the two tiles of 64 channels
+template <int CB, int BITS>
+__device__ __forceinline__ unsigned kt_pack_round(const uint8_t* ctile, int r, uint8_t* at, int lane) {
+    constexpr int LB = len_field_bits(BITS), kMin = 16 * BITS, kLen = 16 * LB;
+    unsigned minword = 0, lenword = 0, lens4 = 0;
+    uint64_t wd[4];
+    int len[4];
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+        const int ch = 4 * lane + j;                       // this lane's channel row and its chunk swizzle
+        const uint8_t* row = ctile + (ch >> 6) * 64 * CB + (ch & 63) * CB;
+        const uint4 cw = *reinterpret_cast<const uint4*>(row + ((r ^ v_swz<CB>(ch & 63)) << 4));
+        unsigned mn1;
+        chunk_to_pack<BITS>(cw, len[j], wd[j], mn1);
+        minword |= (mn1 & ((1u << BITS) - 1u)) << (j * BITS);
+        lenword |= (unsigned)len[j] << (j * LB);
+        lens4 |= (unsigned)len[j] << (8 * j);
+    }
+    store_lane_fields_w<4 * BITS>(at, lane, minword);
+    store_lane_fields_w<4 * LB>(at + kMin, lane, lenword);
+    const unsigned inc = warp_inclusive_sum(lens4);
+    const unsigned tot = __shfl_sync(0xffffffffu, inc, 31);
+    const unsigned exc = inc - lens4;
+    uint8_t* packs = at + kMin + kLen;
+    unsigned before = 0;
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+        store_pack_smem(packs + 2 * (before + ((exc >> (8 * j)) & 0xFFu)), wd[j], len[j]);
+        before += (tot >> (8 * j)) & 0xFFu;
+    }
+    return kMin + kLen + 2 * before;
+}
+
+// What token_params_pass and the one-block kernel keep per token of one block
+template <typename T, int CB>
+__device__ __forceinline__ void put_token_params(const Quantiser<T, false>& qz, float4* prm, int t) {
+    prm[t] = make_float4(qz.scale, qz.zero, qz.rcp, __uint_as_float(qz.packable() ? packed_code_bias(qz, qz) : 0u));   // bias 0 = not packable
+    const HalfQuotient<T> hq(qz, qz);
+    reinterpret_cast<uint4*>(prm + CB)[t] = make_uint4(*reinterpret_cast<const unsigned*>(&hq.r), *reinterpret_cast<const unsigned*>(&hq.nsp),
+                                                       *reinterpret_cast<const unsigned*>(&hq.rp), qz.half_domain() ? hq.kab : 0u);
+}
+
 // Per-token quantisation parameters of one token block over all heads and channels (the
 // reference's token mode reduces over dims [1, 4], utils/compute.py:405-410): half a warp per token.
 // Writes (scale, zero, 1/scale, packed code bias or 0) to prm[] and scale / zero to the caller's arrays.
@@ -560,10 +659,7 @@ __device__ __forceinline__ bool token_params_pass(const FusedArgs& a, const T* x
         const Quantiser<T, false> qz(lo, hi, a.rel);
         bad = bad || qz.degenerate();
         if ((lane & 15) == 0) {
-            prm[t] = make_float4(qz.scale, qz.zero, qz.rcp, __uint_as_float(qz.packable() ? packed_code_bias(qz, qz) : 0u));   // bias 0 = not packable
-            const HalfQuotient<T> hq(qz, qz);
-            reinterpret_cast<uint4*>(prm + CB)[t] = make_uint4(*reinterpret_cast<const unsigned*>(&hq.r), *reinterpret_cast<const unsigned*>(&hq.nsp),
-                                                               *reinterpret_cast<const unsigned*>(&hq.rp), qz.half_domain() ? hq.kab : 0u);
+            put_token_params<T, CB>(qz, prm, t);
             if (WRITE) {
                 const int64_t pi = (int64_t)b * a.param_tokens + a.first_token + cbi * CB + t;
                 reinterpret_cast<T*>(a.scale)[pi] = QT<T>::cvt(qz.scale);
@@ -646,36 +742,7 @@ __global__ void __launch_bounds__(NW * 32, NW == 8 ? 3 : 1) v_fused_encode_kerne
             const uint8_t* row = ctile + ch * CB;
             const int swz = v_swz<CB>(ch);
             for (int r = 0; r < RPW; r++) {
-                unsigned minword = 0, lenword = 0, lens4 = 0;
-                uint64_t wd[4];
-                int len[4];
-#pragma unroll
-                for (int q = 0; q < 4; q++) {
-                    len[q] = 0; wd[q] = 0;
-                    if (q < PPT) {
-                        // word r0 of the chunk: bytes k = tokens r0 + 4k of the pack
-                        const uint4 cw = *reinterpret_cast<const uint4*>(row + (((r * PPT + q) ^ swz) << 4));
-                        unsigned mn1;
-                        chunk_to_pack<BITS>(cw, len[q], wd[q], mn1);
-                        minword |= (mn1 & ((1u << BITS) - 1u)) << (q * BITS);
-                        lenword |= (unsigned)len[q] << (q * LB);
-                        lens4 |= (unsigned)len[q] << (8 * q);
-                    }
-                }
-                store_lane_fields_w<PPT * BITS>(stage + pos, lane, minword);
-                store_lane_fields_w<PPT * LB>(stage + pos + g.min_bytes, lane, lenword);
-                const unsigned inc = warp_inclusive_sum(lens4);
-                const unsigned tot = __shfl_sync(0xffffffffu, inc, 31);
-                const unsigned exc = inc - lens4;
-                uint8_t* packs = stage + pos + g.min_bytes + g.len_bytes;
-                unsigned before = 0;
-#pragma unroll
-                for (int q = 0; q < 4; q++)
-                    if (q < PPT) {
-                        store_pack_smem(packs + 2 * (before + ((exc >> (8 * q)) & 0xFFu)), wd[q], len[q]);
-                        before += (tot >> (8 * q)) & 0xFFu;
-                    }
-                const unsigned seg_size = g.min_bytes + g.len_bytes + 2 * before;
+                const unsigned seg_size = v_pack_segment<CB, BITS>(row, swz, r, stage + pos, lane);
                 seg_end += seg_size;
                 if (lane == 0) *reinterpret_cast<uint16_t*>(stage + 2 * (w * RPW + r)) = (uint16_t)seg_end;
                 pos += seg_size;
@@ -741,43 +808,10 @@ __global__ void __launch_bounds__(256, 2) kt_fused_encode_kernel(FusedArgs a) {
                              : all_packed ? v_quantise_tile<T, CB, 1>(src + 64 * half, a.ss, prm, ord, ctile + half * 64 * CB, lane)
                                           : v_quantise_tile<T, CB, 0>(src + 64 * half, a.ss, prm, ord, ctile + half * 64 * CB, lane);
         __syncwarp();
-        // this lane's four channel rows and their chunk swizzles
-        const uint8_t* row[4];
-        int swz[4];
-#pragma unroll
-        for (int j = 0; j < 4; j++) {
-            const int ch = 4 * lane + j;
-            row[j] = ctile + (ch >> 6) * 64 * CB + (ch & 63) * CB;
-            swz[j] = v_swz<CB>(ch & 63);
-        }
         int pos = g.head_bytes;
         unsigned round_end = 0;
         for (int r = 0; r < g.rounds; r++) {
-            unsigned minword = 0, lenword = 0, lens4 = 0;
-            uint64_t wd[4];
-            int len[4];
-#pragma unroll
-            for (int j = 0; j < 4; j++) {
-                const uint4 cw = *reinterpret_cast<const uint4*>(row[j] + ((r ^ swz[j]) << 4));
-                unsigned mn1;
-                chunk_to_pack<BITS>(cw, len[j], wd[j], mn1);
-                minword |= (mn1 & ((1u << BITS) - 1u)) << (j * BITS);
-                lenword |= (unsigned)len[j] << (j * LB);
-                lens4 |= (unsigned)len[j] << (8 * j);
-            }
-            store_lane_fields_w<4 * BITS>(stage + pos, lane, minword);
-            store_lane_fields_w<4 * LB>(stage + pos + g.min_bytes, lane, lenword);
-            const unsigned inc = warp_inclusive_sum(lens4);
-            const unsigned tot = __shfl_sync(0xffffffffu, inc, 31);
-            const unsigned exc = inc - lens4;
-            uint8_t* packs = stage + pos + g.min_bytes + g.len_bytes;
-            unsigned before = 0;
-#pragma unroll
-            for (int j = 0; j < 4; j++) {
-                store_pack_smem(packs + 2 * (before + ((exc >> (8 * j)) & 0xFFu)), wd[j], len[j]);
-                before += (tot >> (8 * j)) & 0xFFu;
-            }
-            const unsigned round_size = g.min_bytes + g.len_bytes + 2 * before;
+            const unsigned round_size = kt_pack_round<CB, BITS>(ctile, r, stage + pos, lane);
             round_end += round_size;
             if (lane == 0) *reinterpret_cast<uint16_t*>(stage + 2 * r) = (uint16_t)round_end;
             pos += round_size;
@@ -794,6 +828,247 @@ __global__ void __launch_bounds__(256, 2) kt_fused_encode_kernel(FusedArgs a) {
     if (direct)
         chain_store(a, b, cbi, sh_sizes, a.heads, &sh_word, (int64_t)(a.first_cb + cbi) * a.heads, 8,
                     [&](int j) { return smem + 32 * CB + j * (CB * 128 + bound16) + CB * 128; });
+    bad = bad || (seen & ~(((1u << BITS) - 1u) * 0x00010001u)) != 0;
+    if (__any_sync(0xffffffffu, bad) && lane == 0) atomicOr(a.flags, kFlagCodeRange);
+}
+
+// ------------------------------------------------------------------- one block of every sequence
+// Launches of one token block per sequence (what leaves the residual in a decode step): their time is the latency of one CTA's
+// chain of loads, quantising, packing and storing, so the block is spread over a cluster of `heads` CTAs of four warps, one head
+// to a CTA.  A warp holds its rows in registers from one round of loads, packs a round (K) or segments (V) of its own into shared
+// memory, and stores it where the sizes of the parts before it put it: inside the CTA through shared memory, across the heads
+// through distributed shared memory (no look-back, no scratch).  16 sequences x 64 tokens x 8 heads, four layers' K and V: 98 us
+// with one CTA per sequence, 49 us this way.
+constexpr int kOneWarps = 4;
+constexpr int kOneBlockCtas = 4 * kSmCount;
+
+// Launched under programmatic stream serialisation: its CTAs are placed while the launch before drains, and touch nothing before
+// that one is complete; the launch after it may be placed from here on.
+__device__ __forceinline__ void one_block_begin() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
+// The CTA's `n` parts (sizes[], packed at part(i)) of `blocks` equal blocks, n / blocks parts each: tables of part ends, table
+// entries and bytes to the stream.  All threads call; two cluster barriers.  `total`: shared word that the other CTAs read.
+template <typename Part>
+__device__ __forceinline__ void one_block_store(const FusedArgs& a, int b, int blocks, const unsigned* sizes, int n, unsigned* total, int64_t info_first, Part part) {
+    cg::cluster_group cluster = cg::this_cluster();
+    const int lane = lane_id(), wic = threadIdx.x >> 5, rank = (int)cluster.block_rank(), per = n / blocks, head = 2 * per;
+    const unsigned base = a.first_cb == 0 ? 0u : a.stream_bytes[b];    // read by all before the last CTA writes it
+    __syncthreads();                                                   // the parts and their sizes are there
+    if (threadIdx.x == 0) {
+        unsigned sum = (unsigned)(blocks * head);
+        for (int i = 0; i < n; i++) sum += sizes[i];
+        *total = sum;
+    }
+    cluster.sync();
+    const unsigned other = lane < (int)cluster.num_blocks() ? *cluster.map_shared_rank(total, lane) : 0u;
+    const unsigned first = base + warp_sum(lane < rank ? other : 0u), all = base + warp_sum(other);
+    if (rank == (int)cluster.num_blocks() - 1 && threadIdx.x == 0) a.stream_bytes[b] = all;
+    unsigned off = first;
+    for (int blk = 0; blk < blocks; blk++) {
+        unsigned size = (unsigned)head;
+        for (int i = 0; i < per; i++) size += sizes[blk * per + i];
+        if (wic == 0 && lane == 0) {
+            uint32_t* bi = a.info + ((int64_t)b * a.info_seq_stride + info_first + blk) * 2;
+            bi[0] = off; bi[1] = size;
+        }
+        if ((int64_t)off + size > a.capacity) {
+            if (wic == 0 && lane == 0) atomicOr(a.flags, kFlagStreamOverflow);
+        } else {
+            uint8_t* dst = a.stream + (int64_t)b * a.stream_seq_stride + off;
+            unsigned end = 0;
+            for (int i = 0; i < per; i++) {
+                const unsigned bytes = sizes[blk * per + i];
+                if ((blk * per + i) % kOneWarps == wic) {
+                    store_block(dst + head + end, part(blk * per + i), (int)bytes, lane);
+                    if (lane == 0) *reinterpret_cast<uint16_t*>(dst + 2 * i) = (uint16_t)(end + bytes);
+                }
+                end += bytes;
+            }
+        }
+        off += size;
+    }
+    cluster.sync();                                                    // the others have read `total`
+}
+
+// K with per-channel parameters, CB / 16 rounds of 16 tokens dealt to the warps
+template <typename T, int BITS, int CB>
+__global__ void __launch_bounds__(kOneWarps * 32) k_one_block_kernel(FusedArgs a) {
+    one_block_begin();
+    constexpr int kRounds = CB / 16, kMine = (kRounds + kOneWarps - 1) / kOneWarps, kBound = (16 * BITS + 16 * len_field_bits(BITS) + 256 * BITS + 15) & ~15;
+    using T2 = typename QT<T>::T2;
+    __shared__ __align__(16) uint8_t stage[kRounds][kBound];
+    __shared__ uint4 extremes[kOneWarps][kLanes];
+    __shared__ unsigned sizes[kRounds], total;
+    const int lane = lane_id(), wic = threadIdx.x >> 5, h = blockIdx.x, b = blockIdx.y;
+    const T* x = reinterpret_cast<const T*>(a.x) + (int64_t)b * a.sb + (int64_t)h * a.sh + 4 * lane;
+    uint2 rows[kMine][16];
+    T2 lo01 = QT<T>::init2(INFINITY), lo23 = lo01, hi01 = QT<T>::init2(-INFINITY), hi23 = hi01;
+#pragma unroll
+    for (int i = 0; i < kMine; i++) {
+        const int r = wic + kOneWarps * i;
+        if (r < kRounds) {
+#pragma unroll
+            for (int t = 0; t < 16; t++) {
+                const int row = a.order ? a.order[(int64_t)b * CB + 16 * r + t] : 16 * r + t;
+                rows[i][t] = *reinterpret_cast<const uint2*>(x + (int64_t)row * a.ss);
+            }
+#pragma unroll
+            for (int t = 0; t < 16; t++) {
+                const T2 v01 = *reinterpret_cast<const T2*>(&rows[i][t].x), v23 = *reinterpret_cast<const T2*>(&rows[i][t].y);
+                lo01 = QT<T>::min2(lo01, v01); hi01 = QT<T>::max2(hi01, v01);
+                lo23 = QT<T>::min2(lo23, v23); hi23 = QT<T>::max2(hi23, v23);
+            }
+        }
+    }
+    extremes[wic][lane] = make_uint4(*reinterpret_cast<unsigned*>(&lo01), *reinterpret_cast<unsigned*>(&lo23), *reinterpret_cast<unsigned*>(&hi01),
+                                     *reinterpret_cast<unsigned*>(&hi23));
+    __syncthreads();
+#pragma unroll
+    for (int w = 0; w < kOneWarps; w++) {
+        const uint4 e = extremes[w][lane];
+        lo01 = QT<T>::min2(lo01, *reinterpret_cast<const T2*>(&e.x)); lo23 = QT<T>::min2(lo23, *reinterpret_cast<const T2*>(&e.y));
+        hi01 = QT<T>::max2(hi01, *reinterpret_cast<const T2*>(&e.z)); hi23 = QT<T>::max2(hi23, *reinterpret_cast<const T2*>(&e.w));
+    }
+    const Quantiser<T, false> q0(QT<T>::lo_f(lo01), QT<T>::lo_f(hi01), a.rel), q1(QT<T>::hi_f(lo01), QT<T>::hi_f(hi01), a.rel);
+    const Quantiser<T, false> q2(QT<T>::lo_f(lo23), QT<T>::lo_f(hi23), a.rel), q3(QT<T>::hi_f(lo23), QT<T>::hi_f(hi23), a.rel);
+    if (wic == 0) {
+        const int64_t pi = (((int64_t)b * a.heads + h) * a.param_blocks + a.first_block) * 128 + 4 * lane;
+        T sc[4] = {QT<T>::cvt(q0.scale), QT<T>::cvt(q1.scale), QT<T>::cvt(q2.scale), QT<T>::cvt(q3.scale)};
+        T zr[4] = {QT<T>::cvt(q0.zero), QT<T>::cvt(q1.zero), QT<T>::cvt(q2.zero), QT<T>::cvt(q3.zero)};
+        *reinterpret_cast<uint2*>(reinterpret_cast<T*>(a.scale) + pi) = *reinterpret_cast<const uint2*>(sc);
+        *reinterpret_cast<uint2*>(reinterpret_cast<T*>(a.zero) + pi) = *reinterpret_cast<const uint2*>(zr);
+    }
+    bool bad = q0.degenerate() || q1.degenerate() || q2.degenerate() || q3.degenerate();
+    const bool packable = __all_sync(0xffffffffu, q0.packable() && q1.packable() && q2.packable() && q3.packable());
+    const bool half_ok = __all_sync(0xffffffffu, q0.half_domain() && q1.half_domain() && q2.half_domain() && q3.half_domain());
+    const PackedQuantisers<T> pq(q0, q1, q2, q3);
+#pragma unroll
+    for (int i = 0; i < kMine; i++) {
+        const int r = wic + kOneWarps * i;
+        if (r < kRounds) {
+            const auto row = [&](int t) { return rows[i][t]; };
+            unsigned over = 0, size;
+            if (half_ok || packable) {
+                size = half_ok ? k_encode_round_packed<T, BITS, true>(row, q0, q1, q2, q3, pq, stage[r], lane, over)
+                               : k_encode_round_packed<T, BITS, false>(row, q0, q1, q2, q3, pq, stage[r], lane, over);
+                over &= ~(((1u << BITS) - 1u) * 0x00010001u);
+            } else {
+                size = k_encode_round<T, false, BITS, false>(row, q0, q1, q2, q3, stage[r], lane, over);
+            }
+            bad = bad || over != 0;
+            if (lane == 0) sizes[r] = size;
+        }
+    }
+    one_block_store(a, b, 1, sizes, kRounds, &total, (int64_t)a.first_cb * a.heads + h, [&](int i) { return stage[i]; });
+    if (__any_sync(0xffffffffu, bad) && lane == 0) atomicOr(a.flags, kFlagCodeRange);
+}
+
+// Per-token parameters: V (two blocks of 64 channels a head), or K in its own layout (IS_K: one block of 128 channels).  The
+// parameters span the heads: every CTA gets the other heads' minima and maxima through distributed shared memory.
+template <typename T, int BITS, int CB, bool IS_K>
+__global__ void __launch_bounds__(kOneWarps * 32) token_one_block_kernel(FusedArgs a) {
+    one_block_begin();
+    // packs of 16 tokens: two warps to each half of the channels, which take every other half of the packs
+    constexpr int kPacks = CB / 16, kMine = kPacks / 2, kSegs = CB == 128 ? 4 : 2, kParts = IS_K ? kPacks : 2 * kSegs;
+    constexpr int kBound = (16 * BITS + 16 * len_field_bits(BITS) + 256 * BITS + 15) & ~15;
+    using T2 = typename QT<T>::T2;
+    __shared__ __align__(16) uint8_t tile[2 * 64 * CB];
+    __shared__ float4 prm[2 * CB];
+    __shared__ __align__(16) uint8_t stage[kParts][kBound];
+    __shared__ unsigned range[2][CB], sizes[kParts], total;        // range: (minimum, -maximum) of a token, by half; then of this head
+    cg::cluster_group cluster = cg::this_cluster();
+    const int lane = lane_id(), wic = threadIdx.x >> 5, h = blockIdx.x, b = blockIdx.y;
+    const int half = wic & 1, p0 = (wic >> 1) * kMine, r0 = lane >> 3;
+    const T* src = reinterpret_cast<const T*>(a.x) + (int64_t)b * a.sb + (int64_t)h * a.sh + 64 * half + 8 * (lane & 7);
+    uint4 raw[kMine][4];
+#pragma unroll
+    for (int i = 0; i < kMine; i++)
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            const int t = 16 * (p0 + i) + 4 * k + r0;
+            const int row = a.order ? t / a.order_block * a.order_block + a.order[(int64_t)b * CB + t] : t;
+            raw[i][k] = *reinterpret_cast<const uint4*>(src + (int64_t)row * a.ss);
+        }
+    const auto min_of = [](unsigned x, unsigned y) {
+        const T2 m = QT<T>::min2(*reinterpret_cast<const T2*>(&x), *reinterpret_cast<const T2*>(&y));
+        return *reinterpret_cast<const unsigned*>(&m);
+    };
+#pragma unroll
+    for (int i = 0; i < kMine; i++)
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            const T2 v0 = *reinterpret_cast<const T2*>(&raw[i][k].x), v1 = *reinterpret_cast<const T2*>(&raw[i][k].y);
+            const T2 v2 = *reinterpret_cast<const T2*>(&raw[i][k].z), v3 = *reinterpret_cast<const T2*>(&raw[i][k].w);
+            const T2 lo2 = QT<T>::min2(QT<T>::min2(v0, v1), QT<T>::min2(v2, v3)), hi2 = QT<T>::max2(QT<T>::max2(v0, v1), QT<T>::max2(v2, v3));
+            const unsigned l = *reinterpret_cast<const unsigned*>(&lo2), u = *reinterpret_cast<const unsigned*>(&hi2) ^ 0x80008000u;   // -max: one minimum serves both
+            unsigned m = min_of(__byte_perm(l, u, 0x5410), __byte_perm(l, u, 0x7632));
+#pragma unroll
+            for (int s = 4; s > 0; s >>= 1) m = min_of(m, __shfl_xor_sync(0xffffffffu, m, s));
+            if ((lane & 7) == 0) range[half][16 * (p0 + i) + 4 * k + r0] = m;
+        }
+    __syncthreads();
+    for (int t = threadIdx.x; t < CB; t += kOneWarps * 32) range[0][t] = min_of(range[0][t], range[1][t]);
+    cluster.sync();
+    bool bad = false;
+    for (int t = threadIdx.x; t < CB; t += kOneWarps * 32) {
+        // (a minimum of nothing but NaN is infinity, as in token_params_pass)
+        const T2 none = QT<T>::init2(INFINITY);
+        unsigned m = *reinterpret_cast<const unsigned*>(&none);
+        for (int r = 0; r < a.heads; r++) m = min_of(m, cluster.map_shared_rank(&range[0][0], r)[t]);
+        const T2 both = *reinterpret_cast<const T2*>(&m);
+        const Quantiser<T, false> qz(QT<T>::lo_f(both), -QT<T>::hi_f(both), a.rel);
+        bad = bad || qz.degenerate();
+        put_token_params<T, CB>(qz, prm, t);
+        if (h == 0) {
+            const int64_t pi = (int64_t)b * a.param_tokens + a.first_token + t;
+            reinterpret_cast<T*>(a.scale)[pi] = QT<T>::cvt(qz.scale);
+            reinterpret_cast<T*>(a.zero)[pi] = QT<T>::cvt(qz.zero);
+        }
+    }
+    __syncthreads();
+    bool mine_ok = true, mine_half = true;
+    for (int t = threadIdx.x; t < CB; t += kOneWarps * 32) {
+        mine_ok = mine_ok && __float_as_uint(prm[t].w) != 0u;
+        mine_half = mine_half && reinterpret_cast<const uint4*>(prm + CB)[t].w != 0u;
+    }
+    const bool all_packed = __syncthreads_and(mine_ok);
+    const bool all_half = __syncthreads_and(mine_half);
+    unsigned seen = 0;
+    const TileLane<CB> out(tile + half * 64 * CB, lane);
+    const auto quantise = [&](auto mode) {
+#pragma unroll
+        for (int i = 0; i < kMine; i++) {
+            unsigned c[4][4];
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                v_quantise_row<T, CB, decltype(mode)::value>(raw[i][k], prm, 16 * (p0 + i) + 4 * k + r0, c[k]);
+#pragma unroll
+                for (int j = 0; j < 4; j++) seen |= c[k][j];
+            }
+            out.store(p0 + i, c);
+        }
+    };
+    if (all_half) quantise(std::integral_constant<int, 2>{});
+    else if (all_packed) quantise(std::integral_constant<int, 1>{});
+    else quantise(std::integral_constant<int, 0>{});
+    __syncthreads();
+    for (int i = wic; i < kParts; i += kOneWarps) {
+        unsigned size;
+        if (IS_K) {
+            size = kt_pack_round<CB, BITS>(tile, i, stage[i], lane);
+        } else {
+            // segment i % kSegs of block i / kSegs: 32 channels, then the other 32
+            constexpr int kHalfSegs = kSegs / 2;
+            const int s = i % kSegs, ch = 32 * (s / kHalfSegs) + lane;
+            size = v_pack_segment<CB, BITS>(tile + (i / kSegs) * 64 * CB + ch * CB, v_swz<CB>(ch), s % kHalfSegs, stage[i], lane);
+        }
+        if (lane == 0) sizes[i] = size;
+    }
+    constexpr int kBlocks = IS_K ? 1 : 2;
+    one_block_store(a, b, kBlocks, sizes, kParts, &total, ((int64_t)a.first_cb * a.heads + h) * kBlocks, [&](int i) { return stage[i]; });
     bad = bad || (seen & ~(((1u << BITS) - 1u) * 0x00010001u)) != 0;
     if (__any_sync(0xffffffffu, bad) && lane == 0) atomicOr(a.flags, kFlagCodeRange);
 }
@@ -999,6 +1274,34 @@ static int launch_fused_t(const FusedEncodeRequest& r, uint8_t* slots, const uin
     static const bool env_slots = [] { const char* v = std::getenv("PKV_ENCODE_PATH"); return v && std::string(v) == "slots"; }();
     const bool per_token_kernel = r.which == 1 || r.mode == 1;
     const bool k_one = !per_token_kernel && nctx * r.heads <= kKWarpsOne;
+    // One token block per sequence and few sequences: one head to a CTA of a cluster (see k_one_block_kernel).
+    if (!env_slots && nctx == 1 && r.heads <= 8 && (int64_t)r.batch * r.heads <= kOneBlockCtas) {
+        a.stream = r.stream; a.stream_seq_stride = r.stream_seq_stride; a.capacity = r.capacity; a.stream_bytes = reinterpret_cast<unsigned*>(r.stream_bytes);
+        const auto by_block = [&](auto cb) {
+            constexpr int CB = decltype(cb)::value;
+            void (*kern)(FusedArgs) = r.which == 1 ? token_one_block_kernel<T, BITS, CB, false>
+                                      : r.mode == 1 ? token_one_block_kernel<T, BITS, CB, true> : k_one_block_kernel<T, BITS, CB>;
+            cudaLaunchConfig_t cfg = {};
+            cfg.gridDim = dim3(r.heads, r.batch, 1);
+            cfg.blockDim = dim3(kOneWarps * 32, 1, 1);
+            cfg.stream = st;
+            cudaLaunchAttribute attr[2];
+            attr[0].id = cudaLaunchAttributeClusterDimension;
+            attr[0].val.clusterDim.x = r.heads;
+            attr[0].val.clusterDim.y = 1;
+            attr[0].val.clusterDim.z = 1;
+            attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+            attr[1].val.programmaticStreamSerializationAllowed = 1;
+            cfg.attrs = attr;
+            cfg.numAttrs = 2;
+            if (cudaLaunchKernelEx(&cfg, kern, a) == cudaSuccess) return (int)kOk;
+            cudaGetLastError();
+            return (int)kCudaError;
+        };
+        if (r.cb == 32) return by_block(std::integral_constant<int, 32>{});
+        if (r.cb == 64) return by_block(std::integral_constant<int, 64>{});
+        return by_block(std::integral_constant<int, 128>{});
+    }
     const int links = per_token_kernel ? nctx : k_one ? 1 : (nctx * r.heads + kKWarps - 1) / kKWarps;
     const int64_t chain_bytes = 256 + (int64_t)r.batch * links * 8;
     // (128-token blocks in the per-token kernels: a second staging buffer per warp would leave one CTA per SM; measured

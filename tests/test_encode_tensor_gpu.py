@@ -159,3 +159,44 @@ def test_launch_forms_by_size(cuda_device, which, mode, H, S, block, bits):
         assert np.array_equal(bufs["info"][b].cpu().numpy().view(np.uint32), wi)
     assert torch.equal(bufs["scale"].cpu().view(torch.int16), s.reshape(bufs["scale"].shape).contiguous().view(torch.int16))
     assert torch.equal(bufs["zero"].cpu().view(torch.int16), z.reshape(bufs["zero"].shape).contiguous().view(torch.int16))
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("which,mode", [("k", ops.K_CHANNEL), ("v", ops.K_TOKEN), ("k", ops.K_TOKEN)])
+@pytest.mark.parametrize("values", ["synthetic", "wide", "tiny", "special"])
+def test_one_block_of_every_sequence(cuda_device, which, mode, dtype, values):
+    """A call of one token block per sequence (a cluster of one-head CTAs) writes what a call of two blocks does: every block size and bit
+    width, 1 to 8 heads, rows in any strides and through an order, parameters outside of the half-precision domain and without valid
+    codes, the flags among the outputs; and a stream that is too small is flagged."""
+    dev, gen = cuda_device, torch.Generator(device=cuda_device).manual_seed(7)
+    for cb, bits, H in ((32, 4, 3), (64, 4, 8), (64, 3, 1), (64, 2, 5), (128, 4, 8), (128, 2, 2)):
+        B, S = 3, 2 * cb
+        x = torch.randn(B, S, H, 128, generator=gen, device=dev)
+        if values == "wide":
+            x = x * 900 + 3000
+        elif values == "tiny":
+            x = x * 1e-6
+        elif values == "special":
+            x[0, 3] = 0.0
+            x[1, 5, 0, 7] = float("nan")
+            x[1, cb + 1] = float("nan")
+            x[2, 9, H - 1, 100] = float("inf")
+            x[2, 2] = -0.0
+        x = x.to(dtype).transpose(1, 2)                             # (B, H, S, 128), token-major in memory
+        rel = synth.rel_for_bits(bits)
+        order = None
+        if cb == 64 and bits == 4:
+            order = torch.stack([torch.randperm(cb, generator=torch.Generator().manual_seed(i)) for i in range(2 * B)]).view(B, 2, cb).to(torch.uint8).to(dev)
+        two, one = (_bufs(B, H, S, cb, bits, which, mode, dtype, dev) for _ in range(2))
+        ops.encode_tensor(which, x, cb, rel, mode, bits, cb, **two, **({} if order is None else dict(order=order, order_block=cb)))
+        for i in range(2):
+            ops.encode_tensor(which, x[:, :, i * cb: (i + 1) * cb], cb, rel, mode, bits, cb, first_token=i * cb, **one,
+                              **({} if order is None else dict(order=order[:, i].contiguous(), order_block=cb)))
+        for name in two:
+            assert torch.equal(one[name].view(torch.uint8), two[name].view(torch.uint8)), (cb, bits, H, name)
+        if values == "synthetic":
+            assert int(one["flags"].item()) == 0
+            small = _bufs(B, H, S, cb, bits, which, mode, dtype, dev)
+            small["stream"] = torch.zeros(B, 256, dtype=torch.uint8, device=dev)
+            ops.encode_tensor(which, x[:, :, :cb], cb, rel, mode, bits, cb, **small, **({} if order is None else dict(order=order[:, 0].contiguous(), order_block=cb)))
+            assert int(small["flags"].item()) == 1 and torch.equal(small["info"][:, : one["info"].shape[1] // 2], one["info"][:, : one["info"].shape[1] // 2])
