@@ -268,6 +268,7 @@ struct AttnDev {
     int slot;            // bytes of one staging slot
     int nslots;          // staging slots per warp: 2 = the next block is copied while this one is unpacked
     int team;            // single launch: the warps of a CTA share its tiles (see TEAM)
+    int serial;          // launched under programmatic stream serialisation: waits for the launch before by itself (launch_attention)
     int early;           // single launch that may start while the one before drains (launch_attention)
     int dim;             // channels of q's rows and of the new token's: 128, or a narrow head's 64 .. 120 (the stored rows repeat their first ones behind them)
     int vpair;           // 64-token V blocks: an item is the pair of blocks of one token block (both channel halves)
@@ -389,9 +390,9 @@ __global__ void __launch_bounds__(kAW * 32, PASS == 1 ? PKV_ATTN_CTAS_SCORES : P
     __syncthreads();
     asm volatile("" : "+r"(lutm_a) :: "memory");        // reads of the table stay behind the barrier
     if (PASS != kValues) {
-        // Small single launches are started under programmatic stream serialisation (P.early): the lines above overlap the
-        // end of the launch before; nothing it may have written (q, tables, residual) is touched before it is complete, and
-        // the launch after this one may be set up from here on.
+        // Launches are started under programmatic stream serialisation (P.serial): the lines above overlap the end of the launch
+        // before; nothing it may have written (q, tables, residual) is touched before it is complete.  Where P.early, the
+        // launch after this one may be set up from here on.
         asm volatile("griddepcontrol.wait;" ::: "memory");
         if (PASS == kFused && P.early) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     }
@@ -1261,8 +1262,9 @@ __global__ void __launch_bounds__(kAW * 32, PASS == 1 ? PKV_ATTN_CTAS_SCORES : P
         }
     }
     __syncwarp();
-    // a launch that follows under programmatic stream serialisation (the exchange's wait) may be set up from here on
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    // the exchange's wait, launched under programmatic stream serialisation, may be set up from here on; other launches are placed once
+    // every CTA of this one has ended (see launch_attention)
+    if (P.x.n_ranks > 0) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     if (TEAM) {
 #pragma unroll
         for (int mt = 0; mt < 8; mt++)
@@ -1410,10 +1412,10 @@ static int launch_one(const AttnDev& P, dim3 grid, int smem, cudaStream_t st) {
     attr[0].val.clusterDim.y = 1;
     attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
-    // a launch may start while the one before it drains; it waits for it on the device (griddepcontrol.wait): the second of
-    // two launches with its first copies under way, a small single launch with its shared memory set up
+    // a launch may be placed before the one before it is complete; it waits for it on the device (griddepcontrol.wait): the second of
+    // two launches with its first copies under way, the others with their shared memory set up
     cfg.numAttrs = 1;
-    if (PASS == kValues || P.early) {
+    if (PASS == kValues || P.serial) {
         attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
         attr[1].val.programmaticStreamSerializationAllowed = 1;
         cfg.numAttrs = 2;
@@ -1799,9 +1801,13 @@ int launch_attention(const AttnArgs& a, const AttnExchange* xch, const AttnAppen
     P.team = best_launches == 1 && team_wins(best_cl);
     const int smem = plan_smem(P, best_cl, best_split, best_ns, slot);
     P.extra = best_extra;
-    // At most one CTA per SM: 8 KV heads x 700 tokens 14.3 -> 13.0 us a launch.  Fuller launches stay ordered: their CTAs would
-    // be placed around those still running, unevenly (11 x 2154: 30 -> 34 us; two launches 0 to 5 % slower).  So do launches
-    // with an exchange, which were not measured.
+    // Launches without an exchange are placed as soon as every CTA of the launch before has ended, and wait for its completion on the
+    // device: in stream order they start when the whole launch is known to be complete, up to 2 us later on launches of 10 to 40 us
+    // (4 x 500 tokens 12.4 -> 9.6 us a launch, 5 x 5333 in two launches 26.7 -> 24.8, 16 x 8k 115.7 -> 113.3).  At most one CTA per SM:
+    // as soon as every CTA of the launch before has begun (8 KV heads x 700 tokens 14.3 -> 13.0 us).  Fuller launches would be placed
+    // around those still running, unevenly (11 x 2154: 30 -> 34 us; two launches 0 to 5 % slower).  Launches with an exchange stay in
+    // stream order: they were not measured.
+    P.serial = !xch;
     P.early = best_launches == 1 && !xch && pairs * best_cl <= kSmCount;
     if (best_launches == 2) {
         const ScratchLayout L = scratch_layout(pairs, best_cl, best_extra >= 0 ? best_split + 1 : best_split, P.dump_bytes);

@@ -8,7 +8,8 @@ import pytest
 import torch
 
 from oracle import quant as Q
-from packkv_b200 import ops, synth
+from packkv_b200 import encode, ops, synth
+from packkv_b200.config import QuantMode
 from tests.helpers import layer_from_oracle
 
 pytestmark = pytest.mark.gpu
@@ -473,6 +474,77 @@ def test_back_to_back_steps_equal_synchronised_steps(cuda_device, n_comp, plan):
         torch.cuda.synchronize()
         for n in range(steps):
             ops.decode_attention(x, layer, k_res, v_res, n0 + n + 1, out=y, flags=flags, append=(new[0][n], new[1][n], None, None), scratch=scratch, plan=plan,
+                                 scaling=1.0)
+            x, y = y, x
+            if wait:
+                torch.cuda.synchronize()
+        torch.cuda.synchronize()
+        assert int(flags.item()) == 0
+        got.append((x, y, k_res, v_res))
+    for a, b in zip(*got):
+        assert torch.equal(a.view(torch.int16), b.view(torch.int16))
+
+
+@pytest.mark.parametrize("cl", range(1, 17))
+def test_every_cluster_size(cuda_device, cl):
+    """The cluster's CTAs share out the output rows and gather one another's maxima and sums: every cluster size, groups that give
+    its CTAs several, one or no rows each, in one launch and in two."""
+    for G, n_comp, plan in ((8, 1536, (cl, 1, 1)), (1, 192, (cl, 1, 1)), (7, 1024, (cl, 3, 2))):
+        err = _run_case(cuda_device, torch.bfloat16, 2, 1, G, n_comp, 140, block=64, cbk=64, cbv=64, bits_k=4, bits_v=3, k_mode="channel", seed=80 + G,
+                        plan=plan, repeats=2)
+        assert err <= TOL, (G, err)
+
+
+def test_plans_do_not_depend_on_what_was_planned_before(cuda_device):
+    """The last few plans of a thread are kept: shapes asked for in turn, again, and by other threads get the plan of a first call, and
+    launches that need more and less shared memory than the ones before them run."""
+    from concurrent.futures import ThreadPoolExecutor
+    dev, dtype, H = cuda_device, torch.float16, 2
+    scratch = ops.new_attention_scratch(dev)
+    res = torch.randn(6, H, 192, 128, device=dev).to(dtype)
+    k, v = synth.synth_kv(6, H, 1024, 128, seed=9, dtype=dtype, device=dev)
+    layers = {(B, n): encode.compress_kv(k[:B, :, :n], v[:B, :, :n], block=64, bits_k=4, bits_v=4, k_rel=1 / 14, v_rel=1 / 14, k_mode=QuantMode.ChannelQuant,
+                                         cbk=64, cbv=64) for B in (1, 6) for n in (64, 1024)}
+    asked = [(B, n, G, n_res, s) for B, n in layers for G in (1, 8) for n_res in (1, 191) for s in (None, scratch)]
+
+    def ask(x, launch=False):
+        B, n, G, n_res, s = x
+        q = torch.ones(B, H * G, 128, device=dev, dtype=dtype)
+        return ops.decode_attention(q, layers[B, n], res[:B], res[:B], n_res, scratch=s, plan_only=not launch)
+
+    first = []
+    for x in asked:                                          # each by a thread of its own
+        with ThreadPoolExecutor(1) as pool:
+            first.append(pool.submit(ask, x).result())
+    assert [ask(x) for x in asked] == first and [ask(x) for x in reversed(asked)] == first[::-1]
+    with ThreadPoolExecutor(1) as pool:
+        assert [pool.submit(ask, x).result() for x in asked for _ in range(2)] == [p for p in first for _ in range(2)]
+    out = [ask(x, True) for x in asked]
+    again = [ask(x, True) for x in reversed(asked)][::-1]
+    assert all(torch.equal(a, b) for a, b in zip(out, again))
+
+
+@pytest.mark.parametrize("n_comp,plan", [(512, None), (512, (12, 1, 1)), (1024, (1, 1, 1)), (1024, (1, 3, 2))])
+def test_steps_behind_one_another_on_a_full_gpu(cuda_device, n_comp, plan):
+    """Launches of more CTAs than SMs are placed when the CTAs of the launch before have ended, not when it is complete: steps whose
+    query is the step before's output, behind launches of one CTA to an SM, give the bits of steps that wait."""
+    dev, dtype, B, H, G, steps = cuda_device, torch.bfloat16, 20, 8, 2, 12
+    k, v = synth.synth_kv(B, H, n_comp, 128, seed=8, dtype=dtype, device=dev)
+    layer = encode.compress_kv(k, v, block=64, bits_k=4, bits_v=4, k_rel=1 / 14, v_rel=1 / 14, k_mode=QuantMode.ChannelQuant, cbk=64, cbv=64)
+    few = encode.compress_kv(k[:1, :, :64], v[:1, :, :64], block=64, bits_k=4, bits_v=4, k_rel=1 / 14, v_rel=1 / 14, k_mode=QuantMode.ChannelQuant, cbk=64, cbv=64)
+    g = torch.Generator(device=dev).manual_seed(3)
+    res = [torch.randn(B, H, 192, 128, generator=g, device=dev).to(dtype) for _ in range(2)]
+    new = [torch.randn(steps, B, H, 1, 128, generator=g, device=dev).to(dtype) for _ in range(2)]
+    x0 = torch.randn(B, H * G, 128, generator=g, device=dev).to(dtype)
+    got = []
+    for wait in (True, False):
+        k_res, v_res = (t.clone() for t in res)
+        x, y, flags, scratch = x0.clone(), torch.empty_like(x0), ops.new_flags(dev), ops.new_attention_scratch(dev)
+        torch.cuda.synchronize()
+        for n in range(steps):
+            if n % 3 == 0:
+                ops.decode_attention(x[:1], few, k_res[:1], v_res[:1], 129 + n, out=x[:1], flags=flags, scratch=scratch)
+            ops.decode_attention(x, layer, k_res, v_res, 130 + n, out=y, flags=flags, append=(new[0][n], new[1][n], None, None), scratch=scratch, plan=plan,
                                  scaling=1.0)
             x, y = y, x
             if wait:
