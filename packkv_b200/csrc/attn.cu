@@ -298,7 +298,8 @@ struct AttnDev {
 struct CtaShared {
     float cl_m[8];       // this CTA's max per head
     float cl_l[8];       // this CTA's sum of exp(s - cl_m) per head
-    float wm[kAW][8];    // per-warp scratch
+    float wm[kAW][8];    // per-warp maxima; scratch
+    float wl[kAW][8];    // a team's per-warp sums of exp(s - wm)
     float gM[kAW][8], gInvL[kAW][8];   // global maximum and reciprocal sum, a copy for every warp
     unsigned lutm[8];    // (2^len - 1) * 0x00010001 per pack length 0..4 (see unpack8)
     unsigned last;       // two-launch form: this cluster is the pair's last one to deliver its rows
@@ -548,8 +549,21 @@ __global__ void __launch_bounds__(kAW * 32, PASS == 1 ? PKV_ATTN_CTAS_SCORES : P
 
     unsigned cur_pk0 = 0, cur_pk1 = 0, nxt_pk0 = 0, nxt_pk1 = 0;
     uint4 inf = make_uint4(0, 0, 0, 0);
-    if (total_items > 0) issue(0, load_info(0), nxt_pk0, nxt_pk1);
-    if (total_items > 1) inf = load_info(1);
+    // a team's launch: the first two items' table entries and q are under way together, before the first copy waits for its entry
+    uint4 qv[4];
+    if constexpr (TEAM) {
+        uint4 inf0 = inf;
+        if (total_items > 0) inf0 = load_info(0);
+        if (total_items > 1) inf = load_info(1);
+        const uint4* qp = reinterpret_cast<const uint4*>(
+            reinterpret_cast<const T*>(a.q) + ((int64_t)(b * q_heads + h * G + min(g, G - 1))) * P.dim + 8 * c);
+#pragma unroll
+        for (int m = 0; m < 4; m++) qv[m] = g < G && 32 * m + 8 * c < P.dim ? __ldg(qp + 4 * m) : make_uint4(0, 0, 0, 0);
+        if (total_items > 0) issue(0, inf0, nxt_pk0, nxt_pk1);
+    } else {
+        if (total_items > 0) issue(0, load_info(0), nxt_pk0, nxt_pk1);
+        if (total_items > 1) inf = load_info(1);
+    }
 
     // q fragments for the compressed tiles.  The mma step (j, ap) contracts the 16 channels
     // 64 ap + 32 hf + 8 c' + 4 e + j  (k = 8 hf + 2 c' + e): plane j of the exchange tile, lanes 16 ap .. 16 ap + 15.
@@ -562,7 +576,9 @@ __global__ void __launch_bounds__(kAW * 32, PASS == 1 ? PKV_ATTN_CTAS_SCORES : P
 #pragma unroll
         for (int m = 0; m < 4; m++) {
             // the repeated channels behind a narrow head's own add nothing to its scores: q is 0 there
-            const uint4 v = g < G && 32 * m + 8 * c < P.dim ? __ldg(qp + 4 * m) : make_uint4(0, 0, 0, 0);
+            uint4 v;
+            if constexpr (TEAM) v = qv[m];
+            else v = g < G && 32 * m + 8 * c < P.dim ? __ldg(qp + 4 * m) : make_uint4(0, 0, 0, 0);
             unsigned f0[2], f1[2];
             pair_shuffle(v, f0, f1);
             qf[0][m >> 1][m & 1] = f0[0]; qf[1][m >> 1][m & 1] = f0[1];
@@ -590,6 +606,7 @@ __global__ void __launch_bounds__(kAW * 32, PASS == 1 ? PKV_ATTN_CTAS_SCORES : P
         return at;
     };
 
+    bool v_params = false;                             // the first V tile's parameters are in pair order already
     T2 mpk0 = as_t2<T2>(Tr<T>::pack2(-INFINITY, -INFINITY)), mpk1 = mpk0;   // running max of this lane's scores, heads 2c and 2c+1
 
     // ============================================================================ phase 1: K tiles
@@ -845,6 +862,67 @@ __global__ void __launch_bounds__(kAW * 32, PASS == 1 ? PKV_ATTN_CTAS_SCORES : P
         }
     }
 
+    if constexpr (TEAM) {
+        // A launch of little work per warp: the first V tile's parameters (their copy began with the last K block) are put in order
+        // before the exchange, and the sums are taken relative to the warp's own maxima, over the scores that it wrote itself, so
+        // that one CTA barrier is left between the scores and the exchange (three before: with the loads above, 8 KV heads x 700
+        // tokens 11.65 -> 10.85 us; launches of several tiles to a warp keep the form below, 16 x 8k tokens 115.7 us against 116.6).
+        if (v_items > 0 && P.nslots == 2 && !dead) {
+            wait_item(k_items);
+            if (!dead) { permute_params(); v_params = true; }
+        }
+#pragma unroll
+        for (int d = 4; d < 32; d <<= 1) {
+            mloc0 = fmaxf(mloc0, __shfl_xor_sync(0xffffffffu, mloc0, d));
+            mloc1 = fmaxf(mloc1, __shfl_xor_sync(0xffffffffu, mloc1, d));
+        }
+        if (g == 0) {
+            cs->wm[wic][2 * c] = mloc0;                 // columns >= rows carry -inf or the score of a zero q
+            cs->wm[wic][2 * c + 1] = mloc1;
+        }
+        __syncwarp();
+        // the 16 tokens of a round are eight pairs: lane = pair lane & 7 of the rows lane >> 3 and (lane >> 3) + 4
+        const int ra = lane >> 3, rb = ra + 4;
+        const float ma = cs->wm[wic][ra], mb = cs->wm[wic][rb];
+        float la = 0.f, lb = 0.f;
+        const auto add = [&](float& sum, float m, unsigned at) {
+            const float2 x = Tr<T>::unpack2(lds32(at));
+            // a masked token holds -inf; if the whole warp is masked m is -inf too and the term must be 0
+            sum += (x.x == -INFINITY ? 0.f : fast_exp(x.x - m)) + (x.y == -INFINITY ? 0.f : fast_exp(x.y - m));
+        };
+        for (int tl = 0; tl < my_tiles; tl++)
+            for (int rd = wic; rd < (P.tile >> 4); rd += kAW) {      // round rd of the tile: every K block's rounds are dealt alike
+                const unsigned at = stile_a + tl * P.rows * P.prow + 32 * rd + 4 * (lane & 7);
+                if (ra < P.rows) add(la, ma, at + ra * P.prow);
+                if (rb < P.rows) add(lb, mb, at + rb * P.prow);
+            }
+        for (int k = 0; k < my_rt; k++) {
+            const unsigned at = rst_a + k * P.rows * 32 + 4 * (lane & 7);
+            if (ra < P.rows) add(la, ma, at + ra * 32);
+            if (rb < P.rows) add(lb, mb, at + rb * 32);
+        }
+#pragma unroll
+        for (int d = 4; d > 0; d >>= 1) {
+            la += __shfl_xor_sync(0xffffffffu, la, d);
+            lb += __shfl_xor_sync(0xffffffffu, lb, d);
+        }
+        if ((lane & 7) == 0) { cs->wl[wic][ra] = la; cs->wl[wic][rb] = lb; }
+        __syncthreads();
+        if (threadIdx.x < 8) {
+            float m = cs->wm[0][threadIdx.x], l = 0.f;
+#pragma unroll
+            for (int w = 1; w < kAW; w++) m = fmaxf(m, cs->wm[w][threadIdx.x]);
+            if ((int)threadIdx.x < P.rows) {
+#pragma unroll
+                for (int w = 0; w < kAW; w++) {
+                    const float mw = cs->wm[w][threadIdx.x];
+                    if (mw != -INFINITY) l += cs->wl[w][threadIdx.x] * fast_exp(mw - m);
+                }
+            }
+            cs->cl_m[threadIdx.x] = m;
+            cs->cl_l[threadIdx.x] = l;
+        }
+    } else {
     // ---- warp max -> CTA max --------------------------------------------------------------------
 #pragma unroll
     for (int d = 4; d < 32; d <<= 1) {
@@ -873,7 +951,7 @@ __global__ void __launch_bounds__(kAW * 32, PASS == 1 ? PKV_ATTN_CTAS_SCORES : P
             const unsigned st = stile_a + tl * P.rows * P.prow + 4 * lane;
 #pragma unroll
             for (int r = 0; r < 8; r++) {
-                if (r < P.rows && (!TEAM || (r & (kAW - 1)) == wic)) {   // a team's rows are shared out
+                if (r < P.rows) {
                     const float m = cs->cl_m[r];
                     for (int ch = 0; ch < chunks; ch++) {
                         const float2 x = Tr<T>::unpack2(lds32(st + r * P.prow + 128 * ch));
@@ -913,6 +991,7 @@ __global__ void __launch_bounds__(kAW * 32, PASS == 1 ? PKV_ATTN_CTAS_SCORES : P
         }
         cs->cl_l[threadIdx.x] = l;
     }
+    }   // not a team
     }   // PASS != kValues
     auto report_flags = [&]() {
         if (__any_sync(0xffffffffu, bad_len) && lane == 0) atomicOr(a.flags, kFlagBadStream);
@@ -1155,7 +1234,7 @@ __global__ void __launch_bounds__(kAW * 32, PASS == 1 ? PKV_ATTN_CTAS_SCORES : P
 
         if (vi == 0 && !dead) {
             // the tile's V scales and zero-points, pair order
-            permute_params();
+            if (!TEAM || n != k_items || !v_params) permute_params();
             // the tile's probabilities: loads of up to four units per lane, a warp barrier, then the stores
             for (int u0 = 0; !TEAM && u0 < units; u0 += 128) {
                 unsigned w0[4], w1[4];
