@@ -685,14 +685,27 @@ __device__ __forceinline__ void load_row_order(const FusedArgs& a, uint8_t* ord,
     __syncthreads();
 }
 
+// Warps of a V CTA.  A launch ends with the CTAs of its last, partly filled wave, so the form is taken whose waves fit the number of CTAs:
+// three CTAs of 8 warps on every SM take about 30 us and a last wave of one or two to an SM 22 and 32, two of 16 warps 22, one 17
+// (us at 8 heads, 4 bits; V of 160 token blocks 25.4 and 23.1 us, 384: 31.9 and 40.3, 504: 53.0 and 43.8, 640: 64.0 and 60.0,
+// 2048: 147 and 150).  128-token blocks leave room for one CTA of 16 warps only, which pays up to one to an SM.
+static int v_warps(int64_t ctas, int heads, int cb) {
+    if (2 * heads <= 8) return 8;
+    if (cb == 128) return ctas <= kSmCount ? 16 : 8;
+    const auto time = [&](int64_t per_sm, int full, int one, int two) {
+        const int64_t wave = per_sm * kSmCount, rest = ctas % wave;
+        return (int64_t)full * (ctas / wave) + (rest == 0 ? 0 : rest <= kSmCount ? one : rest <= 2 * kSmCount ? two : full);
+    };
+    return time(2, 22, 17, 22) < time(3, 30, 22, 32) ? 16 : 8;
+}
+
 // finished blocks that a warp of the V kernel holds in the direct form until their offsets are known
 __host__ __device__ constexpr int v_slots(int heads, int nw) { return (2 * heads + nw - 1) / nw; }
 
-// NW warps: 8, or 16 for launches of no more CTAs than SMs, whose time is that of one CTA (every warp then packs one block
-// of an 8-head token block instead of two, and the parameter pass has half the rows to a warp): with the K kernel's
-// single-CTA form, 16 sequences x 64 tokens take 98 us for four layers' K and V instead of 121
+// NW warps: 8, three CTAs to an SM, or 16, two to an SM at 64 registers: every warp then packs one block of an 8-head token block
+// instead of two, and a CTA takes little more than half the time (see v_warps)
 template <typename T, bool HP, int BITS, int CB, int NW>
-__global__ void __launch_bounds__(NW * 32, NW == 8 ? 3 : 1) v_fused_encode_kernel(FusedArgs a) {
+__global__ void __launch_bounds__(NW * 32, NW == 8 ? 3 : CB == 128 ? 1 : 2) v_fused_encode_kernel(FusedArgs a) {
     extern __shared__ __align__(16) uint8_t smem[];
     constexpr int LB = len_field_bits(BITS);
     const int lane = lane_id(), wic = threadIdx.x >> 5;
@@ -1352,7 +1365,7 @@ static int launch_fused_t(const FusedEncodeRequest& r, uint8_t* slots, const uin
         bound16 = (g.head_bytes + g.nseg * (g.min_bytes + g.len_bytes + 32 * g.ppt * 2 * BITS) + 15) & ~15;
         a.slot_stride = bound16;
         blocks_per_seq = nctx * 2 * r.heads;
-        const int nw = 2 * r.heads > 8 && (int64_t)nctx * r.batch <= kSmCount ? 16 : 8;
+        const int nw = v_warps((int64_t)nctx * r.batch, r.heads, r.cb);
         const int smem = 32 * r.cb + nw * (r.cb * 64 + (direct ? v_slots(r.heads, nw) : 1) * bound16) + r.cb + 16;
         auto launch_v = [&](auto kern) {
             if (opt_in_smem(kern, smem)) return (int)kCudaError;

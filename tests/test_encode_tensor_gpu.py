@@ -200,3 +200,20 @@ def test_one_block_of_every_sequence(cuda_device, which, mode, dtype, values):
             small["stream"] = torch.zeros(B, 256, dtype=torch.uint8, device=dev)
             ops.encode_tensor(which, x[:, :, :cb], cb, rel, mode, bits, cb, **small, **({} if order is None else dict(order=order[:, 0].contiguous(), order_block=cb)))
             assert int(small["flags"].item()) == 1 and torch.equal(small["info"][:, : one["info"].shape[1] // 2], one["info"][:, : one["info"].shape[1] // 2])
+
+
+@pytest.mark.parametrize("cb,bits", [(64, 4), (64, 3), (32, 2)])
+def test_v_forms_write_the_same(cuda_device, cb, bits):
+    """V CTAs of 8 and of 16 warps, by the number of token blocks a call has (more than 296 and up to 444: 8, a few and 504: 16): the
+    sequences of one call equal the same sequences in calls of one sequence each."""
+    dev, dtype, H, rel = cuda_device, torch.float16, 8, synth.rel_for_bits(bits)
+    for B, blocks in ((4, 126), (6, 60), (2, 100), (37, 12)):           # 504, 360, 200 and 444 token blocks
+        _, v = synth.synth_kv(B, H, blocks * cb, 128, seed=B, dtype=dtype, device=dev)
+        all_ = _bufs(B, H, blocks * cb, cb, bits, "v", ops.K_TOKEN, dtype, dev)
+        ops.encode_tensor("v", v, cb, rel, ops.K_TOKEN, bits, cb, **all_)
+        assert int(all_["flags"].item()) == 0
+        for b in (0, B - 1):
+            one = _bufs(1, H, blocks * cb, cb, bits, "v", ops.K_TOKEN, dtype, dev)
+            ops.encode_tensor("v", v[b: b + 1], cb, rel, ops.K_TOKEN, bits, cb, **one)
+            for name in ("scale", "zero", "stream", "info", "stream_bytes"):
+                assert torch.equal(one[name][0], all_[name][b]), (B, b, name)
