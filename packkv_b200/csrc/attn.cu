@@ -1744,10 +1744,10 @@ int launch_attention(const AttnArgs& a, const AttnExchange* xch, const AttnAppen
         const long on_gpu = ctas < slots ? ctas : slots;
         const int sm_warps = (int)((on_gpu + kSmCount - 1) / kSmCount) * kAW;
         // On a busy SM it makes no difference who holds the residual tiles; on an idle one it is the longest warp's time,
-        // and so are the hand-over and the second start of two launches.  Powers of two only: that, like the 6 % of a team
-        // below, is fitted to short launches, where 4, 8 and 16 CTAs to a cluster beat their neighbours by up to 2 us
-        // (one sequence x 700 tokens, 8 KV heads, us for 3..16: 19.0 14.2 14.9 15.1 14.2 12.4 13.6 14.3 14.9 13.8 14.6 15.5
-        // 15.8 13.8; two x 825: 19.5 17.1 15.2 15.5 16.1 13.2 14.4 15.5 16.0 15.0 15.9 17.2 17.6 15.5).
+        // and so are the hand-over and the second start of two launches.  Powers of two only.
+        // (The factors here were fitted to 30 shapes timed at every cluster size after the reduction was shared out and the launches
+        // were placed early: the chosen plan is 1.2 % from the best on average, 2.7 % with the factors before; e.g. 4 KV heads x 8192
+        // tokens 26.8 -> 24.7 us, 2 x 4 heads x 900 with 7 heads to a group 12.7 -> 11.3, 40 pairs x 3000 28.9 -> 24.4.)
         const bool idle = sm_warps <= 8;
         const double upw_max = team || (idle && !(cl & (cl - 1))) ? upw_placed : upw_dealt;
         if (idle && launches == 2) fixed += 1.0;
@@ -1758,9 +1758,10 @@ int launch_attention(const AttnArgs& a, const AttnExchange* xch, const AttnAppen
         const double lat = upw_max + fixed;
         double cost = (double)waves * (thr > lat ? thr : lat);
         if (ns == 1) cost *= 1.02;                              // the copy of the next block is not overlapped (it comes from L2)
-        if (cl > 8) cost *= 2 * ctas > slots ? 1.4 : 1.1;
+        if (cl > 8) cost *= 2 * ctas > slots ? 1.15 : 1.05;
+        // CTAs that need no company fill the places that come free (8 x 32k tokens, 16 CTAs to a pair: 8 x 2 214 us, 2 x 8 204)
+        if (waves > 1) cost *= 1 + 0.004 * (cl - 1);
         if (team && sm_warps > 8) cost *= 1.15;                 // a team's extra instructions count once the SM is busy (11 x 2154, 2 bits: 39 us against 35)
-        if (team && (cl & (cl - 1))) cost *= 1.06;
         return cost;
     };
     // Units of the longest warp.  Compressed tiles are dealt from the first owner (warp, or CTA of a team) on, residual
