@@ -40,6 +40,11 @@ def _require(cond: bool, msg: str) -> None:
 _CHUNK = 2 << 20
 
 
+def _staged(host: torch.Tensor) -> bool:
+    """Whether a uint8 tensor goes through the chunks: in host memory, ordinary, and of a chunk or more."""
+    return host.numel() >= _CHUNK and not host.is_cuda and not host.is_pinned()
+
+
 def _bytes(t: torch.Tensor) -> torch.Tensor:
     return t.view(-1).view(torch.uint8)
 
@@ -54,7 +59,7 @@ def _chunks(n: int):
 def _upload(src: torch.Tensor, dst: torch.Tensor) -> None:
     """Contiguous host tensor -> device tensor of as many bytes, on the current stream."""
     src, dst = _bytes(src), _bytes(dst)
-    if src.numel() < _CHUNK or src.is_pinned():
+    if not _staged(src):
         dst.copy_(src)
         return
     for i, (at, n, buf, event) in enumerate(_chunks(src.numel())):
@@ -66,11 +71,11 @@ def _upload(src: torch.Tensor, dst: torch.Tensor) -> None:
 
 
 def _download(src: torch.Tensor, dst: torch.Tensor) -> None:
-    """Device tensor -> contiguous host tensor of as many bytes; complete on return."""
-    src, dst = _bytes(src), _bytes(dst)
-    if src.numel() < _CHUNK or dst.is_pinned():
+    """Device tensor -> contiguous uint8 host tensor of its size; complete on return."""
+    if not _staged(dst):
         dst.copy_(src)
         return
+    src, dst = _bytes(src), _bytes(dst)
     chunks = _chunks(src.numel())
 
     def start(at, n, buf, event):
@@ -112,10 +117,11 @@ def _check_codec_args(which, codes, compressed, info, ctx_len, hidden_dim, cb, h
 def _encode(which, codes, compressed, info, ctx_len, hidden_dim, cb, hb, bits) -> int:
     _check_codec_args(which, codes, compressed, info, ctx_len, hidden_dim, cb, hb, bits)
     dev = codes.device if codes.is_cuda else _dev()
-    d_codes = codes
-    if not codes.is_cuda:
+    if _staged(codes):
         d_codes = torch.empty(codes.shape, dtype=torch.uint8, device=dev)
         _upload(codes, d_codes)
+    else:
+        d_codes = codes.to(dev)
     d_codes = d_codes.unsqueeze(0)
     staged = not compressed.is_cuda
     cap = compressed.numel()
@@ -145,17 +151,17 @@ def _decode(which, compressed, info, codes, ctx_len, hidden_dim, cb, hb, bits) -
     _check_codec_args(which, codes, compressed, info, ctx_len, hidden_dim, cb, hb, bits)
     dev = compressed.device if compressed.is_cuda else _dev()
     flat = compressed.reshape(-1)
-    used = flat.numel()
-    if not compressed.is_cuda and not info.is_cuda:
-        # no more of the buffer than the block table refers to (entries beyond the buffer are the kernel's to report)
+    if _staged(flat) and not info.is_cuda:
+        # no more of the buffer than the block table refers to (entries beyond the buffer are the kernel's to report); on a small one
+        # the look at the table takes longer than the bytes it saves
         ends = info.view(torch.int32).to(torch.int64) & 0xFFFFFFFF
-        used = min(used, int(ends.sum(dim=1).max()) if ends.numel() else 0)
-    d_stream = torch.empty((used + 31) // 16 * 16, dtype=torch.uint8, device=dev)
-    d_stream[used:].zero_()
-    if compressed.is_cuda:
-        d_stream[:used].copy_(flat)
-    else:
+        used = min(flat.numel(), int(ends.sum(dim=1).max()) if ends.numel() else 0)
+        d_stream = torch.empty((used + 31) // 16 * 16, dtype=torch.uint8, device=dev)
+        d_stream[used:].zero_()
         _upload(flat[:used], d_stream[:used])
+    else:
+        d_stream = torch.zeros((flat.numel() + 31) // 16 * 16, dtype=torch.uint8, device=dev)
+        d_stream[: flat.numel()].copy_(flat)
     d_info = info.view(torch.int32).to(dev).unsqueeze(0)
     d_codes = codes if codes.is_cuda else torch.zeros(codes.shape, dtype=torch.uint8, device=dev)
     flags = ops.new_flags(dev)
