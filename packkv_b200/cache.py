@@ -227,8 +227,7 @@ class PackKVCache(_HFCache):
             return self._update_dense(L, key_states, value_states, cos, sin, layer_idx)
         total = L.n_res + T
         n_c = compress_block_count(total, cfg.block_size, cfg.buffer_size) * cfg.block_size
-        if n_c == 0 and L.k_res is not None and T == 1 and not self.materialize and key_states.dtype in (torch.float16, torch.bfloat16) \
-                and (D == 128 or self._narrow_step(L, key_states, value_states, cos, sin)):
+        if n_c == 0 and L.k_res is not None and T == 1 and D == 128 and not self.materialize and key_states.dtype in (torch.float16, torch.bfloat16):
             # the common decode step: the fused attention to follow writes the token into the residual itself (attend() below)
             if cos is not None:
                 cos, sin = cos.to(key_states.dtype).contiguous(), sin.to(key_states.dtype).contiguous()
@@ -296,15 +295,6 @@ class PackKVCache(_HFCache):
         return L.k_res, L.v_res
 
     @staticmethod
-    def _narrow_step(L: "_Layer", k: torch.Tensor, v: torch.Tensor, cos, sin) -> bool:
-        """Whether a decode step's token of a narrow head can wait for attend(): anything the attention launch would not take goes through
-        _append at once, which converts it or refuses it."""
-        if not k.is_cuda or k.stride(3) != 1 or v.stride(3) != 1 or v.dtype != k.dtype or v.shape != k.shape or k.shape[:2] != L.k_res.shape[:2]:
-            return False
-        return (sin is None) if cos is None else (sin is not None and cos.is_cuda and sin.is_cuda and cos.dim() == 3 and sin.shape == cos.shape
-                                                  and cos.shape[1:] == k.shape[2:] and cos.shape[0] in (1, k.shape[0]))
-
-    @staticmethod
     def _append(k_rows: torch.Tensor, v_rows: torch.Tensor, position: int, k: torch.Tensor, v: torch.Tensor, cos, sin) -> None:
         """Tokens (B, H, T, D) into rows [position, position + T) of 128 channels: K rotated when cos is given; rows of
         64 <= D < 128 are widened, the tail repeating the first 128 - D channels.  The streams are built from 128-channel
@@ -328,8 +318,7 @@ class PackKVCache(_HFCache):
         if L.pending is not None:
             k_new, v_new, cos, sin = L.pending
             L.pending = None
-            write = ops.append_residual if k_new.shape[3] == 128 else ops.widen_rows
-            write(k_new, v_new, L.k_res, L.v_res, L.n_res - 1, cos, sin)
+            ops.append_residual(k_new, v_new, L.k_res, L.v_res, L.n_res - 1, cos, sin)
 
     def flush(self) -> None:
         """Makes the residual buffers of every layer complete (call before reading them from outside)."""
@@ -375,15 +364,14 @@ class PackKVCache(_HFCache):
             # few (sequence, KV head) pairs: let the library split each over several clusters (all layers share the
             # area: their launches are ordered on one stream)
             self._scratch = ops.new_attention_scratch(q.device)
-        if L.pending is not None and L.pending[0].shape[3] != D:
-            self._flush(L)                                     # a query of another width than the rows: they are written as they are
         if D != 128:
+            self._flush(L)                                     # (of a token of 128 channels; narrow heads' rows are written by update())
             if q.data_ptr() % 16:
                 q = q.clone()
-            # the launch reads q's D channels as if zeros stood behind them (the copied channels of K add nothing) and widens the
-            # pending token's rows itself: 4 sequences x 32 heads x ~1100 tokens 31 us a step and layer, 38 with both as launches
+            # the launch reads q's D channels as if zeros stood behind them (the copied channels of K add nothing).  It could widen the
+            # step's rows too, but update() would then have to keep the caller's tensors instead of their contents until here.
             out = ops.decode_attention_narrow(q, L.comp if L.n_comp else None, L.k_res, L.v_res, L.n_res, scaling=D ** -0.5 if scaling is None else scaling,
-                                              flags=self.flags, kv_heads=kv_heads, append=self._take_pending(L), scratch=self._scratch)
+                                              flags=self.flags, kv_heads=kv_heads, scratch=self._scratch)
             return out.view(B, 1, Hq, 128)[..., :D]
         pending = self._take_pending(L)
         out = ops.decode_attention(q, L.comp if L.n_comp else None, L.k_res, L.v_res, L.n_res, scaling=scaling,

@@ -278,19 +278,18 @@ def test_update_refuses_rotation_tables_of_another_length(cuda_device, D):
 @pytest.mark.parametrize("D", [64, 72, 96, 120])
 @pytest.mark.parametrize("tables", ["row", "rows", None])
 def test_narrow_decode_step_inside_the_attention_launch(cuda_device, D, dtype, tables):
-    """Heads below 128 channels: the launch that attends widens the step's rows and reads the narrow q.  Residual rows bit for bit those of
-    widen_rows (halves of 32 .. 60 channels, rows at odd addresses, tables for one or all sequences), outputs those of a q that is padded
-    and rows that are written beforehand, with and without packed blocks and without an attend() between two steps."""
+    """Heads below 128 channels: an attention launch that is handed the step's token widens its rows and reads the narrow q.  Residual rows bit
+    for bit those of widen_rows (halves of 32 .. 60 channels, rows at odd addresses, tables for one or all sequences), outputs those of a q that
+    is padded and rows that are written beforehand, with and without packed blocks.  A cache writes the rows in update(), with and without an
+    attend() between two steps."""
     dev, B, H, G = cuda_device, 2, 2, 3
     C.PackKVCacheConfigStatic.config = _cfg(QuantMethod.PackKV)
     try:
         for S0 in (3, 270):
-            new, old = C.PackKVCache(B, H * G, D, 1), C.PackKVCache(B, H * G, D, 1)
-            old._narrow_step = lambda *a: False                    # its rows are written by update()
-            new._scratch = ops.new_attention_scratch(dev)
+            cache = C.PackKVCache(B, H * G, D, 1)
+            cache._scratch = ops.new_attention_scratch(dev)
             k, v = synth.synth_kv(B, H, S0, D, seed=S0, dtype=dtype, device=dev)
-            for cache in (new, old):
-                cache.update(k, v, 0)
+            cache.update(k, v, 0)
             for t in range(5):
                 gen = torch.Generator(device=dev).manual_seed(t)
                 buf = torch.randn(2, B, H, D + 1, generator=gen, device=dev).to(dtype)
@@ -300,23 +299,59 @@ def test_narrow_decode_step_inside_the_attention_launch(cuda_device, D, dtype, t
                 if tables:
                     cs = torch.randn(2, B if tables == "rows" else 1, 1, D, generator=gen, device=dev).to(dtype)
                     kw = {"cos": cs[0], "sin": cs[1]}
-                for cache in (new, old):
-                    cache.update(kn, vn, 0, kw)
-                assert new._layers[0].pending is not None and old._layers[0].pending is None
+                cache.update(kn, vn, 0, kw)
+                assert cache._layers[0].pending is None
                 if t == 2:
-                    continue                                       # the next update writes the row itself
+                    continue
                 wide = torch.zeros(B, H * G, 128, dtype=dtype, device=dev)
                 wide[..., :D] = q[:, :, 0]
-                L = old._layers[0]
-                want = ops.decode_attention(wide, L.comp if L.n_comp else None, L.k_res, L.v_res, L.n_res, scaling=D ** -0.5, kv_heads=H, scratch=new._scratch)
-                got = new.attend(q, 0)
+                L = cache._layers[0]
+                layer = L.comp if L.n_comp else None
+                want = ops.decode_attention(wide, layer, L.k_res, L.v_res, L.n_res, scaling=D ** -0.5, kv_heads=H, scratch=cache._scratch)
+                got = cache.attend(q, 0)
                 assert got.shape == (B, 1, H * G, D) and torch.equal(got[:, 0], want[..., :D])
-                N = new._layers[0]
-                assert torch.equal(N.k_res[:, :, : N.n_res], L.k_res[:, :, : L.n_res]) and torch.equal(N.v_res[:, :, : N.n_res], L.v_res[:, :, : L.n_res])
-            new.check_flags()
+                k_res, v_res = L.k_res.clone(), L.v_res.clone()
+                k_res[:, :, L.n_res - 1], v_res[:, :, L.n_res - 1] = float("nan"), float("nan")
+                got = ops.decode_attention_narrow(q[:, :, 0].contiguous(), layer, k_res, v_res, L.n_res, scaling=D ** -0.5, kv_heads=H, scratch=cache._scratch,
+                                                  append=(kn, vn, *(cs if tables else (None, None))))
+                assert torch.equal(got[..., :D], want[..., :D])
+                assert torch.equal(k_res[:, :, : L.n_res], L.k_res[:, :, : L.n_res]) and torch.equal(v_res[:, :, : L.n_res], L.v_res[:, :, : L.n_res])
+            cache.check_flags()
         other = torch.randn(B, H * G, 1, 128, device=dev).to(dtype)
-        new.update(kn, vn, 0, kw)
-        old.update(kn, vn, 0, kw)
-        assert torch.equal(new.attend(other, 0), old.attend(other, 0))   # a wider query than the rows of the step
+        L = cache._layers[0]
+        want = ops.decode_attention(other[:, :, 0], L.comp, L.k_res, L.v_res, L.n_res, kv_heads=H, scratch=cache._scratch)
+        assert torch.equal(cache.attend(other, 0)[:, 0], want)           # a wider query than the rows of the step
+    finally:
+        C.PackKVCacheConfigStatic.config = None
+
+
+@pytest.mark.parametrize("D", [64, 96])
+def test_narrow_steps_from_one_buffer(cuda_device, D):
+    """A caller that keeps one projection buffer and one pair of table rows for all steps of a narrow-headed model: update() has taken what they
+    held when it was called, whether attend() follows, follows after the buffers are written again, or not at all."""
+    dev, dtype, B, H, G, steps = cuda_device, torch.bfloat16, 2, 2, 4, 6
+    C.PackKVCacheConfigStatic.config = _cfg(QuantMethod.KIVI)
+    try:
+        one, own = C.PackKVCache(B, H * G, D, 1), C.PackKVCache(B, H * G, D, 1)
+        k, v = synth.synth_kv(B, H, 300 + steps, D, seed=3, dtype=dtype, device=dev)
+        cos, sin = synth.rope_tables(300 + steps, D, device=dev, dtype=dtype)
+        for cache in (one, own):
+            cache.update(k[:, :, :300], v[:, :, :300], 0, {"cos": cos[:, :300], "sin": sin[:, :300]})
+        buf = [torch.empty(B, H, 1, D, dtype=dtype, device=dev) for _ in range(2)] + [torch.empty(1, 1, D, dtype=dtype, device=dev) for _ in range(2)]
+        for n in range(steps):
+            t = 300 + n
+            row = [k[:, :, t:t + 1].clone(), v[:, :, t:t + 1].clone(), cos[:, t:t + 1].clone(), sin[:, t:t + 1].clone()]
+            for b, x in zip(buf, row):
+                b.copy_(x)
+            one.update(buf[0], buf[1], 0, {"cos": buf[2], "sin": buf[3]})
+            own.update(row[0], row[1], 0, {"cos": row[2], "sin": row[3]})
+            if n % 3 != 2:
+                if n % 3 == 1:
+                    for b in buf:
+                        b.fill_(float("nan"))
+                q = synth.synth_q(B, H * G, D, seed=n, dtype=dtype).to(dev)
+                assert torch.equal(one.attend(q, 0), own.attend(q, 0)), n
+        a, b = one._layers[0], own._layers[0]
+        assert a.n_res == b.n_res and torch.equal(a.k_res[:, :, : a.n_res], b.k_res[:, :, : b.n_res]) and torch.equal(a.v_res[:, :, : a.n_res], b.v_res[:, :, : b.n_res])
     finally:
         C.PackKVCacheConfigStatic.config = None
