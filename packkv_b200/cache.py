@@ -317,8 +317,8 @@ class PackKVCache(_HFCache):
         """Writes a decode step's token that no attend() has consumed into the residual (one launch)."""
         if L.pending is not None:
             k_new, v_new, cos, sin = L.pending
-            L.pending = None
             ops.append_residual(k_new, v_new, L.k_res, L.v_res, L.n_res - 1, cos, sin)
+            L.pending = None
 
     def flush(self) -> None:
         """Makes the residual buffers of every layer complete (call before reading them from outside)."""
@@ -344,11 +344,6 @@ class PackKVCache(_HFCache):
         block = self._config().block_size
         return (ops.dense("k", L.comp, L.k_res, L.n_res, D, block, self.flags), ops.dense("v", L.comp, L.v_res, L.n_res, D, block, self.flags))
 
-    @staticmethod
-    def _take_pending(L: "_Layer"):
-        pending, L.pending = L.pending, None
-        return pending
-
     def attend(self, query_states: torch.Tensor, layer_idx: int, scaling: Optional[float] = None) -> torch.Tensor:
         """Decode attention for one new token: query_states (B, Hq, 1, 128) after RoPE ->
         (B, 1, Hq, 128), the layout the reference's eager attention returns (llama.py:210-212)."""
@@ -373,9 +368,9 @@ class PackKVCache(_HFCache):
             out = ops.decode_attention_narrow(q, L.comp if L.n_comp else None, L.k_res, L.v_res, L.n_res, scaling=D ** -0.5 if scaling is None else scaling,
                                               flags=self.flags, kv_heads=kv_heads, scratch=self._scratch)
             return out.view(B, 1, Hq, 128)[..., :D]
-        pending = self._take_pending(L)
         out = ops.decode_attention(q, L.comp if L.n_comp else None, L.k_res, L.v_res, L.n_res, scaling=scaling,
-                                   flags=self.flags, kv_heads=kv_heads, append=pending, scratch=self._scratch)
+                                   flags=self.flags, kv_heads=kv_heads, append=L.pending, scratch=self._scratch)
+        L.pending = None                                       # not before: a call that was refused has not written the token
         return out.view(B, 1, Hq, 128)[..., :D]
 
     def get_seq_length(self, layer_idx: Optional[int] = 0) -> int:

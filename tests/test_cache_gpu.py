@@ -355,3 +355,37 @@ def test_narrow_steps_from_one_buffer(cuda_device, D):
         assert a.n_res == b.n_res and torch.equal(a.k_res[:, :, : a.n_res], b.k_res[:, :, : b.n_res]) and torch.equal(a.v_res[:, :, : a.n_res], b.v_res[:, :, : b.n_res])
     finally:
         C.PackKVCacheConfigStatic.config = None
+
+
+@pytest.mark.parametrize("D", [96, 128])
+def test_refused_attend_keeps_the_step(cuda_device, D):
+    """An attend() that is refused (a query of another type, q heads that are no multiple of the KV heads, a group above 8) leaves the step's
+    token in place: the attend() that is corrected, dense() and the next steps find its row."""
+    dev, dtype, B, H = cuda_device, torch.float16, 2, 2
+    C.PackKVCacheConfigStatic.config = _cfg(QuantMethod.KIVI)
+    try:
+        cache, plain = C.PackKVCache(B, H * 2, D, 1), C.PackKVCache(B, H * 2, D, 1)
+        k, v = synth.synth_kv(B, H, 303, D, seed=4, dtype=dtype, device=dev)
+        cos, sin = synth.rope_tables(303, D, device=dev, dtype=dtype)
+        kw = lambda a, b: {"cos": cos[:, a:b], "sin": sin[:, a:b]}
+        for c in (cache, plain):
+            c.update(k[:, :, :300], v[:, :, :300], 0, kw(0, 300))
+        for t in range(300, 303):
+            q = synth.synth_q(B, H * 2, D, seed=t, dtype=dtype).to(dev)
+            for c in (cache, plain):
+                c.update(k[:, :, t:t + 1], v[:, :, t:t + 1], 0, kw(t, t + 1))
+            plain.flush()
+            L = cache._layers[0]
+            if L.pending is not None:                    # what the row holds until the launch writes it
+                L.k_res[:, :, L.n_res - 1], L.v_res[:, :, L.n_res - 1] = 7.0, 7.0
+            for bad in (q.bfloat16(), q[:, :3], q.repeat(1, 5, 1, 1)[:, : H * 9]):
+                with pytest.raises((ValueError, RuntimeError)):
+                    cache.attend(bad, 0)
+            if t == 301:
+                assert all(torch.equal(a, b) for a, b in zip(cache.dense(0), plain.dense(0)))
+            else:
+                assert torch.equal(cache.attend(q, 0), plain.attend(q, 0))
+        a, b = cache._layers[0], plain._layers[0]
+        assert torch.equal(a.k_res[:, :, : a.n_res], b.k_res[:, :, : b.n_res]) and torch.equal(a.v_res[:, :, : a.n_res], b.v_res[:, :, : b.n_res])
+    finally:
+        C.PackKVCacheConfigStatic.config = None
