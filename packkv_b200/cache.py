@@ -227,10 +227,10 @@ class PackKVCache(_HFCache):
             return self._update_dense(L, key_states, value_states, cos, sin, layer_idx)
         total = L.n_res + T
         n_c = compress_block_count(total, cfg.block_size, cfg.buffer_size) * cfg.block_size
-        if n_c == 0 and L.k_res is not None and T == 1 and D == 128 and not self.materialize and key_states.dtype in (torch.float16, torch.bfloat16):
-            # the common decode step: the fused attention to follow writes the token into the residual itself (attend() below)
-            if cos is not None:
-                cos, sin = cos.to(key_states.dtype).contiguous(), sin.to(key_states.dtype).contiguous()
+        if n_c == 0 and L.k_res is not None and T == 1 and D == 128 and not self.materialize \
+                and ops.waiting_step(L.k_res, key_states, value_states, cos, sin) is not None:
+            # the common decode step: the fused attention to follow writes the token into the residual itself (attend() below).  What the
+            # launch would not take goes through _append at once, which converts it, or refuses it before the token is counted.
             L.pending = (key_states, value_states, cos, sin)
             L.n_res = total
             return self._step_result(layer_idx, T)

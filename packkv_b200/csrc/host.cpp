@@ -478,6 +478,30 @@ PyObject* widen_rows(PyObject* const* p) {
     Py_RETURN_NONE;
 }
 
+// k_res, k_new, v_new, cos, sin -> the current stream of k_new's device if the attention launch can take the step's rows where they are (what
+// fill_append and the launch ask of them), None if they have to be converted or refused first
+PyObject* waiting_step(PyObject* const* p) {
+    for (int i = 0; i < 3; i++)
+        if (!THPVariable_Check(p[i])) Py_RETURN_NONE;
+    const at::Tensor &res = THPVariable_Unpack(p[0]), &k = THPVariable_Unpack(p[1]), &v = THPVariable_Unpack(p[2]);
+    const auto aligned = [](const at::Tensor& t) { return reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0; };
+    const auto row = [&](const at::Tensor& t) {
+        return t.is_cuda() && t.device() == res.device() && t.scalar_type() == res.scalar_type() && t.dim() == 4 && t.size(0) == res.size(0) &&
+               t.size(1) == res.size(1) && t.size(2) == 1 && t.size(3) == 128 && t.stride(3) == 1 && t.stride(0) % 8 == 0 && t.stride(1) % 8 == 0 && aligned(t);
+    };
+    if (res.dim() != 4 || !half_type(res) || !row(k) || !row(v)) Py_RETURN_NONE;
+    if (p[3] != Py_None) {
+        if (!THPVariable_Check(p[3]) || !THPVariable_Check(p[4])) Py_RETURN_NONE;
+        const at::Tensor &cos = THPVariable_Unpack(p[3]), &sin = THPVariable_Unpack(p[4]);
+        const auto table = [&](const at::Tensor& t) {
+            return t.is_cuda() && t.device() == res.device() && t.scalar_type() == res.scalar_type() && t.dim() >= 2 && t.size(-2) == 1 && t.size(-1) == 128 &&
+                   t.is_contiguous() && (t.size(0) == 1 || t.numel() >= res.size(0) * 128) && aligned(t);
+        };
+        if (!table(cos) || !table(sin) || cos.sizes() != sin.sizes()) Py_RETURN_NONE;
+    }
+    return PyLong_FromVoidPtr(c10::cuda::getCurrentCUDAStream(res.get_device()).stream());
+}
+
 // x, cos, sin, out -> out
 PyObject* rope(PyObject* const* p) {
     const at::Tensor &x = cuda(p[0], "x"), &cos = cuda(p[1], "cos"), &sin = cuda(p[2], "sin");
@@ -544,6 +568,7 @@ PyMethodDef methods[] = {
     FAST(encode_tensor, 18, "ops.encode_tensor / ops.encode_tensor_static"),
     FAST(value_median_order, 4, "ops.value_median_order"),
     FAST(append_residual, 7, "ops.append_residual"),
+    FAST(waiting_step, 5, "whether a decode step's rows can wait for the attention launch"),
     FAST(rope, 4, "ops.rope"),
     FAST(widen_rows, 8, "ops.widen_rows"),
     {nullptr, nullptr, 0, nullptr}};

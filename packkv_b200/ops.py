@@ -310,6 +310,12 @@ def append_residual(k_new: torch.Tensor, v_new: torch.Tensor, k_res: torch.Tenso
     _lib.host().append_residual(k_new, v_new, k_res, v_res, position, cos, sin)
 
 
+def waiting_step(k_res: torch.Tensor, k_new: torch.Tensor, v_new: torch.Tensor, cos: Optional[torch.Tensor], sin: Optional[torch.Tensor]) -> Optional[int]:
+    """The current stream (its handle) if decode_attention(append=(k_new, v_new, cos, sin)) over residual buffers like k_res can take these
+    tensors as they are; None if they have to be converted, or refused, first."""
+    return _lib.host().waiting_step(k_res, k_new, v_new, cos, sin)
+
+
 def widen_rows(k: torch.Tensor, v: Optional[torch.Tensor], k_out: torch.Tensor, v_out: Optional[torch.Tensor], position: int = 0,
                cos: Optional[torch.Tensor] = None, sin: Optional[torch.Tensor] = None, zero_tail: bool = False) -> None:
     """append_residual for heads of 64 <= D < 128 channels (B, H, T, D): the rows of k_out / v_out (B, H, capacity, 128) are

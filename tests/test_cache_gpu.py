@@ -389,3 +389,47 @@ def test_refused_attend_keeps_the_step(cuda_device, D):
         assert torch.equal(a.k_res[:, :, : a.n_res], b.k_res[:, :, : b.n_res]) and torch.equal(a.v_res[:, :, : a.n_res], b.v_res[:, :, : b.n_res])
     finally:
         C.PackKVCacheConfigStatic.config = None
+
+
+@pytest.mark.parametrize("form", ["odd address", "odd strides", "v channels apart", "v of another type", "tables of another type", "tables apart", "k of another type", "heads"])
+def test_step_that_the_attention_launch_does_not_take(cuda_device, form):
+    """A step of 128 channels whose tensors the attention launch cannot read as they are: written (converted) by update() like a step of any
+    other length, or refused there, with the token not counted and the cache as it was."""
+    dev, dtype, B, H, G = cuda_device, torch.bfloat16, 2, 2, 2
+    C.PackKVCacheConfigStatic.config = _cfg(QuantMethod.KIVI)
+    try:
+        cache, plain = C.PackKVCache(B, H * G, 128, 1), C.PackKVCache(B, H * G, 128, 1)
+        k, v = synth.synth_kv(B, H, 301, 128, seed=6, dtype=dtype, device=dev)
+        cos, sin = synth.rope_tables(301, 128, device=dev, dtype=dtype)
+        for c in (cache, plain):
+            c.update(k[:, :, :300], v[:, :, :300], 0, {"cos": cos[:, :300], "sin": sin[:, :300]})
+        row = [k[:, :, 300:].clone(), v[:, :, 300:].clone(), cos[:, 300:].clone(), sin[:, 300:].clone()]
+        plain.update(row[0], row[1], 0, {"cos": row[2], "sin": row[3]})
+        plain.flush()
+        if form == "odd address":
+            row[0] = torch.empty(B * H * 128 + 1, dtype=dtype, device=dev)[1:].view(B, H, 1, 128).copy_(row[0])
+        elif form == "odd strides":
+            row[1] = torch.empty(B, H, 1, 129, dtype=dtype, device=dev)[..., :128].copy_(row[1])
+        elif form == "v channels apart":
+            row[1] = torch.empty(B, H, 1, 128, 2, dtype=dtype, device=dev)[..., 0].copy_(row[1])
+        elif form == "v of another type":
+            row[1] = row[1].float()
+        elif form == "tables of another type":
+            row[2], row[3] = row[2].float(), row[3].float()
+        elif form == "tables apart":
+            row[2] = torch.empty(1, 1, 128, 2, dtype=dtype, device=dev)[..., 0].copy_(row[2])
+        q = synth.synth_q(B, H * G, 128, seed=1, dtype=dtype).to(dev)
+        if form in ("k of another type", "heads"):
+            bad = row[0].half() if form[0] == "k" else row[0].repeat(1, 2, 1, 1)
+            with pytest.raises(ValueError):
+                cache.update(bad, row[1].half() if form[0] == "k" else row[1].repeat(1, 2, 1, 1), 0, {"cos": row[2], "sin": row[3]})
+            assert cache.get_seq_length(0) == 300 and cache._layers[0].pending is None
+            cache.update(row[0], row[1], 0, {"cos": row[2], "sin": row[3]})
+        else:
+            cache.update(row[0], row[1], 0, {"cos": row[2], "sin": row[3]})
+            assert cache._layers[0].pending is None
+        assert torch.equal(cache.attend(q, 0), plain.attend(q, 0))
+        a, b = cache._layers[0], plain._layers[0]
+        assert a.n_res == b.n_res and torch.equal(a.k_res[:, :, : a.n_res], b.k_res[:, :, : b.n_res]) and torch.equal(a.v_res[:, :, : a.n_res], b.v_res[:, :, : b.n_res])
+    finally:
+        C.PackKVCacheConfigStatic.config = None
