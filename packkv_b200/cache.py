@@ -82,6 +82,7 @@ class _Layer:
         self.n_res = 0
         self.n_comp = 0
         self.pending = None        # (k_new, v_new, cos, sin) of a decode step whose token the next attend() writes into row n_res - 1
+        self.pending_on = 0        # the stream that update() was called on with them
 
 
 class PackKVCache(_HFCache):
@@ -227,13 +228,14 @@ class PackKVCache(_HFCache):
             return self._update_dense(L, key_states, value_states, cos, sin, layer_idx)
         total = L.n_res + T
         n_c = compress_block_count(total, cfg.block_size, cfg.buffer_size) * cfg.block_size
-        if n_c == 0 and L.k_res is not None and T == 1 and D == 128 and not self.materialize \
-                and ops.waiting_step(L.k_res, key_states, value_states, cos, sin) is not None:
-            # the common decode step: the fused attention to follow writes the token into the residual itself (attend() below).  What the
-            # launch would not take goes through _append at once, which converts it, or refuses it before the token is counted.
-            L.pending = (key_states, value_states, cos, sin)
-            L.n_res = total
-            return self._step_result(layer_idx, T)
+        if n_c == 0 and L.k_res is not None and T == 1 and D == 128 and not self.materialize:
+            on = ops.waiting_step(L.k_res, key_states, value_states, cos, sin)
+            if on is not None:
+                # the common decode step: the fused attention to follow writes the token into the residual itself (attend() below).  What the
+                # launch would not take goes through _append at once, which converts it, or refuses it before the token is counted.
+                L.pending, L.pending_on = (key_states, value_states, cos, sin), on
+                L.n_res = total
+                return self._step_result(layer_idx, T)
         if key_states.stride(3) != 1 or value_states.stride(3) != 1:
             key_states, value_states = key_states.contiguous(), value_states.contiguous()
         if value_states.dtype != key_states.dtype:
@@ -318,6 +320,17 @@ class PackKVCache(_HFCache):
         if L.pending is not None:
             k_new, v_new, cos, sin = L.pending
             ops.append_residual(k_new, v_new, L.k_res, L.v_res, L.n_res - 1, cos, sin)
+            self._written(L)
+
+    @staticmethod
+    def _written(L: "_Layer") -> None:
+        """The launch that reads a step's tensors has been made: they are let go.  On another stream than update()'s the allocator is told
+        first, or it would give their memory to that stream's next tensors while the launch still waits or reads."""
+        if L.pending is not None:
+            if ops.stream_of(L.k_res) != L.pending_on:
+                for t in L.pending:
+                    if t is not None:
+                        t.record_stream(torch.cuda.current_stream(L.k_res.device))
             L.pending = None
 
     def flush(self) -> None:
@@ -370,7 +383,7 @@ class PackKVCache(_HFCache):
             return out.view(B, 1, Hq, 128)[..., :D]
         out = ops.decode_attention(q, L.comp if L.n_comp else None, L.k_res, L.v_res, L.n_res, scaling=scaling,
                                    flags=self.flags, kv_heads=kv_heads, append=L.pending, scratch=self._scratch)
-        L.pending = None                                       # not before: a call that was refused has not written the token
+        self._written(L)                                       # not before: a call that was refused has not written the token
         return out.view(B, 1, Hq, 128)[..., :D]
 
     def get_seq_length(self, layer_idx: Optional[int] = 0) -> int:

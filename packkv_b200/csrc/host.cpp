@@ -502,6 +502,9 @@ PyObject* waiting_step(PyObject* const* p) {
     return PyLong_FromVoidPtr(c10::cuda::getCurrentCUDAStream(res.get_device()).stream());
 }
 
+// tensor -> the handle of its device's current stream
+PyObject* stream_of(PyObject* const* p) { return PyLong_FromVoidPtr(c10::cuda::getCurrentCUDAStream(cuda(p[0], "tensor").get_device()).stream()); }
+
 // x, cos, sin, out -> out
 PyObject* rope(PyObject* const* p) {
     const at::Tensor &x = cuda(p[0], "x"), &cos = cuda(p[1], "cos"), &sin = cuda(p[2], "sin");
@@ -569,6 +572,7 @@ PyMethodDef methods[] = {
     FAST(value_median_order, 4, "ops.value_median_order"),
     FAST(append_residual, 7, "ops.append_residual"),
     FAST(waiting_step, 5, "whether a decode step's rows can wait for the attention launch"),
+    FAST(stream_of, 1, "handle of the current stream of a tensor's device"),
     FAST(rope, 4, "ops.rope"),
     FAST(widen_rows, 8, "ops.widen_rows"),
     {nullptr, nullptr, 0, nullptr}};

@@ -316,6 +316,11 @@ def waiting_step(k_res: torch.Tensor, k_new: torch.Tensor, v_new: torch.Tensor, 
     return _lib.host().waiting_step(k_res, k_new, v_new, cos, sin)
 
 
+def stream_of(t: torch.Tensor) -> int:
+    """Handle of the current stream of t's device (torch.cuda.current_stream(t.device).cuda_stream, without building the Python objects)."""
+    return _lib.host().stream_of(t)
+
+
 def widen_rows(k: torch.Tensor, v: Optional[torch.Tensor], k_out: torch.Tensor, v_out: Optional[torch.Tensor], position: int = 0,
                cos: Optional[torch.Tensor] = None, sin: Optional[torch.Tensor] = None, zero_tail: bool = False) -> None:
     """append_residual for heads of 64 <= D < 128 channels (B, H, T, D): the rows of k_out / v_out (B, H, capacity, 128) are

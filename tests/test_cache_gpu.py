@@ -433,3 +433,46 @@ def test_step_that_the_attention_launch_does_not_take(cuda_device, form):
         assert a.n_res == b.n_res and torch.equal(a.k_res[:, :, : a.n_res], b.k_res[:, :, : b.n_res]) and torch.equal(a.v_res[:, :, : a.n_res], b.v_res[:, :, : b.n_res])
     finally:
         C.PackKVCacheConfigStatic.config = None
+
+
+@pytest.mark.parametrize("flush", [False, True])
+def test_update_and_attend_on_two_streams(cuda_device, flush):
+    """A step goes to update() on one stream, to attend() (or flush()) on another that is ordered behind it and busy, and its tensors are let go:
+    the first stream's next tensors must not get their memory before the row is written."""
+    dev, dtype, B, H, G = cuda_device, torch.bfloat16, 2, 2, 2
+    C.PackKVCacheConfigStatic.config = _cfg(QuantMethod.KIVI)
+    try:
+        cache, plain = C.PackKVCache(B, H * G, 128, 1), C.PackKVCache(B, H * G, 128, 1)
+        k, v = synth.synth_kv(B, H, 301, 128, seed=6, dtype=dtype, device=dev)
+        cos, sin = synth.rope_tables(301, 128, device=dev, dtype=dtype)
+        for c in (cache, plain):
+            c.update(k[:, :, :300], v[:, :, :300], 0, {"cos": cos[:, :300], "sin": sin[:, :300]})
+        plain.update(k[:, :, 300:], v[:, :, 300:], 0, {"cos": cos[:, 300:], "sin": sin[:, 300:]})
+        q = synth.synth_q(B, H * G, 128, seed=1, dtype=dtype).to(dev)
+        want = plain.attend(q, 0)
+        plain.flush()
+        torch.cuda.synchronize()
+        first, second = torch.cuda.Stream(), torch.cuda.Stream()
+        with torch.cuda.stream(second):
+            cache.attend(q, 0)                                     # buffers and kernels are there: nothing below waits for an allocation
+        torch.full((1,), float("nan"), dtype=dtype, device=dev)
+        torch.cuda.synchronize()
+        with torch.cuda.stream(first):
+            row = [k[:, :, 300:].clone(), v[:, :, 300:].clone(), cos[:, 300:].clone(), sin[:, 300:].clone()]
+            cache.update(row[0], row[1], 0, {"cos": row[2], "sin": row[3]})
+            shapes = [t.shape for t in row]
+            del row
+        assert cache._layers[0].pending is not None
+        second.wait_stream(first)
+        with torch.cuda.stream(second):
+            torch.cuda._sleep(20_000_000)                          # about 10 ms
+            got = cache.flush() if flush else cache.attend(q, 0)
+        with torch.cuda.stream(first):
+            new = [torch.full(s, float("nan"), dtype=dtype, device=dev) for s in shapes for _ in range(4)]
+        torch.cuda.synchronize()
+        del new
+        a, b = cache._layers[0], plain._layers[0]
+        assert torch.equal(a.k_res[:, :, : a.n_res], b.k_res[:, :, : b.n_res]) and torch.equal(a.v_res[:, :, : a.n_res], b.v_res[:, :, : b.n_res])
+        assert flush or torch.equal(got, want)
+    finally:
+        C.PackKVCacheConfigStatic.config = None
