@@ -210,6 +210,11 @@ class PackKVCache(_HFCache):
     # ---------------------------------------------------------------------------------------------
     def update(self, key_states: torch.Tensor, value_states: torch.Tensor, layer_idx: int,
                cache_kwargs: Optional[Dict[str, Any]] = None, **_unused) -> Tuple[Optional[torch.Tensor], Optional[torch.Tensor]]:
+        """Adds T tokens, (B, KV heads, T, D) each, to a layer; the module's description says what is returned.
+
+        A single token of 128 channels is written into the residual by the launch that attends: its tensors, cos and sin among them, must stay
+        as they are until this layer's attend(), flush(), dense() or next update() has been called.  Those of every other call (prompts, narrow
+        heads, materialize) have been read, in stream order, when update() returns."""
         cfg = self._config()
         if PackKVCacheConfigStatic.extract_cache is not None:
             assert not cfg.enable_quant, "Disable quant to enable cache collect."
@@ -359,7 +364,8 @@ class PackKVCache(_HFCache):
 
     def attend(self, query_states: torch.Tensor, layer_idx: int, scaling: Optional[float] = None) -> torch.Tensor:
         """Decode attention for one new token: query_states (B, Hq, 1, 128) after RoPE ->
-        (B, 1, Hq, 128), the layout the reference's eager attention returns (llama.py:210-212)."""
+        (B, 1, Hq, 128), the layout the reference's eager attention returns (llama.py:210-212).  Writes the token that update() left for it;
+        a call that raises leaves it in place."""
         L = self._layers[layer_idx]
         B, Hq, T, D = query_states.shape
         if T != 1:

@@ -325,6 +325,41 @@ def test_narrow_decode_step_inside_the_attention_launch(cuda_device, D, dtype, t
         C.PackKVCacheConfigStatic.config = None
 
 
+def test_steps_from_one_buffer(cuda_device):
+    """A caller that keeps one projection buffer and one pair of table rows for all steps of 128 channels, and writes them again once attend(),
+    flush() or dense() has been called for the step before."""
+    dev, dtype, B, H, G, steps = cuda_device, torch.bfloat16, 2, 2, 4, 6
+    C.PackKVCacheConfigStatic.config = _cfg(QuantMethod.KIVI)
+    try:
+        one, own = C.PackKVCache(B, H * G, 128, 1), C.PackKVCache(B, H * G, 128, 1)
+        k, v = synth.synth_kv(B, H, 300 + steps, 128, seed=3, dtype=dtype, device=dev)
+        cos, sin = synth.rope_tables(300 + steps, 128, device=dev, dtype=dtype)
+        for cache in (one, own):
+            cache.update(k[:, :, :300], v[:, :, :300], 0, {"cos": cos[:, :300], "sin": sin[:, :300]})
+        buf = [torch.empty(B, H, 1, 128, dtype=dtype, device=dev) for _ in range(2)] + [torch.empty(1, 1, 128, dtype=dtype, device=dev) for _ in range(2)]
+        for n in range(steps):
+            t = 300 + n
+            row = [k[:, :, t:t + 1].clone(), v[:, :, t:t + 1].clone(), cos[:, t:t + 1].clone(), sin[:, t:t + 1].clone()]
+            for b, x in zip(buf, row):
+                b.copy_(x)
+            one.update(buf[0], buf[1], 0, {"cos": buf[2], "sin": buf[3]})
+            own.update(row[0], row[1], 0, {"cos": row[2], "sin": row[3]})
+            q = synth.synth_q(B, H * G, 128, seed=n, dtype=dtype).to(dev)
+            if n % 3 == 0:
+                assert torch.equal(one.attend(q, 0), own.attend(q, 0)), n
+            elif n % 3 == 1:
+                one.flush()
+            else:
+                one.dense(0)
+            for b in buf:
+                b.fill_(float("nan"))
+        own.flush()
+        a, b = one._layers[0], own._layers[0]
+        assert a.n_res == b.n_res and torch.equal(a.k_res[:, :, : a.n_res], b.k_res[:, :, : b.n_res]) and torch.equal(a.v_res[:, :, : a.n_res], b.v_res[:, :, : b.n_res])
+    finally:
+        C.PackKVCacheConfigStatic.config = None
+
+
 @pytest.mark.parametrize("D", [64, 96])
 def test_narrow_steps_from_one_buffer(cuda_device, D):
     """A caller that keeps one projection buffer and one pair of table rows for all steps of a narrow-headed model: update() has taken what they
