@@ -1768,6 +1768,10 @@ int launch_attention(const AttnArgs& a, const AttnExchange* xch, const AttnAppen
         // CTAs that need no company fill the places that come free (8 x 32k tokens, 16 CTAs to a pair: 8 x 2 214 us, 2 x 8 204)
         if (waves > 1) cost *= 1 + 0.004 * (cl - 1);
         if (team && sm_warps > 8) cost *= 1.15;                 // a team's extra instructions count once the SM is busy (11 x 2154, 2 bits: 39 us against 35)
+        // and so does how its tiles divide: three to a CTA of a cluster that is no power of two, or a third CTA that leaves the longest with the
+        // two tiles it has without (8 heads, us at 2, 3, 4 CTAs: 18 x 600 tokens 20.7 23.4 29.0, 14 x 600 20.4 20.9 18.4, 18 x 420 17.5 18.5 22.8;
+        // 18 x 521, two tiles each: 20.5 18.5 28.7)
+        if (team && sm_warps > 8 && (cl & (cl - 1)) && (P.tiles_total > 2 * cl || (cl == 3 && P.tiles_total == 4))) cost *= 1.05;
         return cost;
     };
     // Units of the longest warp.  Compressed tiles are dealt from the first owner (warp, or CTA of a team) on, residual
