@@ -393,7 +393,8 @@ __global__ void __launch_bounds__(kAW * 32, PASS == 1 ? PKV_ATTN_CTAS_SCORES : P
     if (PASS != kValues) {
         // Launches are started under programmatic stream serialisation (P.serial): the lines above overlap the end of the launch
         // before; nothing it may have written (q, tables, residual) is touched before it is complete.  Where P.early, the
-        // launch after this one may be set up from here on.
+        // launch after this one may be set up from here on.  What is read of these is read by ordinary loads: the read-only path is for
+        // data that nobody writes while the kernel runs, and this kernel runs already while the one before still writes.
         asm volatile("griddepcontrol.wait;" ::: "memory");
         if (PASS == kFused && P.early) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     }
@@ -435,21 +436,21 @@ __global__ void __launch_bounds__(kAW * 32, PASS == 1 ? PKV_ATTN_CTAS_SCORES : P
     auto load_info = [&](int n) -> uint4 {
         if (n < k_items) {
             const int tl = n >> P.nkb_shift, i = n & (nkb - 1);
-            const uint2 e = __ldg(kinfo_h + (((tw + tl * tstep) << P.nkb_shift) + i) * a.kv_heads);
+            const uint2 e = kinfo_h[(((tw + tl * tstep) << P.nkb_shift) + i) * a.kv_heads];
             return make_uint4(e.x, e.y, 0, 0);
         }
         const int m = n - k_items;
         const int tl = m >> nvi_shift, vi = m & (nvi - 1);
         if (TEAM) {
-            const uint2 e = __ldg(vinfo_h + (((tw + tl * tstep) << nvi_shift) + vi) * (2 * a.kv_heads) + (wic >> 1));
+            const uint2 e = vinfo_h[(((tw + tl * tstep) << nvi_shift) + vi) * (2 * a.kv_heads) + (wic >> 1)];
             return make_uint4(e.x, e.y, 0, 0);
         }
         if (P.vpair) {
             const uint2* p = vinfo_h + (((gw + tl * n_warps) << nvi_shift) + vi) * (2 * a.kv_heads);
-            const uint2 e0 = __ldg(p), e1 = __ldg(p + 1);
+            const uint2 e0 = p[0], e1 = p[1];
             return make_uint4(e0.x, e0.y, e1.x, e1.y);
         }
-        const uint2 e = __ldg(vinfo_h + (gw + tl * n_warps) * (2 * a.kv_heads) + vi);   // one 128-token block per tile: vi = half
+        const uint2 e = vinfo_h[(gw + tl * n_warps) * (2 * a.kv_heads) + vi];   // one 128-token block per tile: vi = half
         return make_uint4(e.x, e.y, 0, 0);
     };
     // (size << 4 | 16-byte phase) of a block that can be copied, 0 for a table entry that points outside the stream
@@ -558,7 +559,7 @@ __global__ void __launch_bounds__(kAW * 32, PASS == 1 ? PKV_ATTN_CTAS_SCORES : P
         const uint4* qp = reinterpret_cast<const uint4*>(
             reinterpret_cast<const T*>(a.q) + ((int64_t)(b * q_heads + h * G + min(g, G - 1))) * P.dim + 8 * c);
 #pragma unroll
-        for (int m = 0; m < 4; m++) qv[m] = g < G && 32 * m + 8 * c < P.dim ? __ldg(qp + 4 * m) : make_uint4(0, 0, 0, 0);
+        for (int m = 0; m < 4; m++) qv[m] = g < G && 32 * m + 8 * c < P.dim ? qp[4 * m] : make_uint4(0, 0, 0, 0);
         if (total_items > 0) issue(0, inf0, nxt_pk0, nxt_pk1);
     } else {
         if (total_items > 0) issue(0, load_info(0), nxt_pk0, nxt_pk1);
@@ -578,7 +579,7 @@ __global__ void __launch_bounds__(kAW * 32, PASS == 1 ? PKV_ATTN_CTAS_SCORES : P
             // the repeated channels behind a narrow head's own add nothing to its scores: q is 0 there
             uint4 v;
             if constexpr (TEAM) v = qv[m];
-            else v = g < G && 32 * m + 8 * c < P.dim ? __ldg(qp + 4 * m) : make_uint4(0, 0, 0, 0);
+            else v = g < G && 32 * m + 8 * c < P.dim ? qp[4 * m] : make_uint4(0, 0, 0, 0);
             unsigned f0[2], f1[2];
             pair_shuffle(v, f0, f1);
             qf[0][m >> 1][m & 1] = f0[0]; qf[1][m >> 1][m & 1] = f0[1];
@@ -824,7 +825,7 @@ __global__ void __launch_bounds__(kAW * 32, PASS == 1 ? PKV_ATTN_CTAS_SCORES : P
             reinterpret_cast<const T*>(a.q) + ((int64_t)(b * q_heads + h * G + min(g, G - 1))) * P.dim + 8 * c);
 #pragma unroll
         for (int m = 0; m < 4; m++) {
-            const uint4 v = g < G && 32 * m + 8 * c < P.dim ? __ldg(qp + 4 * m) : make_uint4(0, 0, 0, 0);
+            const uint4 v = g < G && 32 * m + 8 * c < P.dim ? qp[4 * m] : make_uint4(0, 0, 0, 0);
             pair_shuffle(v, qr[2 * m], qr[2 * m + 1]);
         }
         for (int k = 0; k < my_rt; k++) {
