@@ -195,22 +195,24 @@ void fill_layer(PyObject* layer, const at::Tensor& q, int64_t batch, int64_t n_c
     a.k_mode = extent(mode); a.high_precision_zero = truth(h_hp.o);
 }
 
+const char* const kAppendRows = "append needs k_new / v_new of shape (B, Hkv, 1, %lld) in q's dtype with contiguous channels";
+
 void fill_append(PyObject* append, const at::Tensor& q, const at::Tensor& k_res, int64_t batch, int64_t kv_heads, int64_t n_res, int64_t dim, pkv_attn_append& ap) {
     check(PySequence_Fast_GET_SIZE(append) == 4, "append is (k_new, v_new, cos, sin)");
     PyObject** it = PySequence_Fast_ITEMS(append);
     const at::Tensor &k = cuda(it[0], "k_new"), &v = cuda(it[1], "v_new");
     const at::Tensor *cos = maybe_cuda(it[2], "cos"), *sin = maybe_cuda(it[3], "sin");
-    check(n_res >= 1 && k.dim() == 4 && k.size(0) == batch && k.size(1) == kv_heads && k.size(2) == 1 && k.size(3) == dim && v.sizes() == k.sizes() &&
-              k.stride(3) == 1 && v.stride(3) == 1 && k.scalar_type() == q.scalar_type() && v.scalar_type() == q.scalar_type(),
-          "append needs k_new / v_new of shape (B, Hkv, 1, 128) in q's dtype with contiguous channels");
+    if (!(n_res >= 1 && k.dim() == 4 && k.size(0) == batch && k.size(1) == kv_heads && k.size(2) == 1 && k.size(3) == dim && v.sizes() == k.sizes() &&
+          k.stride(3) == 1 && v.stride(3) == 1 && k.scalar_type() == q.scalar_type() && v.scalar_type() == q.scalar_type()))
+        fail(PyExc_ValueError, kAppendRows, (long long)dim);
     ap.new_k = k.data_ptr(); ap.new_v = v.data_ptr();
     ap.k_stride_b = k.stride(0); ap.k_stride_h = k.stride(1); ap.v_stride_b = v.stride(0); ap.v_stride_h = v.stride(1);
     if (cos) {
-        check(sin && cos->scalar_type() == q.scalar_type() && sin->scalar_type() == q.scalar_type() && cos->dim() >= 2 && cos->size(-2) == 1 &&
-                  cos->size(-1) == dim && sin->sizes() == cos->sizes() && cos->is_contiguous() && sin->is_contiguous(),
-              "cos / sin must be contiguous (B or 1, 1, 128) tensors of q's dtype");
+        if (!(sin && cos->scalar_type() == q.scalar_type() && sin->scalar_type() == q.scalar_type() && cos->dim() >= 2 && cos->size(-2) == 1 &&
+              cos->size(-1) == dim && sin->sizes() == cos->sizes() && cos->is_contiguous() && sin->is_contiguous() &&
+              (cos->size(0) == 1 || cos->numel() >= batch * dim)))
+            fail(PyExc_ValueError, "cos / sin must be contiguous (B or 1, 1, %lld) tensors of q's dtype", (long long)dim);
         ap.cos = cos->data_ptr(); ap.sin = sin->data_ptr(); ap.cs_stride_b = cos->size(0) == 1 ? 0 : dim;
-        check(ap.cs_stride_b == 0 || cos->numel() >= batch * dim, "cos / sin must be contiguous (B or 1, 1, 128) tensors of q's dtype");
     }
     ap.res_capacity = extent(k_res.size(2));
 }
@@ -260,13 +262,13 @@ template <bool NARROW> PyObject* decode_attention_of(PyObject* const* p) {
     }
     a.n_res = extent(n_res); a.batch = extent(batch); a.kv_heads = extent(kv_heads); a.group = extent(q_heads / kv_heads); a.n_comp = extent(n_comp);
     a.is_bf16 = is_bf16(q);
-    a.scaling = p[5] == Py_None ? (float)std::pow(128.0, -0.5) : (float)number(p[5]);
+    a.scaling = p[5] == Py_None ? (float)std::pow((double)q.size(2), -0.5) : (float)number(p[5]);
     a.flags = status_word(*flags);
     pkv_attn_append ap{};
     const bool has_append = p[10] != Py_None;
     const Held append(has_append ? PySequence_Fast(p[10], "append is (k_new, v_new, cos, sin)") : Py_NewRef(Py_None));   // any iterable
     if (has_append) {
-        check(n_res >= 1 && k_res, "append needs k_new / v_new of shape (B, Hkv, 1, 128) in q's dtype with contiguous channels");
+        if (n_res < 1 || !k_res) fail(PyExc_ValueError, kAppendRows, (long long)q.size(2));
         fill_append(append.o, q, *k_res, batch, kv_heads, n_res, q.size(2), ap);
     }
     const pkv_attn_exchange* xch = p[9] == Py_None ? nullptr : reinterpret_cast<const pkv_attn_exchange*>(integer(p[9]));

@@ -271,10 +271,11 @@ def decode_attention(q: torch.Tensor, layer: Optional[CompressedLayer], k_res: O
 
 
 def decode_attention_narrow(q: torch.Tensor, layer: Optional[CompressedLayer], k_res: Optional[torch.Tensor], v_res: Optional[torch.Tensor], n_res: int, *,
-                            scaling: float, flags: Optional[torch.Tensor] = None, kv_heads: Optional[int] = None, append: Optional[tuple] = None,
+                            scaling: Optional[float], flags: Optional[torch.Tensor] = None, kv_heads: Optional[int] = None, append: Optional[tuple] = None,
                             scratch: Optional[torch.Tensor] = None) -> torch.Tensor:
     """decode_attention for heads of D channels, 64 <= D < 128, a multiple of 8, whose stored rows are widened (widen_rows): q (B, Hq, D)
-    from a 16-byte aligned address; the appended rows (B, Hkv, 1, D) and cos / sin (B or 1, 1, D) are widened as they are written.
+    from a 16-byte aligned address; the appended rows (B, Hkv, 1, D) and cos / sin (B or 1, 1, D) are widened as they are written.  scaling: the
+    factor of the scores, None for 1 / sqrt(D).
     Returns (B, Hq, 128): the first D channels of a row are the head's."""
     return _lib.host().decode_attention_narrow(q, layer, k_res, v_res, n_res, scaling, flags, kv_heads, append, scratch)
 

@@ -554,3 +554,20 @@ def test_steps_behind_one_another_on_a_full_gpu(cuda_device, n_comp, plan):
         got.append((x, y, k_res, v_res))
     for a, b in zip(*got):
         assert torch.equal(a.view(torch.int16), b.view(torch.int16))
+
+
+@pytest.mark.parametrize("D", [64, 96, 120])
+def test_narrow_scaling_and_refusals(cuda_device, D):
+    """scaling=None of the narrow form is 1 / sqrt(D), and a refusal names the width that was expected."""
+    dev, B, H, G = cuda_device, 2, 2, 3
+    res = [torch.randn(B, H, 64, 128, device=dev).half() for _ in range(2)]
+    q, row = torch.randn(B, H * G, D, device=dev).half(), torch.randn(B, H, 1, D, device=dev).half()
+    got, want = (ops.decode_attention_narrow(q, None, *res, 50, scaling=s) for s in (None, D ** -0.5))
+    assert torch.equal(got, want)
+    wide = torch.randn(B, H, 1, 128, device=dev).half()
+    with pytest.raises(ValueError, match=rf"\(B, Hkv, 1, {D}\)"):
+        ops.decode_attention_narrow(q, None, *res, 50, scaling=None, append=(wide, wide, None, None))
+    with pytest.raises(ValueError, match=rf"\(B or 1, 1, {D}\)"):
+        ops.decode_attention_narrow(q, None, *res, 50, scaling=None, append=(row, row, wide[0], wide[0]))
+    with pytest.raises(ValueError, match=r"\(B, Hkv, 1, 128\)"):
+        ops.decode_attention(wide.view(B, H, 128), None, *res, 50, append=(row, row, None, None))
