@@ -853,7 +853,18 @@ __global__ void __launch_bounds__(256, 2) kt_fused_encode_kernel(FusedArgs a) {
 // through distributed shared memory (no look-back, no scratch).  16 sequences x 64 tokens x 8 heads, four layers' K and V: 98 us
 // with one CTA per sequence, 49 us this way.
 constexpr int kOneWarps = 4;
-constexpr int kOneBlockCtas = 4 * kSmCount;
+
+// Most CTAs of a one-block launch.  Blocks of 64 and 128 tokens: up to four to an SM this form takes 0.17 to 0.93 of the other's time (us at 592
+// CTAs, 64 tokens, 8 heads: K 11.7 and 8.9, V 13.2 and 10.3; at 888 it is still ahead, 12.0 and 9.4, but the line was not moved).  Blocks of 32
+// tokens are little work: the form loses once its clusters do not all fit at once, which depends on what a CTA holds and on how many make a
+// cluster, unless the other's one CTA per sequence needs a second wave by then (K, 4 heads: 444 CTAs 5.4 and 4.9, 516 5.4 and 6.6; 2 heads: 518
+// 6.0 and 5.0, 592 6.1 and 6.6; 1 head: 592 9.4 and 6.5.  V, 4 heads: 516 6.6 and 5.6, 592 6.6 and 7.6; 2 heads: 592 7.0 and 5.7.  K with
+// parameters per token, 592: 4 heads 6.3 and 7.0, 8 heads 7.9 and 7.3).
+static int one_block_ctas(int heads, int cb, bool is_v, bool per_token) {
+    if (cb != 32 || heads == 1) return 4 * kSmCount;
+    if (per_token) return heads <= 3 || (!is_v && heads > 4) ? 4 * kSmCount : 7 * kSmCount / 2;
+    return heads == 2 ? 7 * kSmCount / 2 : 3 * kSmCount;
+}
 
 // Launched under programmatic stream serialisation: its CTAs are placed while the launch before drains, and touch nothing before
 // that one is complete; the launch after it may be placed from here on.
@@ -1288,7 +1299,7 @@ static int launch_fused_t(const FusedEncodeRequest& r, uint8_t* slots, const uin
     const bool per_token_kernel = r.which == 1 || r.mode == 1;
     const bool k_one = !per_token_kernel && nctx * r.heads <= kKWarpsOne;
     // One token block per sequence and few sequences: one head to a CTA of a cluster (see k_one_block_kernel).
-    if (!env_slots && nctx == 1 && r.heads <= 8 && (int64_t)r.batch * r.heads <= kOneBlockCtas) {
+    if (!env_slots && nctx == 1 && r.heads <= 8 && (int64_t)r.batch * r.heads <= one_block_ctas(r.heads, r.cb, r.which == 1, per_token_kernel)) {
         a.stream = r.stream; a.stream_seq_stride = r.stream_seq_stride; a.capacity = r.capacity; a.stream_bytes = reinterpret_cast<unsigned*>(r.stream_bytes);
         const auto by_block = [&](auto cb) {
             constexpr int CB = decltype(cb)::value;

@@ -217,3 +217,21 @@ def test_v_forms_write_the_same(cuda_device, cb, bits):
             ops.encode_tensor("v", v[b: b + 1], cb, rel, ops.K_TOKEN, bits, cb, **one)
             for name in ("scale", "zero", "stream", "info", "stream_bytes"):
                 assert torch.equal(one[name][0], all_[name][b]), (B, b, name)
+
+
+@pytest.mark.parametrize("which,mode", [("k", ops.K_CHANNEL), ("v", ops.K_TOKEN), ("k", ops.K_TOKEN)])
+@pytest.mark.parametrize("cb", [32, 64, 128])
+def test_one_block_at_the_limits_of_the_form(cuda_device, which, mode, cb):
+    """Calls of one token block per sequence around the numbers of one-head CTAs up to which a cluster takes a sequence, every number of heads:
+    both forms write what a call of two blocks per sequence does."""
+    dev, dtype, rel = cuda_device, torch.bfloat16, synth.rel_for_bits(3)
+    for H in range(1, 9):
+        for ctas in (444, 518, 592) if cb == 32 else (592,):
+            for B in (ctas // H, ctas // H + 1):
+                x = torch.randn(B, H, 2 * cb, 128, generator=torch.Generator(device=dev).manual_seed(B), device=dev).to(dtype)
+                two, one = (_bufs(B, H, 2 * cb, cb, 3, which, mode, dtype, dev) for _ in range(2))
+                ops.encode_tensor(which, x, cb, rel, mode, 3, cb, **two)
+                for i in range(2):
+                    ops.encode_tensor(which, x[:, :, i * cb: (i + 1) * cb], cb, rel, mode, 3, cb, first_token=i * cb, **one)
+                for name in two:
+                    assert torch.equal(one[name].view(torch.uint8), two[name].view(torch.uint8)), (H, B, name)
