@@ -685,27 +685,40 @@ __device__ __forceinline__ void load_row_order(const FusedArgs& a, uint8_t* ord,
     __syncthreads();
 }
 
-// Warps of a V CTA.  A launch ends with the CTAs of its last, partly filled wave, so the form is taken whose waves fit the number of CTAs:
-// three CTAs of 8 warps on every SM take about 30 us and a last wave of one or two to an SM 22 and 32, two of 16 warps 22, one 17
-// (us at 8 heads, 4 bits; V of 160 token blocks 25.4 and 23.1 us, 384: 31.9 and 40.3, 504: 53.0 and 43.8, 640: 64.0 and 60.0,
-// 2048: 147 and 150).  128-token blocks leave room for one CTA of 16 warps only, which pays up to one to an SM.
-static int v_warps(int64_t ctas, int heads, int cb) {
-    if (2 * heads <= 8) return 8;
-    if (cb == 128) return ctas <= kSmCount ? 16 : 8;
-    const auto time = [&](int64_t per_sm, int full, int one, int two) {
-        const int64_t wave = per_sm * kSmCount, rest = ctas % wave;
-        return (int64_t)full * (ctas / wave) + (rest == 0 ? 0 : rest <= kSmCount ? one : rest <= 2 * kSmCount ? two : full);
-    };
-    return time(2, 22, 17, 22) < time(3, 30, 22, 32) ? 16 : 8;
+// Form of a V launch: the warps of a CTA and how many CTAs an SM's registers hold.  Up to one CTA to an SM, 16 warps.  Beyond, a launch ends with
+// the CTAs of its last, partly filled wave, and the form is taken whose waves fit the number of CTAs: 8 warps, three to an SM (waves of 444), or
+// 16, two to an SM (waves of 296).  us with 8 and with 16 warps:
+//   8 heads, 4 bits, 64 tokens: 148 CTAs 26.0 22.1, 296 32.3 30.5, 298 35.5 38.1, 444 39.9 48.8, 500 56.6 47.0, 740 68.5 67.1, 888 72.5 73.9,
+//     1036 92.4 86.8, 1332 102 107, 1500 122 116, 2048 154 154, 4096 275 288; 5 heads: 296 28.2 25.2, 444 32.4 38.1, 592 47.2 38.8, 1500 95.1 90.8
+//   8 heads, 4 bits, 32 tokens: 296 24.5 22.1, 360 26.7 30.4, 592 39.9 34.6, 900 47.4 48.5, 1332 65.2 69.3, 2048 99.2 99.1
+//   16 heads, 4 bits, 64 tokens: 296 58.5 55.4, 298 67.1 70.7, 592 108 104, 888 151 151, 2048 322 332; 32 heads: 148 73.7 58.0, 660 236 246, 1500
+//     486 523; 16 heads, 2 bits: 298 57.8 57.9, 888 128 117, 2048 274 251; 12 heads: 360 47.7 48.5, 444 53.9 52.4, 1500 158 154
+// 128-token blocks leave room for one CTA of 16 warps only, which pays up to one to an SM.  Up to four heads make no more than 8 blocks a CTA.
+struct VForm { int warps, per_sm; };
+static VForm v_form(int64_t ctas, int heads, int bits, int cb) {
+    const VForm narrow{8, 3}, wide{16, 2};
+    if (2 * heads <= 8) return narrow;
+    // (with all registers, for one CTA to an SM, 64-token blocks take 19.6 us instead of 20.3 at 5 heads, 56.6 instead of 58.0 at 32 and the same at 8;
+    // 32-token blocks gain nothing by it: 18.1 and 17.6 at 8 heads)
+    if (ctas <= kSmCount) return cb == 32 ? wide : VForm{16, 1};
+    if (cb == 128) return narrow;
+    const int64_t two = 2 * kSmCount, three = 3 * kSmCount;
+    if (heads <= 8)                                           // 16 where the last wave of 444 is up to two of their CTAs to an SM; of many waves, or of
+        return ctas <= (cb == 32 ? 5 : 12) * kSmCount && (ctas - 1) % three < two ? wide : narrow;     // little work each, 8 do as well or better
+    // above 8 heads the blocks go through the scratch and a warp packs several: 8 warps where 16 would add a wave of their own, and, for the largest
+    // blocks, in launches of many waves
+    const bool added = ctas > two && ctas <= three;
+    if (bits == 4 && cb == 64) return !added && ctas <= 4 * kSmCount ? wide : narrow;
+    return added && heads < 16 ? narrow : wide;
 }
 
 // finished blocks that a warp of the V kernel holds in the direct form until their offsets are known
 __host__ __device__ constexpr int v_slots(int heads, int nw) { return (2 * heads + nw - 1) / nw; }
 
-// NW warps: 8, three CTAs to an SM, or 16, two to an SM at 64 registers: every warp then packs one block of an 8-head token block
-// instead of two, and a CTA takes little more than half the time (see v_warps)
-template <typename T, bool HP, int BITS, int CB, int NW>
-__global__ void __launch_bounds__(NW * 32, NW == 8 ? 3 : CB == 128 ? 1 : 2) v_fused_encode_kernel(FusedArgs a) {
+// NW warps: 8, three CTAs to an SM, or 16, one to an SM or two at 64 registers: every warp then packs one block of an 8-head token block
+// instead of two, and a CTA takes little more than half the time (see v_form)
+template <typename T, bool HP, int BITS, int CB, int NW, int PER_SM>
+__global__ void __launch_bounds__(NW * 32, PER_SM) v_fused_encode_kernel(FusedArgs a) {
     extern __shared__ __align__(16) uint8_t smem[];
     constexpr int LB = len_field_bits(BITS);
     const int lane = lane_id(), wic = threadIdx.x >> 5;
@@ -1376,7 +1389,8 @@ static int launch_fused_t(const FusedEncodeRequest& r, uint8_t* slots, const uin
         bound16 = (g.head_bytes + g.nseg * (g.min_bytes + g.len_bytes + 32 * g.ppt * 2 * BITS) + 15) & ~15;
         a.slot_stride = bound16;
         blocks_per_seq = nctx * 2 * r.heads;
-        const int nw = v_warps((int64_t)nctx * r.batch, r.heads, r.cb);
+        const VForm form = v_form((int64_t)nctx * r.batch, r.heads, BITS, r.cb);
+        const int nw = form.warps;
         const int smem = 32 * r.cb + nw * (r.cb * 64 + (direct ? v_slots(r.heads, nw) : 1) * bound16) + r.cb + 16;
         auto launch_v = [&](auto kern) {
             if (opt_in_smem(kern, smem)) return (int)kCudaError;
@@ -1384,9 +1398,17 @@ static int launch_fused_t(const FusedEncodeRequest& r, uint8_t* slots, const uin
             return (int)kOk;
         };
         int rc = kOk;
-        if (r.cb == 32) rc = nw == 16 ? launch_v(v_fused_encode_kernel<T, HP, BITS, 32, 16>) : launch_v(v_fused_encode_kernel<T, HP, BITS, 32, 8>);
-        else if (r.cb == 64) rc = nw == 16 ? launch_v(v_fused_encode_kernel<T, HP, BITS, 64, 16>) : launch_v(v_fused_encode_kernel<T, HP, BITS, 64, 8>);
-        else rc = nw == 16 ? launch_v(v_fused_encode_kernel<T, HP, BITS, 128, 16>) : launch_v(v_fused_encode_kernel<T, HP, BITS, 128, 8>);
+        const auto by_form = [&](auto cb) {
+            constexpr int CB = decltype(cb)::value;
+            if (nw == 8) return launch_v(v_fused_encode_kernel<T, HP, BITS, CB, 8, 3>);
+            if constexpr (CB != 128)
+                if (CB == 32 || form.per_sm == 2) return launch_v(v_fused_encode_kernel<T, HP, BITS, CB, 16, 2>);
+            if constexpr (CB != 32) return launch_v(v_fused_encode_kernel<T, HP, BITS, CB, 16, 1>);
+            return (int)kUnsupported;
+        };
+        if (r.cb == 32) rc = by_form(std::integral_constant<int, 32>{});
+        else if (r.cb == 64) rc = by_form(std::integral_constant<int, 64>{});
+        else rc = by_form(std::integral_constant<int, 128>{});
         if (rc != kOk) return rc;
     }
     if (direct) return cudaGetLastError() == cudaSuccess ? kOk : kCudaError;

@@ -235,3 +235,23 @@ def test_one_block_at_the_limits_of_the_form(cuda_device, which, mode, cb):
                     ops.encode_tensor(which, x[:, :, i * cb: (i + 1) * cb], cb, rel, mode, 3, cb, first_token=i * cb, **one)
                 for name in two:
                     assert torch.equal(one[name].view(torch.uint8), two[name].view(torch.uint8)), (H, B, name)
+
+
+@pytest.mark.parametrize("heads,cb,bits,ordered", [(5, 64, 4, True), (6, 32, 3, False), (9, 64, 2, False), (16, 64, 4, True), (16, 32, 4, False), (8, 128, 4, False),
+                                                   (5, 128, 2, True)])
+def test_v_forms_of_other_heads_and_blocks(cuda_device, heads, cb, bits, ordered):
+    """The forms of the V launch for other numbers of heads, 128-token blocks, bf16 and rows read through an order write the same; numbers of token
+    blocks on both sides of each line between them: 148, 296, 444, 592 and 888."""
+    dev, dtype, rel = cuda_device, torch.bfloat16, synth.rel_for_bits(bits)
+    g = torch.Generator(device=dev).manual_seed(1)
+    for blocks in (148, 149, 296, 297, 444, 445, 592, 593, 889):
+        v = torch.randn(1, blocks * cb, heads, 128, generator=g, device=dev).to(dtype).transpose(1, 2)
+        order = torch.argsort(torch.rand(blocks, cb, generator=g, device=dev)).to(torch.uint8) if ordered else None
+        more = lambda lo, hi: {} if order is None else dict(order=order[lo:hi].contiguous(), order_block=cb)
+        all_, parts = (_bufs(1, heads, blocks * cb, cb, bits, "v", ops.K_TOKEN, dtype, dev) for _ in range(2))
+        ops.encode_tensor("v", v, cb, rel, ops.K_TOKEN, bits, cb, **all_, **more(0, blocks))
+        for lo in range(0, blocks, 100):                            # calls of up to 100 token blocks: one CTA of 16 warps to an SM
+            hi = min(blocks, lo + 100)
+            ops.encode_tensor("v", v[:, :, lo * cb: hi * cb], cb, rel, ops.K_TOKEN, bits, cb, first_token=lo * cb, **parts, **more(lo, hi))
+        for name in all_:
+            assert torch.equal(all_[name].view(torch.uint8), parts[name].view(torch.uint8)), (blocks, name)
