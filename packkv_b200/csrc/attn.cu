@@ -27,7 +27,8 @@
 //   phase 2  scores -> probabilities in place; V packs are fetched by the lane whose mma fragment
 //            needs them (a pack is 16 tokens of one channel = one row segment of the A operand), so
 //            V needs no transposition at all.
-//   reduce   warps -> CTA in shared memory, CTAs -> rank 0 through distributed shared memory.
+//   reduce   warps -> CTA in shared memory, then the cluster's CTAs share out the sums through distributed shared memory
+//            (with an exchange its first CTA adds them all).
 //
 // Unpack, per pack (16 codes of `len` bits, token 0 in the top bits): one 8-byte window at a 2-byte
 // aligned offset (warp scan of the lengths), then per 8 codes one shift-and-select that puts codes
@@ -288,7 +289,7 @@ struct AttnDev {
     int extra;           // two-launch form with cluster 1: the first `extra` pairs have nsplit + 1 CTAs, so that the CTAs of
                          // all pairs together fill the GPU's CTA slots exactly (grid = (total CTAs, 1, 1)); -1 = uniform
     int dump_bytes;      // bytes of a warp's score region (compressed + residual tiles), a multiple of 16
-    unsigned* sc_count;  // [pairs] arrivals of the pair's clusters in the second launch (zero between launches)
+    unsigned* sc_count;  // [pairs] arrivals in the second launch: of the pair's CTAs, with an exchange of its clusters (zero between launches)
     float* sc_ml;        // [pairs][cluster * nsplit][16] per-CTA max (8 rows) and sum (8 rows)
     uint8_t* sc_scores;  // [pairs][cluster * nsplit * kAW][dump_bytes]
     float* sc_part;      // [pairs][nsplit][8][kD] per-cluster unnormalised output rows
@@ -302,11 +303,11 @@ struct CtaShared {
     float wl[kAW][8];    // a team's per-warp sums of exp(s - wm)
     float gM[kAW][8], gInvL[kAW][8];   // global maximum and reciprocal sum, a copy for every warp
     unsigned lutm[8];    // (2^len - 1) * 0x00010001 per pack length 0..4 (see unpack8)
-    unsigned last;       // two-launch form: this cluster is the pair's last one to deliver its rows
+    unsigned last;       // two-launch form: this CTA (with an exchange: its cluster) is the pair's last one to deliver its rows
     unsigned pad_[3];
     unsigned long long mbar[kAW][2];
 };
-// The CTA's reduced accumulators out[head][channel] (read by rank 0 through distributed shared
+// The CTA's reduced accumulators out[head][channel] (read by the cluster's CTAs through distributed shared
 // memory) live in the warps' regions, which are idle by then: head hd -> warp hd % kAW,
 // float offset (hd / kAW) * kD (at most 8 / kAW rows of 512 bytes per warp: the 2 KB behind out_off hold them).
 __device__ __forceinline__ float* cta_out_row(uint8_t* smem, int warp_smem, int out_off, int hd) {
@@ -328,7 +329,7 @@ __device__ __forceinline__ unsigned deq(unsigned biased, typename Tr<T>::T2 add,
 // =================================================================================================
 // PASS: kFused = everything in one launch (one cluster per pair); kScores = first launch of the two-launch
 // form: K phase, per-CTA max and sum and the score tiles go to the scratch; kValues = second launch: scores
-// come back, global max and sum, V phase, per-cluster rows to the scratch, the pair's last cluster adds them up.
+// come back, global max and sum, V phase, per-cluster rows to the scratch, the pair's last CTA to arrive adds them up.
 enum AttnPass : int { kFused = 0, kScores = 1, kValues = 2 };
 
 // TEAM (single launch only): the four warps of a CTA share its tiles instead of owning tiles each.  Warp w takes the K rounds
@@ -1364,7 +1365,7 @@ __global__ void __launch_bounds__(kAW * 32, PASS == 1 ? PKV_ATTN_CTAS_SCORES : P
     }
     __syncwarp();
     __syncthreads();
-    // ---- CTA reduce, then cluster reduce on rank 0 ---------------------------------------------
+    // ---- CTA reduce, then cluster reduce --------------------------------------------------------
     constexpr int kThreads = kAW * 32;
     for (int d = threadIdx.x; d < kD; d += kThreads) {
         for (int hd = 0; hd < G; hd++) {
@@ -1723,7 +1724,7 @@ int launch_attention(const AttnArgs& a, const AttnExchange* xch, const AttnAppen
     }
     // Cluster size, clusters per pair and staging depth: the (sequence, KV head) pairs times their CTAs should
     // fill the 148 SMs' CTA slots in whole waves, every warp should have work, and a warp's scores must fit in
-    // shared memory.  Cost model: waves x (work units per warp + a fixed part) x (resident warps beyond about 9
+    // shared memory.  Cost model: waves x (work units per warp + a fixed part) x (resident warps beyond about 13
     // per SM share the issue slots).  Several clusters per pair need the scratch and two launches.
     static const int env_cl = env_int("PKV_ATTN_CLUSTER"), env_slots = env_int("PKV_ATTN_SLOTS");
     const int want_cl = plan_io && plan_io->cluster > 0 ? plan_io->cluster : env_cl;
@@ -1752,9 +1753,9 @@ int launch_attention(const AttnArgs& a, const AttnExchange* xch, const AttnAppen
         const int sm_warps = (int)((on_gpu + kSmCount - 1) / kSmCount) * kAW;
         // On a busy SM it makes no difference who holds the residual tiles; on an idle one it is the longest warp's time,
         // and so are the hand-over and the second start of two launches.  Powers of two only.
-        // (The factors here were fitted to 30 shapes timed at every cluster size after the reduction was shared out and the launches
-        // were placed early: the chosen plan is 1.2 % from the best on average, 2.7 % with the factors before; e.g. 4 KV heads x 8192
-        // tokens 26.8 -> 24.7 us, 2 x 4 heads x 900 with 7 heads to a group 12.7 -> 11.3, 40 pairs x 3000 28.9 -> 24.4.)
+        // (The factors were fitted to 30 shapes timed at every cluster size.  Over 264 others, 1 to 500 pairs of 300 to 32768 tokens with every
+        // bit width, block size and K mode, each timed in 16 to 60 plans, the chosen one is 2.5 % from the best on average, 14 % at the 95th
+        // percentile and 22 % at worst: 39 x 8 heads x 575 tokens, 2-bit K, groups of 7, 42.5 us where the best takes 34.7.)
         const bool idle = sm_warps <= 8;
         const double upw_max = team || (idle && !(cl & (cl - 1))) ? upw_placed : upw_dealt;
         if (idle && launches == 2) fixed += 1.0;

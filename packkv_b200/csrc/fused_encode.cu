@@ -6,7 +6,10 @@
 // the separate quantise + pack kernels.
 //
 // The stream format lays blocks back to back, so a block's byte offset is the sum of all earlier
-// block sizes of its sequence.  Two forms:
+// block sizes of its sequence.  Three forms:
+//   one block: ONE launch, for calls of one token block per sequence (what leaves the residual in a decode
+//            step; up to 8 heads, see one_block_ctas): a cluster of one CTA per head takes a sequence, and
+//            they get their offsets from one another's sizes through distributed shared memory.
 //   direct : ONE launch.  A CTA builds its blocks (consecutive in the stream) in shared memory, then
 //            learns the offset of its first block from the CTAs before it in the sequence by a
 //            decoupled look-back over a small status array (every CTA publishes the bytes of its own
@@ -16,7 +19,8 @@
 //            and a CTA that gives up raises the timeout flag and writes nothing.
 //            HBM traffic per element: 2 B read (the second read of a tile comes from L1/L2) + the
 //            block bytes written once (~0.56 B at 4 bit).
-//   slots  : three launches, no device-side waiting (more than 8 heads, or on request): encode into
+//   slots  : three launches, no device-side waiting (more than 8 heads or 128-token blocks in the kernels
+//            with per-token parameters, or on request): encode into
 //            fixed-stride SLOTS in scratch memory with the size in block_info[blk][1]; per-sequence
 //            exclusive scan (scan_sizes_kernel, pack.cu); one warp per block copies its slot to its
 //            final offset.  The block bytes are written, read and written once more.
@@ -187,9 +191,9 @@ __device__ __forceinline__ void store_slot(uint8_t* slot, const uint8_t* stage, 
 // ------------------------------------------------------------------------------------------ K
 // One round of a K block: quantise 16 tokens x 4 channels per lane and pack them at `at`: minima, lengths, packs.  row(t) gives the
 // lane's four elements of the round's token t.  Returns the round's bytes.
-template <typename T, bool HP, int BITS, bool FAST, typename Row>
-__device__ __forceinline__ unsigned k_encode_round(Row row, const Quantiser<T, HP>& q0, const Quantiser<T, HP>& q1, const Quantiser<T, HP>& q2,
-                                                   const Quantiser<T, HP>& q3, uint8_t* at, int lane, unsigned& over) {
+template <typename T, int BITS, typename Row>
+__device__ __forceinline__ unsigned k_encode_round(Row row, const Quantiser<T, false>& q0, const Quantiser<T, false>& q1, const Quantiser<T, false>& q2,
+                                                   const Quantiser<T, false>& q3, uint8_t* at, int lane, unsigned& over) {
     constexpr int LB = len_field_bits(BITS), kMin = 16 * BITS, kLen = 16 * LB;
     const int z0 = (int)q0.zero, z1 = (int)q1.zero, z2 = (int)q2.zero, z3 = (int)q3.zero;
     unsigned u[16];                                   // four channel codes per token, one byte each
@@ -198,8 +202,8 @@ __device__ __forceinline__ unsigned k_encode_round(Row row, const Quantiser<T, H
     for (int t = 0; t < 16; t++) {
         const uint2 raw = row(t);
         const T* e = reinterpret_cast<const T*>(&raw);
-        const unsigned c0 = q0.template code_u8<FAST>(QT<T>::ld(e), z0), c1 = q1.template code_u8<FAST>(QT<T>::ld(e + 1), z1);
-        const unsigned c2 = q2.template code_u8<FAST>(QT<T>::ld(e + 2), z2), c3 = q3.template code_u8<FAST>(QT<T>::ld(e + 3), z3);
+        const unsigned c0 = q0.template code_u8<false>(QT<T>::ld(e), z0), c1 = q1.template code_u8<false>(QT<T>::ld(e + 1), z1);
+        const unsigned c2 = q2.template code_u8<false>(QT<T>::ld(e + 2), z2), c3 = q3.template code_u8<false>(QT<T>::ld(e + 3), z3);
         mnj[0] = min(mnj[0], c0); mxj[0] = max(mxj[0], c0);
         mnj[1] = min(mnj[1], c1); mxj[1] = max(mxj[1], c1);
         mnj[2] = min(mnj[2], c2); mxj[2] = max(mxj[2], c2);
@@ -330,7 +334,7 @@ __device__ __forceinline__ int k_encode_rounds(const T* x, int64_t ss, const uin
             const int at = ORDERED ? (int)((ow[t >> 2] >> (8 * (t & 3))) & 0xFFu) : r * 16 + t;
             return __ldg(reinterpret_cast<const uint2*>(x + (int64_t)at * ss));
         };
-        pos += MODE == 0 ? k_encode_round<T, false, BITS, false>(row, q0, q1, q2, q3, stage + pos, lane, over)
+        pos += MODE == 0 ? k_encode_round<T, BITS>(row, q0, q1, q2, q3, stage + pos, lane, over)
                          : k_encode_round_packed<T, BITS, MODE == 2>(row, q0, q1, q2, q3, pq, stage + pos, lane, over);
         if (lane == 0) *reinterpret_cast<uint16_t*>(stage + 2 * r) = (uint16_t)(pos - g.head_bytes);
     }
@@ -349,10 +353,8 @@ constexpr int kKWarps = PKV_K_WARPS;   // warps (= consecutive blocks of a seque
 constexpr int kKWarpsOne = 8;          // and when that many blocks are all there is of a sequence: one CTA then needs no look-back
 template <typename T, bool CONTIG, int BITS, bool ORDERED, int NW>
 __global__ void __launch_bounds__(NW * 32, 768 / (NW * 32)) k_fused_encode_kernel(FusedArgs a) {
-    constexpr bool HP = false;
     const int64_t ss = CONTIG ? 128 : a.ss;
     extern __shared__ __align__(16) uint8_t smem[];
-    constexpr int LB = len_field_bits(BITS);
     const int lane = lane_id(), wic = threadIdx.x >> 5;
     const int nctx = a.tokens / a.cb;
     const int64_t per_seq = (int64_t)nctx * a.heads;
@@ -393,7 +395,7 @@ __global__ void __launch_bounds__(NW * 32, 768 / (NW * 32)) k_fused_encode_kerne
     }
     const float lo[4] = {QT<T>::lo_f(lo01), QT<T>::hi_f(lo01), QT<T>::lo_f(lo23), QT<T>::hi_f(lo23)};
     const float hi[4] = {QT<T>::lo_f(hi01), QT<T>::hi_f(hi01), QT<T>::lo_f(hi23), QT<T>::hi_f(hi23)};
-    const Quantiser<T, HP> q0(lo[0], hi[0], a.rel), q1(lo[1], hi[1], a.rel), q2(lo[2], hi[2], a.rel), q3(lo[3], hi[3], a.rel);
+    const Quantiser<T, false> q0(lo[0], hi[0], a.rel), q1(lo[1], hi[1], a.rel), q2(lo[2], hi[2], a.rel), q3(lo[3], hi[3], a.rel);
     {
         const int64_t pi = (((int64_t)b * a.heads + h) * a.param_blocks + a.first_block + cbi) * 128 + 4 * lane;
         T sc[4] = {QT<T>::cvt(q0.scale), QT<T>::cvt(q1.scale), QT<T>::cvt(q2.scale), QT<T>::cvt(q3.scale)};
@@ -717,10 +719,9 @@ __host__ __device__ constexpr int v_slots(int heads, int nw) { return (2 * heads
 
 // NW warps: 8, three CTAs to an SM, or 16, one to an SM or two at 64 registers: every warp then packs one block of an 8-head token block
 // instead of two, and a CTA takes little more than half the time (see v_form)
-template <typename T, bool HP, int BITS, int CB, int NW, int PER_SM>
+template <typename T, int BITS, int CB, int NW, int PER_SM>
 __global__ void __launch_bounds__(NW * 32, PER_SM) v_fused_encode_kernel(FusedArgs a) {
     extern __shared__ __align__(16) uint8_t smem[];
-    constexpr int LB = len_field_bits(BITS);
     const int lane = lane_id(), wic = threadIdx.x >> 5;
     const int nctx = a.tokens / CB;
     __shared__ unsigned sh_word, sh_sizes[16];
@@ -797,7 +798,6 @@ __global__ void __launch_bounds__(NW * 32, PER_SM) v_fused_encode_kernel(FusedAr
 template <typename T, int BITS, int CB>
 __global__ void __launch_bounds__(256, 2) kt_fused_encode_kernel(FusedArgs a) {
     extern __shared__ __align__(16) uint8_t smem[];
-    constexpr int LB = len_field_bits(BITS);
     const int lane = lane_id(), wic = threadIdx.x >> 5;
     const int nctx = a.tokens / CB;
     __shared__ unsigned sh_word, sh_sizes[8];
@@ -993,7 +993,7 @@ __global__ void __launch_bounds__(kOneWarps * 32) k_one_block_kernel(FusedArgs a
                                : k_encode_round_packed<T, BITS, false>(row, q0, q1, q2, q3, pq, stage[r], lane, over);
                 over &= ~(((1u << BITS) - 1u) * 0x00010001u);
             } else {
-                size = k_encode_round<T, false, BITS, false>(row, q0, q1, q2, q3, stage[r], lane, over);
+                size = k_encode_round<T, BITS>(row, q0, q1, q2, q3, stage[r], lane, over);
             }
             bad = bad || over != 0;
             if (lane == 0) sizes[r] = size;
@@ -1291,7 +1291,7 @@ int64_t fused_encode_scratch_bytes(const FusedEncodeRequest& r) {
     return (int64_t)r.batch * nblk * ((bound + 15) & ~15);
 }
 
-template <typename T, bool HP, int BITS>
+template <typename T, int BITS>
 static int launch_fused_t(const FusedEncodeRequest& r, uint8_t* slots, const uint8_t* order, int order_block, cudaStream_t st) {
     FusedArgs a{};
     a.order = order; a.order_block = order_block;
@@ -1400,10 +1400,10 @@ static int launch_fused_t(const FusedEncodeRequest& r, uint8_t* slots, const uin
         int rc = kOk;
         const auto by_form = [&](auto cb) {
             constexpr int CB = decltype(cb)::value;
-            if (nw == 8) return launch_v(v_fused_encode_kernel<T, HP, BITS, CB, 8, 3>);
+            if (nw == 8) return launch_v(v_fused_encode_kernel<T, BITS, CB, 8, 3>);
             if constexpr (CB != 128)
-                if (CB == 32 || form.per_sm == 2) return launch_v(v_fused_encode_kernel<T, HP, BITS, CB, 16, 2>);
-            if constexpr (CB != 32) return launch_v(v_fused_encode_kernel<T, HP, BITS, CB, 16, 1>);
+                if (CB == 32 || form.per_sm == 2) return launch_v(v_fused_encode_kernel<T, BITS, CB, 16, 2>);
+            if constexpr (CB != 32) return launch_v(v_fused_encode_kernel<T, BITS, CB, 16, 1>);
             return (int)kUnsupported;
         };
         if (r.cb == 32) rc = by_form(std::integral_constant<int, 32>{});
@@ -1426,12 +1426,12 @@ static int launch_fused_t(const FusedEncodeRequest& r, uint8_t* slots, const uin
     return cudaGetLastError() == cudaSuccess ? kOk : kCudaError;
 }
 
-template <typename T, bool HP>
+template <typename T>
 static int launch_fused_b(const FusedEncodeRequest& r, uint8_t* slots, const uint8_t* order, int order_block, cudaStream_t st) {
     switch (r.bits) {
-        case 2: return launch_fused_t<T, HP, 2>(r, slots, order, order_block, st);
-        case 3: return launch_fused_t<T, HP, 3>(r, slots, order, order_block, st);
-        case 4: return launch_fused_t<T, HP, 4>(r, slots, order, order_block, st);
+        case 2: return launch_fused_t<T, 2>(r, slots, order, order_block, st);
+        case 3: return launch_fused_t<T, 3>(r, slots, order, order_block, st);
+        case 4: return launch_fused_t<T, 4>(r, slots, order, order_block, st);
     }
     return kUnsupported;
 }
@@ -1448,7 +1448,7 @@ int launch_fused_encode(const FusedEncodeRequest& r, uint8_t* slots, const uint8
     if ((int64_t)r.batch * r.tokens == 0) return kOk;
     if (!r.x || !r.scale || !r.zero || !r.stream || !r.block_info || !r.stream_bytes || !r.flags || !slots) return kBadArgument;
     if ((reinterpret_cast<uintptr_t>(slots) & 15) || (reinterpret_cast<uintptr_t>(r.stream) & 1) || (r.stream_seq_stride & 1)) return kBadArgument;
-    return r.is_bf16 ? launch_fused_b<__nv_bfloat16, false>(r, slots, order, order_block, st) : launch_fused_b<__half, false>(r, slots, order, order_block, st);
+    return r.is_bf16 ? launch_fused_b<__nv_bfloat16>(r, slots, order, order_block, st) : launch_fused_b<__half>(r, slots, order, order_block, st);
 }
 
 #ifdef PKV_DEBUG_CHAIN
