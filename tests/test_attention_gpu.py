@@ -571,3 +571,70 @@ def test_narrow_scaling_and_refusals(cuda_device, D):
         ops.decode_attention_narrow(q, None, *res, 50, scaling=None, append=(row, row, wide[0], wide[0]))
     with pytest.raises(ValueError, match=r"\(B, Hkv, 1, 128\)"):
         ops.decode_attention(wide.view(B, H, 128), None, *res, 50, append=(row, row, None, None))
+
+
+@pytest.mark.parametrize("plan", [(4, 1, 1), (1, 3, 2), None])
+def test_encode_then_attend_without_waiting(cuda_device, plan):
+    """Every launch may be placed while the one before it still runs: steps that pack one token block of K and V into the buffers that are there and
+    at once attend over them, the query being the step before's output, give the bits of steps that wait after every call; so do the same calls
+    in a captured graph, replayed twice."""
+    import copy
+    dev, dtype, B, H, G, n0, steps = cuda_device, torch.bfloat16, 3, 4, 2, 256, 5
+    cap, rel = n0 + 64 * steps, synth.rel_for_bits(4)
+    k, v = synth.synth_kv(B, H, cap, 128, seed=12, dtype=dtype, device=dev)
+    g = torch.Generator(device=dev).manual_seed(5)
+    k_res, v_res = (torch.randn(B, H, 64, 128, generator=g, device=dev).to(dtype) for _ in range(2))
+    x0 = torch.randn(B, H * G, 128, generator=g, device=dev).to(dtype)
+
+    def buffers():
+        info = lambda n: torch.zeros(B, n, 2, dtype=torch.int32, device=dev)
+        par = lambda *s: torch.zeros(*s, dtype=dtype, device=dev)
+        stream = lambda w: torch.zeros(B, encode.stream_capacity(w, cap, H, 64, 4), dtype=torch.uint8, device=dev)
+        count = lambda: torch.zeros(B, dtype=torch.int32, device=dev)
+        L = ops.CompressedLayer(k_stream=stream("k"), k_info=info(cap // 64 * H), k_bytes=count(), k_scale=par(B, H, cap // 64, 128), k_zero=par(B, H, cap // 64, 128),
+                                v_stream=stream("v"), v_info=info(cap // 64 * 2 * H), v_bytes=count(), v_scale=par(B, cap), v_zero=par(B, cap),
+                                n_comp=0, kv_heads=H, cbk=64, cbv=64, bits_k=4, bits_v=4, k_mode=ops.K_CHANNEL, high_precision_zero=False)
+        return L, ops.new_flags(dev), ops.new_attention_scratch(dev), [torch.empty_like(x0) for _ in range(steps + 1)]
+
+    def pack(L, flags, lo, hi):
+        for which, x, mode in (("k", k, ops.K_CHANNEL), ("v", v, ops.K_TOKEN)):
+            ops.encode_tensor(which, x[:, :, lo:hi], 64, rel, mode, 4, 64, first_token=lo, flags=flags, scratch=work,
+                              **{name: getattr(L, f"{which}_{field}") for name, field in
+                                 (("scale", "scale"), ("zero", "zero"), ("stream", "stream"), ("info", "info"), ("stream_bytes", "bytes"))})
+
+    def run(state, sync):
+        L, flags, scratch, xs = state
+        xs[0].copy_(x0)
+        for n in range(steps):
+            pack(L, flags, n0 + 64 * n, n0 + 64 * (n + 1))
+            sync()
+            at = copy.copy(L)
+            at.n_comp = n0 + 64 * (n + 1)
+            ops.decode_attention(xs[n], at, k_res, v_res, 50, out=xs[n + 1], flags=flags, scratch=scratch, plan=plan, scaling=1.0)
+            sync()
+
+    work = torch.empty(B * cap * H * 128, dtype=torch.uint8, device=dev)
+    states = [buffers() for _ in range(3)]
+    for L, flags, _, _ in states:
+        pack(L, flags, 0, n0)
+    torch.cuda.synchronize()
+    run(states[0], torch.cuda.synchronize)
+    run(states[1], lambda: None)
+    torch.cuda.synchronize()
+    L = states[2][0]
+    first = [L.k_bytes.clone(), L.v_bytes.clone()]
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        L.k_bytes.copy_(first[0])
+        L.v_bytes.copy_(first[1])
+        run(states[2], lambda: None)
+    for _ in range(2):
+        for x in states[2][3]:
+            x.fill_(float("nan"))
+        graph.replay()
+    torch.cuda.synchronize()
+    for state in states[1:]:
+        assert int(state[1].item()) == 0
+        for a, b in zip(state[3], states[0][3]):
+            assert torch.equal(a.view(torch.int16), b.view(torch.int16))
+        assert torch.equal(state[0].v_stream, states[0][0].v_stream) and torch.equal(state[0].k_stream, states[0][0].k_stream)
