@@ -262,7 +262,7 @@ template <bool NARROW> PyObject* decode_attention_of(PyObject* const* p) {
     }
     a.n_res = extent(n_res); a.batch = extent(batch); a.kv_heads = extent(kv_heads); a.group = extent(q_heads / kv_heads); a.n_comp = extent(n_comp);
     a.is_bf16 = is_bf16(q);
-    a.scaling = p[5] == Py_None ? (float)std::pow((double)q.size(2), -0.5) : (float)number(p[5]);
+    a.scaling = p[5] == Py_None ? (float)std::pow(NARROW ? (double)q.size(2) : 128.0, -0.5) : (float)number(p[5]);   // (a constant for 128)
     a.flags = status_word(*flags);
     pkv_attn_append ap{};
     const bool has_append = p[10] != Py_None;
