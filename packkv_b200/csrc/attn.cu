@@ -1384,19 +1384,25 @@ __global__ void __launch_bounds__(kAW * 32, PASS == 1 ? PKV_ATTN_CTAS_SCORES : P
     if (spread || rank == 0) {
         const int first = (spread ? rank : 0) * kThreads + (int)threadIdx.x, stride = (spread ? P.cluster : 1) * kThreads;
         const auto cluster_sum = [&](int e) {
-            // (as many loads as the cluster has CTAs, nearly: with sixteen for every size, fifteen of them predicated off, launches of one CTA to a
-            // cluster took 2 to 3 % longer than with one load after the other: 48 x 8 heads x 925 tokens in groups of 8 57.0 us, 55.1 this way)
+            // (in fours, as far as the cluster goes: with sixteen for every size, fifteen of them predicated off, launches of one CTA to a
+            // cluster took 2 to 3 % longer than with one load after the other: 48 x 8 heads x 925 tokens in groups of 8 57.0 us, 55.1 without.
+            // One copy of the loads: a second one for small clusters cost launches of few warps, which wait for their code, 0.1 of 9 to 10 us)
             float* row = cta_out_row(smem, P.warp_smem, P.out_off, e / kD) + e % kD;
             if (P.cluster == 1) return *row;
-            const auto sum_of = [&](auto most) {
-                float x[decltype(most)::value], v = 0.f;
+            float x[16], v = 0.f;
 #pragma unroll
-                for (int r = 0; r < decltype(most)::value; r++) x[r] = r < P.cluster ? *cluster.map_shared_rank(row, r) : 0.f;
+            for (int r0 = 0; r0 < 16; r0 += 4) {
 #pragma unroll
-                for (int r = 0; r < decltype(most)::value; r++) v += x[r];
-                return v;
-            };
-            return P.cluster <= 4 ? sum_of(std::integral_constant<int, 4>{}) : sum_of(std::integral_constant<int, 16>{});
+                for (int r = r0; r < r0 + 4; r++) x[r] = 0.f;
+                if (r0 < P.cluster) {
+#pragma unroll
+                    for (int r = r0; r < r0 + 4; r++)
+                        if (r < P.cluster) x[r] = *cluster.map_shared_rank(row, r);
+                }
+            }
+#pragma unroll
+            for (int r = 0; r < 16; r++) v += x[r];
+            return v;
         };
         const auto put = [&](int e, float v) {
             const T r = Tr<T>::from_float(v);
