@@ -19,7 +19,7 @@
 //            and a CTA that gives up raises the timeout flag and writes nothing.
 //            HBM traffic per element: 2 B read (the second read of a tile comes from L1/L2) + the
 //            block bytes written once (~0.56 B at 4 bit).
-//   slots  : three launches, no device-side waiting (more than 8 heads or 128-token blocks in the kernels
+//   slots  : three launches, no device-side waiting (more than 8 heads in the kernels
 //            with per-token parameters, or on request): encode into
 //            fixed-stride SLOTS in scratch memory with the size in block_info[blk][1]; per-sequence
 //            exclusive scan (scan_sizes_kernel, pack.cu); one warp per block copies its slot to its
@@ -134,21 +134,21 @@ __device__ __forceinline__ bool chain_offset(const FusedArgs& a, int b, int link
 
 // One warp copies a finished block from shared memory (16-byte aligned) to its place in the stream (even address).
 __device__ __forceinline__ void store_block(uint8_t* dst, const uint8_t* stage, int size, int lane) {
-    const int phase = (int)(reinterpret_cast<uintptr_t>(dst) & 15);   // even
-    const int head = min((16 - phase) & 15, size);                    // bytes before the first aligned chunk
-    for (int j = 2 * lane; j < head; j += 64) *reinterpret_cast<uint16_t*>(dst + j) = *reinterpret_cast<const uint16_t*>(stage + j);
+    const int head = min((int)(0u - (unsigned)reinterpret_cast<uintptr_t>(dst)) & 15, size);   // bytes before the first aligned chunk, even
     const int nfull = (size - head) >> 4;
-    const unsigned* s32 = reinterpret_cast<const unsigned*>(stage);
-    const int sw = head >> 2;                                          // first source word of the body
-    const unsigned sh = (unsigned)(head & 3) * 8;                      // 0 or 16: byte offset inside that word
-    for (int c = lane; c < nfull; c += 32) {
-        const unsigned* p = s32 + sw + 4 * c;                          // aligned 32-bit loads, realigned by funnel shifts
-        const unsigned w0 = p[0], w1 = p[1], w2 = p[2], w3 = p[3], w4 = sh ? p[4] : 0u;
-        *reinterpret_cast<uint4*>(dst + head + 16 * c) = make_uint4(__funnelshift_r(w0, w1, sh), __funnelshift_r(w1, w2, sh),
-                                                                    __funnelshift_r(w2, w3, sh), __funnelshift_r(w3, w4, sh));
+    // the halfwords before the first chunk (at most seven, lanes 0 ..) and behind the last one (at most seven, lanes 8 ..)
+    {
+        const int at = lane < 8 ? 2 * lane : head + 16 * nfull + 2 * (lane - 8);
+        if (at < (lane < 8 ? head : lane < 16 ? size : 0)) *reinterpret_cast<uint16_t*>(dst + at) = *reinterpret_cast<const uint16_t*>(stage + at);
     }
-    for (int j = head + 16 * nfull + 2 * lane; j < size; j += 64)
-        *reinterpret_cast<uint16_t*>(dst + j) = *reinterpret_cast<const uint16_t*>(stage + j);
+    const unsigned sh = (unsigned)(head & 3) * 8;                      // 0 or 16: byte offset inside the first source word of a chunk
+    const unsigned* p = reinterpret_cast<const unsigned*>(stage + (head & ~3)) + 4 * lane;
+    uint4* d = reinterpret_cast<uint4*>(dst + head) + lane;
+    for (int c = lane; c < nfull; c += 32, p += 128, d += 32) {
+        // aligned 32-bit loads, realigned by funnel shifts (the fifth word counts only where sh is not 0: then it is inside the block)
+        const unsigned w0 = p[0], w1 = p[1], w2 = p[2], w3 = p[3], w4 = sh ? p[4] : 0u;
+        *d = make_uint4(__funnelshift_r(w0, w1, sh), __funnelshift_r(w1, w2, sh), __funnelshift_r(w2, w3, sh), __funnelshift_r(w3, w4, sh));
+    }
 }
 
 // Direct form, after every warp of the CTA has put the sizes of its blocks into sizes[0..n): warp 0 gets the
@@ -180,6 +180,53 @@ __device__ __forceinline__ void chain_store(const FusedArgs& a, int b, int link,
             continue;
         }
         store_block(a.stream + (int64_t)b * a.stream_seq_stride + off, stage_of(j), (int)size, lane);
+    }
+}
+
+// A V block that lies in PARTS segments (part i at part(i), its bytes in sizes[i]) to dst: the table of segment ends, then the segments.
+template <int PARTS, typename Part>
+__device__ __forceinline__ void store_parts(uint8_t* dst, const unsigned* sizes, int lane, Part part) {
+    unsigned end = 0;
+#pragma unroll
+    for (int i = 0; i < PARTS; i++) {
+        store_block(dst + 2 * PARTS + end, part(i), (int)sizes[i], lane);
+        end += sizes[i];
+        if (lane == 0) *reinterpret_cast<uint16_t*>(dst + 2 * i) = (uint16_t)end;
+    }
+}
+template <int PARTS>
+__device__ __forceinline__ unsigned parts_size(const unsigned* sizes) {
+    unsigned size = 2 * PARTS;
+#pragma unroll
+    for (int i = 0; i < PARTS; i++) size += sizes[i];
+    return size;
+}
+
+// chain_store for n <= 32 blocks that lie in PARTS segments each (see store_parts): segment i of block j at part(j, i).
+template <int PARTS, typename Part>
+__device__ __forceinline__ void chain_store_parts(const FusedArgs& a, int b, int link, const unsigned* sizes, int n, unsigned* sh_word, int64_t info_first,
+                                                  int nwarps, Part part) {
+    const int lane = lane_id(), wic = threadIdx.x >> 5;
+    __syncthreads();
+    const unsigned mine = lane < n ? parts_size<PARTS>(sizes + lane * PARTS) : 0u;      // lane: block
+    const unsigned incl = warp_inclusive_sum(mine);
+    if (wic == 0) {
+        unsigned off;
+        const bool ok = chain_offset(a, b, link, __shfl_sync(0xffffffffu, incl, 31), off);
+        if (lane == 0) *sh_word = ok ? off : 0xFFFFFFFFu;
+    }
+    __syncthreads();
+    const unsigned base = *sh_word;
+    if (base == 0xFFFFFFFFu) return;
+    for (int j = wic; j < n; j += nwarps) {
+        const unsigned size = __shfl_sync(0xffffffffu, mine, j), off = base + __shfl_sync(0xffffffffu, incl, j) - size;
+        uint32_t* bi = a.info + ((int64_t)b * a.info_seq_stride + info_first + j) * 2;
+        if (lane == 0) { bi[0] = off; bi[1] = size; }
+        if ((int64_t)off + size > a.capacity) {
+            if (lane == 0) atomicOr(a.flags, kFlagStreamOverflow);
+            continue;
+        }
+        store_parts<PARTS>(a.stream + (int64_t)b * a.stream_seq_stride + off, sizes + j * PARTS, lane, [&](int i) { return part(j, i); });
     }
 }
 
@@ -248,6 +295,105 @@ __device__ __forceinline__ unsigned k_encode_round(Row row, const Quantiser<T, f
     return kMin + kLen + 2 * before;
 }
 
+// A pack's len halfwords to shared memory (even address): four predicated stores, 13 instructions less than with branches
+__device__ __forceinline__ void sts_pack(unsigned at, uint64_t w, int len) {
+    const unsigned lo = (unsigned)w, hi = (unsigned)(w >> 32);
+    asm volatile(
+        "{ .reg .pred a, b, c, d; .reg .b16 l0, l1, h0, h1;\n"
+        "mov.b32 {l0, l1}, %1; mov.b32 {h0, h1}, %2;\n"
+        "setp.gt.s32 a, %3, 0; setp.gt.s32 b, %3, 1; setp.gt.s32 c, %3, 2; setp.gt.s32 d, %3, 3;\n"
+        "@a st.shared.u16 [%0], l0; @b st.shared.u16 [%0+2], l1; @c st.shared.u16 [%0+4], h0; @d st.shared.u16 [%0+6], h1; }"
+        ::"r"(at), "r"(lo), "r"(hi), "r"(len) : "memory");
+}
+// The lanes' words of W bits (8, 12 or 16) as a bit string at shared address at (even).  All 32 lanes call.
+template <int W>
+__device__ __forceinline__ void sts_lane_fields(unsigned at, int lane, unsigned word) {
+    static_assert(W == 8 || W == 12 || W == 16, "header fields of four channels");
+    if (W == 8) {
+        asm volatile("st.shared.u8 [%0], %1;" ::"r"(at + lane), "r"(word) : "memory");
+    } else if (W == 16) {
+        sts16(at + 2 * lane, (unsigned short)word);
+    } else {                                             // four lanes' words are three halfwords: lanes 0, 1, 2 of four store one each
+        const unsigned next = __shfl_down_sync(0xffffffffu, word, 1);
+        const int i = lane & 3;
+        if (i < 3) sts16(at + 6 * (lane >> 2) + 2 * i, (unsigned short)((word >> (4 * i)) | (next << (12 - 4 * i))));
+    }
+}
+
+// A pack's word from its four groups of four tokens, 4 len bits each, in 16-bit lanes: tokens 0 .. 3 above 4 .. 7 in za, 8 .. 11 above 12 .. 15 in
+// zb; step4 = 2^(4 len).
+__device__ __forceinline__ uint64_t join_lanes(unsigned za, unsigned zb, int len, unsigned step4) {
+    const unsigned close = step4 - 65536u, wt = (za >> 16) * close + za, wb = (zb >> 16) * close + zb;   // upper lane * 2^(4 len) + lower lane
+    const unsigned step8 = step4 * step4;                                                               // 2^(8 len), 0 for len 4
+    return (uint64_t)__funnelshift_lc(wt, 0u, 8 * len) << 32 | (wt * step8 + wb);
+}
+
+// The packs of four channels from the codes of 16 tokens and their minima and maxima (two channels to a word, 16-bit lanes): lengths
+// (one to a byte in lens4) and words (token 0 in the top bits).  codes(j, t): channel j's codes of tokens t and t + 4, t's above.
+template <int BITS, typename Codes>
+__device__ __forceinline__ void pack_words(Codes codes, unsigned mn01, unsigned mx01, unsigned mn23, unsigned mx23,
+                                           int (&len)[4], unsigned& lens4, uint64_t (&w)[4]) {
+    const unsigned d01 = mx01 - mn01, d23 = mx23 - mn23;     // lane-wise: no borrow, max >= min
+    const unsigned dj[4] = {d01 & 0xFFFFu, d01 >> 16, d23 & 0xFFFFu, d23 >> 16};
+    lens4 = 0;
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+        len[j] = min(bit_length_u32(dj[j]), BITS);
+        lens4 |= (unsigned)len[j] << (8 * j);
+        // 16-bit lanes, four tokens each (tokens 0 .. 3 above 4 .. 7, 8 .. 11 above 12 .. 15): z = z * 2^len + code for two of them per
+        // multiply-add, then the minimum is taken off all four fields at once (min * (1 + 2^len + ... + 2^(3 len))); modulo 2^32, so
+        // that the codes may carry a common offset that the minimum carries too.
+        // In the end a lane is below 2^16: four codes below 2^4 at steps of at most 2^4.  Against one multiply-add and one
+        // extraction per code: 1.6 instead of 2.8 instructions per code.
+        unsigned step = 1u << len[j];
+        asm("" : "+r"(step));                             // a number, or the compiler makes a shift and an addition of every multiply-add
+        unsigned za = codes(j, 0), zb = codes(j, 8);
+#pragma unroll
+        for (int t = 1; t < 4; t++) {
+            za = za * step + codes(j, t);
+            zb = zb * step + codes(j, t + 8);
+        }
+        const unsigned step2 = step * step, off = 0u - (step2 * step + step2) - step - 1u, both = __byte_perm(j < 2 ? mn01 : mn23, 0, j & 1 ? 0x3232 : 0x1010);
+        za += both * off;
+        zb += both * off;
+        w[j] = join_lanes(za, zb, len[j], step2 * step2);
+    }
+}
+
+// A round of a K block (16 tokens x 128 channels, four channels to a lane) at `at`: minima, lengths, packs.  Returns its bytes.
+template <int BITS>
+__device__ __forceinline__ unsigned k_store_round(unsigned at, int lane, unsigned minword, unsigned lenword, unsigned lens4, const int (&len)[4],
+                                                  const uint64_t (&w)[4]) {
+    constexpr int LB = len_field_bits(BITS), kMin = 16 * BITS, kLen = 16 * LB;
+    sts_lane_fields<4 * BITS>(at, lane, minword);
+    sts_lane_fields<4 * LB>(at + kMin, lane, lenword);
+    const unsigned inc = warp_inclusive_sum(lens4);
+    const unsigned tot = __shfl_sync(0xffffffffu, inc, 31);
+    const unsigned exc2 = (inc - lens4) << 1;            // bytes: at most 2 * 31 * 4
+    unsigned packs = at + kMin + kLen;
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+        sts_pack(packs + __byte_perm(exc2, 0, 0x4440 + j), w[j], len[j]);
+        packs += 2 * __byte_perm(tot, 0, 0x4440 + j);
+    }
+    return packs - at;
+}
+
+// The same from the codes, as pack_words takes them; min01, min23: the minima without an offset that the codes may carry
+template <int BITS, typename Codes>
+__device__ __forceinline__ unsigned k_pack_round(Codes codes, unsigned min01, unsigned min23, unsigned mn01, unsigned mx01, unsigned mn23, unsigned mx23, unsigned at,
+                                                 int lane) {
+    constexpr unsigned kMask = (1u << BITS) - 1u;
+    unsigned lenword = 0, lens4;
+    int len[4];
+    uint64_t w[4];
+    pack_words<BITS>(codes, mn01, mx01, mn23, mx23, len, lens4, w);
+#pragma unroll
+    for (int j = 0; j < 4; j++) lenword |= (unsigned)len[j] << (j * len_field_bits(BITS));
+    const unsigned minword = (min01 & kMask) | ((min01 >> 16 & kMask) << BITS) | ((min23 & kMask) << (2 * BITS)) | ((min23 >> 16 & kMask) << (3 * BITS));
+    return k_store_round<BITS>(at, lane, minword, lenword, lens4, len, w);
+}
+
 // The same round for blocks whose four quantisers are packable(): two channels per instruction
 // from the conversion to the pack minimum / maximum (16-bit lanes), then one multiply-add per code
 // into the pack words.
@@ -260,61 +406,23 @@ struct PackedQuantisers {
 };
 template <typename T, int BITS, bool HALF, typename Row>
 __device__ __forceinline__ unsigned k_encode_round_packed(Row row, const Quantiser<T, false>& q0, const Quantiser<T, false>& q1, const Quantiser<T, false>& q2,
-                                                          const Quantiser<T, false>& q3, const PackedQuantisers<T>& pq, uint8_t* at, int lane, unsigned& over) {
-    constexpr int LB = len_field_bits(BITS), kMin = 16 * BITS, kLen = 16 * LB;
-    unsigned c01[16], c23[16];
+                                                          const Quantiser<T, false>& q3, const PackedQuantisers<T>& pq, unsigned at, int lane, unsigned& over) {
+    unsigned c01[16], c23[16];                        // HALF: with their channels' bias, which pack_words takes off with the minimum
     unsigned mn01 = 0xFFFFFFFFu, mx01 = 0u, mn23 = 0xFFFFFFFFu, mx23 = 0u;
 #pragma unroll
     for (int t = 0; t < 16; t++) {
         const uint2 raw = row(t);
-        c01[t] = HALF ? pq.h01.codes(raw.x) : packed_codes<T>(raw.x, q0, q1, pq.k01);
-        c23[t] = HALF ? pq.h23.codes(raw.y) : packed_codes<T>(raw.y, q2, q3, pq.k23);
+        c01[t] = HALF ? pq.h01.raw(raw.x) : packed_codes<T>(raw.x, q0, q1, pq.k01);
+        c23[t] = HALF ? pq.h23.raw(raw.y) : packed_codes<T>(raw.y, q2, q3, pq.k23);
         mn01 = min_u16x2(mn01, c01[t]); mx01 = max_u16x2(mx01, c01[t]);
         mn23 = min_u16x2(mn23, c23[t]); mx23 = max_u16x2(mx23, c23[t]);
     }
-    over |= mx01 | mx23;
-    const unsigned mnj[4] = {mn01 & 0xFFFFu, mn01 >> 16, mn23 & 0xFFFFu, mn23 >> 16};
-    const unsigned d01 = mx01 - mn01, d23 = mx23 - mn23;     // lane-wise: no borrow, max >= min
-    const unsigned dj[4] = {d01 & 0xFFFFu, d01 >> 16, d23 & 0xFFFFu, d23 >> 16};
-    unsigned minword = 0, lenword = 0, lens4 = 0;
-    int len[4];
-#pragma unroll
-    for (int j = 0; j < 4; j++) {
-        len[j] = min(bit_length_u32(dj[j]), BITS);
-        minword |= (mnj[j] & ((1u << BITS) - 1u)) << (j * BITS);
-        lenword |= (unsigned)len[j] << (j * LB);
-        lens4 |= (unsigned)len[j] << (8 * j);
-    }
-    store_lane_fields_w<4 * BITS>(at, lane, minword);
-    store_lane_fields_w<4 * LB>(at + kMin, lane, lenword);
-    const unsigned inc = warp_inclusive_sum(lens4);
-    const unsigned tot = __shfl_sync(0xffffffffu, inc, 31);
-    const unsigned exc = inc - lens4;
-    uint8_t* packs = at + kMin + kLen;
-    unsigned before = 0;
-#pragma unroll
-    for (int j = 0; j < 4; j++) {
-        // 16-bit lanes, four tokens each (token 0 and 4, 8 and 12 highest): w = w * 2^len + code for two of them per
-        // multiply-add, then the minimum is taken off all four fields at once (min * (1 + 2^len + ... + 2^(3 len))).
-        // A lane stays below 2^16: four codes below 2^4 at steps of at most 2^4.  Against one multiply-add and one
-        // extraction per code: 1.6 instead of 2.8 instructions per code.
-        const unsigned step = 1u << len[j], sel = (j & 1) ? 0x7632u : 0x5410u;
-        const unsigned(&cj)[16] = j < 2 ? c01 : c23;
-        unsigned za = __byte_perm(cj[0], cj[4], sel), zb = __byte_perm(cj[8], cj[12], sel);
-#pragma unroll
-        for (int t = 1; t < 4; t++) {
-            za = za * step + __byte_perm(cj[t], cj[t + 4], sel);
-            zb = zb * step + __byte_perm(cj[t + 8], cj[t + 12], sel);
-        }
-        const unsigned low = mnj[j] * ((1u + step) * (1u + step * step)) * 0x00010001u;
-        za -= low;
-        zb -= low;
-        const unsigned wt = ((za & 0xFFFFu) << (4 * len[j])) | (za >> 16), wb = ((zb & 0xFFFFu) << (4 * len[j])) | (zb >> 16);
-        const uint64_t w = ((uint64_t)wt << (8 * len[j])) | wb;
-        store_pack_smem(packs + 2 * (before + ((exc >> (8 * j)) & 0xFFu)), w, len[j]);
-        before += (tot >> (8 * j)) & 0xFFu;
-    }
-    return kMin + kLen + 2 * before;
+    const unsigned k01 = HALF ? pq.k01 : 0u, k23 = HALF ? pq.k23 : 0u, min01 = mn01 - k01, min23 = mn23 - k23;
+    over |= min01 | min23 | (mx01 - k01) | (mx23 - k23);      // a code below zero leaves its lane too
+    const auto codes = [&](int j, int t) {
+        return j < 2 ? __byte_perm(c01[t + 4], c01[t], j & 1 ? 0x7632 : 0x5410) : __byte_perm(c23[t + 4], c23[t], j & 1 ? 0x7632 : 0x5410);
+    };
+    return k_pack_round<BITS>(codes, min01, min23, mn01, mx01, mn23, mx23, at, lane);
 }
 
 // rounds of one K block, appended to `stage` behind the table of round ends
@@ -324,6 +432,8 @@ template <typename T, int BITS, int MODE, bool ORDERED>
 __device__ __forceinline__ int k_encode_rounds(const T* x, int64_t ss, const uint8_t* ordp, const Quantiser<T, false>& q0, const Quantiser<T, false>& q1,
                                                const Quantiser<T, false>& q2, const Quantiser<T, false>& q3, const KGeom& g, uint8_t* stage, int lane, bool& bad) {
     const PackedQuantisers<T> pq(q0, q1, q2, q3);
+    const uint64_t row_bytes = 2 * (uint64_t)ss;
+    const unsigned stage_a = smem_addr(stage);
     int pos = g.head_bytes;
     unsigned over = 0;
     for (int r = 0; r < g.rounds; r++) {
@@ -331,11 +441,11 @@ __device__ __forceinline__ int k_encode_rounds(const T* x, int64_t ss, const uin
         if (ORDERED) ob = __ldg(reinterpret_cast<const uint4*>(ordp + 16 * r));
         const unsigned ow[4] = {ob.x, ob.y, ob.z, ob.w};
         const auto row = [&](int t) {
-            const int at = ORDERED ? (int)((ow[t >> 2] >> (8 * (t & 3))) & 0xFFu) : r * 16 + t;
-            return __ldg(reinterpret_cast<const uint2*>(x + (int64_t)at * ss));
+            const int at = ORDERED ? (int)__byte_perm(ow[t >> 2], 0, 0x4440 + (t & 3)) : r * 16 + t;
+            return __ldg(reinterpret_cast<const uint2*>(reinterpret_cast<const uint8_t*>(x) + (uint64_t)(unsigned)at * row_bytes));
         };
         pos += MODE == 0 ? k_encode_round<T, BITS>(row, q0, q1, q2, q3, stage + pos, lane, over)
-                         : k_encode_round_packed<T, BITS, MODE == 2>(row, q0, q1, q2, q3, pq, stage + pos, lane, over);
+                         : k_encode_round_packed<T, BITS, MODE == 2>(row, q0, q1, q2, q3, pq, stage_a + pos, lane, over);
         if (lane == 0) *reinterpret_cast<uint16_t*>(stage + 2 * r) = (uint16_t)(pos - g.head_bytes);
     }
     bad = bad || (MODE == 0 ? over : over & ~(((1u << BITS) - 1u) * 0x00010001u)) != 0;
@@ -427,11 +537,12 @@ __global__ void __launch_bounds__(NW * 32, 768 / (NW * 32)) k_fused_encode_kerne
 
 // ------------------------------------------------------------------------------------------ V
 // one CTA per (sequence, token block): pass 1 computes the per-token parameters over all heads
-// (one warp per token); pass 2 gives each warp whole V blocks (cb tokens x 64 channels): rows are
-// quantised as they are loaded (8 channels of one token per lane, so the token's parameters are
-// fetched once per 8 elements) into a uint8 tile in shared memory, from which the lane <-> channel
-// packing reads its columns.
-// Tile of one V block in shared memory, transposed for the packing stage: one row of CB bytes per
+// (one warp per token); pass 2 gives each warp whole V blocks (cb tokens x 64 channels), two packs of 16 tokens
+// at a time: a lane quantises four channels of the 16 tokens of one pack, two channels to an instruction, and
+// forms their pack words in registers as K's rounds do; the words then change lanes through shared memory, so that
+// a store covers the adjacent packs of 32 channels as the stream has them.
+//
+// (One-block launches go through a tile of codes instead.)  Tile of one V block in shared memory, transposed for the packing stage: one row of CB bytes per
 // channel, made of 16-byte chunks (one per pack); chunk p of channel ch is stored at chunk position
 // p ^ v_swz(ch) so that both the word stores of the quantising stage and the 16-byte row reads of the
 // packing stage spread over the banks.  Inside a chunk, byte 4*r0 + k holds token r0 + 4*k of the
@@ -500,31 +611,6 @@ struct TileLane {
     }
 };
 
-// Quantises one V block into the tile.  Lane (r0 = lane >> 3, cg = lane & 7) loads 8 channels
-// (16 bytes) of tokens r0, r0+4, r0+8, ...
-// Returns the OR of all codes in 16-bit lanes for the range check.
-template <typename T, int CB, int MODE>
-__device__ __forceinline__ unsigned v_quantise_tile(const T* src, int64_t ss, const float4* prm, const uint8_t* ord, uint8_t* tile, int lane) {
-    const int r0 = lane >> 3;
-    unsigned seen = 0;
-    const TileLane<CB> out(tile, lane);
-    const T* lsrc = src + 8 * (lane & 7);
-#pragma unroll 1
-    for (int p = 0; p < CB / 16; p++) {
-        unsigned c[4][4];
-#pragma unroll
-        for (int k = 0; k < 4; k++) {
-            const int tok = 16 * p + 4 * k + r0;
-            const uint4 raw = __ldg(reinterpret_cast<const uint4*>(lsrc + (int64_t)ord[tok] * ss));
-            v_quantise_row<T, CB, MODE>(raw, prm, tok, c[k]);
-#pragma unroll
-            for (int i = 0; i < 4; i++) seen |= c[k][i];
-        }
-        out.store(p, c);
-    }
-    return seen;
-}
-
 // One 16-byte tile chunk (word r0: bytes k = codes of tokens r0 + 4k of the pack) -> the pack's
 // minimum, bit length and 2*len-byte word (token 0 in the top bits).
 template <int BITS>
@@ -540,18 +626,18 @@ __device__ __forceinline__ void chunk_to_pack(const uint4& cw, int& len, uint64_
     mn1 = min(mn & 0xFFFFu, mn >> 16);
     const unsigned mx1 = max(mx & 0xFFFFu, mx >> 16);
     len = min(bit_length_u32(mx1 - mn1), BITS);
-    const unsigned step = 1u << len, rep = mn1 * 0x01010101u;
-    // 16-bit slots: slot k collects tokens 4k..4k+3 (r0 = 0 highest) by Horner steps over the words
-    unsigned zlo = 0, zhi = 0;
+    unsigned step = 1u << len;
+    asm("" : "+r"(step));                                 // see pack_words
+    const unsigned rep = mn1 * 0x01010101u, step2 = step * step;
+    // 16-bit lanes: tokens 0..3 above 4..7, 8..11 above 12..15, by Horner steps over the words (r0 = 0 highest)
+    unsigned za = 0, zb = 0;
 #pragma unroll
     for (int i = 0; i < 4; i++) {
         const unsigned v = wv[i] - rep;
-        zlo = zlo * step + __byte_perm(v, 0, 0x4140);
-        zhi = zhi * step + __byte_perm(v, 0, 0x4342);
+        za = za * step + __byte_perm(v, 0, 0x4041);
+        zb = zb * step + __byte_perm(v, 0, 0x4243);
     }
-    const unsigned wt = ((zlo & 0xFFFFu) << (4 * len)) | (zlo >> 16);     // tokens 0..7
-    const unsigned wb = ((zhi & 0xFFFFu) << (4 * len)) | (zhi >> 16);     // tokens 8..15
-    wd = ((uint64_t)wt << (8 * len)) | wb;
+    wd = join_lanes(za, zb, len, step2 * step2);
 }
 
 // One segment of a V block (PPT packs of 16 tokens for each of 32 channels) from the tile: this lane's channel row and swizzle.
@@ -580,12 +666,12 @@ __device__ __forceinline__ unsigned v_pack_segment(const uint8_t* row, int swz, 
     const unsigned inc = warp_inclusive_sum(lens4);
     const unsigned tot = __shfl_sync(0xffffffffu, inc, 31);
     const unsigned exc = inc - lens4;
-    uint8_t* packs = at + kMin + kLen;
+    const unsigned packs = smem_addr(at) + kMin + kLen;
     unsigned before = 0;
 #pragma unroll
     for (int q = 0; q < 4; q++)
         if (q < PPT) {
-            store_pack_smem(packs + 2 * (before + ((exc >> (8 * q)) & 0xFFu)), wd[q], len[q]);
+            sts_pack(packs + 2 * (before + ((exc >> (8 * q)) & 0xFFu)), wd[q], len[q]);
             before += (tot >> (8 * q)) & 0xFFu;
         }
     return kMin + kLen + 2 * before;
@@ -594,7 +680,7 @@ __device__ __forceinline__ unsigned v_pack_segment(const uint8_t* row, int swz, 
 // One round (16 tokens x 128 channels) of a K block with per-token parameters from the two tiles of 64 channels
 template <int CB, int BITS>
 __device__ __forceinline__ unsigned kt_pack_round(const uint8_t* ctile, int r, uint8_t* at, int lane) {
-    constexpr int LB = len_field_bits(BITS), kMin = 16 * BITS, kLen = 16 * LB;
+    constexpr int LB = len_field_bits(BITS);
     unsigned minword = 0, lenword = 0, lens4 = 0;
     uint64_t wd[4];
     int len[4];
@@ -609,19 +695,7 @@ __device__ __forceinline__ unsigned kt_pack_round(const uint8_t* ctile, int r, u
         lenword |= (unsigned)len[j] << (j * LB);
         lens4 |= (unsigned)len[j] << (8 * j);
     }
-    store_lane_fields_w<4 * BITS>(at, lane, minword);
-    store_lane_fields_w<4 * LB>(at + kMin, lane, lenword);
-    const unsigned inc = warp_inclusive_sum(lens4);
-    const unsigned tot = __shfl_sync(0xffffffffu, inc, 31);
-    const unsigned exc = inc - lens4;
-    uint8_t* packs = at + kMin + kLen;
-    unsigned before = 0;
-#pragma unroll
-    for (int j = 0; j < 4; j++) {
-        store_pack_smem(packs + 2 * (before + ((exc >> (8 * j)) & 0xFFu)), wd[j], len[j]);
-        before += (tot >> (8 * j)) & 0xFFu;
-    }
-    return kMin + kLen + 2 * before;
+    return k_store_round<BITS>(smem_addr(at), lane, minword, lenword, lens4, len, wd);
 }
 
 // What token_params_pass and the one-block kernel keep per token of one block
@@ -634,42 +708,223 @@ __device__ __forceinline__ void put_token_params(const Quantiser<T, false>& qz, 
 }
 
 // Per-token quantisation parameters of one token block over all heads and channels (the
-// reference's token mode reduces over dims [1, 4], utils/compute.py:405-410): half a warp per token.
-// Writes (scale, zero, 1/scale, packed code bias or 0) to prm[] and scale / zero to the caller's arrays.
-// ord[t] = source row (inside the block) of stored row t; WRITE = false keeps the parameters in shared memory only.
+// reference's token mode reduces over dims [1, 4], utils/compute.py:405-410): half a warp per token takes its minimum and
+// maximum, then thread t forms token t's parameters.  Writes (scale, zero, 1/scale, packed code bias or 0) to prm[] and, with WRITE, scale /
+// zero to the caller's arrays; ord[t] = source row (inside the block) of stored row t.  One CTA barrier inside; the caller's next one must come
+// before prm[] is read.  (Parameters formed by the half warp, every lane alike: 400 of a warp's 4700 instructions per block of 64 tokens x 8 heads.)
+struct TokenState { bool bad, packed, half; };           // of this thread's token: degenerate; parameters that the two faster conversions take
 template <typename T, int CB, bool WRITE = true, int NW = 8>
-__device__ __forceinline__ bool token_params_pass(const FusedArgs& a, const T* xb, float4* prm, const uint8_t* ord, int b, int cbi, int lane, int wic) {
-    bool bad = false;
+__device__ __forceinline__ TokenState token_params_pass(const FusedArgs& a, const T* xb, float4* prm, const uint8_t* ord, int b, int cbi, int lane, int wic) {
+    using T2 = typename QT<T>::T2;
+    static_assert(NW * 32 >= CB, "a thread to a token");
+    const auto min_of = [](unsigned x, unsigned y) {
+        const T2 m = QT<T>::min2(*reinterpret_cast<const T2*>(&x), *reinterpret_cast<const T2*>(&y));
+        return *reinterpret_cast<const unsigned*>(&m);
+    };
     for (int t = 2 * wic + (lane >> 4); t < CB; t += 2 * NW) {     // 8 channels per lane
-        const T* xt = xb + (int64_t)ord[t] * a.ss + 8 * (lane & 15);
-        using T2 = typename QT<T>::T2;
+        const uint8_t* xt = reinterpret_cast<const uint8_t*>(xb + 8 * (lane & 15)) + (uint64_t)ord[t] * (2 * (uint64_t)a.ss);
         T2 lo2 = QT<T>::init2(INFINITY), hi2 = QT<T>::init2(-INFINITY);
-#pragma unroll 4
-        for (int h = 0; h < a.heads; h++) {
-            const uint4 raw = __ldg(reinterpret_cast<const uint4*>(xt + (int64_t)h * a.sh));
-            const T2 v0 = *reinterpret_cast<const T2*>(&raw.x), v1 = *reinterpret_cast<const T2*>(&raw.y);
-            const T2 v2 = *reinterpret_cast<const T2*>(&raw.z), v3 = *reinterpret_cast<const T2*>(&raw.w);
-            lo2 = QT<T>::min2(lo2, QT<T>::min2(QT<T>::min2(v0, v1), QT<T>::min2(v2, v3)));
-            hi2 = QT<T>::max2(hi2, QT<T>::max2(QT<T>::max2(v0, v1), QT<T>::max2(v2, v3)));
-        }
-        float lo = fminf(QT<T>::lo_f(lo2), QT<T>::hi_f(lo2)), hi = fmaxf(QT<T>::lo_f(hi2), QT<T>::hi_f(hi2));
+        for (int h0 = 0; h0 < a.heads; h0 += 8) {          // eight heads' loads in flight together
+            uint4 raw[8];
 #pragma unroll
-        for (int s = 8; s > 0; s >>= 1) {
-            lo = fminf(lo, __shfl_xor_sync(0xffffffffu, lo, s));
-            hi = fmaxf(hi, __shfl_xor_sync(0xffffffffu, hi, s));
-        }
-        const Quantiser<T, false> qz(lo, hi, a.rel);
-        bad = bad || qz.degenerate();
-        if ((lane & 15) == 0) {
-            put_token_params<T, CB>(qz, prm, t);
-            if (WRITE) {
-                const int64_t pi = (int64_t)b * a.param_tokens + a.first_token + cbi * CB + t;
-                reinterpret_cast<T*>(a.scale)[pi] = QT<T>::cvt(qz.scale);
-                reinterpret_cast<T*>(a.zero)[pi] = QT<T>::cvt(qz.zero);
+            for (int i = 0; i < 8; i++) {
+                if (i == 0 || h0 + i < a.heads) raw[i] = __ldg(reinterpret_cast<const uint4*>(xt + (uint64_t)(unsigned)(h0 + i) * (2 * (uint64_t)a.sh)));
+                else raw[i] = raw[0];
+            }
+#pragma unroll
+            for (int i = 0; i < 8; i++) {
+                const T2 v0 = *reinterpret_cast<const T2*>(&raw[i].x), v1 = *reinterpret_cast<const T2*>(&raw[i].y);
+                const T2 v2 = *reinterpret_cast<const T2*>(&raw[i].z), v3 = *reinterpret_cast<const T2*>(&raw[i].w);
+                lo2 = QT<T>::min2(lo2, QT<T>::min2(QT<T>::min2(v0, v1), QT<T>::min2(v2, v3)));
+                hi2 = QT<T>::max2(hi2, QT<T>::max2(QT<T>::max2(v0, v1), QT<T>::max2(v2, v3)));
             }
         }
+        // (minimum, -maximum) of the lane, then of the token: one minimum serves both
+        const unsigned l = *reinterpret_cast<const unsigned*>(&lo2), u = *reinterpret_cast<const unsigned*>(&hi2) ^ 0x80008000u;
+        unsigned m = min_of(__byte_perm(l, u, 0x5410), __byte_perm(l, u, 0x7632));
+#pragma unroll
+        for (int s = 8; s > 0; s >>= 1) m = min_of(m, __shfl_xor_sync(0xffffffffu, m, s));
+        if ((lane & 15) == 0) prm[t].x = __uint_as_float(m);
     }
-    return bad;
+    __syncthreads();
+    const int t = threadIdx.x;
+    if (t >= CB) return TokenState{false, true, true};
+    const unsigned m = __float_as_uint(prm[t].x);
+    const T2 both = *reinterpret_cast<const T2*>(&m);
+    const Quantiser<T, false> qz(QT<T>::lo_f(both), -QT<T>::hi_f(both), a.rel);
+    put_token_params<T, CB>(qz, prm, t);
+    if (WRITE) {
+        const int64_t pi = (int64_t)b * a.param_tokens + a.first_token + cbi * CB + t;
+        reinterpret_cast<T*>(a.scale)[pi] = QT<T>::cvt(qz.scale);
+        reinterpret_cast<T*>(a.zero)[pi] = QT<T>::cvt(qz.zero);
+    }
+    // (half_domain() implies packable(); a bias of 0 marks parameters that are not)
+    return TokenState{qz.degenerate(), __float_as_uint(prm[t].w) != 0u, reinterpret_cast<const uint4*>(prm + CB)[t].w != 0u};
+}
+
+// Codes of a lane's four channels (at src) of the 16 tokens from tok0 on, with the tokens' parameters prm[], and their minima and maxima
+// in 16-bit lanes.  ord: source row of every stored row (16-byte aligned).  The codes are kept as bytes, a word for two channels of
+// tokens t and t + 4 (16 registers; with 16-bit lanes, 32 of them, the V kernel spills).
+struct PackCodes {
+    unsigned c01[8], c23[8], mn01, mx01, mn23, mx23;               // word 4 (t / 8) + t % 4: (t, t + 4) of the even channel, then of the odd one
+    unsigned largest;                                              // OR of the maxima, before a code that is no byte (an error) lost its upper bits
+    __device__ __forceinline__ unsigned operator()(int j, int t) const {
+        const int at = 4 * (t >> 3) + (t & 3);
+        return j < 2 ? __byte_perm(c01[at], 0, j & 1 ? 0x4243 : 0x4041) : __byte_perm(c23[at], 0, j & 1 ? 0x4243 : 0x4041);
+    }
+};
+template <typename T, int CB, int MODE>     // MODE 0: scalar conversion, 1: two elements per instruction in fp32, 2: in the element type
+__device__ __forceinline__ void quantise_pack(const uint8_t* src, uint64_t row_bytes, const float4* prm, const uint8_t* ord, int tok0, PackCodes& p) {
+    const uint4* prmh = reinterpret_cast<const uint4*>(prm + CB);   // per token: r, -128*scale, r/128 (element-type pairs), code bias
+    const uint4 ob = *reinterpret_cast<const uint4*>(ord + tok0);
+    const unsigned ow[4] = {ob.x, ob.y, ob.z, ob.w};
+    p.mn01 = 0xFFFFFFFFu; p.mx01 = 0u; p.mn23 = 0xFFFFFFFFu; p.mx23 = 0u;
+    uint2 raw[16];
+#pragma unroll
+    for (int t = 0; t < 16; t++) raw[t] = __ldg(reinterpret_cast<const uint2*>(src + (uint64_t)__byte_perm(ow[t >> 2], 0, 0x4440 + (t & 3)) * row_bytes));
+#pragma unroll
+    for (int at = 0; at < 8; at++) {
+        unsigned c[2][2];
+#pragma unroll
+        for (int e = 0; e < 2; e++) {
+            const int t = 8 * (at >> 2) + (at & 3) + 4 * e;
+            if (MODE == 2) {
+                const uint4 ph = prmh[tok0 + t];
+                HalfQuotient<T> hq;
+                hq.r = *reinterpret_cast<const typename QT<T>::T2*>(&ph.x);
+                hq.nsp = *reinterpret_cast<const typename QT<T>::T2*>(&ph.y);
+                hq.rp = *reinterpret_cast<const typename QT<T>::T2*>(&ph.z);
+                hq.kab = ph.w;
+                hq.magic = QT<T>::dup((float)(QT<T>::kIntBits == 0x6600u ? 1536 : 192));
+                hq.pre = QT<T>::dup(QT<T>::kPre);
+                c[e][0] = hq.codes(raw[t].x);
+                c[e][1] = hq.codes(raw[t].y);
+            } else {
+                const float4 pr = prm[tok0 + t];                    // scale, zero, 1/scale, packed code bias
+                Quantiser<T, false> qz;
+                qz.scale = pr.x; qz.zero = pr.y; qz.rcp = pr.z;
+                if (MODE == 1) {
+                    c[e][0] = packed_codes<T>(raw[t].x, qz, qz, __float_as_uint(pr.w));
+                    c[e][1] = packed_codes<T>(raw[t].y, qz, qz, __float_as_uint(pr.w));
+                } else {
+                    const int zi = (int)pr.y;
+                    const float2 f01 = QT<T>::to_float2(raw[t].x), f23 = QT<T>::to_float2(raw[t].y);
+                    c[e][0] = qz.template code_u8<false>(f01.x, zi) | (qz.template code_u8<false>(f01.y, zi) << 16);
+                    c[e][1] = qz.template code_u8<false>(f23.x, zi) | (qz.template code_u8<false>(f23.y, zi) << 16);
+                }
+            }
+            p.mn01 = min_u16x2(p.mn01, c[e][0]); p.mx01 = max_u16x2(p.mx01, c[e][0]);
+            p.mn23 = min_u16x2(p.mn23, c[e][1]); p.mx23 = max_u16x2(p.mx23, c[e][1]);
+        }
+        p.c01[at] = __byte_perm(c[0][0], c[1][0], 0x6240);
+        p.c23[at] = __byte_perm(c[0][1], c[1][1], 0x6240);
+    }
+    p.largest = p.mx01 | p.mx23;
+    if (p.largest & 0xFF00FF00u) {                                 // reported by the caller; the bytes are those of every form of the encoder
+        p.mn01 = 0xFFFFFFFFu; p.mx01 = 0u; p.mn23 = 0xFFFFFFFFu; p.mx23 = 0u;
+#pragma unroll
+        for (int at = 0; at < 8; at++) {
+            const unsigned e01 = __byte_perm(p.c01[at], 0, 0x4240), o01 = __byte_perm(p.c01[at], 0, 0x4341);
+            const unsigned e23 = __byte_perm(p.c23[at], 0, 0x4240), o23 = __byte_perm(p.c23[at], 0, 0x4341);
+            p.mn01 = min_u16x2(p.mn01, min_u16x2(e01, o01)); p.mx01 = max_u16x2(p.mx01, max_u16x2(e01, o01));
+            p.mn23 = min_u16x2(p.mn23, min_u16x2(e23, o23)); p.mx23 = max_u16x2(p.mx23, max_u16x2(e23, o23));
+        }
+    }
+}
+
+// Four fields of W bits (the 16-bit lanes of f01, f23) as W / 2 bytes at `at` (even; 4-byte aligned for W = 8 and 16): the fields of
+// four adjacent channels in a segment's header.
+template <int W>
+__device__ __forceinline__ void put_fields(uint8_t* at, unsigned f01, unsigned f23) {
+    static_assert(W == 4 || W == 6 || W == 8 || W == 12 || W == 16, "header fields of one channel");
+    const unsigned lo = W == 16 ? f01 : (f01 & 0xFFFFu) | (f01 >> 16 << W), hi = W == 16 ? f23 : (f23 & 0xFFFFu) | (f23 >> 16 << W);
+    if (W == 16) {
+        reinterpret_cast<unsigned*>(at)[0] = lo; reinterpret_cast<unsigned*>(at)[1] = hi;
+    } else if (W == 12) {
+        uint16_t* h = reinterpret_cast<uint16_t*>(at);
+        h[0] = (uint16_t)lo; h[1] = (uint16_t)((lo >> 16) | (hi << 8)); h[2] = (uint16_t)(hi >> 8);
+    } else if (W == 8) {
+        *reinterpret_cast<unsigned*>(at) = lo | (hi << 16);
+    } else if (W == 6) {
+        const unsigned v = lo | (hi << 12);
+        at[0] = (uint8_t)v; at[1] = (uint8_t)(v >> 8); at[2] = (uint8_t)(v >> 16);
+    } else {
+        *reinterpret_cast<uint16_t*>(at) = (uint16_t)(lo | (hi << 8));
+    }
+}
+
+template <int CB, int BITS> struct VSegment {
+    static constexpr int kPacks = CB == 32 ? 2 : 4, kGroups = CB == 128 ? 2 : 1, kCount = 2 * kGroups;   // packs per channel; 64-token groups; segments
+    static constexpr int kMin = BITS * kPacks * 4, kLen = len_field_bits(BITS) * kPacks * 4, kBound = (kMin + kLen + 64 * kPacks * BITS + 15) & ~15;
+};
+
+// One V block (CB tokens x 64 channels at src) into its segments: segment i at stage + i * kBound, its bytes in sizes[i].
+// Lane (par = lane >> 4, cg = lane & 15) takes channels 4cg .. 4cg + 3 of every other pack.  xch: 1280 bytes of the warp's, 16-byte aligned, in
+// which the words change lanes.  Against codes transposed through a tile of bytes (two header fields, a row of codes and a scan for every
+// segment) a round takes 670 instructions for 64 elements of a lane.  Returns the OR of the packs' largest codes in 16-bit lanes.
+template <typename T, int CB, int BITS, int MODE>
+__device__ __forceinline__ unsigned v_block_segments(const T* src, uint64_t row_bytes, const float4* prm, const uint8_t* ord, uint8_t* stage, uint8_t* xch, unsigned* sizes,
+                                                     int lane) {
+    using S = VSegment<CB, BITS>;
+    constexpr int LB = len_field_bits(BITS);
+    const int par = lane >> 4, cg = lane & 15, w = cg >> 3;
+    const uint8_t* lsrc = reinterpret_cast<const uint8_t*>(src + 4 * cg);
+    const unsigned stage_a = smem_addr(stage);
+    uint2* words = reinterpret_cast<uint2*>(xch);                 // [128] pack words: pack 4 * lane + j (parity, channel) at a swizzled place
+    uint16_t* places = reinterpret_cast<uint16_t*>(xch + 1024);   // [128] halfword offset in its segment's packs | length << 12
+    unsigned over = 0;
+#pragma unroll 1
+    for (int r = 0; r < S::kGroups; r++) {
+        unsigned cum = 0, min01 = 0, min23 = 0, len01 = 0, len23 = 0;   // packs of this lane's segment so far (halfwords); its channels' header fields
+#pragma unroll 1
+        for (int rr = 0; rr < S::kPacks / 2; rr++) {
+            PackCodes p;
+            unsigned lens4;
+            int len[4];
+            uint64_t wd[4];
+            const int q = 2 * rr + par;
+            quantise_pack<T, CB, MODE>(lsrc, row_bytes, prm, ord, 64 * r + 16 * q, p);
+            over |= p.largest;
+            pack_words<BITS>(p, p.mn01, p.mx01, p.mn23, p.mx23, len, lens4, wd);
+            constexpr unsigned kMask = ((1u << BITS) - 1u) * 0x00010001u;
+            const unsigned l01 = (unsigned)len[0] | ((unsigned)len[1] << 16), l23 = (unsigned)len[2] | ((unsigned)len[3] << 16);
+            min01 |= (p.mn01 & kMask) << (q * BITS); min23 |= (p.mn23 & kMask) << (q * BITS);
+            len01 |= l01 << (q * LB); len23 |= l23 << (q * LB);
+            // packs of the segment and q before this lane's: the other eight lanes', and all of q - 1's for the odd q
+            const unsigned sum = (lens4 * 0x01010101u) >> 24;
+            unsigned inc = sum;
+#pragma unroll
+            for (int d = 1; d < 8; d <<= 1) {
+                const unsigned n = __shfl_up_sync(0xffffffffu, inc, d, 8);
+                if ((lane & 7) >= d) inc += n;
+            }
+            const unsigned tot = __shfl_sync(0xffffffffu, inc, lane | 7), other = __shfl_xor_sync(0xffffffffu, tot, 16);
+            const unsigned at0 = cum + (par ? other : 0u) + inc - sum;
+            const unsigned p01 = at0 * 0x00010001u + ((unsigned)len[0] << 16) + (l01 << 12);
+            const unsigned p23 = (at0 + len[0] + len[1]) * 0x00010001u + ((unsigned)len[2] << 16) + (l23 << 12);
+            cum += tot + other;
+            __syncwarp();                                          // the round before has read its words
+#pragma unroll
+            for (int j = 0; j < 4; j++) words[4 * lane + ((j + (lane >> 2)) & 3)] = make_uint2((unsigned)wd[j], (unsigned)(wd[j] >> 32));
+            reinterpret_cast<uint2*>(places)[lane] = make_uint2(p01, p23);
+            __syncwarp();
+#pragma unroll
+            for (int i = 0; i < 4; i++) {                          // the 32 channels of segment i & 1, pack 2 rr + (i >> 1)
+                const unsigned place = places[32 * i + lane];
+                const uint2 v = words[32 * i + (lane & ~3) + (((lane & 3) + 2 * i + (lane >> 4)) & 3)];
+                sts_pack(stage_a + ((i & 1) * S::kGroups + r) * S::kBound + S::kMin + S::kLen + 2 * (place & 0xFFFu), (uint64_t)v.y << 32 | v.x, (int)(place >> 12));
+            }
+        }
+        // the even packs' fields and the odd ones' belong together; half of the lanes store minima, half lengths
+        const unsigned m01 = min01 | __shfl_xor_sync(0xffffffffu, min01, 16), m23 = min23 | __shfl_xor_sync(0xffffffffu, min23, 16);
+        const unsigned n01 = len01 | __shfl_xor_sync(0xffffffffu, len01, 16), n23 = len23 | __shfl_xor_sync(0xffffffffu, len23, 16);
+        uint8_t* seg = stage + (w * S::kGroups + r) * S::kBound;
+        if (par == 0) put_fields<S::kPacks * BITS>(seg + (cg & 7) * (S::kPacks * BITS / 2), m01, m23);
+        else put_fields<S::kPacks * LB>(seg + S::kMin + (cg & 7) * (S::kPacks * LB / 2), n01, n23);
+        if ((lane & 23) == 0) sizes[w * S::kGroups + r] = S::kMin + S::kLen + 2 * cum;
+    }
+    __syncwarp();
+    return over;
 }
 
 // Source row (inside a block of CB tokens) of every stored row: the identity, or the caller's reorder of every
@@ -687,116 +942,91 @@ __device__ __forceinline__ void load_row_order(const FusedArgs& a, uint8_t* ord,
     __syncthreads();
 }
 
-// Form of a V launch: the warps of a CTA and how many CTAs an SM's registers hold.  Up to one CTA to an SM, 16 warps.  Beyond, a launch ends with
-// the CTAs of its last, partly filled wave, and the form is taken whose waves fit the number of CTAs: 8 warps, three to an SM (waves of 444), or
-// 16, two to an SM (waves of 296).  us with 8 and with 16 warps:
-//   8 heads, 4 bits, 64 tokens: 148 CTAs 26.0 22.1, 296 32.3 30.5, 298 35.5 38.1, 444 39.9 48.8, 500 56.6 47.0, 740 68.5 67.1, 888 72.5 73.9,
-//     1036 92.4 86.8, 1332 102 107, 1500 122 116, 2048 154 154, 4096 275 288; 5 heads: 296 28.2 25.2, 444 32.4 38.1, 592 47.2 38.8, 1500 95.1 90.8
-//   8 heads, 4 bits, 32 tokens: 296 24.5 22.1, 360 26.7 30.4, 592 39.9 34.6, 900 47.4 48.5, 1332 65.2 69.3, 2048 99.2 99.1
-//   16 heads, 4 bits, 64 tokens: 296 58.5 55.4, 298 67.1 70.7, 592 108 104, 888 151 151, 2048 322 332; 32 heads: 148 73.7 58.0, 660 236 246, 1500
-//     486 523; 16 heads, 2 bits: 298 57.8 57.9, 888 128 117, 2048 274 251; 12 heads: 360 47.7 48.5, 444 53.9 52.4, 1500 158 154
-// 128-token blocks leave room for one CTA of 16 warps only, which pays up to one to an SM.  Up to four heads make no more than 8 blocks a CTA.
+// Form of a V launch: the warps of a CTA and how many CTAs an SM's registers hold.  Up to one CTA to an SM: 16 warps with all registers, so that
+// a warp has few blocks.  Beyond, 8 warps: three to an SM (waves of 444 CTAs), or four with 64 registers (waves of 592), which are slower where both
+// make the same number of waves, unless a CTA has little work.  us with 8 x 3, 8 x 4 and 16 x 1 (16 warps, two to an SM, was at most 3 % ahead of the
+// best of them between 149 and 296 CTAs and is not built):
+//   8 heads x 64 tokens: 148 CTAs 24.8 28.1 21.1, 296 30.8 34.0 35.9, 444 37.5 40.0 50.8, 500 53.3 42.6 51.6, 592 58.2 46.4 60.9, 740 62.0 76.4 71.5,
+//     1184 89.4 92.0 109, 2048 141 159 185
+//   4 x 64: 148 19.9 20.4 17.9, 444 27.9 29.6 40.7, 592 38.3 27.8 47.4, 888 42.8 47.6 65.6, 1184 58.9 52.7 86.4, 2048 95.4 90.5 146
+//   8 x 32: 444 25.8 25.8 36.8, 592 33.6 25.5 41.8, 888 41.0 42.9 57.0, 1500 66.7 62.4 94.6; 1 x 64: 592 26.9 19.9 36.0, 2048 65.6 59.7 109;
+//   2 x 128: 592 51.4 36.5 62.9, 740 54.8 61.4 75.0, 2048 132 125 201
+// Of more than 8 heads x 64 tokens, blocks of 128 tokens leave room for two CTAs of 8 warps only (8 x 128: 370 CTAs 89.5 and 71.1 with 16, 740 140 and
+// 118, 2048 327 and 305; 16 x 128: 592 241 and 198); smaller ones go through the scratch, a few waves of 16 warps (16 x 64: 100 CTAs 35.8 and 27.8,
+// 592 113 and 111, 740 130 and 137; 32 x 64: 444 153 and 158, 592 220 and 209, 740 251 and 258).
 struct VForm { int warps, per_sm; };
-static VForm v_form(int64_t ctas, int heads, int bits, int cb) {
-    const VForm narrow{8, 3}, wide{16, 2};
-    if (2 * heads <= 8) return narrow;
-    // (with all registers, for one CTA to an SM, 64-token blocks take 19.6 us instead of 20.3 at 5 heads, 56.6 instead of 58.0 at 32 and the same at 8;
-    // 32-token blocks gain nothing by it: 18.1 and 17.6 at 8 heads)
-    if (ctas <= kSmCount) return cb == 32 ? wide : VForm{16, 1};
-    if (cb == 128) return narrow;
-    const int64_t two = 2 * kSmCount, three = 3 * kSmCount;
-    if (heads <= 8)                                           // 16 where the last wave of 444 is up to two of their CTAs to an SM; of many waves, or of
-        return ctas <= (cb == 32 ? 5 : 12) * kSmCount && (ctas - 1) % three < two ? wide : narrow;     // little work each, 8 do as well or better
-    // above 8 heads the blocks go through the scratch and a warp packs several: 8 warps where 16 would add a wave of their own, and, for the largest
-    // blocks, in launches of many waves
-    const bool added = ctas > two && ctas <= three;
-    if (bits == 4 && cb == 64) return !added && ctas <= 4 * kSmCount ? wide : narrow;
-    return added && heads < 16 ? narrow : wide;
+static VForm v_form(int64_t ctas, int heads, int cb) {
+    const VForm narrow{8, 3}, dense{8, 4}, wide{16, 1};
+    if (ctas <= kSmCount) return wide;
+    if (heads * cb > 512) return cb == 128 || ctas <= 4 * kSmCount ? wide : narrow;
+    const bool one_wave = ctas > 3 * kSmCount && ctas <= 4 * kSmCount, light = heads * cb <= 256;
+    return one_wave || (light && ctas > 6 * kSmCount) ? dense : narrow;
 }
 
 // finished blocks that a warp of the V kernel holds in the direct form until their offsets are known
 __host__ __device__ constexpr int v_slots(int heads, int nw) { return (2 * heads + nw - 1) / nw; }
 
-// NW warps: 8, three CTAs to an SM, or 16, one to an SM or two at 64 registers: every warp then packs one block of an 8-head token block
-// instead of two, and a CTA takes little more than half the time (see v_form)
+constexpr int kVExchange = 1280;   // bytes of a warp's exchange area (see v_block_segments)
+
+// NW warps, PER_SM CTAs to an SM: see v_form.  Bound by instructions and the latency of its loads (134 M elements, 8 heads x 64 tokens, 4 bits: 130 us,
+// 17 instructions per element at 47 % of the issue slots; 145 us when codes went through a transposed tile).  What each form of the stages costs,
+// per 16 tokens x 4 channels of a lane: quantiser about 300 instructions, pack words 150, exchange, offsets and stores 200.
 template <typename T, int BITS, int CB, int NW, int PER_SM>
 __global__ void __launch_bounds__(NW * 32, PER_SM) v_fused_encode_kernel(FusedArgs a) {
     extern __shared__ __align__(16) uint8_t smem[];
     const int lane = lane_id(), wic = threadIdx.x >> 5;
     const int nctx = a.tokens / CB;
-    __shared__ unsigned sh_word, sh_sizes[16];
+    __shared__ unsigned sh_word, sh_sizes[64];   // bytes of the segments: of all blocks, in the slots form of a warp's own
     const bool direct = a.status != nullptr;                 // then a warp keeps both of its blocks until the offsets are known
     int cbi = blockIdx.x, b = blockIdx.y;
     if (direct) chain_place(a, &sh_word, b, cbi);
-    constexpr int PPT = CB == 32 ? 2 : 4, RPW = CB == 128 ? 2 : 1;
-    const VGeom g(CB, BITS);
-    const int bound16 = (g.head_bytes + g.nseg * (g.min_bytes + g.len_bytes + 32 * PPT * 2 * BITS) + 15) & ~15;
-    const int wstride = CB * 64 + (direct ? v_slots(a.heads, NW) : 1) * bound16;
+    using S = VSegment<CB, BITS>;
+    constexpr int kBlock = S::kCount * S::kBound;            // a finished block's segments
+    const int wstride = kVExchange + (direct ? v_slots(a.heads, NW) : 1) * kBlock;
     float4* prm = reinterpret_cast<float4*>(smem);           // [cb] (scale, zero, 1/scale, fast)
     uint8_t* wbase = smem + 32 * CB + wic * wstride;
-    uint8_t* ctile = wbase;                                  // [cb][64] codes
     const T* xb = reinterpret_cast<const T*>(a.x) + (int64_t)b * a.sb + (int64_t)cbi * CB * a.ss;
     uint8_t* ord = smem + 32 * CB + NW * wstride;
     load_row_order<CB, NW>(a, ord, b, cbi);
 
     // pass 1: per-token statistics across every head and channel
-    bool bad = token_params_pass<T, CB, true, NW>(a, xb, prm, ord, b, cbi, lane, wic);
-    // one decision for the whole CTA: the packed conversion needs every token's parameters in range
-    __syncthreads();
-    bool mine_ok = true, mine_half = true;
-    for (int t = threadIdx.x; t < CB; t += 32 * NW) {
-        mine_ok = mine_ok && __float_as_uint(prm[t].w) != 0u;
-        mine_half = mine_half && reinterpret_cast<const uint4*>(prm + CB)[t].w != 0u;
-    }
-    const bool all_packed = __syncthreads_and(mine_ok);
-    const bool all_half = __syncthreads_and(mine_half);
+    const TokenState mine = token_params_pass<T, CB, true, NW>(a, xb, prm, ord, b, cbi, lane, wic);
+    // one decision for the whole CTA: the faster conversions need every token's parameters in range
+    const bool all_packed = __syncthreads_and(mine.packed);
+    const bool all_half = __syncthreads_and(mine.half);
 
     // pass 2: quantise + pack, one warp per V block
     unsigned seen = 0;
     const int nvb = 2 * a.heads;
     for (int vb = wic; vb < nvb; vb += NW) {
-        const int h = vb >> 1, half = vb & 1;
-        const T* src = xb + (int64_t)h * a.sh + 64 * half;
-        uint8_t* stage = wbase + CB * 64 + (direct ? (vb / NW) * bound16 : 0);
+        const T* src = xb + (int64_t)(vb >> 1) * a.sh + 64 * (vb & 1);
+        uint8_t* stage = wbase + kVExchange + (direct ? (vb / NW) * kBlock : 0);
+        unsigned* sizes = sh_sizes + (direct ? vb : wic) * S::kCount;
         __syncwarp();
-        seen |= all_half ? v_quantise_tile<T, CB, 2>(src, a.ss, prm, ord, ctile, lane)
-                         : all_packed ? v_quantise_tile<T, CB, 1>(src, a.ss, prm, ord, ctile, lane) : v_quantise_tile<T, CB, 0>(src, a.ss, prm, ord, ctile, lane);
-        __syncwarp();
-        int pos = g.head_bytes;
-        unsigned seg_end = 0;
-        for (int w = 0; w < 2; w++) {
-            const int ch = 32 * w + lane;
-            const uint8_t* row = ctile + ch * CB;
-            const int swz = v_swz<CB>(ch);
-            for (int r = 0; r < RPW; r++) {
-                const unsigned seg_size = v_pack_segment<CB, BITS>(row, swz, r, stage + pos, lane);
-                seg_end += seg_size;
-                if (lane == 0) *reinterpret_cast<uint16_t*>(stage + 2 * (w * RPW + r)) = (uint16_t)seg_end;
-                pos += seg_size;
-            }
-        }
-        __syncwarp();
-        if (direct) {
-            if (lane == 0) sh_sizes[vb] = (unsigned)pos;
-        } else {
+        seen |= all_half ? v_block_segments<T, CB, BITS, 2>(src, 2 * (uint64_t)a.ss, prm, ord, stage, wbase, sizes, lane)
+                         : all_packed ? v_block_segments<T, CB, BITS, 1>(src, 2 * (uint64_t)a.ss, prm, ord, stage, wbase, sizes, lane)
+                                      : v_block_segments<T, CB, BITS, 0>(src, 2 * (uint64_t)a.ss, prm, ord, stage, wbase, sizes, lane);
+        if (!direct) {
             const int64_t blk = ((int64_t)b * nctx + cbi) * nvb + vb;
-            store_slot(a.slots + blk * a.slot_stride, stage, pos, lane);
-            if (lane == 0) a.info[((int64_t)b * a.info_seq_stride + (int64_t)(a.first_cb + cbi) * nvb + vb) * 2 + 1] = (unsigned)pos;
+            store_parts<S::kCount>(a.slots + blk * a.slot_stride, sizes, lane, [&](int i) { return stage + i * S::kBound; });
+            if (lane == 0)
+                a.info[((int64_t)b * a.info_seq_stride + (int64_t)(a.first_cb + cbi) * nvb + vb) * 2 + 1] = parts_size<S::kCount>(sizes);
         }
     }
     if (direct)
-        chain_store(a, b, cbi, sh_sizes, nvb, &sh_word, (int64_t)(a.first_cb + cbi) * nvb, NW,
-                    [&](int j) { return smem + 32 * CB + (j % NW) * wstride + CB * 64 + (j / NW) * bound16; });
-    bad = bad || (seen & ~(((1u << BITS) - 1u) * 0x00010001u)) != 0;
+        chain_store_parts<S::kCount>(a, b, cbi, sh_sizes, nvb, &sh_word, (int64_t)(a.first_cb + cbi) * nvb, NW, [&](int j, int i) {
+            return smem + 32 * CB + (j % NW) * wstride + kVExchange + (j / NW) * kBlock + i * S::kBound;
+        });
+    const bool bad = mine.bad || (seen & ~(((1u << BITS) - 1u) * 0x00010001u)) != 0;
     if (__any_sync(0xffffffffu, bad) && lane == 0) atomicOr(a.flags, kFlagCodeRange);
 }
 
 // ------------------------------------------------------------------------- K, token mode
 // K with per-token parameters (the reference's QuantMethod.PackKV pairing): the parameter pass and
-// the quantising stage are V's; each warp then packs one K block (CB tokens x 128 channels of one
+// the quantiser are V's; each warp packs one K block (CB tokens x 128 channels of one
 // head) in the K layout, lane = channels 4*lane..4*lane+3, one round per 16 tokens.
 template <typename T, int BITS, int CB>
-__global__ void __launch_bounds__(256, 2) kt_fused_encode_kernel(FusedArgs a) {
+__global__ void __launch_bounds__(256, 3) kt_fused_encode_kernel(FusedArgs a) {
     extern __shared__ __align__(16) uint8_t smem[];
     const int lane = lane_id(), wic = threadIdx.x >> 5;
     const int nctx = a.tokens / CB;
@@ -807,41 +1037,35 @@ __global__ void __launch_bounds__(256, 2) kt_fused_encode_kernel(FusedArgs a) {
     const KGeom g(CB, BITS);
     const int bound16 = (g.head_bytes + g.rounds * (g.min_bytes + g.len_bytes + 128 * 2 * BITS) + 15) & ~15;
     float4* prm = reinterpret_cast<float4*>(smem);
-    uint8_t* wbase = smem + 32 * CB + wic * (CB * 128 + bound16);
-    uint8_t* ctile = wbase;                                  // two 64-channel halves of [64][CB] codes
-    uint8_t* stage = wbase + CB * 128;
+    uint8_t* stage = smem + 32 * CB + wic * bound16;
     const T* xb = reinterpret_cast<const T*>(a.x) + (int64_t)b * a.sb + (int64_t)cbi * CB * a.ss;
-    uint8_t* ord = smem + 32 * CB + 8 * (CB * 128 + bound16);
+    uint8_t* ord = smem + 32 * CB + 8 * bound16;
     load_row_order<CB>(a, ord, b, cbi);
 
-    bool bad = token_params_pass<T, CB>(a, xb, prm, ord, b, cbi, lane, wic);
-    __syncthreads();
-    bool mine_ok = true, mine_half = true;
-    for (int t = threadIdx.x; t < CB; t += 256) {
-        mine_ok = mine_ok && __float_as_uint(prm[t].w) != 0u;
-        mine_half = mine_half && reinterpret_cast<const uint4*>(prm + CB)[t].w != 0u;
-    }
-    const bool all_packed = __syncthreads_and(mine_ok);
-    const bool all_half = __syncthreads_and(mine_half);
+    const TokenState mine = token_params_pass<T, CB>(a, xb, prm, ord, b, cbi, lane, wic);
+    // one decision for the whole CTA: the faster conversions need every token's parameters in range
+    const bool all_packed = __syncthreads_and(mine.packed);
+    const bool all_half = __syncthreads_and(mine.half);
 
     unsigned seen = 0;
     for (int h = wic; h < a.heads; h += 8) {
-        const T* src = xb + (int64_t)h * a.sh;
+        const T* src = xb + (int64_t)h * a.sh + 4 * lane;
         __syncwarp();
-#pragma unroll 1
-        for (int half = 0; half < 2; half++)
-            seen |= all_half ? v_quantise_tile<T, CB, 2>(src + 64 * half, a.ss, prm, ord, ctile + half * 64 * CB, lane)
-                             : all_packed ? v_quantise_tile<T, CB, 1>(src + 64 * half, a.ss, prm, ord, ctile + half * 64 * CB, lane)
-                                          : v_quantise_tile<T, CB, 0>(src + 64 * half, a.ss, prm, ord, ctile + half * 64 * CB, lane);
-        __syncwarp();
+        const unsigned stage_a = smem_addr(stage);
         int pos = g.head_bytes;
-        unsigned round_end = 0;
-        for (int r = 0; r < g.rounds; r++) {
-            const unsigned round_size = kt_pack_round<CB, BITS>(ctile, r, stage + pos, lane);
-            round_end += round_size;
-            if (lane == 0) *reinterpret_cast<uint16_t*>(stage + 2 * r) = (uint16_t)round_end;
-            pos += round_size;
-        }
+        const auto rounds = [&](auto mode) {
+#pragma unroll 1
+            for (int r = 0; r < g.rounds; r++) {
+                PackCodes p;
+                quantise_pack<T, CB, decltype(mode)::value>(reinterpret_cast<const uint8_t*>(src), 2 * (uint64_t)a.ss, prm, ord, 16 * r, p);
+                seen |= p.largest;
+                pos += k_pack_round<BITS>(p, p.mn01, p.mn23, p.mn01, p.mx01, p.mn23, p.mx23, stage_a + pos, lane);
+                if (lane == 0) *reinterpret_cast<uint16_t*>(stage + 2 * r) = (uint16_t)(pos - g.head_bytes);
+            }
+        };
+        if (all_half) rounds(std::integral_constant<int, 2>{});
+        else if (all_packed) rounds(std::integral_constant<int, 1>{});
+        else rounds(std::integral_constant<int, 0>{});
         __syncwarp();
         if (direct) {
             if (lane == 0) sh_sizes[h] = (unsigned)pos;     // direct form: at most 8 heads, one block per warp
@@ -853,8 +1077,8 @@ __global__ void __launch_bounds__(256, 2) kt_fused_encode_kernel(FusedArgs a) {
     }
     if (direct)
         chain_store(a, b, cbi, sh_sizes, a.heads, &sh_word, (int64_t)(a.first_cb + cbi) * a.heads, 8,
-                    [&](int j) { return smem + 32 * CB + j * (CB * 128 + bound16) + CB * 128; });
-    bad = bad || (seen & ~(((1u << BITS) - 1u) * 0x00010001u)) != 0;
+                    [&](int j) { return smem + 32 * CB + j * bound16; });
+    const bool bad = mine.bad || (seen & ~(((1u << BITS) - 1u) * 0x00010001u)) != 0;
     if (__any_sync(0xffffffffu, bad) && lane == 0) atomicOr(a.flags, kFlagCodeRange);
 }
 
@@ -989,8 +1213,8 @@ __global__ void __launch_bounds__(kOneWarps * 32) k_one_block_kernel(FusedArgs a
             const auto row = [&](int t) { return rows[i][t]; };
             unsigned over = 0, size;
             if (half_ok || packable) {
-                size = half_ok ? k_encode_round_packed<T, BITS, true>(row, q0, q1, q2, q3, pq, stage[r], lane, over)
-                               : k_encode_round_packed<T, BITS, false>(row, q0, q1, q2, q3, pq, stage[r], lane, over);
+                size = half_ok ? k_encode_round_packed<T, BITS, true>(row, q0, q1, q2, q3, pq, smem_addr(stage[r]), lane, over)
+                               : k_encode_round_packed<T, BITS, false>(row, q0, q1, q2, q3, pq, smem_addr(stage[r]), lane, over);
                 over &= ~(((1u << BITS) - 1u) * 0x00010001u);
             } else {
                 size = k_encode_round<T, BITS>(row, q0, q1, q2, q3, stage[r], lane, over);
@@ -1305,8 +1529,8 @@ static int launch_fused_t(const FusedEncodeRequest& r, uint8_t* slots, const uin
     const int nctx = r.tokens / r.cb;
     int bound16, blocks_per_seq;
     // Direct form: the scratch holds only the ticket and the status array of the look-back.  The slots form stays
-    // for more than 8 heads (a CTA of the per-token kernels would not hold all blocks of its token block), for
-    // 128-token blocks in those kernels, for a scratch too small for the status array, and on request
+    // for more than 8 heads (a CTA of the per-token kernels would not hold all blocks of its token block), for a scratch
+    // too small for the status array, and on request
     // (PKV_ENCODE_PATH=slots: measurements, tests).
     static const bool env_slots = [] { const char* v = std::getenv("PKV_ENCODE_PATH"); return v && std::string(v) == "slots"; }();
     const bool per_token_kernel = r.which == 1 || r.mode == 1;
@@ -1341,9 +1565,7 @@ static int launch_fused_t(const FusedEncodeRequest& r, uint8_t* slots, const uin
     }
     const int links = per_token_kernel ? nctx : k_one ? 1 : (nctx * r.heads + kKWarps - 1) / kKWarps;
     const int64_t chain_bytes = 256 + (int64_t)r.batch * links * 8;
-    // (128-token blocks in the per-token kernels: a second staging buffer per warp would leave one CTA per SM; measured
-    // 2.55 ms against 2.28 ms for the slots form on the 4-bit sweep configuration)
-    const bool direct = !env_slots && (!per_token_kernel || (r.heads <= 8 && r.cb != 128)) && chain_bytes <= fused_encode_scratch_bytes(r) &&
+    const bool direct = !env_slots && (!per_token_kernel || r.heads <= 8) && chain_bytes <= fused_encode_scratch_bytes(r) &&
                         r.stream_bytes != nullptr;
     if (direct) {
         a.ticket = reinterpret_cast<unsigned*>(slots);
@@ -1361,7 +1583,7 @@ static int launch_fused_t(const FusedEncodeRequest& r, uint8_t* slots, const uin
         const int nw = direct && k_one ? kKWarpsOne : kKWarps, smem = nw * bound16 + 16;
         const unsigned grid = direct ? (unsigned)links * r.batch : (unsigned)((nwarps + nw - 1) / nw);
         if (r.mode == 1) {                       // per-token parameters: CTA per (sequence, token block)
-            const int smem_t = 32 * r.cb + 8 * (r.cb * 128 + bound16) + r.cb + 16;
+            const int smem_t = 32 * r.cb + 8 * bound16 + r.cb + 16;
             auto launch_kt = [&](auto kern) {
                 if (opt_in_smem(kern, smem_t)) return (int)kCudaError;
                 kern<<<dim3(nctx, r.batch), 256, smem_t, st>>>(a);
@@ -1389,9 +1611,10 @@ static int launch_fused_t(const FusedEncodeRequest& r, uint8_t* slots, const uin
         bound16 = (g.head_bytes + g.nseg * (g.min_bytes + g.len_bytes + 32 * g.ppt * 2 * BITS) + 15) & ~15;
         a.slot_stride = bound16;
         blocks_per_seq = nctx * 2 * r.heads;
-        const VForm form = v_form((int64_t)nctx * r.batch, r.heads, BITS, r.cb);
+        const VForm form = v_form((int64_t)nctx * r.batch, r.heads, r.cb);
         const int nw = form.warps;
-        const int smem = 32 * r.cb + nw * (r.cb * 64 + (direct ? v_slots(r.heads, nw) : 1) * bound16) + r.cb + 16;
+        const int seg_bound = (g.min_bytes + g.len_bytes + 32 * g.ppt * 2 * BITS + 15) & ~15;     // VSegment::kBound
+        const int smem = 32 * r.cb + nw * (kVExchange + (direct ? v_slots(r.heads, nw) : 1) * g.nseg * seg_bound) + r.cb + 16;
         auto launch_v = [&](auto kern) {
             if (opt_in_smem(kern, smem)) return (int)kCudaError;
             kern<<<dim3(nctx, r.batch), nw * 32, smem, st>>>(a);
@@ -1400,11 +1623,8 @@ static int launch_fused_t(const FusedEncodeRequest& r, uint8_t* slots, const uin
         int rc = kOk;
         const auto by_form = [&](auto cb) {
             constexpr int CB = decltype(cb)::value;
-            if (nw == 8) return launch_v(v_fused_encode_kernel<T, BITS, CB, 8, 3>);
-            if constexpr (CB != 128)
-                if (CB == 32 || form.per_sm == 2) return launch_v(v_fused_encode_kernel<T, BITS, CB, 16, 2>);
-            if constexpr (CB != 32) return launch_v(v_fused_encode_kernel<T, BITS, CB, 16, 1>);
-            return (int)kUnsupported;
+            if (nw == 16) return launch_v(v_fused_encode_kernel<T, BITS, CB, 16, 1>);
+            return form.per_sm == 3 ? launch_v(v_fused_encode_kernel<T, BITS, CB, 8, 3>) : launch_v(v_fused_encode_kernel<T, BITS, CB, 8, 4>);
         };
         if (r.cb == 32) rc = by_form(std::integral_constant<int, 32>{});
         else if (r.cb == 64) rc = by_form(std::integral_constant<int, 64>{});

@@ -165,14 +165,16 @@ struct HalfQuotient {
         pre = QT<T>::dup(QT<T>::kPre);
         kab = packed_code_bias(qa, qb);
     }
-    __device__ __forceinline__ unsigned codes(unsigned pair_bits) const {
+    __device__ __forceinline__ unsigned codes(unsigned pair_bits) const { return raw(pair_bits) - kab; }
+    // the codes and the bias kab, which keeps their order as 16-bit lanes
+    __device__ __forceinline__ unsigned raw(unsigned pair_bits) const {
         using T2 = typename QT<T>::T2;
         const T2 x = *reinterpret_cast<const T2*>(&pair_bits);
         const T2 xp = QT<T>::kPre == 1.f ? x : __hmul2(x, pre);
         const T2 q0 = __hmul2(x, r);
         const T2 e = __hfma2(nsp, q0, xp);
         const T2 m = __hadd2(__hfma2(e, rp, q0), magic);
-        return *reinterpret_cast<const unsigned*>(&m) - kab;
+        return *reinterpret_cast<const unsigned*>(&m);
     }
 };
 

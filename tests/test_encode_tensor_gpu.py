@@ -255,3 +255,21 @@ def test_v_forms_of_other_heads_and_blocks(cuda_device, heads, cb, bits, ordered
             ops.encode_tensor("v", v[:, :, lo * cb: hi * cb], cb, rel, ops.K_TOKEN, bits, cb, first_token=lo * cb, **parts, **more(lo, hi))
         for name in all_:
             assert torch.equal(all_[name].view(torch.uint8), parts[name].view(torch.uint8)), (blocks, name)
+
+
+@pytest.mark.parametrize("heads,cb,bits", [(4, 64, 4), (1, 64, 3), (2, 128, 4), (4, 128, 3), (3, 32, 2)])
+def test_v_forms_of_little_work(cuda_device, heads, cb, bits):
+    """V launches of little work per CTA on both sides of the lines between their forms (148, 444, 592 and 888 token blocks), in blocks of every size:
+    the calls' results equal those of calls of at most 100 token blocks."""
+    dev, dtype, rel = cuda_device, torch.float16, synth.rel_for_bits(bits)
+    g = torch.Generator(device=dev).manual_seed(2)
+    for blocks in (148, 149, 444, 445, 592, 593, 888, 889):
+        v = torch.randn(1, heads, blocks * cb, 128, generator=g, device=dev).to(dtype)
+        all_, parts = (_bufs(1, heads, blocks * cb, cb, bits, "v", ops.K_TOKEN, dtype, dev) for _ in range(2))
+        ops.encode_tensor("v", v, cb, rel, ops.K_TOKEN, bits, cb, **all_)
+        for lo in range(0, blocks, 100):
+            hi = min(blocks, lo + 100)
+            ops.encode_tensor("v", v[:, :, lo * cb: hi * cb], cb, rel, ops.K_TOKEN, bits, cb, first_token=lo * cb, **parts)
+        assert int(all_["flags"].item()) == 0
+        for name in all_:
+            assert torch.equal(all_[name].view(torch.uint8), parts[name].view(torch.uint8)), (blocks, name)
