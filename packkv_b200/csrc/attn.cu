@@ -23,7 +23,7 @@
 //            unpacked and dequantised by the lane that owns the channel, transposed through a
 //            small shared-memory tile into mma fragments and contracted with q on the tensor cores;
 //            scores stay in the warp's shared memory.
-//   exchange per-CTA (max, sum) go through distributed shared memory, one cluster barrier.
+//   exchange per-CTA (max, sum) go through distributed shared memory: sent, or read behind a cluster barrier (PUSH).
 //   phase 2  scores -> probabilities in place; V packs are fetched by the lane whose mma fragment
 //            needs them (a pack is 16 tokens of one channel = one row segment of the A operand), so
 //            V needs no transposition at all.
@@ -150,6 +150,20 @@ __device__ __forceinline__ bool mbar_try_wait(unsigned bar, unsigned parity) {
         "{ .reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }"
         : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
     return ok != 0;
+}
+__device__ __forceinline__ bool mbar_try_wait_cluster(unsigned bar, unsigned parity) {   // for what other CTAs of the cluster have sent
+    unsigned ok;
+    asm volatile(
+        "{ .reg .pred p; mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }"
+        : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+    return ok != 0;
+}
+// 16 bytes to the shared memory of CTA `rank` of the cluster, counted on its mbarrier; dst and bar are this CTA's own addresses of the places
+__device__ __forceinline__ void send16(unsigned dst, unsigned bar, int rank, float4 v) {
+    asm volatile(
+        "{ .reg .b32 d, b; mapa.shared::cluster.u32 d, %0, %2; mapa.shared::cluster.u32 b, %1, %2;\n"
+        "st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.f32 [d], {%3, %4, %5, %6}, [b]; }"
+        ::"r"(dst), "r"(bar), "r"(rank), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w) : "memory");
 }
 __device__ __forceinline__ void bulk_g2s(unsigned dst, const void* src, unsigned bytes, unsigned bar) {
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
@@ -278,6 +292,9 @@ struct AttnDev {
     int warp_smem;       // bytes of per-warp shared memory
     int off_xch, off_raw, off_perm, off_desc, off_stile, off_rst;   // byte offsets inside a warp's region
     int cta_off;         // byte offset of the CTA-shared block
+    int push;            // the cluster's CTAs send one another their sums (see CtaShared); 0: they read them
+    int rx_off;          // push: byte offset of the area they are received in
+    int rx_per, rx_inv;  // push: units of four sums that a CTA delivers, ceil(2^16 / rx_per)
     int out_off;         // byte offset, inside a warp's region, of its rows of the CTA's reduced output
     int tile_shift, cbk_shift, cbv_shift;   // log2 of tile, cbk, cbv
     int nkb_shift, nvi_shift;               // log2 of K blocks per tile and of V blocks (2 halves x token blocks) per tile
@@ -306,7 +323,15 @@ struct CtaShared {
     unsigned last;       // two-launch form: this CTA (with an exchange: its cluster) is the pair's last one to deliver its rows
     unsigned pad_[3];
     unsigned long long mbar[kAW][2];
+    unsigned long long rx_ml, rx_out;   // push: all CTAs' maxima and sums, their rows of the output, have arrived
 };
+static_assert(sizeof(CtaShared) % 16 == 0, "the receive area behind it holds 16-byte units");
+// What crosses the cluster.  With PUSH a CTA sends its maxima and sums to every other one, and its sums of the output to the one that delivers
+// them, into a receive area behind the CTA-shared block ([16 CTAs][16] maxima and sums, then [CTAs][rx_per] units of four sums); the receiver
+// waits on its own mbarrier.  Written where they are and read from there, both cost a cluster barrier and a remote load's round trip more, and
+// nobody may leave before a third barrier (us a launch: 10 pairs x 5333 tokens 25.5 -> 24.3, 4 x 32 heads x 1025 26.4 -> 24.5, 8 x 8 x 2000
+// 24.0 -> 23.0; 16 x 8 x 8192 114.3 and 114.6).  Kernels of their own: with both ways in one, 16 x 8 x 8192 took 1 % longer and a team 3 %.
+
 // The CTA's reduced accumulators out[head][channel] (read by the cluster's CTAs through distributed shared
 // memory) live in the warps' regions, which are idle by then: head hd -> warp hd % kAW,
 // float offset (hd / kAW) * kD (at most 8 / kAW rows of 512 bytes per warp: the 2 KB behind out_off hold them).
@@ -336,7 +361,8 @@ enum AttnPass : int { kFused = 0, kScores = 1, kValues = 2 };
 // w, w + 4, ... of a block and, of the head's 128 V channels, w's 32 (the block headers say where a round or segment starts);
 // the scores of a tile lie in the first warp's region.  For launches whose time is the latency of one warp's tile: with one
 // tile to a warp and one warp to a scheduler, a round or segment of 16 x 128 codes is about 1 us of dependent instructions.
-template <typename T, int KMODE, bool HP, int PASS, bool TEAM>
+// PUSH: the cluster's CTAs send one another their sums instead of reading them (see CtaShared).
+template <typename T, int KMODE, bool HP, int PASS, bool TEAM, bool PUSH>
 __global__ void __launch_bounds__(kAW * 32, PASS == 1 ? PKV_ATTN_CTAS_SCORES : PASS == 2 ? PKV_ATTN_CTAS_VALUES : kMaxCtasPerSm) attn_decode_kernel(const AttnDev P) {
     using T2 = typename Tr<T>::T2;
     constexpr unsigned MAGIC = Tr<T>::kMagic2;
@@ -384,12 +410,22 @@ __global__ void __launch_bounds__(kAW * 32, PASS == 1 ? PKV_ATTN_CTAS_SCORES : P
         const unsigned L = threadIdx.x;
         cs->lutm[L] = ((1u << L) - 1u) * 0x00010001u;
     }
+    static_assert(!PUSH || (PASS != kScores && !TEAM), "a score launch sends nothing; teams read (see launch_attention)");
+    constexpr bool push = PUSH;
+    const int rx_mine = min(max(G * (kD / 4) - rank * P.rx_per, 0), P.rx_per);   // push: units that this CTA delivers
+    const unsigned rx_a = smem_addr(smem) + P.rx_off, rx_ml_bar = smem_addr(&cs->rx_ml), rx_out_bar = smem_addr(&cs->rx_out);
     if (lane == 0) {
         mbar_init(bar_a, 1);
         mbar_init(bar_a + 8, 1);
+        if (push && wic == 0) { mbar_init(rx_ml_bar, 1); mbar_init(rx_out_bar, 1); }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        if (push && wic == 0) {
+            mbar_expect_tx(rx_ml_bar, PASS == kFused ? P.cluster * 64 : 0);
+            mbar_expect_tx(rx_out_bar, P.cluster * rx_mine * 16);
+        }
     }
     __syncthreads();
+    if (push) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");    // the others may send from here on
     asm volatile("" : "+r"(lutm_a) :: "memory");        // reads of the table stay behind the barrier
     if (PASS != kValues) {
         // Launches are started under programmatic stream serialisation (P.serial): the lines above overlap the end of the launch
@@ -527,6 +563,14 @@ __global__ void __launch_bounds__(kAW * 32, PASS == 1 ? PKV_ATTN_CTAS_SCORES : P
             dead = __any_sync(0xffffffffu, dead);
             if (dead && lane == 0) atomicOr(a.flags, kFlagTimeout);
         }
+    };
+    // what the other CTAs of the cluster send; they run beside this one, so that the wait ends by itself, but it is bounded all the same
+    auto wait_received = [&](unsigned bar) {
+        unsigned spins = 0;
+        while (!mbar_try_wait_cluster(bar, 0)) {
+            if (++spins > kWaitSpins) { atomicOr(a.flags, kFlagTimeout); break; }
+        }
+        __syncwarp();
     };
     // natural-order per-token parameters (raw) -> pair order (perm); zero-points take the conversion bias
     auto permute_params = [&]() {
@@ -1001,17 +1045,32 @@ __global__ void __launch_bounds__(kAW * 32, PASS == 1 ? PKV_ATTN_CTAS_SCORES : P
     };
     if constexpr (PASS == kFused) {
         // ---- cluster exchange: global max and sum ---------------------------------------------------
-        cluster.sync();
         // lane: head lane & 7 of the CTAs (lane >> 3) + 4 i, all remote loads in flight together; every warp for itself, so that no
         // barrier follows
         float mr[4], lr[4], M = -INFINITY, L = 0.f;
+        if (push) {
+            asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");        // every CTA is ready to receive (since long)
+            if (wic == 0) {
+                __syncwarp();                              // the CTA's maxima and sums are this warp's
+                for (int i = lane; i < 4 * P.cluster; i += 32)
+                    send16(rx_a + rank * 64 + 16 * (i & 3), rx_ml_bar, i >> 2, reinterpret_cast<const float4*>(cs->cl_m)[i & 3]);   // cl_l follows cl_m
+            }
+            wait_received(rx_ml_bar);
+        } else {
+            cluster.sync();
+        }
 #pragma unroll
         for (int i = 0; i < 4; i++) {
             const int r = (lane >> 3) + 4 * i;
             mr[i] = -INFINITY; lr[i] = 0.f;
             if (r < P.cluster) {
-                const CtaShared* o = cluster.map_shared_rank(cs, r);
-                mr[i] = o->cl_m[lane & 7]; lr[i] = o->cl_l[lane & 7];
+                if (push) {
+                    const float* o = reinterpret_cast<const float*>(smem + P.rx_off) + 16 * r + (lane & 7);
+                    mr[i] = o[0]; lr[i] = o[8];
+                } else {
+                    const CtaShared* o = cluster.map_shared_rank(cs, r);
+                    mr[i] = o->cl_m[lane & 7]; lr[i] = o->cl_l[lane & 7];
+                }
             }
         }
 #pragma unroll
@@ -1367,15 +1426,29 @@ __global__ void __launch_bounds__(kAW * 32, PASS == 1 ? PKV_ATTN_CTAS_SCORES : P
     __syncthreads();
     // ---- CTA reduce, then cluster reduce --------------------------------------------------------
     constexpr int kThreads = kAW * 32;
-    for (int d = threadIdx.x; d < kD; d += kThreads) {
-        for (int hd = 0; hd < G; hd++) {
-            float v = 0.f;
+    if (push) {
+        if (PASS == kValues) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+        for (int u = threadIdx.x; u < G * (kD / 4); u += kThreads) {       // four sums of the CTA's warps, to the CTA that delivers them
+            float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-            for (int w = 0; w < kAW; w++) v += reinterpret_cast<const float*>(smem + w * P.warp_smem)[hd * kD + d];
-            cta_out_row(smem, P.warp_smem, P.out_off, hd)[d] = v;
+            for (int w = 0; w < kAW; w++) {
+                const float4 x = reinterpret_cast<const float4*>(smem + w * P.warp_smem)[u];
+                v.x += x.x; v.y += x.y; v.z += x.z; v.w += x.w;
+            }
+            const int to = (u * P.rx_inv) >> 16;                           // u / rx_per
+            send16(rx_a + 1024 + (rank * P.rx_per + u - to * P.rx_per) * 16, rx_out_bar, to, v);
         }
+    } else {
+        for (int d = threadIdx.x; d < kD; d += kThreads) {
+            for (int hd = 0; hd < G; hd++) {
+                float v = 0.f;
+#pragma unroll
+                for (int w = 0; w < kAW; w++) v += reinterpret_cast<const float*>(smem + w * P.warp_smem)[hd * kD + d];
+                cta_out_row(smem, P.warp_smem, P.out_off, hd)[d] = v;
+            }
+        }
+        cluster.sync();
     }
-    cluster.sync();
     // The cluster's CTAs share out the G * 128 sums, one to a thread, whose remote loads are in flight together.  With the first CTA adding
     // them all, one remote load after the other, this was the last 1.7 us of 13 (8 KV heads x 700 tokens, 4 heads to a group; 11.5 now) and
     // 8 of the 31 us of two launches with 7 heads to a group (10 pairs x 5333 tokens; 26.7 now).  With an exchange the first CTA
@@ -1412,11 +1485,25 @@ __global__ void __launch_bounds__(kAW * 32, PASS == 1 ? PKV_ATTN_CTAS_SCORES : P
             for (int p = 0; p < P.x.n_ranks; p++)
                 reinterpret_cast<T*>(P.x.gathered[p])[(int64_t)P.x.rank * a.batch * q_heads * kD + idx] = r;
         };
+        // push: the CTA's units, `store` takes four sums
+        const auto received = [&](auto store) {
+            if (rx_mine > 0) wait_received(rx_out_bar);
+            for (int t = threadIdx.x; t < rx_mine; t += kThreads) {
+                float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 4
+                for (int r = 0; r < P.cluster; r++) {
+                    const float4 x = reinterpret_cast<const float4*>(smem + P.rx_off + 1024)[r * P.rx_per + t];
+                    v.x += x.x; v.y += x.y; v.z += x.z; v.w += x.w;
+                }
+                store(4 * (rank * P.rx_per + t), v);
+            }
+        };
         bool deliver = true;
         if constexpr (PASS == kValues) {
             // this cluster's rows go to the scratch; the CTA that finds all the others' there adds them up
             float* part = P.sc_part + ((int64_t)pair * part_stride + split) * 8 * kD;
-            for (int e = first; e < G * kD; e += stride) __stcg(part + e, cluster_sum(e));
+            if (push) received([&](int e, const float4& v) { __stcg(reinterpret_cast<float4*>(part + e), v); });
+            else for (int e = first; e < G * kD; e += stride) __stcg(part + e, cluster_sum(e));
             __threadfence();
             __syncthreads();
             if (threadIdx.x == 0) cs->last = atomicAdd(P.sc_count + pair, 1u) == (unsigned)((spread ? n_vctas : n_splits) - 1) ? 1u : 0u;
@@ -1442,7 +1529,15 @@ __global__ void __launch_bounds__(kAW * 32, PASS == 1 ? PKV_ATTN_CTAS_SCORES : P
                 if (threadIdx.x == 0) P.sc_count[pair] = 0u;   // ready for the next launch on this scratch
             }
         } else {
-            for (int e = first; e < G * kD; e += stride) put(e, cluster_sum(e));
+            if (push) received([&](int e, const float4& v) {
+                T* to = reinterpret_cast<T*>(a.out) + (int64_t)(b * q_heads + h * G) * kD + e;
+                if ((reinterpret_cast<uintptr_t>(a.out) & 7) == 0) {
+                    *reinterpret_cast<uint2*>(to) = make_uint2(Tr<T>::pack2(v.x, v.y), Tr<T>::pack2(v.z, v.w));
+                } else {
+                    put(e, v.x); put(e + 1, v.y); put(e + 2, v.z); put(e + 3, v.w);
+                }
+            });
+            else for (int e = first; e < G * kD; e += stride) put(e, cluster_sum(e));
         }
         if (deliver && P.x.n_ranks > 0) {
             __threadfence_system();                // the rows are visible to the other GPUs before the arrival is
@@ -1450,7 +1545,7 @@ __global__ void __launch_bounds__(kAW * 32, PASS == 1 ? PKV_ATTN_CTAS_SCORES : P
             if ((int)threadIdx.x < P.x.n_ranks) atomicAdd_system(P.x.arrivals[threadIdx.x] + P.x.rank, 1u);
         }
     }
-    cluster.sync();   // keep every CTA's shared memory alive until the others have read it
+    if (!push) cluster.sync();   // keep every CTA's shared memory alive until the others have read it; what is sent here has been received
     }   // PASS != kScores
 }
 
@@ -1487,9 +1582,9 @@ struct LaunchRoom {
     }
 };
 
-template <typename T, int KM, bool HPV, int PASS, bool TEAM>
+template <typename T, int KM, bool HPV, int PASS, bool TEAM, bool PUSH>
 static int launch_one(const AttnDev& P, dim3 grid, int smem, cudaStream_t st) {
-    auto kern = attn_decode_kernel<T, KM, HPV, PASS, TEAM>;
+    auto kern = attn_decode_kernel<T, KM, HPV, PASS, TEAM, PUSH>;
     static LaunchRoom room;
     int device = -1;
     if (cudaGetDevice(&device) != cudaSuccess) { cudaGetLastError(); return kCudaError; }
@@ -1531,24 +1626,29 @@ static int launch_one(const AttnDev& P, dim3 grid, int smem, cudaStream_t st) {
     return cudaLaunchKernelEx(&cfg, kern, P) == cudaSuccess ? kOk : kCudaError;
 }
 
-template <typename T, int PASS, bool TEAM = false>
+template <typename T, int PASS, bool TEAM = false, bool PUSH = false>
 static int launch_pass(const AttnDev& P, dim3 grid, int smem, cudaStream_t st) {
     const AttnArgs& a = P.a;
     if (a.k_mode == kKChannel)
-        return a.high_precision_zero ? launch_one<T, kKChannel, true, PASS, TEAM>(P, grid, smem, st) : launch_one<T, kKChannel, false, PASS, TEAM>(P, grid, smem, st);
-    return a.high_precision_zero ? launch_one<T, kKToken, true, PASS, TEAM>(P, grid, smem, st) : launch_one<T, kKToken, false, PASS, TEAM>(P, grid, smem, st);
+        return a.high_precision_zero ? launch_one<T, kKChannel, true, PASS, TEAM, PUSH>(P, grid, smem, st) : launch_one<T, kKChannel, false, PASS, TEAM, PUSH>(P, grid, smem, st);
+    return a.high_precision_zero ? launch_one<T, kKToken, true, PASS, TEAM, PUSH>(P, grid, smem, st) : launch_one<T, kKToken, false, PASS, TEAM, PUSH>(P, grid, smem, st);
 }
 
 template <typename T>
 static int launch_typed(const AttnDev& P, dim3 grid, int smem, cudaStream_t st) {
-    if (P.nsplit == 1 && P.sc_count == nullptr) return P.team ? launch_pass<T, kFused, true>(P, grid, smem, st) : launch_pass<T, kFused>(P, grid, smem, st);
+    const auto fused = [&]() {
+        if (P.team) return launch_pass<T, kFused, true>(P, grid, smem, st);
+        return P.push ? launch_pass<T, kFused, false, true>(P, grid, smem, st) : launch_pass<T, kFused>(P, grid, smem, st);
+    };
+    const auto values = [&]() { return P.push ? launch_pass<T, kValues, false, true>(P, grid, smem, st) : launch_pass<T, kValues>(P, grid, smem, st); };
+    if (P.nsplit == 1 && P.sc_count == nullptr) return fused();
 #ifdef PKV_DEBUG_PASS   // measurement builds: one of the two launches alone (the results are then meaningless)
     static const int only = env_int("PKV_ATTN_ONLY_PASS");
     if (only == 1) return launch_pass<T, kScores>(P, grid, smem, st);
-    if (only == 2) return launch_pass<T, kValues>(P, grid, smem, st);
+    if (only == 2) return values();
 #endif
     const int rc = launch_pass<T, kScores>(P, grid, smem, st);
-    return rc != kOk ? rc : launch_pass<T, kValues>(P, grid, smem, st);
+    return rc != kOk ? rc : values();
 }
 
 
@@ -1897,7 +1997,17 @@ int launch_attention(const AttnArgs& a, const AttnExchange* xch, const AttnAppen
         plans[oldest++ % kPlans] = key;
     }
     P.team = best_launches == 1 && team_wins(best_cl);
-    const int smem = plan_smem(P, best_cl, best_split, best_ns, slot);
+    int smem = plan_smem(P, best_cl, best_split, best_ns, slot);
+    // Sums are sent where the receive area takes no CTA off an SM and every CTA of the cluster delivers (with an exchange the first one does);
+    // a team's are read: its launches are short of places for code, not of time at the exchange.
+    if (!xch && best_cl > 1 && !P.team) {
+        const int units = a.group * (kD / 4), per = (units + best_cl - 1) / best_cl, with = smem + 1024 + best_cl * per * 16;
+        const auto per_sm = [](int bytes) { return std::min(kMaxCtasPerSm, (228 * 1024) / (bytes + 1024)); };
+        if (with <= 227 * 1024 && per_sm(with) == per_sm(smem)) {
+            P.push = 1; P.rx_off = smem; P.rx_per = per; P.rx_inv = (65536 + per - 1) / per;
+            smem = with;
+        }
+    }
     P.extra = best_extra;
     // Launches without an exchange are placed as soon as every CTA of the launch before has ended, and wait for its completion on the
     // device: in stream order they start when the whole launch is known to be complete, up to 2 us later on launches of 10 to 40 us

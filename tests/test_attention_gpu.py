@@ -638,3 +638,33 @@ def test_encode_then_attend_without_waiting(cuda_device, plan):
         for a, b in zip(state[3], states[0][3]):
             assert torch.equal(a.view(torch.int16), b.view(torch.int16))
         assert torch.equal(state[0].v_stream, states[0][0].v_stream) and torch.equal(state[0].k_stream, states[0][0].k_stream)
+
+
+@pytest.mark.parametrize("cluster,group", [(2, 8), (3, 7), (4, 1), (5, 3), (8, 4), (13, 6), (16, 8)])
+def test_sums_sent_across_the_cluster(cuda_device, cluster, group):
+    """Launches in which the CTAs of a cluster send one another their maxima, sums and parts of the output (no team: four tiles to a CTA or more):
+    cluster sizes that divide the output's units of four sums and that do not, one launch and two, with and without CTAs that have no unit."""
+    n_comp = 64 * max(4 * cluster, 12)
+    for plan in ((cluster, 1, 1), (cluster, 2, 2)):
+        err = _run_case(cuda_device, torch.bfloat16, 1, 2, group, n_comp, 144, block=64, cbk=64, cbv=64, bits_k=4, bits_v=3, k_mode="channel", seed=cluster,
+                        plan=plan)
+        assert err <= TOL, (plan, err)
+
+
+def test_output_at_an_odd_address(cuda_device):
+    """Rows of the output are written in fours where they start on 8 bytes, one by one elsewhere: the same values."""
+    dev, dtype, B, H, G, n_comp, n_res = cuda_device, torch.float16, 2, 4, 4, 2048, 150
+    k, v = synth.synth_kv(B, H, n_comp + n_res, 128, seed=3, dtype=dtype, device=dev)
+    q = synth.synth_q(B, H * G, 128, seed=3, dtype=dtype)[:, :, 0].contiguous().to(dev)
+    layer = encode.compress_kv(k[:, :, :n_comp], v[:, :, :n_comp], block=64, bits_k=4, bits_v=4, k_rel=1 / 14, v_rel=1 / 14, k_mode=QuantMode.ChannelQuant, cbv=64)
+    rest = [t[:, :, n_comp:].contiguous() for t in (k, v)]
+    store = torch.zeros(q.numel() + 3, dtype=dtype, device=dev)
+    outs = [store[at: at + q.numel()].view(q.shape) for at in (0, 3)]
+    wanted = None
+    for out in outs:
+        flags = ops.new_flags(dev)
+        ops.decode_attention(q, layer, *rest, n_res, out=out, flags=flags, kv_heads=H, plan=(4, 1, 1))
+        torch.cuda.synchronize()
+        assert int(flags.item()) == 0
+        assert wanted is None or torch.equal(out, wanted)
+        wanted = out.clone()
