@@ -330,7 +330,8 @@ static_assert(sizeof(CtaShared) % 16 == 0, "the receive area behind it holds 16-
 // them, into a receive area behind the CTA-shared block ([16 CTAs][16] maxima and sums, then [CTAs][rx_per] units of four sums); the receiver
 // waits on its own mbarrier.  Written where they are and read from there, both cost a cluster barrier and a remote load's round trip more, and
 // nobody may leave before a third barrier (us a launch: 10 pairs x 5333 tokens 25.5 -> 24.3, 4 x 32 heads x 1025 26.4 -> 24.5, 8 x 8 x 2000
-// 24.0 -> 23.0; 16 x 8 x 8192 114.3 and 114.6).  Kernels of their own: with both ways in one, 16 x 8 x 8192 took 1 % longer and a team 3 %.
+// 24.0 -> 23.0; teams: 8 x 700 10.2 -> 9.6, 16 x 8 x 1000 17.2 -> 15.9; 16 x 8 x 8192 113.9 and 114.1).  Kernels of their own: with both ways in one,
+// 16 x 8 x 8192 took 1 % longer and a team 3 %.
 
 // The CTA's reduced accumulators out[head][channel] (read by the cluster's CTAs through distributed shared
 // memory) live in the warps' regions, which are idle by then: head hd -> warp hd % kAW,
@@ -410,7 +411,7 @@ __global__ void __launch_bounds__(kAW * 32, PASS == 1 ? PKV_ATTN_CTAS_SCORES : P
         const unsigned L = threadIdx.x;
         cs->lutm[L] = ((1u << L) - 1u) * 0x00010001u;
     }
-    static_assert(!PUSH || (PASS != kScores && !TEAM), "a score launch sends nothing; teams read (see launch_attention)");
+    static_assert(!PUSH || PASS != kScores, "a score launch sends nothing");
     constexpr bool push = PUSH;
     const int rx_mine = min(max(G * (kD / 4) - rank * P.rx_per, 0), P.rx_per);   // push: units that this CTA delivers
     const unsigned rx_a = smem_addr(smem) + P.rx_off, rx_ml_bar = smem_addr(&cs->rx_ml), rx_out_bar = smem_addr(&cs->rx_out);
@@ -1637,7 +1638,7 @@ static int launch_pass(const AttnDev& P, dim3 grid, int smem, cudaStream_t st) {
 template <typename T>
 static int launch_typed(const AttnDev& P, dim3 grid, int smem, cudaStream_t st) {
     const auto fused = [&]() {
-        if (P.team) return launch_pass<T, kFused, true>(P, grid, smem, st);
+        if (P.team) return P.push ? launch_pass<T, kFused, true, true>(P, grid, smem, st) : launch_pass<T, kFused, true>(P, grid, smem, st);
         return P.push ? launch_pass<T, kFused, false, true>(P, grid, smem, st) : launch_pass<T, kFused>(P, grid, smem, st);
     };
     const auto values = [&]() { return P.push ? launch_pass<T, kValues, false, true>(P, grid, smem, st) : launch_pass<T, kValues>(P, grid, smem, st); };
@@ -1998,12 +1999,13 @@ int launch_attention(const AttnArgs& a, const AttnExchange* xch, const AttnAppen
     }
     P.team = best_launches == 1 && team_wins(best_cl);
     int smem = plan_smem(P, best_cl, best_split, best_ns, slot);
-    // Sums are sent where the receive area takes no CTA off an SM and every CTA of the cluster delivers (with an exchange the first one does);
-    // a team's are read: its launches are short of places for code, not of time at the exchange.
-    if (!xch && best_cl > 1 && !P.team) {
+    // Sums are sent where every CTA of the cluster delivers (with an exchange the first one does) and the receive area takes no CTA off an SM, or
+    // none that the launch has (plan_cost's places for clusters; with one CTA off each SM, 8 pairs x 32768 tokens in two launches of 512 CTAs took
+    // 55 us instead of 39.5).
+    if (!xch && best_cl > 1) {
         const int units = a.group * (kD / 4), per = (units + best_cl - 1) / best_cl, with = smem + 1024 + best_cl * per * 16;
         const auto per_sm = [](int bytes) { return std::min(kMaxCtasPerSm, (228 * 1024) / (bytes + 1024)); };
-        if (with <= 227 * 1024 && per_sm(with) == per_sm(smem)) {
+        if (with <= 227 * 1024 && (per_sm(with) == per_sm(smem) || pairs * best_cl * best_split <= (long)(0.93 * kSmCount * per_sm(with)))) {
             P.push = 1; P.rx_off = smem; P.rx_per = per; P.rx_inv = (65536 + per - 1) / per;
             smem = with;
         }

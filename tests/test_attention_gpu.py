@@ -651,6 +651,16 @@ def test_sums_sent_across_the_cluster(cuda_device, cluster, group):
         assert err <= TOL, (plan, err)
 
 
+@pytest.mark.parametrize("cluster,group,cbv", [(2, 4, 64), (3, 8, 128), (6, 5, 64), (8, 4, 128), (16, 7, 64)])
+def test_sums_sent_by_teams(cuda_device, cluster, group, cbv):
+    """The same with teams (three tiles or fewer to a CTA), some of whose CTAs have no tile."""
+    tile = max(64, cbv)
+    for tiles in (cluster // 2, cluster, 3 * cluster):
+        err = _run_case(cuda_device, torch.float16, 2, 2, group, tile * tiles, 130, block=64, cbk=64, cbv=cbv, bits_k=3, bits_v=4, k_mode="token", seed=tiles,
+                        plan=(cluster, 1, 1))
+        assert err <= TOL, (tiles, err)
+
+
 def test_output_at_an_odd_address(cuda_device):
     """Rows of the output are written in fours where they start on 8 bytes, one by one elsewhere: the same values."""
     dev, dtype, B, H, G, n_comp, n_res = cuda_device, torch.float16, 2, 4, 4, 2048, 150
