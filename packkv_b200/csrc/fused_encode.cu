@@ -975,9 +975,9 @@ __host__ __device__ constexpr int v_slots(int heads, int nw) { return (2 * heads
 
 constexpr int kVExchange = 1280;   // bytes of a warp's exchange area (see v_block_segments)
 
-// NW warps, PER_SM CTAs to an SM: see v_form.  Bound by instructions and the latency of its loads (134 M elements, 8 heads x 64 tokens, 4 bits: 130 us,
-// 17 instructions per element at 47 % of the issue slots; 145 us when codes went through a transposed tile).  What each form of the stages costs,
-// per 16 tokens x 4 channels of a lane: quantiser about 300 instructions, pack words 150, exchange, offsets and stores 200.
+// NW warps, PER_SM CTAs to an SM: see v_form.  Bound by instructions and the latency of its loads and of the look-back (134 M elements, 8 heads x 64
+// tokens, 4 bits: 130 us, 16.6 instructions per element at 57 % of the issue slots; 145 us and 18.9 when codes went through a transposed tile).
+// Per 16 tokens x 4 channels of a lane: quantiser about 300 instructions, pack words 150, exchange, offsets and stores 200.
 template <typename T, int BITS, int CB, int NW, int PER_SM>
 __global__ void __launch_bounds__(NW * 32, PER_SM) v_fused_encode_kernel(FusedArgs a) {
     extern __shared__ __align__(16) uint8_t smem[];
