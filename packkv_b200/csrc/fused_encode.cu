@@ -867,8 +867,7 @@ template <int CB, int BITS> struct VSegment {
 
 // One V block (CB tokens x 64 channels at src) into its segments: segment i at stage + i * kBound, its bytes in sizes[i].
 // Lane (par = lane >> 4, cg = lane & 15) takes channels 4cg .. 4cg + 3 of every other pack.  xch: 1280 bytes of the warp's, 16-byte aligned, in
-// which the words change lanes.  Against codes transposed through a tile of bytes (two header fields, a row of codes and a scan for every
-// segment) a round takes 670 instructions for 64 elements of a lane.  Returns the OR of the packs' largest codes in 16-bit lanes.
+// which the words change lanes.  A round takes about 670 instructions for a lane's 64 elements.  Returns the OR of the packs' largest codes in 16-bit lanes.
 template <typename T, int CB, int BITS, int MODE>
 __device__ __forceinline__ unsigned v_block_segments(const T* src, uint64_t row_bytes, const float4* prm, const uint8_t* ord, uint8_t* stage, uint8_t* xch, unsigned* sizes,
                                                      int lane) {
