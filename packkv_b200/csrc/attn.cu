@@ -330,7 +330,7 @@ static_assert(sizeof(CtaShared) % 16 == 0, "the receive area behind it holds 16-
 // them, into a receive area behind the CTA-shared block ([16 CTAs][16] maxima and sums, then [CTAs][rx_per] units of four sums); the receiver
 // waits on its own mbarrier.  Written where they are and read from there, both cost a cluster barrier and a remote load's round trip more, and
 // nobody may leave before a third barrier (us a launch: 10 pairs x 5333 tokens 25.5 -> 24.3, 4 x 32 heads x 1025 26.4 -> 24.5, 8 x 8 x 2000
-// 24.0 -> 23.0; teams: 8 x 700 10.2 -> 9.6, 16 x 8 x 1000 17.2 -> 15.9; 16 x 8 x 8192 113.9 and 114.1).  Kernels of their own: with both ways in one,
+// 24.0 -> 23.0; teams: 8 x 700 10.2 -> 9.6, 16 x 8 x 1000 17.2 -> 15.9; 16 x 8 x 8192 113.6 and 114.1).  Kernels of their own: with both ways in one,
 // 16 x 8 x 8192 took 1 % longer and a team 3 %.
 
 // The CTA's reduced accumulators out[head][channel] (read by the cluster's CTAs through distributed shared
@@ -2001,8 +2001,9 @@ int launch_attention(const AttnArgs& a, const AttnExchange* xch, const AttnAppen
     int smem = plan_smem(P, best_cl, best_split, best_ns, slot);
     // Sums are sent where every CTA of the cluster delivers (with an exchange the first one does) and the receive area takes no CTA off an SM, or
     // none that the launch has (plan_cost's places for clusters; with one CTA off each SM, 8 pairs x 32768 tokens in two launches of 512 CTAs took
-    // 55 us instead of 39.5).
-    if (!xch && best_cl > 1) {
+    // 55 us instead of 39.5).  Single launches of 512 tokens to a warp and more read: their time is in the tiles (us read and sent: 16 x 8 x 8192
+    // 113.6 114.1, 17 x 8 x 8192 114.4 115.4, 8 x 8 x 16384 112.7 112.1; of less work 16 x 8 x 4096 62.7 62.0, 32 x 4 x 3000 57.6 55.1).
+    if (!xch && best_cl > 1 && (best_launches == 2 || P.tpw * P.tile < 512)) {
         const int units = a.group * (kD / 4), per = (units + best_cl - 1) / best_cl, with = smem + 1024 + best_cl * per * 16;
         const auto per_sm = [](int bytes) { return std::min(kMaxCtasPerSm, (228 * 1024) / (bytes + 1024)); };
         if (with <= 227 * 1024 && (per_sm(with) == per_sm(smem) || pairs * best_cl * best_split <= (long)(0.93 * kSmCount * per_sm(with)))) {
