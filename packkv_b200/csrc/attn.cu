@@ -61,6 +61,7 @@ constexpr int kAW = PKV_ATTN_WARPS;   // warps per CTA (1, 2 or 4)
 constexpr int kMaxCtasPerSm = PKV_ATTN_CTAS;  // register budget: 65536 / (128 * 4) -> 128 per thread, 96 for 5
 constexpr int kD = 128;           // head dimension
 constexpr unsigned kWaitSpins = 1u << 22;   // bounded mbarrier wait (each try suspends for a while by itself)
+constexpr unsigned kReceiveTries = 4 * kWaitSpins;   // for what another CTA sends, which may have run out of one such wait first
 #ifndef PKV_ATTN_CTAS_SCORES
 #define PKV_ATTN_CTAS_SCORES PKV_ATTN_CTAS   // the two-launch form's kernels may take other register budgets
 #endif
@@ -295,6 +296,7 @@ struct AttnDev {
     int push;            // the cluster's CTAs send one another their sums (see CtaShared); 0: they read them
     int rx_off;          // push: byte offset of the area they are received in
     int rx_per, rx_inv;  // push: units of four sums that a CTA delivers, ceil(2^16 / rx_per)
+    unsigned rx_tries;   // push: kReceiveTries
     int out_off;         // byte offset, inside a warp's region, of its rows of the CTA's reduced output
     int tile_shift, cbk_shift, cbv_shift;   // log2 of tile, cbk, cbv
     int nkb_shift, nvi_shift;               // log2 of K blocks per tile and of V blocks (2 halves x token blocks) per tile
@@ -321,7 +323,8 @@ struct CtaShared {
     float gM[kAW][8], gInvL[kAW][8];   // global maximum and reciprocal sum, a copy for every warp
     unsigned lutm[8];    // (2^len - 1) * 0x00010001 per pack length 0..4 (see unpack8)
     unsigned last;       // two-launch form: this CTA (with an exchange: its cluster) is the pair's last one to deliver its rows
-    unsigned pad_[3];
+    unsigned late;       // push: a wait of the first warp for what others send has run out
+    unsigned pad_[2];
     unsigned long long mbar[kAW][2];
     unsigned long long rx_ml, rx_out;   // push: all CTAs' maxima and sums, their rows of the output, have arrived
 };
@@ -418,7 +421,7 @@ __global__ void __launch_bounds__(kAW * 32, PASS == 1 ? PKV_ATTN_CTAS_SCORES : P
     if (lane == 0) {
         mbar_init(bar_a, 1);
         mbar_init(bar_a + 8, 1);
-        if (push && wic == 0) { mbar_init(rx_ml_bar, 1); mbar_init(rx_out_bar, 1); }
+        if (push && wic == 0) { mbar_init(rx_ml_bar, 1); mbar_init(rx_out_bar, 1); cs->late = 0u; }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         if (push && wic == 0) {
             mbar_expect_tx(rx_ml_bar, PASS == kFused ? P.cluster * 64 : 0);
@@ -565,11 +568,16 @@ __global__ void __launch_bounds__(kAW * 32, PASS == 1 ? PKV_ATTN_CTAS_SCORES : P
             if (dead && lane == 0) atomicOr(a.flags, kFlagTimeout);
         }
     };
-    // what the other CTAs of the cluster send; they run beside this one, so that the wait ends by itself, but it is bounded all the same
+    // what the other CTAs of the cluster send; they run beside this one, so that the wait ends by itself, but it is bounded all the same.
+    // When it has run out the CTA goes on, so that the others get what it sends; it leaves last (see the end)
     auto wait_received = [&](unsigned bar) {
-        unsigned spins = 0;
-        while (!mbar_try_wait_cluster(bar, 0)) {
-            if (++spins > kWaitSpins) { atomicOr(a.flags, kFlagTimeout); break; }
+        for (unsigned tries = 0; ; tries++) {
+            if (tries >= P.rx_tries) {
+                atomicOr(a.flags, kFlagTimeout);
+                if (wic == 0) *reinterpret_cast<volatile unsigned*>(&cs->late) = 1u;
+                break;
+            }
+            if (mbar_try_wait_cluster(bar, 0)) break;
         }
         __syncwarp();
     };
@@ -1546,7 +1554,15 @@ __global__ void __launch_bounds__(kAW * 32, PASS == 1 ? PKV_ATTN_CTAS_SCORES : P
             if ((int)threadIdx.x < P.x.n_ranks) atomicAdd_system(P.x.arrivals[threadIdx.x] + P.x.rank, 1u);
         }
     }
-    if (!push) cluster.sync();   // keep every CTA's shared memory alive until the others have read it; what is sent here has been received
+    if (!push) {
+        cluster.sync();   // keep every CTA's shared memory alive until the others have read it
+    } else if (wic == 0 && *reinterpret_cast<volatile unsigned*>(&cs->late)) {
+        // What is sent here may not all have arrived: this CTA's shared memory has to stay until it has.  (Every warp waits for the same; the first one
+        // stays for the CTA.)  It waits for the threads of the cluster that have not ended, whose own waits are bounded: all has been sent then; and
+        // for its arrival, which the barrier says nothing about.
+        asm volatile("barrier.cluster.arrive.release;\nbarrier.cluster.wait.acquire;" ::: "memory");
+        for (unsigned tries = 0; tries < kWaitSpins && !(mbar_try_wait_cluster(rx_ml_bar, 0) && mbar_try_wait_cluster(rx_out_bar, 0)); tries++) { }
+    }
     }   // PASS != kScores
 }
 
@@ -2007,7 +2023,9 @@ int launch_attention(const AttnArgs& a, const AttnExchange* xch, const AttnAppen
         const int units = a.group * (kD / 4), per = (units + best_cl - 1) / best_cl, with = smem + 1024 + best_cl * per * 16;
         const auto per_sm = [](int bytes) { return std::min(kMaxCtasPerSm, (228 * 1024) / (bytes + 1024)); };
         if (with <= 227 * 1024 && (per_sm(with) == per_sm(smem) || pairs * best_cl * best_split <= (long)(0.93 * kSmCount * per_sm(with)))) {
+            static const int env_tries = env_int("PKV_ATTN_RECEIVE_TRIES");          // tests: -1 = every wait runs out at once
             P.push = 1; P.rx_off = smem; P.rx_per = per; P.rx_inv = (65536 + per - 1) / per;
+            P.rx_tries = env_tries < 0 ? 0u : env_tries > 0 ? (unsigned)env_tries : kReceiveTries;
             smem = with;
         }
     }

@@ -4,6 +4,10 @@ packkv_assert (include/utils.h:8-16), throws "not supported" for shapes it does 
 (src/kernels.cu:586-589).  Here every such condition is a status code (-> ValueError /
 RuntimeError("not supported")) or a bit in the device flag word; nothing aborts and no kernel
 reads or writes outside its buffers."""
+import os
+import subprocess
+import sys
+
 import pytest
 import torch
 
@@ -75,3 +79,40 @@ def test_status_codes_map_to_exceptions(cuda_device):
         ops.decode_attention(torch.zeros(1, 8, 96, dtype=torch.float16, device=cuda_device), None, None, None, 0)
     lib = _lib.lib()
     assert lib.pkv_decode_attention(None, None) == _lib.PKV_ERR_BAD_ARGUMENT        # null argument block: a status, not a crash
+
+
+RUN_OUT = """
+import torch
+from packkv_b200 import _lib, encode, ops, synth
+from packkv_b200.config import QuantMode
+dev, dtype, B, H, G, n_comp, n_res = "cuda:0", torch.float16, 2, 2, 4, 2048, 150
+k, v = synth.synth_kv(B, H, n_comp + n_res, 128, seed=3, dtype=dtype, device=dev)
+q = synth.synth_q(B, H * G, 128, seed=3, dtype=dtype)[:, :, 0].contiguous().to(dev)
+layer = encode.compress_kv(k[:, :, :n_comp], v[:, :, :n_comp], block=64, bits_k=4, bits_v=4, k_rel=1 / 14, v_rel=1 / 14, k_mode=QuantMode.ChannelQuant, cbv=64)
+rest = [t[:, :, n_comp:].contiguous() for t in (k, v)]
+scratch = ops.new_attention_scratch(dev)
+
+def step(plan, times=1):
+    flags = ops.new_flags(dev)
+    for _ in range(times):
+        out = ops.decode_attention(q, layer, *rest, n_res, flags=flags, kv_heads=H, plan=plan, scratch=scratch)
+    torch.cuda.synchronize()
+    return out, int(flags.item())
+
+alone = [step(plan) for plan in ((1, 1, 1), (1, 3, 2))]                     # clusters of one CTA: nothing is sent
+assert all(flags == 0 for _, flags in alone)
+for plan in ((2, 1, 1), (8, 1, 1), (13, 1, 1), (16, 1, 1), (2, 2, 2), (8, 3, 2), (13, 2, 2)):
+    assert step(plan, 3)[1] == _lib.FLAG_TIMEOUT, plan
+for plan, (out, _) in zip(((1, 1, 1), (1, 3, 2)), alone):                     # the device and the scratch's counters are as before
+    again, flags = step(plan)
+    assert flags == 0 and torch.equal(again, out), plan
+print("as expected")
+"""
+
+
+def test_receive_waits_that_run_out():
+    """The CTAs of a cluster that send one another their sums, with a limit of no tries at all: every wait for them runs out.  The launches end and
+    say so in the status word, one behind another too, and later launches on the same buffers are right."""
+    r = subprocess.run([sys.executable, "-c", RUN_OUT], capture_output=True, text=True, timeout=300, cwd=os.path.dirname(os.path.dirname(__file__)),
+                       env={**os.environ, "PKV_ATTN_RECEIVE_TRIES": "-1"})
+    assert r.returncode == 0 and "as expected" in r.stdout, r.stdout + r.stderr
