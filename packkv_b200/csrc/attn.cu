@@ -1058,9 +1058,9 @@ __global__ void __launch_bounds__(kAW * 32, PASS == 1 ? PKV_ATTN_CTAS_SCORES : P
         // barrier follows
         float mr[4], lr[4], M = -INFINITY, L = 0.f;
         if (push) {
+            __syncwarp();                                  // the barrier is the warp's as one; the CTA's maxima and sums are the first warp's lanes'
             asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");        // every CTA is ready to receive (since long)
             if (wic == 0) {
-                __syncwarp();                              // the CTA's maxima and sums are this warp's
                 for (int i = lane; i < 4 * P.cluster; i += 32)
                     send16(rx_a + rank * 64 + 16 * (i & 3), rx_ml_bar, i >> 2, reinterpret_cast<const float4*>(cs->cl_m)[i & 3]);   // cl_l follows cl_m
             }

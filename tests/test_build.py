@@ -30,3 +30,13 @@ def test_host_extension_is_rebuilt_for_another_torch_python_or_command(tmp_path,
     assert not build._host_stale()
     os.utime(lib, (0, 0))                                    # older than its source
     assert build._host_stale()
+
+
+def test_cluster_barriers_of_a_whole_warp_follow_a_convergence_point():
+    """barrier.cluster with .aligned is executed by the threads of a warp as one: a __syncwarp() or __syncthreads() stands on the lines before it."""
+    with open(os.path.join(build.CSRC, "attn.cu")) as f:
+        lines = [line for line in f.read().splitlines() if line.strip() and not line.strip().startswith("//")]
+    at = [i for i, line in enumerate(lines) if "barrier.cluster." in line and ".aligned" in line]
+    assert at
+    for i in at:
+        assert any("__syncwarp()" in line or "__syncthreads()" in line for line in lines[i - 4: i]), lines[i].strip()
