@@ -427,7 +427,8 @@ int32_t pkv_decode_attention_append(const pkv_attn_args* args_host, const pkv_at
  *   scratch   device memory, 256-byte aligned, ZERO before its first use (the library leaves its counters at
  *             zero after every call); launches that share it must be ordered on one stream.  NULL: single launch.
  * pkv_attention_plan fills plan_io the same way and launches nothing (scratch_bytes alone decides what fits;
- * with_exchange != 0: plan as for a launch with an exchange block).
+ * with_exchange != 0: plan as for a launch with an exchange block).  pkv_attention_sends does the same and says how the CTAs
+ * of a cluster would hand over their sums: sends_host = 1 sent, 0 read behind a barrier (the same results).
  * append_host and exchange_host may be NULL.
  */
 typedef struct pkv_attn_plan {
@@ -442,6 +443,8 @@ int32_t pkv_decode_attention_split(const pkv_attn_args* args_host, const pkv_att
                                    void* scratch, int64_t scratch_bytes, void* cuda_stream);
 int32_t pkv_attention_plan(const pkv_attn_args* args_host, pkv_attn_plan* plan_io, int64_t scratch_bytes,
                            int32_t with_exchange);
+int32_t pkv_attention_sends(const pkv_attn_args* args_host, pkv_attn_plan* plan_io, int64_t scratch_bytes,
+                            int32_t with_exchange, int32_t* sends_host);
 
 /*
  * The same step for heads of head_dim channels, 64 <= head_dim < 128, a multiple of 8, whose stored rows are widened to 128

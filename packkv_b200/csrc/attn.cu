@@ -1775,9 +1775,18 @@ int launch_exchange_wait(uint32_t* arrivals, int n_ranks, unsigned expected, uns
     return kOk;
 }
 
-// plan_io: in: cluster / nsplit / launches to force (0 = choose); out: what was chosen.  dry_run: plan only.
+// Clusters of `cl` CTAs that fit the GPU at once with `per_sm` CTAs to an SM.  A cluster lies in one GPC: three of 20 SMs, four of 18 and one of 10 give
+// what cudaOccupancyMaxActiveClusters says for every size and number on the B200s asked (of 148 SMs: 33 clusters of 4 and 15 of 8 with one CTA to an SM,
+// 142 and 71 with four; of 13, 17 with two, which are 221 of 296 CTAs).
+static long clusters_that_fit(int cl, int per_sm) {
+    if (cl <= 2) return (long)(kSmCount / cl) * per_sm;
+    return 3 * (20 * per_sm / cl) + 4 * (18 * per_sm / cl) + (cl <= 10 ? 10 * per_sm / cl : 0);
+}
+
+// plan_io: in: cluster / nsplit / launches to force (0 = choose); out: what was chosen.  dry_run: plan only.  sends: out: whether the launch
+// that delivers sends its sums across the cluster (see CtaShared).
 int launch_attention(const AttnArgs& a, const AttnExchange* xch, const AttnAppend* ap, AttnPlan* plan_io, void* scratch, int64_t scratch_bytes,
-                     bool dry_run, cudaStream_t st, int head_dim) {
+                     bool dry_run, cudaStream_t st, int head_dim, int32_t* sends) {
     if (head_dim < kD / 2 || head_dim > kD || head_dim % 8) return kUnsupported;
     if (a.batch <= 0 || a.kv_heads <= 0 || a.group < 1 || a.group > 8) return a.group > 8 ? kUnsupported : kBadArgument;
     if (a.n_comp < 0 || a.n_res < 0 || a.n_comp + a.n_res == 0) return kBadArgument;
@@ -2016,13 +2025,13 @@ int launch_attention(const AttnArgs& a, const AttnExchange* xch, const AttnAppen
     P.team = best_launches == 1 && team_wins(best_cl);
     int smem = plan_smem(P, best_cl, best_split, best_ns, slot);
     // Sums are sent where every CTA of the cluster delivers (with an exchange the first one does) and the receive area takes no CTA off an SM, or
-    // none that the launch has (plan_cost's places for clusters; with one CTA off each SM, 8 pairs x 32768 tokens in two launches of 512 CTAs took
-    // 55 us instead of 39.5).  Single launches of 512 tokens to a warp and more read: their time is in the tiles (us read and sent: 16 x 8 x 8192
+    // the launch's clusters fit without it (with one CTA off each SM, 8 pairs x 32768 tokens in two launches of 512 CTAs took 55 us instead of 39.5,
+    // 8 heads x 5333 tokens in blocks of 128, eight clusters of 15 where seven fit, 35.9 instead of 21.9).  Single launches of 512 tokens to a warp and more read: their time is in the tiles (us read and sent: 16 x 8 x 8192
     // 113.6 114.1, 17 x 8 x 8192 114.4 115.4, 8 x 8 x 16384 112.7 112.1; of less work 16 x 8 x 4096 62.7 62.0, 32 x 4 x 3000 57.6 55.1).
     if (!xch && best_cl > 1 && (best_launches == 2 || P.tpw * P.tile < 512)) {
         const int units = a.group * (kD / 4), per = (units + best_cl - 1) / best_cl, with = smem + 1024 + best_cl * per * 16;
         const auto per_sm = [](int bytes) { return std::min(kMaxCtasPerSm, (228 * 1024) / (bytes + 1024)); };
-        if (with <= 227 * 1024 && (per_sm(with) == per_sm(smem) || pairs * best_cl * best_split <= (long)(0.93 * kSmCount * per_sm(with)))) {
+        if (with <= 227 * 1024 && (per_sm(with) == per_sm(smem) || pairs * best_split <= clusters_that_fit(best_cl, per_sm(with)))) {
             static const int env_tries = env_int("PKV_ATTN_RECEIVE_TRIES");          // tests: -1 = every wait runs out at once
             P.push = 1; P.rx_off = smem; P.rx_per = per; P.rx_inv = (65536 + per - 1) / per;
             P.rx_tries = env_tries < 0 ? 0u : env_tries > 0 ? (unsigned)env_tries : kReceiveTries;
@@ -2048,6 +2057,7 @@ int launch_attention(const AttnArgs& a, const AttnExchange* xch, const AttnAppen
         P.sc_scores = base + L.scores;
     }
     if (plan_io) { plan_io->cluster = best_cl; plan_io->nsplit = best_split; plan_io->launches = best_launches; plan_io->extra = best_extra > 0 ? best_extra : 0; }
+    if (sends) *sends = P.push;
     if (dry_run) return kOk;
     dim3 grid(P.cluster * P.nsplit, a.kv_heads, a.batch);
     if (best_extra >= 0) grid = dim3((unsigned)(pairs * best_split + best_extra), 1, 1);

@@ -193,7 +193,7 @@ int32_t pkv_decode_attention_narrow(const pkv_attn_args* args_host, const pkv_at
     return launch_attention(*args_host, nullptr, append_host, nullptr, scratch, scratch_bytes, false, static_cast<cudaStream_t>(cuda_stream), head_dim);
 }
 
-int32_t pkv_attention_plan(const pkv_attn_args* args_host, pkv_attn_plan* plan_io, int64_t scratch_bytes, int32_t with_exchange) {
+static int32_t attention_plan(const pkv_attn_args* args_host, pkv_attn_plan* plan_io, int64_t scratch_bytes, int32_t with_exchange, int32_t* sends) {
     if (!args_host || !plan_io) return kBadArgument;
     // the plan depends on sizes only: any non-null, aligned address stands for the scratch, and a block that is never
     // dereferenced (nothing is launched) for the exchange
@@ -202,7 +202,15 @@ int32_t pkv_attention_plan(const pkv_attn_args* args_host, pkv_attn_plan* plan_i
     uint32_t dummy_counter = 0;
     x.gathered[0] = &dummy_counter; x.arrivals[0] = &dummy_counter;
     return launch_attention(*args_host, with_exchange ? &x : nullptr, nullptr, plan_io, scratch_bytes > 0 ? reinterpret_cast<void*>(uintptr_t(256)) : nullptr,
-                            scratch_bytes, true, nullptr);
+                            scratch_bytes, true, nullptr, 128, sends);
+}
+
+int32_t pkv_attention_plan(const pkv_attn_args* args_host, pkv_attn_plan* plan_io, int64_t scratch_bytes, int32_t with_exchange) {
+    return attention_plan(args_host, plan_io, scratch_bytes, with_exchange, nullptr);
+}
+
+int32_t pkv_attention_sends(const pkv_attn_args* args_host, pkv_attn_plan* plan_io, int64_t scratch_bytes, int32_t with_exchange, int32_t* sends_host) {
+    return sends_host ? attention_plan(args_host, plan_io, scratch_bytes, with_exchange, sends_host) : (int32_t)kBadArgument;
 }
 
 int32_t pkv_exchange_wait(const uint32_t* arrivals, int32_t n_ranks, uint32_t expected, uint32_t max_polls, uint32_t* dev_flags,
