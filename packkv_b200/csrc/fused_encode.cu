@@ -544,12 +544,16 @@ __global__ void __launch_bounds__(NW * 32, 768 / (NW * 32)) k_fused_encode_kerne
 
 // ------------------------------------------------------------------------------------------ V
 // one CTA per (sequence, token block): pass 1 computes the per-token parameters over all heads
-// (one warp per token); pass 2 gives each warp whole V blocks (cb tokens x 64 channels), two packs of 16 tokens
-// at a time: a lane quantises four channels of the 16 tokens of one pack, two channels to an instruction, and
-// forms their pack words in registers as K's rounds do; the words then change lanes through shared memory, so that
-// a store covers the adjacent packs of 32 channels as the stream has them.
+// (half a warp per token); pass 2 gives each warp whole V blocks (cb tokens x 64 channels), in one of two ways (v_form says which):
+//   registers  two packs of 16 tokens at a time: a lane quantises four channels of the 16 tokens of one pack, two channels to an instruction,
+//              and forms their pack words in registers as K's rounds do; the words then change lanes through shared memory, so that
+//              a store covers the adjacent packs of 32 channels as the stream has them.  Fewer instructions.
+//   tile       codes of eight channels of a token to a lane (16-byte loads) go to a transposed tile in shared memory, whose rows the packing
+//              stage reads, a channel to a lane; the block comes out whole.  Fewer registers (16 warps twice to an SM without spills), shorter
+//              chains for a warp that is alone, and whole blocks for the scratch of the slots form.
+// One-block launches use the tile.
 //
-// (One-block launches go through a tile of codes instead.)  Tile of one V block in shared memory, transposed for the packing stage: one row of CB bytes per
+// Tile of one V block in shared memory, transposed for the packing stage: one row of CB bytes per
 // channel, made of 16-byte chunks (one per pack); chunk p of channel ch is stored at chunk position
 // p ^ v_swz(ch) so that both the word stores of the quantising stage and the 16-byte row reads of the
 // packing stage spread over the banks.  Inside a chunk, byte 4*r0 + k holds token r0 + 4*k of the
@@ -617,6 +621,31 @@ struct TileLane {
         }
     }
 };
+
+// Quantises one V block into the tile.  Lane (r0 = lane >> 3, cg = lane & 7) loads 8 channels
+// (16 bytes) of tokens r0, r0+4, r0+8, ...
+// Returns the OR of all codes in 16-bit lanes for the range check.
+template <typename T, int CB, int MODE>
+__device__ __forceinline__ unsigned v_quantise_tile(const T* src, int64_t ss, const float4* prm, const uint8_t* ord, uint8_t* tile, int lane) {
+    const int r0 = lane >> 3;
+    unsigned seen = 0;
+    const TileLane<CB> out(tile, lane);
+    const T* lsrc = src + 8 * (lane & 7);
+#pragma unroll 1
+    for (int p = 0; p < CB / 16; p++) {
+        unsigned c[4][4];
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            const int tok = 16 * p + 4 * k + r0;
+            const uint4 raw = __ldg(reinterpret_cast<const uint4*>(lsrc + (int64_t)ord[tok] * ss));
+            v_quantise_row<T, CB, MODE>(raw, prm, tok, c[k]);
+#pragma unroll
+            for (int i = 0; i < 4; i++) seen |= c[k][i];
+        }
+        out.store(p, c);
+    }
+    return seen;
+}
 
 // One 16-byte tile chunk (word r0: bytes k = codes of tokens r0 + 4k of the pack) -> the pack's
 // minimum, bit length and 2*len-byte word (token 0 in the top bits).
@@ -867,7 +896,7 @@ __device__ __forceinline__ void put_fields(uint8_t* at, unsigned f01, unsigned f
 
 template <int CB, int BITS> struct VSegment {
     static constexpr int kPacks = CB == 32 ? 2 : 4, kGroups = CB == 128 ? 2 : 1, kCount = 2 * kGroups;   // packs per channel; 64-token groups; segments
-    static constexpr int kMin = BITS * kPacks * 4, kLen = len_field_bits(BITS) * kPacks * 4, kBound = (kMin + kLen + 64 * kPacks * BITS + 15) & ~15;
+    static constexpr int kMin = BITS * kPacks * 4, kLen = len_field_bits(BITS) * kPacks * 4, kBytes = kMin + kLen + 64 * kPacks * BITS, kBound = (kBytes + 15) & ~15;
 };
 
 // One V block (CB tokens x 64 channels at src) into its segments: segment i at stage + i * kBound, its bytes in sizes[i].
@@ -953,47 +982,76 @@ __device__ __forceinline__ void load_row_order(const FusedArgs& a, uint8_t* ord,
     __syncthreads();
 }
 
-// Form of a V launch: the warps of a CTA and how many CTAs an SM's registers hold.  Up to one CTA to an SM: 16 warps with all registers, so that
-// a warp has few blocks.  Beyond, 8 warps: three to an SM (waves of 444 CTAs), or four with 64 registers (waves of 592), which are slower where both
-// make the same number of waves, unless a CTA has little work.  us with 8 x 3, 8 x 4 and 16 x 1 (16 warps, two to an SM, was at most 3 % ahead of the
-// best of them between 149 and 296 CTAs and is not built):
-//   8 heads x 64 tokens: 148 CTAs 24.8 28.1 21.1, 296 30.8 34.0 35.9, 444 37.5 40.0 50.8, 500 53.3 42.6 51.6, 592 58.2 46.4 60.9, 740 62.0 76.4 71.5,
-//     1184 89.4 92.0 109, 2048 141 159 185
-//   4 x 64: 148 19.9 20.4 17.9, 444 27.9 29.6 40.7, 592 38.3 27.8 47.4, 888 42.8 47.6 65.6, 1184 58.9 52.7 86.4, 2048 95.4 90.5 146
-//   8 x 32: 444 25.8 25.8 36.8, 592 33.6 25.5 41.8, 888 41.0 42.9 57.0, 1500 66.7 62.4 94.6; 1 x 64: 592 26.9 19.9 36.0, 2048 65.6 59.7 109;
-//   2 x 128: 592 51.4 36.5 62.9, 740 54.8 61.4 75.0, 2048 132 125 201
-// Of more than 8 heads x 64 tokens, blocks of 128 tokens leave room for two CTAs of 8 warps only (8 x 128: 370 CTAs 89.5 and 71.1 with 16, 740 140 and
-// 118, 2048 327 and 305; 16 x 128: 592 241 and 198); smaller ones go through the scratch, a few waves of 16 warps (16 x 64: 100 CTAs 35.8 and 27.8,
-// 592 113 and 111, 740 130 and 137; 32 x 64: 444 153 and 158, 592 220 and 209, 740 251 and 258).
-struct VForm { int warps, per_sm; };
-static VForm v_form(int64_t ctas, int heads, int cb) {
-    const VForm narrow{8, 3}, dense{8, 4}, wide{16, 1};
-    if (ctas <= kSmCount) return wide;
-    if (heads * cb > 512) return cb == 128 || ctas <= 4 * kSmCount ? wide : narrow;
-    const bool one_wave = ctas > 3 * kSmCount && ctas <= 4 * kSmCount, light = heads * cb <= 256;
-    return one_wave || (light && ctas > 6 * kSmCount) ? dense : narrow;
+// Form of a V launch: the warps of a CTA, how many CTAs an SM's registers hold, and which way a block takes.  Up to one CTA to an SM: 16 warps with all
+// registers.  Up to two: 16 warps twice, through the tile (from registers such a CTA spills).  Beyond: 8 warps, three to an SM (waves of 444 CTAs), or from
+// registers four with 64 of them and some spills (waves of 592), where that saves a wave or a CTA has little work.  Of few heads a warp has one block, of
+// which the tile is done sooner; where warps are plenty the instructions count, of which registers need fewer.
+// us, by CTAs of 148, 296, 444, 592, 600, 888, 1036, 1332, 2048 (fp16; r registers, t tile, warps x CTAs to an SM; - not the form of anything near):
+//   4 heads x 64 tokens, 4 bits:  t16x1 17.7 28.7 39.6 46.0 46.2 64.7 74.9 94.9 143   t16x2 17.8 21.8 31.3 32.1 33.1 45.5 54.3 66.4 96.6
+//                                 t8x3 19.6 23.2 26.4 36.2 36.3 41.4 53.4 59.4 91.1   r8x3 20.0 24.6 27.9 38.3 38.4 44.1 55.7 62.0 93.9
+//                                 r8x4 20.8 25.6 29.6 27.6 34.8 47.1 49.9 65.8 89.9   (900: t8x3 44.2, r8x4 47.4)
+//   8 x 64, 4 bits:  t16x1 22.0 35.5 49.6 59.8 60.8 84.2 - 121 183   t16x2 22.1 30.1 48.0 50.2 53.2 71.9 - 103 149   t8x3 24.8 31.6 39.8 62.9 63.2 71.5 - 102 148
+//                    r8x3 25.2 31.2 37.9 58.1 58.4 65.5 - 92.7 139   r8x4 28.8 34.6 40.4 46.8 60.4 81.3 - 114 156   (660: t16x2 58.7, r8x3 60.0; 740: 65.8, 62.2)
+//   8 x 64, 2 bits (a block's packs are fewer stores; 3 bits alike):  t16x2 27.5 at 296, 45.4 at 600, 55.5 at 740, 126 at 2048; r8x3 29.7, 54.7, 57.6, 131
+//   8 x 32:  r16x1 17.0 26.9 36.3 41.7 - 57.5 66.5 - 126   t16x2 17.1 21.3 30.7 32.4 - 44.9 53.5 - 93.7   r8x3 18.5 22.7 26.0 33.9 - 38.1 49.5 - 82.7
+//            r8x4 18.3 22.8 26.5 25.7 - 42.1 44.1 - 77.2;  16 x 32: r8x3 23.7 32.3 44.6 62.4 - 81.7 95.7 - 173, t16x2 20.7 31.1 44.6 56.2 - 80.0 92.2 - 171
+//   4 x 128: r16x1 24.2 41.1 59.0 73.4 - 105 120 - 227   t8x3 28.4 33.1 55.7 58.3 - 85.2 106 - 184 (of a tile of 128 tokens an SM holds two CTAs)
+//            r8x3 29.8 35.5 41.8 68.2 - 75.0 100 - 166   r8x4 33.3 38.1 43.7 52.6 - 93.5 97.0 - 180;  2 x 128 at 2048: r8x3 127, r8x4 125
+//   8 x 128: r16x1 30.6 54.8 78.1 97.0 at 592, 304 at 2048; r8x3 39.7 53.1 93.3 97.5, 322; t8x3 37.3 69.3 96.4 128, 414
+// Above 8 heads blocks go through the scratch, whole from the tile with aligned stores:
+//   16 x 64, 4 bits: t16x1 27.2 at 100, r16x1 27.8; t16x2 54.5 at 296, 102 at 592, 146 at 888, 317 at 2048; t8x3 56.9, 104, 147, 311; r8x3 58.6, 113, 150, 317
+//   16 x 64, 2 bits: t16x2 45.1, 80.1, 113, 241; t8x3 49.5, 91.0, 125, 264; r8x3 51.1, 96.5, 127, 268
+//   12 x 128, 2 bits: t8x3 73.4, 137 at 592, 436 at 2048, r16x1 73.4, 141, 467 (r8x3 97 at 400, t8x3 110);  16 x 128, 4 bits: r16x1 100, 197, 430 at 1332; t8x3 110, 209, 447
+struct VForm { int warps, per_sm; bool tile; };
+static VForm v_form(int64_t ctas, int heads, int bits, int cb) {
+    const VForm regs3{8, 3, false}, regs4{8, 4, false}, regs_wide{16, 1, false}, tile3{8, 3, true}, tile_two{16, 2, true}, tile_wide{16, 1, true};
+    constexpr int64_t n = kSmCount;
+    if (ctas <= n) return cb == 64 ? tile_wide : regs_wide;
+    const bool one_of_four = ctas > 3 * n && ctas <= 4 * n;           // one wave of four to an SM, two of three
+    const bool two_of_four = 4 * ctas > 25 * n && ctas <= 8 * n;      // two, and three of which the last is not near empty
+    if (cb == 32) {
+        if (heads > 12 || ctas <= 2 * n) return tile_two;
+        return one_of_four || (heads <= 8 && ctas > 6 * n) ? regs4 : regs3;
+    }
+    if (cb == 128) {
+        if (heads > 4) return heads <= 8 || heads >= 16 ? regs_wide : ctas > 2 * n && ctas <= 3 * n ? regs3 : tile3;
+        if (ctas <= 2 * n) return tile3;
+        return one_of_four || two_of_four || (heads <= 2 && ctas > 9 * n) ? regs4 : regs3;
+    }
+    if (ctas <= 2 * n) return tile_two;
+    if (heads > 8) return bits < 4 || one_of_four ? tile_two : tile3;
+    if (one_of_four) return regs4;
+    if (heads <= 4) return two_of_four || ctas > 9 * n ? regs4 : tile3;
+    // (of fewer bits, where the last wave of 444 is up to two of its CTAs to an SM)
+    return ctas > 3 * n && (bits < 4 ? (ctas - 1) % (3 * n) < 2 * n : 2 * ctas <= 9 * n) ? tile_two : regs3;
 }
 
 // finished blocks that a warp of the V kernel holds in the direct form until their offsets are known
 __host__ __device__ constexpr int v_slots(int heads, int nw) { return (2 * heads + nw - 1) / nw; }
 
 constexpr int kVExchange = 1280;   // bytes of a warp's exchange area (see v_block_segments)
+// Shared memory of a warp: its tile or exchange area, and `slots` finished blocks, whole or in segments.
+template <int CB, int BITS, bool TILE> struct VWarp {
+    using S = VSegment<CB, BITS>;
+    static constexpr int kWork = TILE ? CB * 64 : kVExchange, kBlock = TILE ? (S::kCount * (2 + S::kBytes) + 15) & ~15 : S::kCount * S::kBound;
+    static __host__ __device__ constexpr int bytes(int slots) { return kWork + slots * kBlock; }
+};
 
-// NW warps, PER_SM CTAs to an SM: see v_form.  Bound by instructions and the latency of its loads and of the look-back (134 M elements, 8 heads x 64
-// tokens, 4 bits: 130 us, 16.6 instructions per element at 57 % of the issue slots; 145 us and 18.9 when codes went through a transposed tile).
-// Per 16 tokens x 4 channels of a lane: quantiser about 300 instructions, pack words 150, exchange, offsets and stores 200.
-template <typename T, int BITS, int CB, int NW, int PER_SM>
+// NW warps, PER_SM CTAs to an SM, through a tile or from registers: see v_form.  Bound by instructions and the latency of its loads and of the look-back
+// (134 M elements, 8 heads x 64 tokens, 4 bits: 130 us from registers, 16.6 instructions per element at 57 % of the issue slots; 138 us through the tile).
+// Per 16 tokens x 4 channels of a lane, from registers: quantiser about 300 instructions, pack words 150, exchange, offsets and stores 200.
+template <typename T, int BITS, int CB, int NW, int PER_SM, bool TILE>
 __global__ void __launch_bounds__(NW * 32, PER_SM) v_fused_encode_kernel(FusedArgs a) {
     extern __shared__ __align__(16) uint8_t smem[];
     const int lane = lane_id(), wic = threadIdx.x >> 5;
     const int nctx = a.tokens / CB;
-    __shared__ unsigned sh_word, sh_sizes[64];   // bytes of the segments: of all blocks, in the slots form of a warp's own
-    const bool direct = a.status != nullptr;                 // then a warp keeps both of its blocks until the offsets are known
+    __shared__ unsigned sh_word, sh_sizes[64];   // bytes of the blocks (TILE), or of the segments of all blocks, in the slots form of a warp's own
+    const bool direct = a.status != nullptr;                 // then a warp keeps all of its blocks until the offsets are known
     int cbi = blockIdx.x, b = blockIdx.y;
     if (direct) chain_place(a, &sh_word, b, cbi);
     using S = VSegment<CB, BITS>;
-    constexpr int kBlock = S::kCount * S::kBound;            // a finished block's segments
-    const int wstride = kVExchange + (direct ? v_slots(a.heads, NW) : 1) * kBlock;
+    using W = VWarp<CB, BITS, TILE>;
+    const int wstride = W::bytes(direct ? v_slots(a.heads, NW) : 1);
     float4* prm = reinterpret_cast<float4*>(smem);           // [cb] (scale, zero, 1/scale, fast)
     uint8_t* wbase = smem + 32 * CB + wic * wstride;
     const T* xb = reinterpret_cast<const T*>(a.x) + (int64_t)b * a.sb + (int64_t)cbi * CB * a.ss;
@@ -1011,23 +1069,44 @@ __global__ void __launch_bounds__(NW * 32, PER_SM) v_fused_encode_kernel(FusedAr
     const int nvb = 2 * a.heads;
     for (int vb = wic; vb < nvb; vb += NW) {
         const T* src = xb + (int64_t)(vb >> 1) * a.sh + 64 * (vb & 1);
-        uint8_t* stage = wbase + kVExchange + (direct ? (vb / NW) * kBlock : 0);
-        unsigned* sizes = sh_sizes + (direct ? vb : wic) * S::kCount;
+        uint8_t* stage = wbase + W::kWork + (direct ? (vb / NW) * W::kBlock : 0);
+        const auto slot = [&]() { return a.slots + (((int64_t)b * nctx + cbi) * nvb + vb) * a.slot_stride; };
+        const auto put_size = [&](unsigned bytes) { a.info[((int64_t)b * a.info_seq_stride + (int64_t)(a.first_cb + cbi) * nvb + vb) * 2 + 1] = bytes; };
         __syncwarp();
-        seen |= all_half ? v_block_segments<T, CB, BITS, 2>(src, 2 * (uint64_t)a.ss, prm, ord, stage, wbase, sizes, lane)
-                         : all_packed ? v_block_segments<T, CB, BITS, 1>(src, 2 * (uint64_t)a.ss, prm, ord, stage, wbase, sizes, lane)
-                                      : v_block_segments<T, CB, BITS, 0>(src, 2 * (uint64_t)a.ss, prm, ord, stage, wbase, sizes, lane);
-        if (!direct) {
-            const int64_t blk = ((int64_t)b * nctx + cbi) * nvb + vb;
-            store_parts<S::kCount>(a.slots + blk * a.slot_stride, sizes, lane, [&](int i) { return stage + i * S::kBound; });
-            if (lane == 0)
-                a.info[((int64_t)b * a.info_seq_stride + (int64_t)(a.first_cb + cbi) * nvb + vb) * 2 + 1] = parts_size<S::kCount>(sizes);
+        if constexpr (TILE) {
+            seen |= all_half ? v_quantise_tile<T, CB, 2>(src, a.ss, prm, ord, wbase, lane)
+                             : all_packed ? v_quantise_tile<T, CB, 1>(src, a.ss, prm, ord, wbase, lane) : v_quantise_tile<T, CB, 0>(src, a.ss, prm, ord, wbase, lane);
+            __syncwarp();
+            int pos = 2 * S::kCount;                         // behind the table of segment ends
+            for (int i = 0; i < S::kCount; i++) {
+                const int ch = 32 * (i / S::kGroups) + lane;
+                pos += v_pack_segment<CB, BITS>(wbase + ch * CB, v_swz<CB>(ch), i % S::kGroups, stage + pos, lane);
+                if (lane == 0) *reinterpret_cast<uint16_t*>(stage + 2 * i) = (uint16_t)(pos - 2 * S::kCount);
+            }
+            __syncwarp();
+            if (direct) {
+                if (lane == 0) sh_sizes[vb] = (unsigned)pos;
+            } else {
+                store_slot(slot(), stage, pos, lane);
+                if (lane == 0) put_size((unsigned)pos);
+            }
+        } else {
+            unsigned* sizes = sh_sizes + (direct ? vb : wic) * S::kCount;
+            seen |= all_half ? v_block_segments<T, CB, BITS, 2>(src, 2 * (uint64_t)a.ss, prm, ord, stage, wbase, sizes, lane)
+                             : all_packed ? v_block_segments<T, CB, BITS, 1>(src, 2 * (uint64_t)a.ss, prm, ord, stage, wbase, sizes, lane)
+                                          : v_block_segments<T, CB, BITS, 0>(src, 2 * (uint64_t)a.ss, prm, ord, stage, wbase, sizes, lane);
+            if (!direct) {
+                store_parts<S::kCount>(slot(), sizes, lane, [&](int i) { return stage + i * S::kBound; });
+                if (lane == 0) put_size(parts_size<S::kCount>(sizes));
+            }
         }
     }
-    if (direct)
-        chain_store_parts<S::kCount>(a, b, cbi, sh_sizes, nvb, &sh_word, (int64_t)(a.first_cb + cbi) * nvb, NW, [&](int j, int i) {
-            return smem + 32 * CB + (j % NW) * wstride + kVExchange + (j / NW) * kBlock + i * S::kBound;
-        });
+    if (direct) {
+        const auto block = [&](int j) { return smem + 32 * CB + (j % NW) * wstride + W::kWork + (j / NW) * W::kBlock; };
+        const int64_t first = (int64_t)(a.first_cb + cbi) * nvb;
+        if constexpr (TILE) chain_store(a, b, cbi, sh_sizes, nvb, &sh_word, first, NW, block);
+        else chain_store_parts<S::kCount>(a, b, cbi, sh_sizes, nvb, &sh_word, first, NW, [&](int j, int i) { return block(j) + i * S::kBound; });
+    }
     const bool bad = mine.bad || (seen & ~(((1u << BITS) - 1u) * 0x00010001u)) != 0;
     if (__any_sync(0xffffffffu, bad) && lane == 0) atomicOr(a.flags, kFlagCodeRange);
 }
@@ -1622,24 +1701,40 @@ static int launch_fused_t(const FusedEncodeRequest& r, uint8_t* slots, const uin
         bound16 = (g.head_bytes + g.nseg * (g.min_bytes + g.len_bytes + 32 * g.ppt * 2 * BITS) + 15) & ~15;
         a.slot_stride = bound16;
         blocks_per_seq = nctx * 2 * r.heads;
-        const VForm form = v_form((int64_t)nctx * r.batch, r.heads, r.cb);
-        const int nw = form.warps;
-        const int seg_bound = (g.min_bytes + g.len_bytes + 32 * g.ppt * 2 * BITS + 15) & ~15;     // VSegment::kBound
-        const int smem = 32 * r.cb + nw * (kVExchange + (direct ? v_slots(r.heads, nw) : 1) * g.nseg * seg_bound) + r.cb + 16;
-        auto launch_v = [&](auto kern) {
+        const VForm form = v_form((int64_t)nctx * r.batch, r.heads, BITS, r.cb);
+        const auto launch = [&](auto cb, auto warps, auto per_sm, auto tile) {
+            constexpr int CB = decltype(cb)::value, NW = decltype(warps)::value;
+            const auto kern = v_fused_encode_kernel<T, BITS, CB, NW, decltype(per_sm)::value, decltype(tile)::value>;
+            const int smem = 32 * CB + NW * VWarp<CB, BITS, decltype(tile)::value>::bytes(direct ? v_slots(r.heads, NW) : 1) + CB + 16;
             if (opt_in_smem(kern, smem)) return (int)kCudaError;
-            kern<<<dim3(nctx, r.batch), nw * 32, smem, st>>>(a);
+            kern<<<dim3(nctx, r.batch), NW * 32, smem, st>>>(a);
             return (int)kOk;
         };
+        using std::integral_constant;
+        constexpr std::true_type tile{};
+        constexpr std::false_type regs{};
+        constexpr integral_constant<int, 1> one{};
+        constexpr integral_constant<int, 2> two{};
+        constexpr integral_constant<int, 3> three{};
+        constexpr integral_constant<int, 4> four{};
+        constexpr integral_constant<int, 8> eight{};
+        constexpr integral_constant<int, 16> sixteen{};
         int rc = kOk;
-        const auto by_form = [&](auto cb) {
+        const auto by_form = [&](auto cb) {                                         // the forms that v_form gives for the block
             constexpr int CB = decltype(cb)::value;
-            if (nw == 16) return launch_v(v_fused_encode_kernel<T, BITS, CB, 16, 1>);
-            return form.per_sm == 3 ? launch_v(v_fused_encode_kernel<T, BITS, CB, 8, 3>) : launch_v(v_fused_encode_kernel<T, BITS, CB, 8, 4>);
+            if (!form.tile && form.warps == 8) return form.per_sm == 3 ? launch(cb, eight, three, regs) : launch(cb, eight, four, regs);
+            if constexpr (CB == 64) {
+                if (form.warps == 8) return launch(cb, eight, three, tile);
+                return form.per_sm == 1 ? launch(cb, sixteen, one, tile) : launch(cb, sixteen, two, tile);
+            } else {
+                if (!form.tile) return launch(cb, sixteen, one, regs);
+                if constexpr (CB == 32) return launch(cb, sixteen, two, tile);
+                else return launch(cb, eight, three, tile);
+            }
         };
-        if (r.cb == 32) rc = by_form(std::integral_constant<int, 32>{});
-        else if (r.cb == 64) rc = by_form(std::integral_constant<int, 64>{});
-        else rc = by_form(std::integral_constant<int, 128>{});
+        if (r.cb == 32) rc = by_form(integral_constant<int, 32>{});
+        else if (r.cb == 64) rc = by_form(integral_constant<int, 64>{});
+        else rc = by_form(integral_constant<int, 128>{});
         if (rc != kOk) return rc;
     }
     if (direct) return cudaGetLastError() == cudaSuccess ? kOk : kCudaError;

@@ -273,3 +273,29 @@ def test_v_forms_of_little_work(cuda_device, heads, cb, bits):
         assert int(all_["flags"].item()) == 0
         for name in all_:
             assert torch.equal(all_[name].view(torch.uint8), parts[name].view(torch.uint8)), (blocks, name)
+
+
+@pytest.mark.parametrize("heads,cb,bits,blocks", [(4, 64, 4, (666, 667, 962, 963, 1184, 1185, 1332, 1333)), (6, 64, 4, (592, 593, 666, 667)), (6, 64, 2, (592, 593)),
+                                                  (10, 64, 4, (296, 297, 444, 445, 592, 593)), (13, 32, 3, (148, 149)), (8, 32, 4, (888, 889)),
+                                                  (3, 128, 3, (296, 297, 888, 889, 1184, 1185)), (2, 128, 4, (1332, 1333)), (10, 128, 2, (148, 149, 296, 297, 444, 445)), (8, 128, 2, (74, 75, 148, 149, 296, 297)),
+                                                  (4, 128, 4, (74, 75, 296, 297))])
+def test_v_blocks_through_a_tile_and_from_registers(cuda_device, heads, cb, bits, blocks):
+    """V launches on both sides of the lines at which the way of a block changes, in calls of several sequences, blocks of every conversion among
+    them: the calls' results equal those of calls of at most 60 token blocks of one sequence."""
+    dev, dtype, rel = cuda_device, torch.bfloat16, synth.rel_for_bits(bits)
+    g = torch.Generator(device=dev).manual_seed(3)
+    for n in blocks:
+        B = next(B for B in (3, 2, 1) if n % B == 0)
+        v = torch.randn(B, n // B * cb, heads, 128, generator=g, device=dev).to(dtype).transpose(1, 2)
+        for i, (spread, middle) in enumerate(((8, 1000), (8, 8000), (3e4, 0))):      # zero-points that the faster conversions do not take
+            at = slice((5 + i) * cb, (6 + i) * cb)
+            v[0, :, at] = (v[0, :, at].float() * spread + middle).to(dtype)
+        all_ = _bufs(B, heads, n // B * cb, cb, bits, "v", ops.K_TOKEN, dtype, dev)
+        ops.encode_tensor("v", v, cb, rel, ops.K_TOKEN, bits, cb, **all_)
+        for b in range(B):
+            one = _bufs(1, heads, n // B * cb, cb, bits, "v", ops.K_TOKEN, dtype, dev)
+            for lo in range(0, n // B, 60):
+                hi = min(n // B, lo + 60)
+                ops.encode_tensor("v", v[b: b + 1, :, lo * cb: hi * cb], cb, rel, ops.K_TOKEN, bits, cb, first_token=lo * cb, **one)
+            for name in ("scale", "zero", "stream", "info", "stream_bytes"):
+                assert torch.equal(one[name].view(torch.uint8), all_[name][b: b + 1].view(torch.uint8)), (n, b, name)
