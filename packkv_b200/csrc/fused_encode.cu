@@ -20,7 +20,7 @@
 //            HBM traffic per element: 2 B read (the second read of a tile comes from L1/L2) + the
 //            block bytes written once (~0.56 B at 4 bit).
 //   slots  : three launches, no device-side waiting (more than 8 heads in the kernels
-//            with per-token parameters, or on request): encode into
+//            with per-token parameters, short launches of V in 128-token blocks, or on request): encode into
 //            fixed-stride SLOTS in scratch memory with the size in block_info[blk][1]; per-sequence
 //            exclusive scan (scan_sizes_kernel, pack.cu); one warp per block copies its slot to its
 //            final offset.  The block bytes are written, read and written once more.
@@ -1619,8 +1619,8 @@ static int launch_fused_t(const FusedEncodeRequest& r, uint8_t* slots, const uin
     const int nctx = r.tokens / r.cb;
     int bound16, blocks_per_seq;
     // Direct form: the scratch holds only the ticket and the status array of the look-back.  The slots form stays
-    // for more than 8 heads (a CTA of the per-token kernels would not hold all blocks of its token block), for a scratch
-    // too small for the status array, and on request
+    // for more than 8 heads (a CTA of the per-token kernels would not hold all blocks of its token block), for short launches of V in
+    // 128-token blocks, for a scratch too small for the status array, and on request
     // (PKV_ENCODE_PATH=slots: measurements, tests).
     static const bool env_slots = [] { const char* v = std::getenv("PKV_ENCODE_PATH"); return v && std::string(v) == "slots"; }();
     const bool per_token_kernel = r.which == 1 || r.mode == 1;
@@ -1655,7 +1655,12 @@ static int launch_fused_t(const FusedEncodeRequest& r, uint8_t* slots, const uin
     }
     const int links = per_token_kernel ? nctx : k_one ? 1 : (nctx * r.heads + kKWarps - 1) / kKWarps;
     const int64_t chain_bytes = 256 + (int64_t)r.batch * links * 8;
-    const bool direct = !env_slots && (!per_token_kernel || r.heads <= 8) && chain_bytes <= fused_encode_scratch_bytes(r) &&
+    // V in 128-token blocks, half a CTA to an SM up to two: all CTAs are there at once, and the chain of their look-backs is the longest part of the launch
+    // (us direct and slots, 2 bits: 8 heads, 148 CTAs 29.1 26.9, 296 50.8 47.2; 5 heads 25.0 23.0, 44.3 39.3; 2 heads 21.1 19.1, 26.6 24.2; 4 heads, 4 bits,
+    // 24.0 23.3, 33.1 32.8, 370 39.9 41.8; 8 heads, 4 bits, 29.9 30.7, 54.7 55.0; 8 heads, 2 bits, 40 CTAs 24.7 23.3, 20 20.4 20.0, 10 18.5 19.6)
+    const bool short_v = r.which == 1 && r.cb == 128 && (BITS < 4 || r.heads <= 4) && 2 * (int64_t)r.batch * nctx > kSmCount &&
+                         (int64_t)r.batch * nctx <= 2 * kSmCount;
+    const bool direct = !env_slots && !short_v && (!per_token_kernel || r.heads <= 8) && chain_bytes <= fused_encode_scratch_bytes(r) &&
                         r.stream_bytes != nullptr;
     if (direct) {
         a.ticket = reinterpret_cast<unsigned*>(slots);
