@@ -333,7 +333,7 @@ static_assert(sizeof(CtaShared) % 16 == 0, "the receive area behind it holds 16-
 // them, into a receive area behind the CTA-shared block ([16 CTAs][16] maxima and sums, then [CTAs][rx_per] units of four sums); the receiver
 // waits on its own mbarrier.  Written where they are and read from there, both cost a cluster barrier and a remote load's round trip more, and
 // nobody may leave before a third barrier (us a launch: 10 pairs x 5333 tokens 25.5 -> 24.3, 4 x 32 heads x 1025 26.4 -> 24.5, 8 x 8 x 2000
-// 24.0 -> 23.0; teams: 8 x 700 10.2 -> 9.6, 16 x 8 x 1000 17.2 -> 15.9; 16 x 8 x 8192 113.6 and 114.1).  Kernels of their own: with both ways in one,
+// 24.0 -> 23.0; teams: 8 x 700 10.2 -> 9.6, 16 x 8 x 1000 17.2 -> 15.9; 16 x 8 x 8192 113.9 -> 112.2).  Kernels of their own: with both ways in one,
 // 16 x 8 x 8192 took 1 % longer and a team 3 %.
 
 // The CTA's reduced accumulators out[head][channel] (read by the cluster's CTAs through distributed shared
@@ -2026,9 +2026,10 @@ int launch_attention(const AttnArgs& a, const AttnExchange* xch, const AttnAppen
     int smem = plan_smem(P, best_cl, best_split, best_ns, slot);
     // Sums are sent where every CTA of the cluster delivers (with an exchange the first one does) and the receive area takes no CTA off an SM, or
     // the launch's clusters fit without it (with one CTA off each SM, 8 pairs x 32768 tokens in two launches of 512 CTAs took 55 us instead of 39.5,
-    // 8 heads x 5333 tokens in blocks of 128, eight clusters of 15 where seven fit, 35.9 instead of 21.9).  Single launches of 512 tokens to a warp and more read: their time is in the tiles (us read and sent: 16 x 8 x 8192
-    // 113.6 114.1, 17 x 8 x 8192 114.4 115.4, 8 x 8 x 16384 112.7 112.1; of less work 16 x 8 x 4096 62.7 62.0, 32 x 4 x 3000 57.6 55.1).
-    if (!xch && best_cl > 1 && (best_launches == 2 || P.tpw * P.tile < 512)) {
+    // 8 heads x 5333 tokens in blocks of 128, eight clusters of 15 where seven fit, 35.9 instead of 21.9).  (us read and
+    // sent, also where the time is in the tiles: 16 x 8 x 4096 62.6 61.4, x 6600 102.5 101.0, x 8192 113.9 112.2, x 11000 161.7 159.0, x 16384 217.9 215.5;
+    // 12 x 8 x 8192 in groups of 8 94.6 94.8; 32 x 4 x 8192 113.9 112.1; over 120 shapes of 4096 to 16384 tokens none is more than 0.3 % slower sent.)
+    if (!xch && best_cl > 1) {
         const int units = a.group * (kD / 4), per = (units + best_cl - 1) / best_cl, with = smem + 1024 + best_cl * per * 16;
         const auto per_sm = [](int bytes) { return std::min(kMaxCtasPerSm, (228 * 1024) / (bytes + 1024)); };
         if (with <= 227 * 1024 && (per_sm(with) == per_sm(smem) || pairs * best_split <= clusters_that_fit(best_cl, per_sm(with)))) {

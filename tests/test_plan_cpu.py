@@ -40,6 +40,7 @@ def test_teams_on_busy_gpus(sequences, n_comp, n_res, cluster):
 @pytest.mark.parametrize("sequences,group,n_comp,plan,sends", [
     (8, 7, 5120, (15, 1, 1), 0), (7, 7, 5120, (15, 1, 1), 1),         # two CTAs to an SM, one with the receive area: seven clusters of 15 fit then
     (8, 8, 5120, (15, 1, 1), 0), (7, 8, 5120, (15, 1, 1), 1),
+    (8, 4, 8192, (4, 1, 1), 1), (8, 4, 16384, (4, 1, 1), 1),          # 512 and 1024 tokens to a warp
     (8, 4, 1024, (1, 1, 1), 0), (8, 4, 1024, (8, 1, 1), 1), (8, 4, 1024, (1, 3, 2), 0), (8, 4, 1024, (3, 3, 2), 1),     # clusters of one CTA send nothing
 ])
 def test_sums_are_sent_where_the_receive_area_costs_no_wave(sequences, group, n_comp, plan, sends):
