@@ -4,11 +4,13 @@ dequantise in the tensor dtype -> eager attention with fp32 softmax.
 
 Tolerance: 2e-3 max-abs error relative to max|reference| (the bar of the task), both dtypes.
 """
+import ctypes
+
 import pytest
 import torch
 
 from oracle import quant as Q
-from packkv_b200 import encode, ops, synth
+from packkv_b200 import _lib, encode, ops, synth
 from packkv_b200.config import QuantMode
 from tests.helpers import layer_from_oracle
 
@@ -643,7 +645,7 @@ def test_encode_then_attend_without_waiting(cuda_device, plan):
 @pytest.mark.parametrize("cluster,group", [(2, 8), (3, 7), (4, 1), (5, 3), (8, 4), (13, 6), (16, 8)])
 def test_sums_sent_across_the_cluster(cuda_device, cluster, group):
     """Launches in which the CTAs of a cluster send one another their maxima, sums and parts of the output (no team: four tiles to a CTA or more):
-    cluster sizes that divide the output's units of four sums and that do not, one launch and two, with and without CTAs that have no unit."""
+    cluster sizes that divide the output's units of four sums and that do not, one launch and two."""
     n_comp = 64 * max(4 * cluster, 12)
     for plan in ((cluster, 1, 1), (cluster, 2, 2)):
         err = _run_case(cuda_device, torch.bfloat16, 1, 2, group, n_comp, 144, block=64, cbk=64, cbv=64, bits_k=4, bits_v=3, k_mode="channel", seed=cluster,
@@ -678,3 +680,43 @@ def test_output_at_an_odd_address(cuda_device):
         assert int(flags.item()) == 0
         assert wanted is None or torch.equal(out, wanted)
         wanted = out.clone()
+
+
+def _sends(layer, dev, B, Hkv, G, n_res, plan):
+    """Whether a launch of this plan sends its sums across the cluster (asked without a launch)."""
+    a = _lib.AttnArgs()
+    for name in ("q", "out", "k_res", "v_res", "flags"):
+        setattr(a, name, 1 << 28)
+    for name in ("k_stream", "k_info", "k_scale", "k_zero", "v_stream", "v_info", "v_scale", "v_zero"):
+        setattr(a, name, getattr(layer, name).data_ptr())
+    a.k_capacity, a.v_capacity = layer.k_stream.shape[1], layer.v_stream.shape[1]
+    a.n_comp, a.n_res, a.batch, a.kv_heads, a.group, a.cbk, a.cbv = layer.n_comp, n_res, B, Hkv, G, layer.cbk, layer.cbv
+    a.bits_k, a.bits_v, a.k_mode, a.scaling = layer.bits_k, layer.bits_v, layer.k_mode, 0.1
+    a.param_tokens, a.param_blocks = layer.v_scale.shape[1], layer.n_comp // layer.cbk
+    forced, sends = _lib.AttnPlan(*plan), ctypes.c_int32(-1)
+    assert _lib.lib().pkv_attention_sends(ctypes.byref(a), ctypes.byref(forced), 32 << 20, 0, ctypes.byref(sends)) == _lib.PKV_OK
+    assert (forced.cluster, forced.nsplit, forced.launches) == plan
+    return sends.value
+
+
+@pytest.mark.parametrize("cluster,group,idle", [(9, 1, 1), (12, 2, 1), (13, 3, 1), (14, 4, 1), (13, 1, 2), (15, 7, 0), (16, 5, 0)])
+def test_sums_sent_to_clusters_with_idle_ctas(cuda_device, cluster, group, idle):
+    """Clusters whose last CTAs deliver no unit of the output (32 x group units of four sums, ceil(units / cluster) to a CTA), or fewer than the others: one
+    launch as a team and not, and two.  The library is asked whether these launches send."""
+    units = 32 * group
+    per = -(-units // cluster)
+    assert sum(per * rank >= units for rank in range(cluster)) == idle
+    for n_comp, plan in ((64 * cluster, (cluster, 1, 1)), (256 * cluster, (cluster, 1, 1)), (64 * 2 * cluster, (cluster, 2, 2))):
+        k, v = synth.synth_kv(2, 1, n_comp + 130, 128, seed=cluster, dtype=torch.bfloat16)
+        layer, kd, vd = layer_from_oracle(k[:, :, :n_comp], v[:, :, :n_comp], block=64, bits_k=4, bits_v=4, k_mode="channel", cbk=64, cbv=64,
+                                          rel_k=synth.rel_for_bits(4), rel_v=synth.rel_for_bits(4), device=cuda_device)
+        assert _sends(layer, cuda_device, 2, 1, group, 130, plan) == 1 and _sends(layer, cuda_device, 2, 1, group, 130, (1, *plan[1:])) == 0
+        q = synth.synth_q(2, group, 128, seed=cluster, dtype=torch.bfloat16)
+        ref = Q.eager_attention(q, torch.cat([kd, k[:, :, n_comp:]], 2), torch.cat([vd, v[:, :, n_comp:]], 2))[:, 0].float()
+        rest = [t[:, :, n_comp:].contiguous().to(cuda_device) for t in (k, v)]
+        flags, scratch = ops.new_flags(cuda_device), ops.new_attention_scratch(cuda_device)
+        for _ in range(2):
+            out = ops.decode_attention(q[:, :, 0].contiguous().to(cuda_device), layer, *rest, 130, flags=flags, kv_heads=1, plan=plan, scratch=scratch)
+        torch.cuda.synchronize()
+        assert int(flags.item()) == 0
+        assert _rel_err(out.float().cpu(), ref, torch.bfloat16) <= TOL, (n_comp, plan)
