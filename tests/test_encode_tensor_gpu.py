@@ -204,8 +204,8 @@ def test_one_block_of_every_sequence(cuda_device, which, mode, dtype, values):
 
 @pytest.mark.parametrize("cb,bits", [(64, 4), (64, 3), (32, 2)])
 def test_v_forms_write_the_same(cuda_device, cb, bits):
-    """V CTAs of 8 and of 16 warps, by the number of token blocks a call has (more than 296 and up to 444: 8, a few and 504: 16): the
-    sequences of one call equal the same sequences in calls of one sequence each."""
+    """V CTAs of 8 and of 16 warps, by the number of token blocks a call has (64-token blocks: up to 148 16 warps, one CTA to an SM; 200: 16, two to an SM;
+    360 and 444: 8, three to an SM; 504: 8, four to an SM): the sequences of one call equal the same sequences in calls of one sequence each."""
     dev, dtype, H, rel = cuda_device, torch.float16, 8, synth.rel_for_bits(bits)
     for B, blocks in ((4, 126), (6, 60), (2, 100), (37, 12)):           # 504, 360, 200 and 444 token blocks
         _, v = synth.synth_kv(B, H, blocks * cb, 128, seed=B, dtype=dtype, device=dev)
@@ -250,7 +250,7 @@ def test_v_forms_of_other_heads_and_blocks(cuda_device, heads, cb, bits, ordered
         more = lambda lo, hi: {} if order is None else dict(order=order[lo:hi].contiguous(), order_block=cb)
         all_, parts = (_bufs(1, heads, blocks * cb, cb, bits, "v", ops.K_TOKEN, dtype, dev) for _ in range(2))
         ops.encode_tensor("v", v, cb, rel, ops.K_TOKEN, bits, cb, **all_, **more(0, blocks))
-        for lo in range(0, blocks, 100):                            # calls of up to 100 token blocks: one CTA of 16 warps to an SM
+        for lo in range(0, blocks, 100):                            # calls of up to 100 token blocks
             hi = min(blocks, lo + 100)
             ops.encode_tensor("v", v[:, :, lo * cb: hi * cb], cb, rel, ops.K_TOKEN, bits, cb, first_token=lo * cb, **parts, **more(lo, hi))
         for name in all_:
