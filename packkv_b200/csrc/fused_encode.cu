@@ -1181,12 +1181,12 @@ __global__ void __launch_bounds__(256, 3) kt_fused_encode_kernel(FusedArgs a) {
 // with one CTA per sequence, 49 us this way.
 constexpr int kOneWarps = 4;
 
-// Most CTAs of a one-block launch.  Blocks of 64 and 128 tokens: up to four to an SM this form takes 0.17 to 0.93 of the other's time (us at 592
-// CTAs, 64 tokens, 8 heads: K 11.7 and 8.9, V 13.2 and 10.3; at 888 it is still ahead, 12.0 and 9.4, but the line was not moved).  Blocks of 32
-// tokens are little work: the form loses once its clusters do not all fit at once, which depends on what a CTA holds and on how many make a
-// cluster, unless the other's one CTA per sequence needs a second wave by then (K, 4 heads: 444 CTAs 5.4 and 4.9, 516 5.4 and 6.6; 2 heads: 518
-// 6.0 and 5.0, 592 6.1 and 6.6; 1 head: 592 9.4 and 6.5.  V, 4 heads: 516 6.6 and 5.6, 592 6.6 and 7.6; 2 heads: 592 7.0 and 5.7.  K with
-// parameters per token, 592: 4 heads 6.3 and 7.0, 8 heads 7.9 and 7.3).
+// Most CTAs of a one-block launch (us of the general form, then of this one, as both are now).  Blocks of 64 and 128 tokens: up to four to an SM this form is
+// ahead, or level (V, 4 heads x 64, 592 CTAs 9.3 and 9.9, 516 8.9 and 7.6); beyond it is ahead still (740 CTAs, 8 heads x 64: K 11.2 and 8.9, V 12.3 and 10.7,
+// K with parameters per token 13.8 and 10.7; x 128: K 19.1 and 15.4, V 19.8 and 17.2), but the line was not moved.  Blocks of 32 tokens are
+// little work: the form loses once its clusters do not all fit at once, which depends on what a CTA holds and on how many make a cluster, unless the other's one
+// CTA per sequence needs a second wave by then.  Where the general form has become faster since the lines were drawn it is up to 12 % ahead below them
+// (V, 2 heads: 148 CTAs 4.5 and 4.9; 3 heads: 591 7.2 and 7.6; K with parameters per token, 592: 3 heads 6.3 and 7.1, 8 heads 6.5 and 7.2), level elsewhere.
 static int one_block_ctas(int heads, int cb, bool is_v, bool per_token) {
     if (cb != 32 || heads == 1) return 4 * kSmCount;
     if (per_token) return heads <= 3 || (!is_v && heads > 4) ? 4 * kSmCount : 7 * kSmCount / 2;
@@ -1620,7 +1620,7 @@ static int launch_fused_t(const FusedEncodeRequest& r, uint8_t* slots, const uin
     int bound16, blocks_per_seq;
     // Direct form: the scratch holds only the ticket and the status array of the look-back.  The slots form stays
     // for more than 8 heads (a CTA of the per-token kernels would not hold all blocks of its token block), for short launches of V in
-    // 128-token blocks, for a scratch too small for the status array, and on request
+    // 128-token blocks (short_v), for a scratch too small for the status array, and on request
     // (PKV_ENCODE_PATH=slots: measurements, tests).
     static const bool env_slots = [] { const char* v = std::getenv("PKV_ENCODE_PATH"); return v && std::string(v) == "slots"; }();
     const bool per_token_kernel = r.which == 1 || r.mode == 1;
@@ -1655,10 +1655,12 @@ static int launch_fused_t(const FusedEncodeRequest& r, uint8_t* slots, const uin
     }
     const int links = per_token_kernel ? nctx : k_one ? 1 : (nctx * r.heads + kKWarps - 1) / kKWarps;
     const int64_t chain_bytes = 256 + (int64_t)r.batch * links * 8;
-    // V in 128-token blocks, half a CTA to an SM up to two: all CTAs are there at once, and the chain of their look-backs is the longest part of the launch
-    // (us direct and slots, 2 bits: 8 heads, 148 CTAs 29.1 26.9, 296 50.8 47.2; 5 heads 25.0 23.0, 44.3 39.3; 2 heads 21.1 19.1, 26.6 24.2; 4 heads, 4 bits,
-    // 24.0 23.3, 33.1 32.8, 370 39.9 41.8; 8 heads, 4 bits, 29.9 30.7, 54.7 55.0; 8 heads, 2 bits, 40 CTAs 24.7 23.3, 20 20.4 20.0, 10 18.5 19.6)
-    const bool short_v = r.which == 1 && r.cb == 128 && (BITS < 4 || r.heads <= 4) && 2 * (int64_t)r.batch * nctx > kSmCount &&
+    // V in 128-token blocks, half a CTA to an SM up to two, of few long sequences: all CTAs are there at once, and the chain of a sequence's look-backs is the
+    // longest part of the launch (us direct and slots, two sequences, 2 bits: 8 heads, 148 CTAs 29.1 26.9, 296 50.8 47.2; 5 heads 25.0 23.0, 44.3 39.3;
+    // 2 heads 21.1 19.1, 26.6 24.2; 4 heads, 4 bits, 24.0 23.3, 33.1 32.8, 370 39.9 41.8; 8 heads, 4 bits, 29.9 30.7, 54.7 55.0; 8 heads, 2 bits, 40 CTAs 24.7 23.3,
+    // 20 20.4 20.0, 10 18.5 19.6).  By the blocks of a sequence, slots take of direct's time, 128 or 148 CTAs: 1 block 1.29 to 1.77, 2 0.98 to 1.14, 8 0.96 to 1.04,
+    // 32 0.93 to 1.01, 64 0.90 to 0.97, 128 0.87 to 0.93.
+    const bool short_v = r.which == 1 && r.cb == 128 && nctx >= 64 && (BITS < 4 || r.heads <= 4) && 2 * (int64_t)r.batch * nctx > kSmCount &&
                          (int64_t)r.batch * nctx <= 2 * kSmCount;
     const bool direct = !env_slots && !short_v && (!per_token_kernel || r.heads <= 8) && chain_bytes <= fused_encode_scratch_bytes(r) &&
                         r.stream_bytes != nullptr;
