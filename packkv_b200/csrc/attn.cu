@@ -1885,9 +1885,10 @@ int launch_attention(const AttnArgs& a, const AttnExchange* xch, const AttnAppen
         const int sm_warps = (int)((on_gpu + kSmCount - 1) / kSmCount) * kAW;
         // On a busy SM it makes no difference who holds the residual tiles; on an idle one it is the longest warp's time,
         // and so are the hand-over and the second start of two launches.  Powers of two only.
-        // (The factors were fitted to 30 shapes timed at every cluster size.  Over 264 others, 1 to 500 pairs of 300 to 32768 tokens with every
-        // bit width, block size and K mode, each timed in 16 to 60 plans, the chosen one is 2.5 % from the best on average, 14 % at the 95th
-        // percentile and 22 % at worst: 39 x 8 heads x 575 tokens, 2-bit K, groups of 7, 42.5 us where the best takes 34.7.)
+        // (The factors were fitted to 30 shapes timed at every cluster size, before launches sent their sums.  Over 225 others, 1 to 500 pairs of 300 to 32768
+        // tokens with every bit width, block size and K mode, each timed in 5 to 84 plans as launches are now, the chosen one is 2.0 % from the best on
+        // average and 10 % at the 95th percentile.  At worst 49 %: 7 x 2 heads x 9857 tokens in groups of 6, 42 clusters of 13 of which 38 fit at once
+        // (see clusters_that_fit; the places counted below hold for clusters of four), 42.3 us where the best takes 28.4; then 22 %.)
         const bool idle = sm_warps <= 8;
         const double upw_max = team || (idle && !(cl & (cl - 1))) ? upw_placed : upw_dealt;
         if (idle && launches == 2) fixed += 1.0;
