@@ -749,7 +749,7 @@ __device__ __forceinline__ void put_token_params(const Quantiser<T, false>& qz, 
 // zero to the caller's arrays; ord[t] = source row (inside the block) of stored row t.  One CTA barrier inside; the caller's next one must come
 // before prm[] is read.  (Parameters formed by the half warp, every lane alike: 400 of a warp's 4700 instructions per block of 64 tokens x 8 heads.)
 struct TokenState { bool bad, packed, half; };           // of this thread's token: degenerate; parameters that the two faster conversions take
-template <typename T, int CB, bool WRITE = true, int NW = 8>
+template <typename T, int CB, bool WRITE = true, int NW = 8, bool FOURS = true>
 __device__ __forceinline__ TokenState token_params_pass(const FusedArgs& a, const T* xb, float4* prm, const uint8_t* ord, int b, int cbi, int lane, int wic) {
     using T2 = typename QT<T>::T2;
     static_assert(NW * 32 >= CB, "a thread to a token");
@@ -760,7 +760,8 @@ __device__ __forceinline__ TokenState token_params_pass(const FusedArgs& a, cons
     for (int t = 2 * wic + (lane >> 4); t < CB; t += 2 * NW) {     // 8 channels per lane
         const uint8_t* xt = reinterpret_cast<const uint8_t*>(xb + 8 * (lane & 15)) + (uint64_t)ord[t] * (2 * (uint64_t)a.ss);
         T2 lo2 = QT<T>::init2(INFINITY), hi2 = QT<T>::init2(-INFINITY);
-        // eight heads' loads in flight together, four where no more are left (eight of a single head: V 3 %, per-token K 4 % slower, 20 to 2048 CTAs)
+        // eight heads' loads in flight together, with FOURS four where no more are left (eight of a single head: V 3 to 7 %, per-token K 4 % slower, 20 to 4096
+        // CTAs; but V of 8 heads x 64 tokens, three CTAs of 8 warps to an SM, 16384 of them, takes 800 us with the second copy of the loads and 795 without)
         const auto take = [&](int h0, auto count) {
             constexpr int N = decltype(count)::value;
             uint4 raw[N];
@@ -778,8 +779,8 @@ __device__ __forceinline__ TokenState token_params_pass(const FusedArgs& a, cons
             }
         };
         int h0 = 0;
-        for (; a.heads - h0 > 4; h0 += 8) take(h0, std::integral_constant<int, 8>{});
-        if (h0 < a.heads) take(h0, std::integral_constant<int, 4>{});
+        for (; a.heads - h0 > (FOURS ? 4 : 0); h0 += 8) take(h0, std::integral_constant<int, 8>{});
+        if (FOURS && h0 < a.heads) take(h0, std::integral_constant<int, 4>{});
         // (minimum, -maximum) of the lane, then of the token: one minimum serves both
         const unsigned l = *reinterpret_cast<const unsigned*>(&lo2), u = *reinterpret_cast<const unsigned*>(&hi2) ^ 0x80008000u;
         unsigned m = min_of(__byte_perm(l, u, 0x5410), __byte_perm(l, u, 0x7632));
@@ -1059,7 +1060,8 @@ __global__ void __launch_bounds__(NW * 32, PER_SM) v_fused_encode_kernel(FusedAr
     load_row_order<CB, NW>(a, ord, b, cbi);
 
     // pass 1: per-token statistics across every head and channel
-    const TokenState mine = token_params_pass<T, CB, true, NW>(a, xb, prm, ord, b, cbi, lane, wic);
+    constexpr bool kFours = TILE || CB != 64 || PER_SM != 3;   // (v_form: that form is for 5 to 8 heads)
+    const TokenState mine = token_params_pass<T, CB, true, NW, kFours>(a, xb, prm, ord, b, cbi, lane, wic);
     // one decision for the whole CTA: the faster conversions need every token's parameters in range
     const bool all_packed = __syncthreads_and(mine.packed);
     const bool all_half = __syncthreads_and(mine.half);
