@@ -57,9 +57,9 @@ MIN_TIMED_S = 1.0   # the timed region is repeated until it is at least this lon
 # captures kept with the repository's profile summaries.  An entry is valid for one revision of the kernel only (the revision is
 # a constant of packkv_b200.ops that changes with the kernel): other revisions report null.
 NCU_TRAFFIC_BYTES = {
-    ("attn", 3, 16, 8192, 8, 4, 4, 64, 128): 160.9e6,      # 155.96 MB read + 4.92 MB written
-    ("encode", 2, 16, 4, 64): 1401e6,                      # K 576 + 151 MB, V 561 + 113 MB
-    ("encode", 2, 64, 4, 64): 4 * 1401e6,                  # the 16-sequence capture scaled by the sequences (traffic is per sequence)
+    ("attn", 3, 16, 8192, 8, 4, 4, 64, 128): 159.7e6,      # 155.98 MB read + 3.73 MB written
+    ("encode", 2, 16, 4, 64): 1376e6,                      # K 561 + 141 MB, V 553 + 121 MB
+    ("encode", 2, 64, 4, 64): 4 * 1376e6,                  # the 16-sequence capture scaled by the sequences (traffic is per sequence)
 }
 
 
